@@ -185,18 +185,18 @@ int vnm_selftest_wait_expiry(vnm_handle_t handle, void *stream);
  * indirection exactly like the reference's compile-time IDEAL_KERNEL experiment
  * (include/spatha/block_sparse/spmm/blockwise_kernel.h:328-642, row = nz_block_idx % 4 at :536);
  * 2 = B is not loaded at all (timing floor; results are meaningless).
- * Producer warps: 4 or 8 warps issue the gather loads (default 8). */
+ * Producer warps: 4 and 8 are accepted for compatibility; sixteen warps issue the gather loads whatever is set. */
 int vnm_set_gather_mode(vnm_handle_t handle, int mode);
 /* Gather mode 3 only: of the 64 gathered rows of every stage, `tma_rows` (0, 16, 32 or 48) are fetched by TMA
  * tile::gather4 and the others by the per-thread copies, so that both paths into the SM are busy at once. */
 int vnm_set_gather_split(vnm_handle_t handle, int tma_rows);
-/* Epilogue of the V:N:M (gather) form.  0 (default): layout MN staged in shared memory and stored as full 128-bit
- * sectors; layout NM as fp16 stores from registers (several destinations -- vnm_spmm_f16_multi -- staged as [n][m] and
- * stored with TMA, boxes of 128 m x 32 n).  1 = layout MN: every thread stores its own row in 32-bit words, the
+/* Epilogue of the V:N:M (gather) form.  0 (default): stored straight from tensor memory, layout MN as full 32-byte
+ * sectors of a row, layout NM as 32-bit words, eight of which fill a sector (several destinations -- vnm_spmm_f16_multi --
+ * staged as [n][m] and stored with TMA).  1 = layout MN: every thread stores its own row in 32-bit words, the
  * reference's OUT_32B experiment (include/spatha/block_sparse/common/epilogue.h:34-61, blockwise_kernel.h:911-943).
  * 2 = layout NM through TMA stores also for a single destination, where ldo % 8 == 0 and out is 16-byte aligned
- * (ablation: measured 1-4 % slower).  All give identical bits.  VNM_ERR_UNSUPPORTED for operands held in dense-B form,
- * whose epilogue always leaves through TMA stores. */
+ * (ablation).  All give identical bits.  VNM_ERR_UNSUPPORTED for operands held in dense-B form, whose epilogue has no
+ * such switch. */
 int vnm_set_epilogue(vnm_handle_t handle, int mode);
 
 /* How vnm_prepare lays the sparse operand out for the kernel (process-wide, applies to later calls):

@@ -139,7 +139,6 @@ struct vnm_prepared_s {
     CUtensorMap tmap_tile;
     CUtensorMap tmap_tile2;  // dense-B kernel: 2-D map for the ragged right edge
     bool tm_wide;            // tmap_tile is the 4-D one-box-per-stage map
-    int producer_warps;
     // device staging of the host-buffer entry point
     void *stage_B;
     size_t stage_B_bytes;
@@ -154,7 +153,7 @@ struct vnm_prepared_s {
     int dense_b;       // 1: A re-expressed as 2:4 over all K columns, B read as plain tiles
     int out32;         // ablation: 32-bit epilogue stores (gather form, layout MN)
     int hybrid_rows;   // gather form: rows of every 64-row stage fetched by TMA gather4 beside the per-thread copies
-    int nm_tma_always; // gather kernel: 1 = the [N,M] result leaves through TMA stores even for a single destination (ablation: measured 1-4 % slower)
+    int nm_tma_always; // gather kernel: 1 = the [N,M] result leaves through TMA stores even for a single destination (ablation)
     int l2_ahead;      // pair kernel: k-tiles of L2 prefetch ahead of the shared-memory loads (0 = none)
     int pair_rows;     // pair kernel: 0 = row tiles per CTA chosen per problem, 1 / 2 = forced where possible (ablation)
     int l2_hints;      // pair kernel: 1 = ask L2 to keep the banded operand (default), 0 = no eviction-priority hints
@@ -264,7 +263,6 @@ int vnm_prepare_as(const void *values, const uint32_t *meta, const uint32_t *col
         h->gather_mode = (m == 4) ? GATHER_CONTIG : GATHER_TMA4;  // with m == 4 every row of B is selected
     }
     h->vblocks_padded = h->mtiles * h->nb;
-    h->producer_warps = 8;
     h->pair_mode = 1;
     h->l2_hints = 1;
     h->device = dev_now;
@@ -386,8 +384,7 @@ int vnm_set_producer_warps(vnm_handle_t h, int warps)
 {
     if (!h) return fail(VNM_ERR_BAD_ARG, "null handle");
     if (warps != 4 && warps != 8) return fail(VNM_ERR_BAD_ARG, "producer warps must be 4 or 8 (got %d)", warps);
-    h->producer_warps = warps;
-    return VNM_OK;
+    return VNM_OK;   // the kernel's sixteen producer warps are part of its layout
 }
 
 int vnm_spmm_config(vnm_handle_t h, int N, int *tile_m, int *tile_n, int *stages, int *grid, int *smem_bytes)
@@ -397,7 +394,7 @@ int vnm_spmm_config(vnm_handle_t h, int N, int *tile_m, int *tile_n, int *stages
     const bool pair = h->dense_b && h->pair_mode && N >= 128 && spmm_dense_b_pair_config(h->M, N, h->K, h->max_ctas, h->pair_rows, &cfg);
     if (pair) { /* cfg filled */ }
     else if (h->dense_b) spmm_dense_b_config(h->M, N, h->max_ctas, &cfg);
-    else if (!spmm_select_config(h->V, N, h->M, h->producer_warps, h->max_ctas, &cfg)) return fail(VNM_ERR_UNSUPPORTED, "unsupported V");
+    else if (!spmm_select_config(h->V, N, h->M, h->max_ctas, &cfg)) return fail(VNM_ERR_UNSUPPORTED, "unsupported V");
     if (tile_m) *tile_m = h->dense_b ? cfg.nb * TILE_M : TILE_M;  // pairs: 512 or 256, one SM per tile: 256 or 128
     if (tile_n) *tile_n = cfg.bn;
     if (stages) *stages = cfg.stages;
@@ -405,6 +402,25 @@ int vnm_spmm_config(vnm_handle_t h, int N, int *tile_m, int *tile_n, int *stages
     if (smem_bytes) *smem_bytes = cfg.smem_bytes;
     return VNM_OK;
 }
+
+}  // extern "C"
+
+// Tensor map of a result buffer: one box is what an epilogue part stores.
+CUresult vnm::encode_out_map(EncodeTiledFn enc, CUtensorMap *map, void *out, int M, int N, int64_t ldo, int layout, int part)
+{
+    cuuint32_t estr[2] = {1, 1};
+    cuuint64_t strides[1] = {(cuuint64_t)ldo * 2};
+    cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)M};
+    cuuint32_t box[2] = {(cuuint32_t)part, 128};
+    if (layout == VNM_LAYOUT_NM) {
+        dims[0] = (cuuint64_t)M; dims[1] = (cuuint64_t)N;
+        box[0] = 128; box[1] = (cuuint32_t)part;
+    }
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, out, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+}
+
+extern "C" {
 
 static int spmm_impl(vnm_handle_t h, const void *B, int64_t ldb, int N, int b_nk, const void *bias, void *out, int64_t ldo, int layout,
                      void *stream, void *const *more_outs = nullptr, int n_more = 0)
@@ -445,7 +461,7 @@ static int spmm_impl(vnm_handle_t h, const void *B, int64_t ldb, int N, int b_nk
     const bool pair = h->dense_b && h->pair_mode && (b_nk || N >= 128) && spmm_dense_b_pair_config(h->M, N, h->K, h->max_ctas, h->pair_rows, &cfg);
     if (pair) { /* cfg filled */ }
     else if (h->dense_b) spmm_dense_b_config(h->M, N, h->max_ctas, &cfg);
-    else if (!spmm_select_config(h->V, N, h->M, h->producer_warps, h->max_ctas, &cfg)) return fail(VNM_ERR_UNSUPPORTED, "unsupported V");
+    else if (!spmm_select_config(h->V, N, h->M, h->max_ctas, &cfg)) return fail(VNM_ERR_UNSUPPORTED, "unsupported V");
     EncodeTiledFn enc = get_encode_fn();
     if (!enc) return fail(VNM_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
 
@@ -467,12 +483,12 @@ static int spmm_impl(vnm_handle_t h, const void *B, int64_t ldb, int N, int b_nk
             h->tm_wide = false;
         } else {
             // B viewed as a 2-D tensor {N (contiguous), K}; one box = 64 columns (128 bytes) of one row
-            // (gather4 picks four such rows) or of 64 consecutive rows (32 for the dense-B kernel), written with
+            // (gather4 picks four such rows) or of 32 consecutive rows (64 for the pair kernel), written with
             // the 128-byte swizzle the MMA's N-major operand layout expects.  Rows >= K and columns >= N read as zeros.
             cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)h->K};
             cuuint64_t strides[1] = {(cuuint64_t)ldb * 2};
             cuuint32_t box_rows[2] = {64, 1};
-            cuuint32_t box_tile[2] = {64, (h->dense_b && !pair) ? 32u : 64u};
+            cuuint32_t box_tile[2] = {64, pair ? 64u : 32u};
             r = enc(&h->tmap_rows, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(B), dims, strides, box_rows, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -531,7 +547,6 @@ static int spmm_impl(vnm_handle_t h, const void *B, int64_t ldb, int N, int b_nk
     p.total_tiles = p.mtiles * p.ntiles;
     p.B = (const __half *)B;
     p.ldb = ldb;
-    p.out32 = h->out32;
     {
         // Band of the tile order (tile_coords) and, for the pair kernel, which operand is asked to stay in L2.  A band
         // keeps either `g` row groups of A (18 KiB per row tile and k-tile) or `q` column panels of B (K x tile-N fp16)
@@ -560,7 +575,8 @@ static int spmm_impl(vnm_handle_t h, const void *B, int64_t ldb, int N, int b_nk
     p.b_wide_ok = h->tm_wide ? 1 : 0;
     p.l2_ahead = h->l2_ahead;
     p.n_out = 1;
-    p.nm_tma = 0;
+    p.tma_out = 1;
+    p.out32 = 0;
     if (h->dense_b) {
         // The result leaves through TMA stores: [M,N] as boxes of 40 columns x 128 rows, [N,M] as boxes of 128
         // columns (m) x 40 rows (n).
@@ -569,44 +585,27 @@ static int spmm_impl(vnm_handle_t h, const void *B, int64_t ldb, int N, int b_nk
         CUtensorMap tmap_out;
         OutMaps more;
         memset(&more, 0, sizeof(more));
-        cuuint32_t oestr[2] = {1, 1};
-        cuuint64_t ostrides[1] = {(cuuint64_t)ldo * 2};
-        cuuint64_t odims[2] = {(cuuint64_t)N, (cuuint64_t)h->M};
-        cuuint32_t obox[2] = {40, 128};
-        if (layout == VNM_LAYOUT_NM) {
-            odims[0] = (cuuint64_t)h->M; odims[1] = (cuuint64_t)N;
-            obox[0] = 128; obox[1] = 40;
-        }
         for (int d = 0; d <= n_more; d++) {
-            CUresult r = enc(d == 0 ? &tmap_out : &more.m[d - 1], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, d == 0 ? out : more_outs[d - 1], odims, ostrides, obox,
-                             oestr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+            CUresult r = encode_out_map(enc, d == 0 ? &tmap_out : &more.m[d - 1], d == 0 ? out : more_outs[d - 1], h->M, N, ldo, layout, cfg.part);
             if (r != CUDA_SUCCESS) return fail(VNM_ERR_CUDA, "cuTensorMapEncodeTiled (output %d) failed with CUresult %d", d, (int)r);
         }
         p.n_out = 1 + n_more;
         if (pair) VNM_CUDA(launch_spmm_dense_b_pair(cfg, h->tmap_tile, h->tmap_tile2, tmap_out, more, p, (cudaStream_t)stream), "spmm launch");
         else VNM_CUDA(launch_spmm_dense_b(cfg, h->tmap_tile, h->tmap_tile2, tmap_out, more, p, (cudaStream_t)stream), "spmm launch");
     } else {
-        // Gather form: the epilogue stores from registers.  Only a [N,M] result with several destinations (or on request)
-        // leaves through shared memory and TMA stores (boxes of 128 m x 32 n; needs ldo % 8 == 0 and 16-byte alignment):
-        // for a single destination that path measured 1-4 % slower.
+        // Gather form: the epilogue stores straight from tensor memory.  Only a [N,M] result with several destinations (or on
+        // request) leaves through shared memory and TMA stores, boxes of 128 columns (m) x cfg.part rows (n).
         CUtensorMap tmap_out;
         OutMaps more;
         memset(&tmap_out, 0, sizeof(tmap_out));
         memset(&more, 0, sizeof(more));
-        p.nm_tma = 0;
-        if (layout == VNM_LAYOUT_NM && ldo % 8 == 0 && ((uintptr_t)out & 15) == 0 && (n_more > 0 || h->nm_tma_always)) {
-            cuuint32_t oestr[2] = {1, 1};
-            cuuint64_t ostrides[1] = {(cuuint64_t)ldo * 2};
-            cuuint64_t odims[2] = {(cuuint64_t)h->M, (cuuint64_t)N};
-            cuuint32_t obox[2] = {128, 32};
+        p.tma_out = layout == VNM_LAYOUT_NM && ldo % 8 == 0 && ((uintptr_t)out & 15) == 0 && (n_more > 0 || h->nm_tma_always);
+        p.out32 = h->out32;
+        if (p.tma_out) {
             for (int d = 0; d <= n_more; d++) {
-                CUresult r = enc(d == 0 ? &tmap_out : &more.m[d - 1], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, d == 0 ? out : more_outs[d - 1], odims, ostrides, obox,
-                                 oestr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                CUresult r = encode_out_map(enc, d == 0 ? &tmap_out : &more.m[d - 1], d == 0 ? out : more_outs[d - 1], h->M, N, ldo, layout, cfg.part);
                 if (r != CUDA_SUCCESS) return fail(VNM_ERR_CUDA, "cuTensorMapEncodeTiled (output %d) failed with CUresult %d", d, (int)r);
             }
-            p.nm_tma = 1;
             p.n_out = 1 + n_more;
         } else if (n_more > 0) {
             return fail(VNM_ERR_UNSUPPORTED, "vnm_spmm_f16_multi: the register-store epilogue of the gather form writes one destination");

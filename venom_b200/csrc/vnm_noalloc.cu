@@ -115,13 +115,13 @@ extern "C" int vnm_spmm_f16_noalloc(const void *values, const uint32_t *meta, co
     if (e != cudaSuccess) return nfail(VNM_ERR_CUDA, "re-pack launch: %s", cudaGetErrorString(e));
 
     SpmmConfig cfg;
-    if (!spmm_select_config(V, N, M, 8, 0, &cfg)) return nfail(VNM_ERR_UNSUPPORTED, "unsupported V");
+    if (!spmm_select_config(V, N, M, 0, &cfg)) return nfail(VNM_ERR_UNSUPPORTED, "unsupported V");
     EncodeTiledFn enc = get_encode_fn();
     if (!enc) return nfail(VNM_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
     CUtensorMap tmap_rows, tmap_tile;
     cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)K};
     cuuint64_t strides[1] = {(cuuint64_t)ldb * 2};
-    cuuint32_t box_rows[2] = {64, 1}, box_tile[2] = {64, 64}, estr[2] = {1, 1};
+    cuuint32_t box_rows[2] = {64, 1}, box_tile[2] = {64, 32}, estr[2] = {1, 1};
     CUresult r = enc(&tmap_rows, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(B), dims, strides, box_rows, estr,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r == CUDA_SUCCESS)
@@ -132,7 +132,6 @@ extern "C" int vnm_spmm_f16_noalloc(const void *values, const uint32_t *meta, co
     SpmmParams p;
     p.n_out = 1;
     p.l2_ahead = 0;
-    p.nm_tma = 0;
     p.am = (const uint8_t *)am;
     p.rows = (const int4 *)rows;
     p.bias = (const __half *)bias;
@@ -146,14 +145,14 @@ extern "C" int vnm_spmm_f16_noalloc(const void *values, const uint32_t *meta, co
     p.total_tiles = p.mtiles * p.ntiles;
     p.B = (const __half *)B;
     p.ldb = ldb;
-    p.out32 = 0;
+    p.tma_out = p.out32 = 0;
     p.hint_a = p.hint_b = L2_EVICT_NORMAL;
     p.group_m = mtiles;  // operands this small fit in L2 whole: row tiles fastest
     p.hybrid_rows = 0;
     p.b_nk = 0;
     p.b_wide_ok = 0;
     {
-        CUtensorMap no_map;   // this entry point keeps the register-store epilogue: no output tensor maps
+        CUtensorMap no_map;   // one destination: the epilogue stores straight from tensor memory
         OutMaps no_maps;
         memset(&no_map, 0, sizeof(no_map));
         memset(&no_maps, 0, sizeof(no_maps));

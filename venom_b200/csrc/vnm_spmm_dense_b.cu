@@ -27,8 +27,6 @@ namespace vnm {
 
 namespace {
 
-constexpr long long WAIT_LIMIT_CYCLES = 4000000000LL;  // ~2 s at B200 clocks
-
 constexpr int RT = 2;            // row tiles per CTA tile the shared-memory and tensor-memory plans are sized for; the kernel
                                  // template runs with R = 2, or R = 1 when the problem has too few tiles to fill the GPU otherwise
 constexpr int BN = 240;          // output columns per CTA tile
@@ -60,39 +58,6 @@ static_assert(SB % NBP == 0 && NBP <= 4, "B producers");
 static_assert(SF >= 4 * SA && SF >= 4 * META_SETS && SF >= 2 * SB && SF % SB == 0, "too few stage barriers: a waiter could miss a phase");
 static_assert(BN <= 240 && META_SETS == 3 && RT == 2 && BN % 16 == 0 && BN == 6 * PART, "tensor-memory column plan");
 static_assert((SA + SB + SF + SR + 2) * 8 + 16 <= BAR_BYTES, "barrier area too small");
-
-__device__ __forceinline__ bool wait_one(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int *status, int code)
-{
-    if (mbar_test_wait(bar, parity)) return true;
-    const long long t0 = clock64();
-    for (uint32_t it = 0;; ++it) {
-        if (mbar_test_wait(bar, parity)) return true;
-        if ((it & 1023u) == 1023u) {
-            if (*abort_flag) return false;
-            if (clock64() - t0 > WAIT_LIMIT_CYCLES) {
-                *abort_flag = 1;
-                atomicOr(status, code);
-                return false;
-            }
-        }
-    }
-}
-
-__device__ __forceinline__ bool wait_warp(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int *status, int code)
-{
-    int ok = 1;
-    if ((threadIdx.x & 31) == 0) ok = wait_one(bar, parity, abort_flag, status, code) ? 1 : 0;
-    return __shfl_sync(0xffffffffu, ok, 0) != 0;
-}
-
-__device__ __forceinline__ void drain_slot(uint64_t *bar, uint32_t parity, int *status)
-{
-    const long long t0 = clock64();
-    while (clock64() - t0 < WAIT_LIMIT_CYCLES / 4) {
-        if (mbar_try_wait(bar, parity)) return;
-    }
-    atomicOr(status, DEV_TIMEOUT_DRAIN);
-}
 
 template <int R>
 __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_kernel(const __grid_constant__ CUtensorMap tmap_tile, const __grid_constant__ CUtensorMap tmap_tile2,
@@ -441,6 +406,7 @@ void spmm_dense_b_config(int M, int N, int max_ctas, SpmmConfig *cfg)
     const int rt = (mtiles >= 2 && cost1 < cost2) ? 1 : 2;
     const long long tiles = rt == 2 ? t2 : t1;
     cfg->bn = BN;
+    cfg->part = PART;
     cfg->nb = rt;  // row tiles per CTA tile
     cfg->stages = 1;
     cfg->smem_bytes = SMEM_BYTES;

@@ -26,8 +26,6 @@ namespace vnm {
 
 namespace {
 
-constexpr long long WAIT_LIMIT_CYCLES = 4000000000LL;  // ~2 s at B200 clocks
-
 constexpr int RT = 2;            // row tiles (accumulators) per CTA; a pair tile has 2 * RT = 4 row tiles
 constexpr int BN = 240;          // output columns per pair tile
 constexpr int PART = 40;         // columns per epilogue part / TMA store
@@ -62,32 +60,6 @@ static_assert(SB % STAGES_PER_KT == 0 && KT_RING == SA && KT_RING == META_SETS &
 static_assert(BN <= 240 && META_SETS == 3 && RT == 2 && BN % 16 == 0 && BN == 6 * PART, "tensor-memory column plan");
 static_assert((SA + SB + SF + SR + 4) * 8 + 16 <= BAR_BYTES, "barrier area too small");
 constexpr int HALF_N = BN / 2;   // columns of a B stage held by each CTA of the pair
-
-__device__ __forceinline__ bool wait_one(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int *status, int code)
-{
-    if (mbar_test_wait(bar, parity)) return true;
-    const long long t0 = clock64();
-    for (uint32_t it = 0;; ++it) {
-        if (mbar_test_wait(bar, parity)) return true;
-        if ((it & 1023u) == 1023u) {
-            if (*abort_flag) return false;
-            if (clock64() - t0 > WAIT_LIMIT_CYCLES) {
-                *abort_flag = 1;
-                atomicOr(status, code);
-                return false;
-            }
-        }
-    }
-}
-
-__device__ __forceinline__ void drain_slot(uint64_t *bar, uint32_t parity, int *status)
-{
-    const long long t0 = clock64();
-    while (clock64() - t0 < WAIT_LIMIT_CYCLES / 4) {
-        if (mbar_try_wait(bar, parity)) return;
-    }
-    atomicOr(status, DEV_TIMEOUT_DRAIN);
-}
 
 // ---- cluster helpers ----
 __device__ __forceinline__ uint32_t cluster_ctarank()
@@ -142,13 +114,6 @@ __device__ __forceinline__ void tc_mma2_sp_f16(uint32_t d_tmem, uint64_t adesc, 
         "tcgen05.mma.sp.cta_group::2.kind::f16 [%0], %1, %2, [%3], %4, {%6, %6, %6, %6, %6, %6, %6, %6}, p;\n\t}" ::"r"(d_tmem),
         "l"(adesc), "l"(bdesc), "r"(meta_tmem), "r"(idesc), "r"(accumulate), "r"(0u)
         : "memory");
-}
-
-__device__ __forceinline__ bool wait_warp(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int *status, int code)
-{
-    int ok = 1;
-    if ((threadIdx.x & 31) == 0) ok = wait_one(bar, parity, abort_flag, status, code) ? 1 : 0;
-    return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
 
 // Warp roles (512 threads per CTA, as in the single-CTA kernel):
@@ -610,6 +575,7 @@ bool spmm_dense_b_pair_config(int M, int N, int K, int max_ctas, int force_rows,
     if (rt == 0) return false;
     const long long tiles = rt == RT ? t2 : t1;
     cfg->bn = BN;
+    cfg->part = PART;
     cfg->nb = 2 * rt;  // row tiles per pair tile
     cfg->stages = 2;
     cfg->smem_bytes = SMEM_BYTES;
