@@ -121,6 +121,16 @@ int vnm_spmm_f16_nk(vnm_handle_t handle, const void *Bt, int64_t ldbt, int N,
                     const void *bias, void *out, int64_t ldo, int layout, void *stream);
 int vnm_operand_form(vnm_handle_t handle, int *dense_b);
 
+/* The same with either form: an operand in gather form multiplies with the transpose of Bt, which the call writes to
+ * `workspace` first (K * N halves, 16-byte aligned, free again when the product is done; not touched in dense-B form).
+ * ldbt must be a multiple of 8. */
+int vnm_spmm_f16_nk_ws(vnm_handle_t handle, const void *Bt, int64_t ldbt, int N,
+                       const void *bias, void *out, int64_t ldo, int layout, void *workspace, void *stream);
+/* The form (VNM_STRATEGY_GATHER or VNM_STRATEGY_DENSE_B) with the smaller estimated time for N columns on the current
+ * device, the dense operand given as [K,N] (b_nk = 0: what VNM_STRATEGY_AUTO takes) or [N,K] (b_nk = 1, the gather form's
+ * transpose included). */
+int vnm_choose_form(int M, int K, int V, int n, int m, int N, int b_nk, int *strategy);
+
 /* Same product with HOST buffers: B (and bias) go up, the product runs on `stream`, the result comes back, and
  * the call returns after synchronising.  The columns are cut into up to eight slices so that the upload of one
  * slice, the product of the previous and the download of the one before run at the same time (two copy streams
@@ -208,17 +218,15 @@ int vnm_set_epilogue(vnm_handle_t handle, int mode);
 enum { VNM_STRATEGY_AUTO = 0, VNM_STRATEGY_GATHER = 1, VNM_STRATEGY_DENSE_B = 2 };
 int vnm_set_strategy(int strategy);
 /* vnm_prepare with the operand form chosen for this one handle (DENSE_B falls back to GATHER where the form does
- * not exist).  The torch op asks for DENSE_B when its dense operand arrives as a transposed [N, K] view, which
- * only that form reads in place. */
+ * not exist).  The torch op chooses with vnm_choose_form. */
 int vnm_prepare_as(const void *values, const uint32_t *meta, const uint32_t *colloc,
                    int M, int K, int V, int n, int m, int strategy, vnm_handle_t *handle, void *stream);
 int vnm_set_producer_warps(vnm_handle_t handle, int warps);
-/* Dense-B form only: 1 (default) = products with at least one full wave of 512 x 240 tiles and M a multiple of 512 run on
- * pairs of SMs (thread-block clusters of two CTAs, tcgen05 cta_group::2: each CTA loads half of every B stage), 0 = always
- * the single-SM kernel, 2 = pairs without the L2 eviction-priority hints that ask the banded operand to stay cached,
- * 3 / 4 = pairs with one / two row tiles per CTA forced where the shape allows (default: two wherever 512-row tiles
- * fill the SM pairs, else one, whose two accumulators alternate between consecutive tiles).  Ablation switches; all
- * give identical bits. */
+/* Dense-B form only: 1 (default) = products with enough tiles run on pairs of SMs (thread-block clusters of two CTAs, tcgen05
+ * cta_group::2: each CTA loads half of every B stage), 0 = one SM per tile wherever the result has a single destination,
+ * 2 = pairs without the L2 eviction-priority hints that ask the banded operand to stay cached,
+ * 3 / 4 = pairs with one / two row tiles per CTA forced (default: whichever has the smaller estimate; with one, the two
+ * accumulators alternate between consecutive tiles).  Ablation switches; all give identical bits for more than 64 columns. */
 int vnm_set_pair_mode(vnm_handle_t handle, int mode);
 /* Host-buffer entry points: number of equal column slices of the upload / product / download pipeline (1 .. 32; slices
  * are multiples of 256 columns and at least 1024 wide; 0 = the default, 8). */
@@ -235,8 +243,8 @@ int vnm_set_max_ctas(vnm_handle_t handle, int max_ctas);
 /* Shape and settings of a prepared operand (any output pointer may be NULL). */
 int vnm_handle_info(vnm_handle_t handle, int *M, int *K, int *V, int *m, int *max_ctas);
 
-/* Kernel configuration that vnm_spmm_f16 would launch for this handle and N (for reporting).  `stages`: for the dense-B
- * form 2 = the kernel on pairs of SMs, 1 = the one-SM kernel; for the gather form the number of producer warps. */
+/* Kernel configuration that vnm_spmm_f16 would launch for this handle and N (for reporting).  `stages`: 2 = the kernel on
+ * pairs of SMs, 1 = the kernel for few tiles, else the number of producer warps of the gather kernel. */
 int vnm_spmm_config(vnm_handle_t handle, int N, int *tile_m, int *tile_n, int *stages, int *grid, int *smem_bytes);
 
 /* ---------------------------------------------------------------------------------------------------------

@@ -53,6 +53,10 @@ def lib():
         L.vnm_host_wait.restype = C.c_int
         L.vnm_spmm_f16_nk.argtypes = L.vnm_spmm_f16.argtypes
         L.vnm_spmm_f16_nk.restype = C.c_int
+        L.vnm_spmm_f16_nk_ws.argtypes = [C.c_void_p, C.c_void_p, C.c_int64, C.c_int, C.c_void_p, C.c_void_p, C.c_int64, C.c_int, C.c_void_p, C.c_void_p]
+        L.vnm_spmm_f16_nk_ws.restype = C.c_int
+        L.vnm_choose_form.argtypes = [C.c_int] * 7 + [C.POINTER(C.c_int)]
+        L.vnm_choose_form.restype = C.c_int
         L.vnm_operand_form.argtypes = [C.c_void_p, C.POINTER(C.c_int)]
         L.vnm_operand_form.restype = C.c_int
         L.vnm_spmm_f16_host.argtypes = [C.c_void_p, C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_int, C.c_void_p]

@@ -37,8 +37,14 @@ struct Key {
 using WeakStorage = c10::weak_intrusive_ptr<c10::StorageImpl>;
 
 struct Entry {
-    vnm_handle_t handle;
+    // the operand re-packed per form (VNM_STRATEGY_GATHER, VNM_STRATEGY_DENSE_B), each when a call first wants it
+    vnm_handle_t handle[2];
+    int last_n, last_t, last_form;   // the form of the last shape of call
     WeakStorage values, meta, idx;   // the storages the operand was re-packed from
+    void release()
+    {
+        for (vnm_handle_t &h : handle) { vnm_destroy(h); h = nullptr; }
+    }
     bool alive() const { return !values.expired() && !meta.expired() && !idx.expired(); }
 };
 
@@ -60,7 +66,7 @@ void sweep_dead_entries()
 {
     for (auto it = g_cache.begin(); it != g_cache.end();) {
         if (!it->second.alive()) {
-            vnm_destroy(it->second.handle);
+            it->second.release();
             it = g_cache.erase(it);
         } else {
             ++it;
@@ -92,8 +98,8 @@ torch::Tensor spmm(torch::Tensor A_metadata, torch::Tensor A_indices, torch::Ten
                 nv, ", metadata ", nm, ", indices ", nc, ")");
     TORCH_CHECK(nnz == nv, "spatha.spmm: nnz must be A_num_rows * padded compressed columns (", nv, ")");
     TORCH_CHECK(rhs_matrix.dim() == 2 && rhs_matrix.size(0) == K && rhs_matrix.size(1) == N, "spatha.spmm: rhs_matrix must be [A_num_cols, B_num_cols]");
-    // A transposed view of a [B_num_cols, A_num_cols] activation (what `flattened_input.T` is) can be consumed
-    // in place when the operand is held in dense-B form; any other non-contiguous rhs is copied like the reference does.
+    // A transposed view of a [B_num_cols, A_num_cols] activation (what `flattened_input.T` is) is consumed as it lies;
+    // any other non-contiguous rhs is copied like the reference does.
     const bool rhs_is_t_view = rhs_matrix.stride(0) == 1 && rhs_matrix.stride(1) >= K && N > 1;
     const bool has_bias = bias.has_value() && bias->defined() && bias->numel() > 0;
     if (has_bias) TORCH_CHECK(bias->is_cuda() && bias->scalar_type() == torch::kFloat16 && bias->numel() == M && bias->is_contiguous(), "spatha.spmm: bias must be fp16 [A_num_rows]");
@@ -103,45 +109,56 @@ torch::Tensor spmm(torch::Tensor A_metadata, torch::Tensor A_indices, torch::Ten
     Key key{A_values.data_ptr(), A_metadata.data_ptr(), A_indices.data_ptr(), M, K, V, (int)n, (int)m, (int)rhs_matrix.device().index(),
             (uint32_t)A_values._version(), (uint32_t)A_metadata._version(), (uint32_t)A_indices._version()};
     vnm_handle_t h = nullptr;
+    int dense_b = 0;
+    const bool in_place = rhs_is_t_view && rhs_matrix.stride(1) % 8 == 0 && (reinterpret_cast<uintptr_t>(rhs_matrix.data_ptr()) & 15) == 0;
     {
         std::lock_guard<std::mutex> lock(g_mutex);
         auto it = g_cache.find(key);
         if (it != g_cache.end() && !(same_storage(it->second.values, A_values) && same_storage(it->second.meta, A_metadata) &&
                                      same_storage(it->second.idx, A_indices))) {
             // same addresses, different (or freed) tensors: the cached copy belongs to an operand that is gone
-            vnm_destroy(it->second.handle);
+            it->second.release();
             g_cache.erase(it);
             it = g_cache.end();
         }
         if (it == g_cache.end()) {
             sweep_dead_entries();
-            // An activation that arrives as a transposed [tokens, features] view is read in place only by the dense-B
-            // form, and the transpose copy it saves costs more than the gather form gains at high sparsity.
-            check(vnm_prepare_as(A_values.data_ptr(), (const uint32_t *)A_metadata.data_ptr(), (const uint32_t *)A_indices.data_ptr(), M, K, V,
-                                 (int)n, (int)m, rhs_is_t_view ? VNM_STRATEGY_DENSE_B : VNM_STRATEGY_AUTO, &h, stream), "vnm_prepare_as");
-            g_cache.emplace(key, Entry{h, weak_of(A_values), weak_of(A_metadata), weak_of(A_indices)});
-        } else {
-            h = it->second.handle;
+            it = g_cache.emplace(key, Entry{{nullptr, nullptr}, -1, 0, 0, weak_of(A_values), weak_of(A_metadata), weak_of(A_indices)}).first;
         }
+        // Dense-B form or gather form: by the estimate for this number of columns and the layout of the activation (a
+        // transposed [tokens, features] view is read in place by the dense-B form and transposed for the gather form).
+        Entry &e = it->second;
+        if (e.last_n != N || e.last_t != (int)in_place) {
+            int strategy = 0;
+            check(vnm_choose_form(M, K, V, (int)n, (int)m, N, in_place ? 1 : 0, &strategy), "vnm_choose_form");
+            e.last_form = strategy == VNM_STRATEGY_DENSE_B ? 1 : 0;
+            e.last_n = N;
+            e.last_t = in_place;
+        }
+        dense_b = e.last_form;
+        if (!e.handle[dense_b])
+            check(vnm_prepare_as(A_values.data_ptr(), (const uint32_t *)A_metadata.data_ptr(), (const uint32_t *)A_indices.data_ptr(), M, K, V,
+                                 (int)n, (int)m, dense_b ? VNM_STRATEGY_DENSE_B : VNM_STRATEGY_GATHER, &e.handle[dense_b], stream), "vnm_prepare_as");
+        h = e.handle[dense_b];
     }
     auto out = torch::empty({N, M}, rhs_matrix.options());
-    int dense_b = 0;
-    check(vnm_operand_form(h, &dense_b), "vnm_operand_form");
-    if (rhs_is_t_view && dense_b && rhs_matrix.stride(1) % 8 == 0 && (reinterpret_cast<uintptr_t>(rhs_matrix.data_ptr()) & 15) == 0) {
-        check(vnm_spmm_f16_nk(h, rhs_matrix.data_ptr(), rhs_matrix.stride(1), N, has_bias ? bias->data_ptr() : nullptr, out.data_ptr(), M,
-                              VNM_LAYOUT_NM, stream), "vnm_spmm_f16_nk");
+    const void *bias_ptr = has_bias ? bias->data_ptr() : nullptr;
+    if (in_place) {
+        torch::Tensor ws;
+        if (!dense_b) ws = torch::empty({K, N}, rhs_matrix.options());
+        check(vnm_spmm_f16_nk_ws(h, rhs_matrix.data_ptr(), rhs_matrix.stride(1), N, bias_ptr, out.data_ptr(), M, VNM_LAYOUT_NM,
+                                 dense_b ? out.data_ptr() : ws.data_ptr(), stream), "vnm_spmm_f16_nk");
         return out;
     }
     torch::Tensor rhs = rhs_matrix.stride(1) == 1 ? rhs_matrix : rhs_matrix.contiguous();
-    check(vnm_spmm_f16(h, rhs.data_ptr(), rhs.stride(0), N, has_bias ? bias->data_ptr() : nullptr, out.data_ptr(), M, VNM_LAYOUT_NM, stream),
-          "vnm_spmm_f16");
+    check(vnm_spmm_f16(h, rhs.data_ptr(), rhs.stride(0), N, bias_ptr, out.data_ptr(), M, VNM_LAYOUT_NM, stream), "vnm_spmm_f16");
     return out;
 }
 
 void clear_cache()
 {
     std::lock_guard<std::mutex> lock(g_mutex);
-    for (auto &kv : g_cache) vnm_destroy(kv.second.handle);
+    for (auto &kv : g_cache) kv.second.release();
     g_cache.clear();
 }
 

@@ -93,24 +93,26 @@ int ensure_kernels_ready(int *device_out)
     std::lock_guard<std::mutex> lock(g_init_mutex);
     if (!g_kernels_ready[dev]) {
         VNM_CUDA(spmm_init_kernels(), "cudaFuncSetAttribute(max dynamic shared memory)");
-        VNM_CUDA(spmm_dense_b_init(), "cudaFuncSetAttribute(max dynamic shared memory)");
         VNM_CUDA(spmm_dense_b_pair_init(), "cudaFuncSetAttribute(max dynamic shared memory)");
+        VNM_CUDA(spmm_small_init(), "cudaFuncSetAttribute(max dynamic shared memory)");
         g_kernels_ready[dev] = true;
     }
     if (device_out) *device_out = dev;
     return VNM_OK;
 }
 
-// Gather form vs dense-B form (see vnm_set_strategy in the header).  Measured on B200: the gather path is
-// bound by the TMA gather rate and pays NB = 128/V times for small vector lengths, the dense-B form costs
-// m/4 times the MMA work but shares B between all vector blocks.
-bool choose_dense_b(int K, int V, int m, int strategy)
+// Gather form vs dense-B form (see vnm_set_strategy in the header).  The gather form multiplies only what the pattern
+// keeps but gathers, and multiplies with masked MMAs, once per vector block of a row tile; the dense-B form costs m/4 times
+// the MMA work and shares B between all blocks.  Measured on B200 (4096 x 4096, N = 16384): V = 128 from m = 16 on 125 us
+// against 240, at m = 8 207 against 245 (and 15.7 against 20.2 ms at 49152 x 12288 x 32768, where the power cap decides and
+// the zeros of the dense-B form cost what they weigh) unless there are only a few row tiles; V = 64 from m = 32 on; V = 32
+// beyond m = 32.
+bool choose_dense_b(int M, int K, int V, int m, int strategy)
 {
     const bool possible = (m % 4 == 0) && (K % m == 0);
     if (!possible || strategy == VNM_STRATEGY_GATHER) return false;
     if (strategy == VNM_STRATEGY_DENSE_B) return true;
-    // measured on B200 (N = 16384): the dense-B kernel wins for every V at m <= 8, at m = 16 for V <= 64 and at
-    // m = 32 for V = 32 (the gather kernel gathers, and multiplies with masked MMAs, once per vector block of a row tile)
+    if (V == 128 && m == 8 && M >= 1024) return false;
     if (m <= 8) return true;
     if (V <= 64 && m <= 16) return true;
     return V == 32 && m <= 32;
@@ -133,7 +135,7 @@ struct vnm_prepared_s {
     int64_t tm_ldb;
     int tm_N;
     int tm_nk;
-    int tm_pair;             // the cached maps are the pair kernel's (half stages)
+    int tm_kind;             // the kernel (and, for the small one, the tile width) that the cached maps belong to
     bool tm_valid;
     CUtensorMap tmap_rows;
     CUtensorMap tmap_tile;
@@ -160,6 +162,31 @@ struct vnm_prepared_s {
     int pair_mode;     // dense-B form: 1 = use the two-SM (cta_group::2) kernel where it applies (default), 0 = never
     int max_ctas;      // 0 = one persistent CTA per SM, else the cap set by vnm_set_max_ctas
 };
+
+namespace {
+
+// Fills in what follows from the shape and the operand form.
+void shape_handle(vnm_prepared_s *h, int M, int K, int V, int n, int m, bool dense_b)
+{
+    h->M = M; h->K = K; h->V = V; h->n = n; h->m = m;
+    h->Ksp = ksp_of(K, m);
+    h->mtiles = (M + TILE_M - 1) / TILE_M;
+    h->dense_b = dense_b ? 1 : 0;
+    if (dense_b) {
+        h->ktiles = (K + 127) / 128;  // a k-tile covers 128 original columns
+        h->nb = 1;
+        h->gather_mode = GATHER_CONTIG;
+    } else {
+        h->ktiles = (int)((h->Ksp + KT_COMP - 1) / KT_COMP);
+        h->nb = TILE_M / V;
+        h->gather_mode = (m == 4) ? GATHER_CONTIG : GATHER_TMA4;  // with m == 4 every row of B is selected
+    }
+    h->vblocks_padded = h->mtiles * h->nb;
+    h->pair_mode = 1;
+    h->l2_hints = 1;
+}
+
+}  // namespace
 
 extern "C" {
 
@@ -221,7 +248,7 @@ int vnm_prepared_bytes(int M, int K, int V, int n, int m, int64_t *bytes)
     if (rc) return rc;
     if (V != 32 && V != 64 && V != 128) return fail(VNM_ERR_UNSUPPORTED, "SpMM supports V in {32, 64, 128} (got %d)", V);
     const int64_t Ksp = ksp_of(K, m);
-    const bool dense_b = choose_dense_b(K, V, m, g_strategy);
+    const bool dense_b = choose_dense_b(M, K, V, m, g_strategy);
     const int64_t mtiles = (M + TILE_M - 1) / TILE_M, ktiles = dense_b ? (K + 127) / 128 : (Ksp + KT_COMP - 1) / KT_COMP;
     const int64_t nb = dense_b ? 1 : TILE_M / V;
     if (bytes) *bytes = mtiles * ktiles * AM_BLOCK_BYTES + mtiles * nb * ktiles * KT_GROUPS * 16 + 256;
@@ -249,22 +276,7 @@ int vnm_prepare_as(const void *values, const uint32_t *meta, const uint32_t *col
     vnm_prepared_s *h = new (std::nothrow) vnm_prepared_s();
     if (!h) return fail(VNM_ERR_CUDA, "out of host memory");
     memset(h, 0, sizeof(*h));
-    h->M = M; h->K = K; h->V = V; h->n = n; h->m = m;
-    h->Ksp = ksp_of(K, m);
-    h->mtiles = (M + TILE_M - 1) / TILE_M;
-    h->dense_b = choose_dense_b(K, V, m, strategy) ? 1 : 0;
-    if (h->dense_b) {
-        h->ktiles = (K + 127) / 128;  // a k-tile covers 128 original columns
-        h->nb = 1;
-        h->gather_mode = GATHER_CONTIG;
-    } else {
-        h->ktiles = (int)((h->Ksp + KT_COMP - 1) / KT_COMP);
-        h->nb = TILE_M / V;
-        h->gather_mode = (m == 4) ? GATHER_CONTIG : GATHER_TMA4;  // with m == 4 every row of B is selected
-    }
-    h->vblocks_padded = h->mtiles * h->nb;
-    h->pair_mode = 1;
-    h->l2_hints = 1;
+    shape_handle(h, M, K, V, n, m, choose_dense_b(M, K, V, m, strategy));
     h->device = dev_now;
     cudaError_t e = cudaMalloc(&h->am, (size_t)h->mtiles * h->ktiles * AM_BLOCK_BYTES);
     if (e == cudaSuccess) e = cudaMalloc(&h->rows, (size_t)h->vblocks_padded * h->ktiles * KT_GROUPS * sizeof(int4));
@@ -387,15 +399,53 @@ int vnm_set_producer_warps(vnm_handle_t h, int warps)
     return VNM_OK;   // the kernel's sixteen producer warps are part of its layout
 }
 
+}  // extern "C"
+
+namespace {
+
+enum Kernel { KERNEL_GATHER, KERNEL_PAIR, KERNEL_SMALL };
+
+// Which kernel multiplies this operand with N columns, and its configuration: the one with the smallest estimate (in
+// microseconds, stored in *us).  False if none can.
+bool choose_kernel(vnm_handle_t h, int N, int n_more, Kernel *kernel, SpmmConfig *cfg, float *us)
+{
+    memset(cfg, 0, sizeof(*cfg));
+    float big = -1.0f;
+    if (!h->dense_b) {
+        big = spmm_select_config(h->V, N, h->M, h->ktiles, h->max_ctas, cfg);
+        *kernel = KERNEL_GATHER;
+    } else {
+        if (h->pair_mode || n_more > 0) big = spmm_dense_b_pair_config(h->M, N, h->K, h->max_ctas, h->pair_rows, cfg);
+        *kernel = KERNEL_PAIR;
+    }
+    *us = big;
+    // The small kernel has one destination, no cap on its CTAs (it is not persistent) and none of the other kernels' ablations.
+    if (n_more == 0 && h->max_ctas == 0 && !h->nm_tma_always && !h->out32 && h->pair_rows == 0 && h->gather_mode != GATHER_CPASYNC) {
+        SpmmConfig small_cfg;
+        const float small = spmm_small_config(h->mtiles, h->ktiles, N, h->nb, h->gather_mode == GATHER_TMA4, &small_cfg);
+        // up to SMALL_SPLIT_N columns it alone is used: its split makes the order of summation its own
+        if (N <= SMALL_SPLIT_N || big < 0.0f || small < big) {
+            *cfg = small_cfg;
+            *kernel = KERNEL_SMALL;
+            *us = small;
+        }
+    }
+    if (*us < 0.0f && h->dense_b) *us = spmm_dense_b_pair_config(h->M, N, h->K, h->max_ctas, h->pair_rows, cfg);   // one SM per tile is not to be had
+    return *us >= 0.0f;
+}
+
+}  // namespace
+
+extern "C" {
+
 int vnm_spmm_config(vnm_handle_t h, int N, int *tile_m, int *tile_n, int *stages, int *grid, int *smem_bytes)
 {
     if (!h) return fail(VNM_ERR_BAD_ARG, "null handle");
     SpmmConfig cfg;
-    const bool pair = h->dense_b && h->pair_mode && N >= 128 && spmm_dense_b_pair_config(h->M, N, h->K, h->max_ctas, h->pair_rows, &cfg);
-    if (pair) { /* cfg filled */ }
-    else if (h->dense_b) spmm_dense_b_config(h->M, N, h->max_ctas, &cfg);
-    else if (!spmm_select_config(h->V, N, h->M, h->max_ctas, &cfg)) return fail(VNM_ERR_UNSUPPORTED, "unsupported V");
-    if (tile_m) *tile_m = h->dense_b ? cfg.nb * TILE_M : TILE_M;  // pairs: 512 or 256, one SM per tile: 256 or 128
+    Kernel kernel;
+    float us;
+    if (!choose_kernel(h, N, 0, &kernel, &cfg, &us)) return fail(VNM_ERR_UNSUPPORTED, "no kernel for this operand and its switches");
+    if (tile_m) *tile_m = kernel == KERNEL_PAIR ? cfg.nb * TILE_M : TILE_M;  // pairs: 512 or 256
     if (tile_n) *tile_n = cfg.bn;
     if (stages) *stages = cfg.stages;
     if (grid) *grid = cfg.grid;
@@ -423,7 +473,7 @@ CUresult vnm::encode_out_map(EncodeTiledFn enc, CUtensorMap *map, void *out, int
 extern "C" {
 
 static int spmm_impl(vnm_handle_t h, const void *B, int64_t ldb, int N, int b_nk, const void *bias, void *out, int64_t ldo, int layout,
-                     void *stream, void *const *more_outs = nullptr, int n_more = 0)
+                     void *stream, void *const *more_outs = nullptr, int n_more = 0, bool after_transpose = false)
 {
     if (!h || !B || !out) return fail(VNM_ERR_BAD_ARG, "vnm_spmm_f16: null pointer");
     if (n_more < 0 || n_more > MAX_OUTS - 1 || (n_more > 0 && !more_outs))
@@ -454,29 +504,33 @@ static int spmm_impl(vnm_handle_t h, const void *B, int64_t ldb, int N, int b_nk
             return fail(VNM_ERR_BAD_ARG, "vnm_spmm_f16: layout MN needs ldo >= N, ldo %% 8 == 0 and a 16-byte aligned out");
     } else if (layout == VNM_LAYOUT_NM) {
         if (ldo < h->M) return fail(VNM_ERR_BAD_ARG, "vnm_spmm_f16: layout NM needs ldo >= M");
+        if (h->dense_b && (ldo % 8 != 0 || ((uintptr_t)out & 15)))
+            return fail(VNM_ERR_BAD_ARG, "vnm_spmm_f16: layout NM needs ldo %% 8 == 0 and a 16-byte aligned out for this operand");
     } else {
         return fail(VNM_ERR_BAD_ARG, "vnm_spmm_f16: unknown layout %d", layout);
     }
     SpmmConfig cfg;
-    const bool pair = h->dense_b && h->pair_mode && (b_nk || N >= 128) && spmm_dense_b_pair_config(h->M, N, h->K, h->max_ctas, h->pair_rows, &cfg);
-    if (pair) { /* cfg filled */ }
-    else if (h->dense_b) spmm_dense_b_config(h->M, N, h->max_ctas, &cfg);
-    else if (!spmm_select_config(h->V, N, h->M, h->max_ctas, &cfg)) return fail(VNM_ERR_UNSUPPORTED, "unsupported V");
+    Kernel kernel;
+    float us;
+    if (!choose_kernel(h, N, n_more, &kernel, &cfg, &us)) return fail(VNM_ERR_UNSUPPORTED, "vnm_spmm_f16: no kernel for this operand and its switches");
+    const bool pair = kernel == KERNEL_PAIR;
+    const int kind = kernel == KERNEL_SMALL ? 1000 * h->gather_mode + cfg.bn : -(int)kernel;
     EncodeTiledFn enc = get_encode_fn();
     if (!enc) return fail(VNM_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
 
-    if (!h->tm_valid || h->tm_B != B || h->tm_ldb != ldb || h->tm_N != N || h->tm_nk != b_nk || h->tm_pair != (pair ? 1 : 0)) {
+    if (!h->tm_valid || h->tm_B != B || h->tm_ldb != ldb || h->tm_N != N || h->tm_nk != b_nk || h->tm_kind != kind) {
         cuuint32_t estr[2] = {1, 1};
         CUresult r;
-        if (b_nk) {
-            // B given as [N, K] (K contiguous): one box of 32 k x 256 rows (n), written with the 64-byte swizzle,
-            // is the K-major operand tile of one MMA (the last 16 rows belong to the next tile and are not read).
+        if (kernel == KERNEL_SMALL) {
+            r = spmm_small_encode(enc, &h->tmap_tile, B, ldb, h->K, N, b_nk, h->gather_mode, cfg.bn);
+            h->tm_wide = false;
+        } else if (b_nk) {
             cuuint64_t dims[2] = {(cuuint64_t)h->K, (cuuint64_t)N};
             cuuint64_t strides[1] = {(cuuint64_t)ldb * 2};
-            // the pair kernel loads each CTA's 128-row half separately, 64 k (two MMA K blocks, 128-byte rows) per box
-            cuuint32_t box[2] = {pair ? 64u : 32u, pair ? 128u : 256u};
+            // B given as [N, K] (K contiguous): a CTA of the pair loads its 128 n-rows, 64 k (two MMA K blocks, 128-byte rows) per box
+            cuuint32_t box[2] = {64, 128};
             r = enc(&h->tmap_tile, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(B), dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, pair ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
             h->tmap_rows = h->tmap_tile;
             h->tmap_tile2 = h->tmap_tile;
@@ -498,7 +552,7 @@ static int spmm_impl(vnm_handle_t h, const void *B, int64_t ldb, int N, int b_nk
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
             h->tmap_tile2 = h->tmap_tile;
             h->tm_wide = false;
-            if (r == CUDA_SUCCESS && pair) {
+            if (r == CUDA_SUCCESS && pair && N >= 128) {
                 // pair kernel: a CTA's half of a stage is {64 columns, 64 rows, 2 slices} starting at any multiple of 8 columns
                 // (pair tiles start at multiples of 240, the peer's half 120 columns further)
                 cuuint64_t dims4[4] = {64, (cuuint64_t)h->K, 2, (cuuint64_t)((N - 128) / 8 + 1)};
@@ -512,25 +566,10 @@ static int spmm_impl(vnm_handle_t h, const void *B, int64_t ldb, int N, int b_nk
                     h->tmap_tile = wide;
                     h->tm_wide = true;
                 }
-            } else if (r == CUDA_SUCCESS && h->dense_b && N >= 256) {
-                // dense-B kernel: {64 columns, K rows, 4 slices of 64 columns, start column / 16}.  A box {64, 32, 4, 1}
-                // lands as [slice][row][64 columns], the N-major operand tile of one MMA, with a single instruction.
-                // Only start columns whose 256 columns lie inside N are addressable; the ragged edge uses the 2-D map.
-                cuuint64_t dims4[4] = {64, (cuuint64_t)h->K, 4, (cuuint64_t)((N - 256) / 16 + 1)};
-                cuuint64_t strides4[3] = {(cuuint64_t)ldb * 2, 128, 32};
-                cuuint32_t box4[4] = {64, 32, 4, 1};
-                cuuint32_t estr4[4] = {1, 1, 1, 1};
-                CUtensorMap wide;
-                if (enc(&wide, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<void *>(B), dims4, strides4, box4, estr4,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS) {
-                    h->tmap_tile = wide;
-                    h->tm_wide = true;
-                }
             }
         }
         if (r != CUDA_SUCCESS) return fail(VNM_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
-        h->tm_B = B; h->tm_ldb = ldb; h->tm_N = N; h->tm_nk = b_nk; h->tm_pair = pair ? 1 : 0; h->tm_valid = true;
+        h->tm_B = B; h->tm_ldb = ldb; h->tm_N = N; h->tm_nk = b_nk; h->tm_kind = kind; h->tm_valid = true;
     }
 
     SpmmParams p;
@@ -577,11 +616,16 @@ static int spmm_impl(vnm_handle_t h, const void *B, int64_t ldb, int N, int b_nk
     p.n_out = 1;
     p.tma_out = 1;
     p.out32 = 0;
-    if (h->dense_b) {
+    p.split_k = 1;
+    p.early = 0;
+    if (kernel == KERNEL_SMALL) {
+        p.tma_out = 0;
+        p.split_k = cfg.split;
+        p.early = after_transpose ? 1 : 0;
+        VNM_CUDA(launch_spmm_small(cfg, h->tmap_tile, p, (cudaStream_t)stream), "spmm launch");
+    } else if (h->dense_b) {
         // The result leaves through TMA stores: [M,N] as boxes of 40 columns x 128 rows, [N,M] as boxes of 128
         // columns (m) x 40 rows (n).
-        if (layout == VNM_LAYOUT_NM && (ldo % 8 != 0 || ((uintptr_t)out & 15)))
-            return fail(VNM_ERR_BAD_ARG, "vnm_spmm_f16: layout NM needs ldo %% 8 == 0 and a 16-byte aligned out for this operand");
         CUtensorMap tmap_out;
         OutMaps more;
         memset(&more, 0, sizeof(more));
@@ -590,8 +634,7 @@ static int spmm_impl(vnm_handle_t h, const void *B, int64_t ldb, int N, int b_nk
             if (r != CUDA_SUCCESS) return fail(VNM_ERR_CUDA, "cuTensorMapEncodeTiled (output %d) failed with CUresult %d", d, (int)r);
         }
         p.n_out = 1 + n_more;
-        if (pair) VNM_CUDA(launch_spmm_dense_b_pair(cfg, h->tmap_tile, h->tmap_tile2, tmap_out, more, p, (cudaStream_t)stream), "spmm launch");
-        else VNM_CUDA(launch_spmm_dense_b(cfg, h->tmap_tile, h->tmap_tile2, tmap_out, more, p, (cudaStream_t)stream), "spmm launch");
+        VNM_CUDA(launch_spmm_dense_b_pair(cfg, h->tmap_tile, h->tmap_tile2, tmap_out, more, p, (cudaStream_t)stream), "spmm launch");
     } else {
         // Gather form: the epilogue stores straight from tensor memory.  Only a [N,M] result with several destinations (or on
         // request) leaves through shared memory and TMA stores, boxes of 128 columns (m) x cfg.part rows (n).
@@ -623,6 +666,43 @@ int vnm_spmm_f16(vnm_handle_t h, const void *B, int64_t ldb, int N, const void *
 int vnm_spmm_f16_nk(vnm_handle_t h, const void *Bt, int64_t ldbt, int N, const void *bias, void *out, int64_t ldo, int layout, void *stream)
 {
     return spmm_impl(h, Bt, ldbt, N, 1, bias, out, ldo, layout, stream);
+}
+
+int vnm_spmm_f16_nk_ws(vnm_handle_t h, const void *Bt, int64_t ldbt, int N, const void *bias, void *out, int64_t ldo, int layout, void *workspace,
+                       void *stream)
+{
+    if (!h || !Bt || !workspace) return fail(VNM_ERR_BAD_ARG, "vnm_spmm_f16_nk_ws: null pointer");
+    if (N <= 0 || N % 8 != 0) return fail(VNM_ERR_BAD_ARG, "vnm_spmm_f16_nk_ws: N (%d) must be a positive multiple of 8", N);
+    if (ldbt < h->K || ldbt % 8 != 0 || ((uintptr_t)Bt & 15) || ((uintptr_t)workspace & 15))
+        return fail(VNM_ERR_BAD_ARG, "vnm_spmm_f16_nk_ws: ldbt (%lld) must be >= K and a multiple of 8, Bt and workspace 16-byte aligned", (long long)ldbt);
+    if (h->dense_b) return spmm_impl(h, Bt, ldbt, N, 1, bias, out, ldo, layout, stream);
+    VNM_CUDA(launch_transpose(Bt, ldbt, N, h->K, workspace, (cudaStream_t)stream), "transpose launch");
+    return spmm_impl(h, workspace, N, N, 0, bias, out, ldo, layout, stream, nullptr, 0, true);
+}
+
+int vnm_choose_form(int M, int K, int V, int n, int m, int N, int b_nk, int *strategy)
+{
+    int rc = check_format(M, K, V, n, m);
+    if (rc) return rc;
+    if (!strategy || N <= 0) return fail(VNM_ERR_BAD_ARG, "vnm_choose_form: bad argument");
+    if (V != 32 && V != 64 && V != 128) return fail(VNM_ERR_UNSUPPORTED, "SpMM supports V in {32, 64, 128} (got %d)", V);
+    if ((rc = ensure_kernels_ready(nullptr))) return rc;
+    *strategy = choose_dense_b(M, K, V, m, g_strategy) ? VNM_STRATEGY_DENSE_B : VNM_STRATEGY_GATHER;
+    if (!b_nk || !choose_dense_b(M, K, V, m, VNM_STRATEGY_DENSE_B)) return VNM_OK;
+    // [N,K] activations: the dense-B form reads them in place, the gather form needs their transpose (read and written once,
+    // at about 4.5 TB/s, and a launch)
+    vnm_prepared_s h;
+    float us[2] = {-1.0f, -1.0f};
+    for (int form = 0; form < 2; form++) {
+        memset(&h, 0, sizeof(h));
+        shape_handle(&h, M, K, V, n, m, form == 1);
+        Kernel kernel;
+        SpmmConfig cfg;
+        if (!choose_kernel(&h, N, 0, &kernel, &cfg, &us[form])) us[form] = -1.0f;
+    }
+    if (us[0] >= 0.0f) us[0] += m == 4 ? 1e6f : 2.0f + 4.0f * (float)N * (float)K / 4.5e6f;
+    *strategy = us[0] >= 0.0f && (us[1] < 0.0f || us[0] < us[1]) ? VNM_STRATEGY_GATHER : VNM_STRATEGY_DENSE_B;
+    return VNM_OK;
 }
 
 int vnm_spmm_f16_multi(vnm_handle_t h, const void *B, int64_t ldb, int N, const void *bias, void *const *outs, int n_outs, int64_t ldo, int layout,

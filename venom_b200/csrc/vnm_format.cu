@@ -876,6 +876,59 @@ __global__ void __launch_bounds__(256) prepare_dense_b_rows_kernel(int K, int mt
     }
 }
 
+// ------------------------------------------------------------------------------------------------
+// Transpose of an activation, [N, K] -> [K, N] (fp16), for the gather form, which needs rows of B.  A block takes 64 n x 64 k:
+// a thread reads 16 bytes (8 k) of two neighbouring n, interleaves them into eight words (n, n + 1) and puts them into shared
+// memory as [k][n pair] (pitch 33 words); then eight threads write the 128 bytes of one k.  Bound by HBM / L2: both
+// sides move 128 contiguous bytes a row.
+// ------------------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(256) transpose_kernel(const __half *__restrict__ src, int64_t ld, int N, int K, __half *__restrict__ dst)
+{
+    __shared__ uint32_t tile[64 * 33];
+    grid_launch_dependents();   // the product's set-up may begin
+    const int k0 = blockIdx.x * 64, n0 = blockIdx.y * 64;
+    {
+        const int c = threadIdx.x & 7, np = threadIdx.x >> 3;   // 8 k at k0 + 8 c of rows n0 + 2 np, + 1 (N is even: both exist or neither)
+        const int k = k0 + 8 * c, n = n0 + 2 * np;
+        if (n < N && k < K) {
+            const __half *r0 = src + (int64_t)n * ld + k, *r1 = r0 + ld;
+            uint32_t a[4] = {0, 0, 0, 0}, b[4] = {0, 0, 0, 0};
+            if (k + 8 <= K) {
+                const uint4 x = __ldg(reinterpret_cast<const uint4 *>(r0)), y = __ldg(reinterpret_cast<const uint4 *>(r1));
+                a[0] = x.x; a[1] = x.y; a[2] = x.z; a[3] = x.w;
+                b[0] = y.x; b[1] = y.y; b[2] = y.z; b[3] = y.w;
+            } else {   // K ends inside the piece
+                for (int i = 0; i < K - k; i++) {
+                    a[i >> 1] |= (uint32_t)__half_as_ushort(r0[i]) << (16 * (i & 1));
+                    b[i >> 1] |= (uint32_t)__half_as_ushort(r1[i]) << (16 * (i & 1));
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                tile[(8 * c + 2 * i) * 33 + np] = __byte_perm(a[i], b[i], 0x5410);
+                tile[(8 * c + 2 * i + 1) * 33 + np] = __byte_perm(a[i], b[i], 0x7632);
+            }
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const int k = (threadIdx.x >> 3) + 32 * i, q = threadIdx.x & 7;
+        const int n = n0 + 8 * q;
+        if (k0 + k < K && n < N) {   // N is a multiple of 8
+            const uint32_t *w = tile + k * 33 + 4 * q;
+            *reinterpret_cast<uint4 *>(dst + (int64_t)(k0 + k) * N + n) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+    }
+}
+
+cudaError_t launch_transpose(const void *src, int64_t ld_src, int N, int K, void *dst, cudaStream_t stream)
+{
+    const dim3 grid((unsigned)((K + 63) / 64), (unsigned)((N + 63) / 64));
+    transpose_kernel<<<grid, 256, 0, stream>>>((const __half *)src, ld_src, N, K, (__half *)dst);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_prepare_dense_b(const void *values, const uint32_t *meta, const uint32_t *colloc, int M, int K, int V, int m,
                                    void *am, void *rows, int mtiles, int ktiles, cudaStream_t stream)
 {

@@ -33,11 +33,13 @@ struct SpmmParams {
     int hybrid_rows;      // gather kernel, GATHER_CPASYNC: of 64 rows of a block, those fetched by TMA gather4 beside the copies (0, 16, 32, 48)
     int group_m;          // band of the tile order (tile_coords): > 0 row groups per band, < 0 column tiles per band
     uint64_t hint_a, hint_b;  // pair kernel: L2 eviction-priority policies of the A and B loads (L2_EVICT_*)
-    int b_nk;             // dense-B kernel only: the dense operand is given as [N, K] row-major (K contiguous)
-    int b_wide_ok;        // dense-B kernel only: the 4-D tensor map exists (column tiles with 256 columns inside N use one box per stage)
+    int b_nk;             // dense-B form only: the dense operand is given as [N, K] row-major (K contiguous)
+    int b_wide_ok;        // pair kernel: the 4-D tensor map exists (halves with 128 columns inside N use one box per stage)
     int l2_ahead;         // pair kernel: k-tiles by which L2 prefetches run ahead of the loads into shared memory (0 = none)
     int out32;            // gather kernel, layout MN: 32-bit stores (ablation)
     int tma_out;          // gather kernel, layout NM: the result leaves through shared memory and TMA stores (tmap_out / OutMaps valid), else from registers
+    int early;            // small kernel: launched before the kernel that writes B has finished (programmatic dependent launch)
+    int split_k;          // small kernel: CTAs of a cluster that share one tile's k-tiles
     int n_out;            // destinations of every output tile stored through TMA (1 = `out` only; more: the OutMaps argument, e.g. peers' buffers)
 };
 
@@ -61,10 +63,12 @@ struct SpmmConfig {
     int bn;      // tile N
     int nb;      // V-blocks per 128-row tile
     int part;    // columns per epilogue part (width of a TMA store box)
-    int stages;  // gather kernel: number of B-producer warps; dense-B kernels: SMs per tile
+    int stages;  // gather kernel: number of B-producer warps; the others: SMs per tile
     int smem_bytes;
     int threads;
-    int grid;    // persistent CTAs
+    int grid;    // CTAs (persistent ones, except in the small kernel)
+    int split;   // small kernel: CTAs that share a tile's k-tiles
+    int resident;  // small kernel: CTAs per SM
 };
 
 // Host-side helpers shared by the translation units that implement C-ABI entry points (defined in vnm_capi.cu).
@@ -86,31 +90,39 @@ cudaError_t launch_prepare(const void *values, const uint32_t *meta, const uint3
 cudaError_t launch_prepare_dense_b(const void *values, const uint32_t *meta, const uint32_t *colloc, int M, int K, int V, int m,
                                    void *am, void *rows, int mtiles, int ktiles, cudaStream_t stream);
 
+cudaError_t launch_transpose(const void *src, int64_t ld_src, int N, int K, void *dst, cudaStream_t stream);  // [N, K] -> [K, N], fp16
+
 cudaError_t launch_prune(const float *w, int64_t ldw, int M, int K, int V, int m, int32_t *mask, int64_t ldm, uint32_t *colloc,
                          cudaStream_t stream);
 
-// Chooses the tile configuration for (V, N).  Returns false for an unsupported V.
-bool spmm_select_config(int V, int N, int M, int max_ctas, SpmmConfig *cfg);  // max_ctas: 0 = one per SM
+// Tile configuration of the gather kernel.
+float spmm_select_config(int V, int N, int M, int ktiles, int max_ctas, SpmmConfig *cfg);  // max_ctas: 0 = one per SM; returns an estimate in microseconds, < 0 for an unsupported V
 // Opt-in to large dynamic shared memory for every kernel instance on the CURRENT device (call once per device).
 cudaError_t spmm_init_kernels();
 cudaError_t launch_spmm(const SpmmConfig &cfg, const CUtensorMap &tmap_rows, const CUtensorMap &tmap_tile, const CUtensorMap &tmap_out,
                         const OutMaps &more_out, const SpmmParams &p,
                         cudaStream_t stream);
 
-// Dense-B form: 256 x 128 tiles, two accumulators sharing every B stage (vnm_spmm_dense_b.cu).
-cudaError_t spmm_dense_b_init();
+// Few columns or few tiles, both operand forms: 128 x (16 .. 128) tiles, several CTAs per SM, k-tiles split over a cluster
+// for N <= SMALL_SPLIT_N (vnm_spmm_small.cu).  nb: vector blocks per row tile (1 for the dense-B form).
+constexpr int SMALL_SPLIT_N = 64;
+cudaError_t spmm_small_init();
 cudaError_t launch_wait_expiry_selftest(int *status, cudaStream_t stream);
-void spmm_dense_b_config(int M, int N, int max_ctas, SpmmConfig *cfg);  // max_ctas: 0 = one per SM
-cudaError_t launch_spmm_dense_b(const SpmmConfig &cfg, const CUtensorMap &tmap_tile, const CUtensorMap &tmap_tile2, const CUtensorMap &tmap_out, const OutMaps &more_out,
-                                const SpmmParams &p, cudaStream_t stream);
+float spmm_small_config(int mtiles, int ktiles, int N, int nb, bool gather, SpmmConfig *cfg);   // returns its estimate in microseconds
+CUresult spmm_small_encode(EncodeTiledFn enc, CUtensorMap *map, const void *B, int64_t ldb, int K, int N, int b_nk, int gather_mode, int bn);
+cudaError_t launch_spmm_small(const SpmmConfig &cfg, const CUtensorMap &tmap_b, const SpmmParams &p, cudaStream_t stream);
 
 // Dense-B form on pairs of SMs (clusters of two CTAs, tcgen05 cta_group::2): 512 x 240 pair tiles (vnm_spmm_dense_b2.cu).
 cudaError_t spmm_dense_b_pair_init();
-bool spmm_dense_b_pair_config(int M, int N, int K, int max_ctas, int force_rows, SpmmConfig *cfg);  // false: use the single-CTA kernel; force_rows: 0 auto, 1 / 2 row tiles per CTA
+float spmm_dense_b_pair_config(int M, int N, int K, int max_ctas, int force_rows, SpmmConfig *cfg);  // < 0: not for this problem, else an estimate in microseconds; force_rows: 0 auto, 1 / 2 row tiles per CTA
 cudaError_t launch_spmm_dense_b_pair(const SpmmConfig &cfg, const CUtensorMap &tmap_tile, const CUtensorMap &tmap_tile2, const CUtensorMap &tmap_out, const OutMaps &more_out,
                                      const SpmmParams &p, cudaStream_t stream);
 
 #if defined(__CUDACC__)
+// Programmatic dependent launch: waits until the kernels this launch depends on have finished; lets dependents start.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- bounded waits of the persistent kernels ----
 constexpr long long WAIT_LIMIT_CYCLES = 4000000000LL;  // ~2 s at B200 clocks
 
@@ -172,93 +184,201 @@ __device__ __forceinline__ void drain_slot(uint64_t *bar, uint32_t parity, int *
 
 // ---- epilogue of one warp straight from tensor memory to global memory (32 accumulator lanes x BN columns) ----
 // Nothing of it passes through shared memory, whose port the mainloop needs: the operand reads of the MMAs and the TMA
-// writes of the rings together keep it busy all the time.  `trow` is the address of the accumulator at this warp's lane
-// quadrant q, `row0` the actual row of accumulator lane 0 of the tile.  `release` runs (converged) once the last column has
-// been read.  Columns >= N and rows >= M are not stored.
+// writes of the rings together keep it busy all the time.  What the stores must not do is flood L2 with small pieces, behind
+// which the loads of the next tile queue: sectors of 32 bytes from 32 different rows cost the next tile about 3500 of its
+// 11000 clocks (4096 x 1024 x 16384, [M,N]).  So lanes exchange words of [M,N] results until an instruction writes 128
+// contiguous bytes of a row.  Accumulators are read in fragment order: thread t holds columns 2 (t % 4), + 1 of every eight for lanes t / 4 and
+// t / 4 + 8 of a 16-lane group, which are the actual rows 2 (t / 4) and 2 (t / 4) + 1.  Work goes in chunks of 64 columns,
+// 32 packed words a thread.  Columns >= N and rows >= M are not stored.
 
-// [M,N]: a lane owns a row and stores 16 columns, one 32-byte sector, at a time (two 16-byte pieces where the rows are
-// not 32-byte aligned or N ends inside; 4-byte words for the `out32` ablation, the reference's OUT_32B build,
-// common/epilogue.h:34-61).
-template <int BN, typename Release>
-__device__ __forceinline__ void store_tile_mn(uint32_t trow, int q, int64_t row0, int n0, const SpmmParams &p, Release release)
+__device__ __forceinline__ void quad_swap(uint32_t &a, uint32_t &b, bool up, int mask)   // exchanges b of the lower lane with a of the upper one
 {
-    constexpr int SPAN = BN % 48 == 0 ? 48 : BN < 32 ? BN : 32;
-    static_assert(BN % SPAN == 0 && SPAN % 16 == 0, "column spans");
-    const int lane = threadIdx.x & 31;
-    const int64_t row = row0 + mma_row_to_actual(q * 32 + lane);
-    __half *orow = p.out + row * p.ldo + n0;
-    const bool row_ok = row < p.M;
-    const bool wide = (p.ldo & 15) == 0 && ((uintptr_t)p.out & 31) == 0;
-#pragma unroll 1
-    for (int c0 = 0; c0 < BN; c0 += SPAN) {
-        uint32_t v[SPAN / 16][16];
+    const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? a : b, mask);
+    if (up) a = got; else b = got;
+}
+
+// [M,N]: a quad of threads holds 64 columns of a row as words (8 j + 2 i, + 1); two 4 x 4 transposes give each thread 16
+// consecutive columns, so that a store instruction (32 bytes a thread) writes 128 contiguous bytes of eight rows.  16-byte pieces
+// where the rows are not 32-byte aligned or N ends inside; 4-byte words for the `out32` ablation, the reference's
+// OUT_32B build, common/epilogue.h:34-61.
+struct TileStoreMN {
+    __half *dst;         // row 2 (t / 4) of the warp's first 16-row group, this thread's 16 columns of the first chunk
+    int64_t ldo;
+    int left;            // columns from there to N
+    bool ok[2], wide, words;   // ok: rows of the two 16-row groups exist (M is a multiple of 32)
+    uint32_t taddr;
+    // `trow`: the accumulator at this warp's lane quadrant q; row0: the actual row of the tile's first lane
+    __device__ __forceinline__ TileStoreMN(uint32_t trow, int q, int64_t row0, int n0, const SpmmParams &p)
+    {
+        const int lane = threadIdx.x & 31;
+        const int64_t row = row0 + q * 32 + (lane >> 2) * 2;
+        const int n = n0 + (lane & 3) * 16;
+        dst = p.out + row * p.ldo + n;
+        ldo = p.ldo;
+        left = p.N - n;
+        ok[0] = row < p.M; ok[1] = row + 16 < p.M;
+        wide = (p.ldo & 15) == 0 && ((uintptr_t)p.out & 31) == 0;
+        words = p.out32 != 0;
+        taddr = trow;
+    }
+    // one group: words pk[0..7] of row 2w, pk[8..15] of row 2w + 1; word j: columns 8 j + 2 (t % 4), + 1 of the chunk
+    __device__ __forceinline__ static void pack(const uint32_t (&v)[32], uint32_t *pk)
+    {
 #pragma unroll
-        for (int i = 0; i < SPAN / 16; i++) tc_ld_32x32b_x16(trow + (uint32_t)(c0 + 16 * i), v[i]);
-        tc_wait_ld();
-        if (c0 == BN - SPAN) release();
+        for (int j = 0; j < 8; j++) {
+            pk[j] = pack_half2(v[4 * j], v[4 * j + 1]);
+            pk[8 + j] = pack_half2(v[4 * j + 2], v[4 * j + 3]);
+        }
+    }
+    __device__ __forceinline__ void store(int c, int g, int cols, uint32_t *pk) const
+    {
+        const int lane = threadIdx.x & 31;
+        const bool odd = (lane & 1) != 0, upper = (lane & 2) != 0;
 #pragma unroll
-        for (int i = 0; i < SPAN / 16; i++) {
-            uint32_t pk[8];
+        for (int r = 0; r < 2; r++) {
+            uint32_t *w = pk + 8 * r;
+            // words of groups 0, 2, 4, 6 and of 1, 3, 5, 7: thread i ends with groups 2 i and 2 i + 1
 #pragma unroll
-            for (int k = 0; k < 8; k++) pk[k] = pack_half2(v[i][2 * k], v[i][2 * k + 1]);
-            const int c = c0 + 16 * i, left = p.N - n0 - c;
-            if (!row_ok || left <= 0) continue;
-            if (p.out32) {
+            for (int h = 0; h < 2; h++) {
+                quad_swap(w[0 + h], w[2 + h], odd, 1);
+                quad_swap(w[4 + h], w[6 + h], odd, 1);
+                quad_swap(w[0 + h], w[4 + h], upper, 2);
+                quad_swap(w[2 + h], w[6 + h], upper, 2);
+            }
+            const uint32_t o[8] = {w[0], w[2], w[4], w[6], w[1], w[3], w[5], w[7]};
+            const int rest = left - c;
+            if (!ok[g] || rest <= 0 || (lane & 3) * 16 >= cols) continue;
+            __half *d = dst + (int64_t)(16 * g + r) * ldo + c;
+            if (words) {
 #pragma unroll
                 for (int k = 0; k < 8; k++)
-                    if (2 * k < left) *reinterpret_cast<uint32_t *>(orow + c + 2 * k) = pk[k];
-            } else if (wide && left >= 16) {
-                st_global_v8(orow + c, pk);
+                    if (2 * k < rest) *reinterpret_cast<uint32_t *>(d + 2 * k) = o[k];
+            } else if (wide && rest >= 16) {
+                st_global_v8(d, o);
             } else {
-                *reinterpret_cast<uint4 *>(orow + c) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                if (left >= 16) *reinterpret_cast<uint4 *>(orow + c + 8) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+                *reinterpret_cast<uint4 *>(d) = make_uint4(o[0], o[1], o[2], o[3]);
+                if (rest >= 16) *reinterpret_cast<uint4 *>(d + 8) = make_uint4(o[4], o[5], o[6], o[7]);
             }
         }
     }
-}
+};
 
-// [N,M] (+ bias): accumulator lanes w and w + 8 of a 16-lane group are the actual rows 2w and 2w + 1, and the fragment
-// order hands both to one thread: a 32-bit word of two neighbouring m.  Eight threads store one 32-byte sector of an n row, a
-// store instruction four of them.
-template <int BN, typename Release>
-__device__ __forceinline__ void store_tile_nm(uint32_t trow, int q, int64_t row0, int n0, const SpmmParams &p, Release release)
-{
-    const int lane = threadIdx.x & 31;
-    const int64_t m0 = row0 + q * 32 + (lane >> 2) * 2;      // rows m0, m0 + 1 of the first 16-row group; + 16 for the second
-    const bool ok[2] = {m0 < p.M, m0 + 16 < p.M};            // M is a multiple of 32
-    const bool words = (p.ldo & 1) == 0 && ((uintptr_t)p.out & 3) == 0;
-    __half2 bias[2];
+// [N,M] (+ bias): a word is two neighbouring m (rows 2w, 2w + 1), so that eight threads fill a 32-byte sector of an n row and a
+// store instruction writes four of them.  (Exchanging words for 64 contiguous bytes of two n rows took 2.4 times as long.)
+struct TileStoreNM {
+    __half *dst;         // first n this thread stores, its two m of the first 16-row group
+    int64_t ldo;
+    int left;
+    bool ok[2], words;   // ok: rows of the two 16-row groups exist (M is a multiple of 32)
+    __half2 bias[2];     // -0 without a bias: x + -0 is x, bit for bit
+    uint32_t taddr;
+    __device__ __forceinline__ TileStoreNM(uint32_t trow, int q, int64_t row0, int n0, const SpmmParams &p)
+    {
+        const int lane = threadIdx.x & 31;
+        const int64_t m0 = row0 + q * 32 + (lane >> 2) * 2;
+        const int n = n0 + (lane & 3) * 2;
+        dst = p.out + (int64_t)n * p.ldo + m0;
+        ldo = p.ldo;
+        left = p.N - n;
+        words = (p.ldo & 1) == 0 && ((uintptr_t)p.out & 3) == 0;
 #pragma unroll
-    for (int g = 0; g < 2; g++) bias[g] = (p.bias && ok[g]) ? __halves2half2(p.bias[m0 + 16 * g], p.bias[m0 + 16 * g + 1]) : __half2half2(__ushort_as_half((unsigned short)0));
-    const bool has_bias = p.bias != nullptr;
-    const int ncol = n0 + (lane & 3) * 2;
-#pragma unroll 1
-    for (int c0 = 0; c0 < BN; c0 += 16) {
-        uint32_t v[2][8];
-        tc_ld_16x256b_x2(trow + (uint32_t)c0, v[0]);
-        tc_ld_16x256b_x2(trow + (16u << 16) + (uint32_t)c0, v[1]);
-        tc_wait_ld();
-        if (c0 == BN - 16) release();
+        for (int g = 0; g < 2; g++) {
+            ok[g] = m0 + 16 * g < p.M;
+            bias[g] = (p.bias && ok[g]) ? __halves2half2(p.bias[m0 + 16 * g], p.bias[m0 + 16 * g + 1]) : __half2half2(__ushort_as_half((unsigned short)0x8000));
+        }
+        taddr = trow;
+    }
+    // one group: word 2 j + e of pk: column 8 j + 2 (t % 4) + e of the chunk
+    __device__ __forceinline__ static void pack(const uint32_t (&v)[32], uint32_t *pk)
+    {
 #pragma unroll
-        for (int j = 0; j < 2; j++)
+        for (int j = 0; j < 8; j++) {
+            pk[2 * j] = pack_half2(v[4 * j], v[4 * j + 2]);
+            pk[2 * j + 1] = pack_half2(v[4 * j + 1], v[4 * j + 3]);
+        }
+    }
+    __device__ __forceinline__ void store(int c, int cols, const uint32_t *pk) const   // both groups
+    {
+        __half *d = dst + (int64_t)c * ldo;
+        if (words && ok[0] && ok[1] && c + 64 <= left) {
+            // whole chunk (columns past `cols` belong to nobody): two adds, a half2 add and a store a word.  With the checks below
+            // around every word the stores of a tile took 11500 clocks, longer than the MMAs of a tile of eight k-tiles.
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                if (8 * j >= cols) break;
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+#pragma unroll
+                    for (int g = 0; g < 2; g++) {
+                        uint32_t w = pk[16 * g + 2 * j + e];
+                        *reinterpret_cast<__half2 *>(d + e * ldo + 16 * g) = __hadd2(*reinterpret_cast<__half2 *>(&w), bias[g]);
+                    }
+                }
+                d += 8 * ldo;
+            }
+            return;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            if (8 * j >= cols) break;
 #pragma unroll
             for (int e = 0; e < 2; e++) {
-                const int n = ncol + c0 + 8 * j + e;
-                if (n >= p.N) continue;
-                __half *dst = p.out + (int64_t)n * p.ldo + m0;
+                if (c + 8 * j + e >= left) continue;
 #pragma unroll
                 for (int g = 0; g < 2; g++) {
-                    __half2 h = __floats2half2_rn(__uint_as_float(v[g][4 * j + e]), __uint_as_float(v[g][4 * j + 2 + e]));
-                    if (has_bias) h = __hadd2(h, bias[g]);
                     if (!ok[g]) continue;
+                    uint32_t w = pk[16 * g + 2 * j + e];
+                    const __half2 h = __hadd2(*reinterpret_cast<__half2 *>(&w), bias[g]);
+                    __half *dd = d + (8 * j + e) * ldo + 16 * g;
                     if (words) {
-                        *reinterpret_cast<__half2 *>(dst + 16 * g) = h;
+                        *reinterpret_cast<__half2 *>(dd) = h;
                     } else {
-                        dst[16 * g] = __low2half(h);
-                        dst[16 * g + 1] = __high2half(h);
+                        dd[0] = __low2half(h);
+                        dd[1] = __high2half(h);
                     }
                 }
             }
+        }
+    }
+};
+__device__ __forceinline__ void store_chunk(const TileStoreMN &st, int c, int cols, uint32_t *pk) { st.store(c, 0, cols, pk); st.store(c, 1, cols, pk + 16); }
+__device__ __forceinline__ void store_chunk(const TileStoreNM &st, int c, int cols, uint32_t *pk) { st.store(c, cols, pk); }
+
+// BN columns in chunks of 64 (a last chunk of fewer reads on into columns that it does not store).  `release` runs
+// (converged) once the last column has been read.  HOLD: all columns are read into registers first, for kernels whose next
+// tile waits for this accumulator.
+template <int BN, bool HOLD, typename Store, typename Release>
+__device__ __forceinline__ void store_tile(const Store &st, Release release)
+{
+    constexpr int CHUNKS = (BN + 63) / 64;
+    if (HOLD) {
+        uint32_t pk[CHUNKS][32];
+#pragma unroll
+        for (int k = 0; k < CHUNKS; k++) {
+            uint32_t v0[32], v1[32];   // both groups in flight before the wait: the next tile's MMAs wait for this
+            tc_ld_16x256b(st.taddr + (uint32_t)(64 * k), v0);
+            tc_ld_16x256b(st.taddr + (16u << 16) + (uint32_t)(64 * k), v1);
+            tc_wait_ld();
+            Store::pack(v0, pk[k]);
+            Store::pack(v1, pk[k] + 16);
+        }
+        release();
+#pragma unroll
+        for (int k = 0; k < CHUNKS; k++) store_chunk(st, 64 * k, BN - 64 * k, pk[k]);
+    } else {
+#pragma unroll 1
+        for (int k = 0; k < CHUNKS; k++) {
+            uint32_t pk[32];
+#pragma unroll
+            for (int g = 0; g < 2; g++) {
+                uint32_t v[32];
+                tc_ld_16x256b(st.taddr + ((uint32_t)(16 * g) << 16) + (uint32_t)(64 * k), v);
+                tc_wait_ld();
+                Store::pack(v, pk + 16 * g);
+            }
+            if (k == CHUNKS - 1) release();
+            store_chunk(st, 64 * k, BN - 64 * k, pk);
+        }
     }
 }
 #endif  // __CUDACC__

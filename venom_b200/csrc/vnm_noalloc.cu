@@ -115,7 +115,7 @@ extern "C" int vnm_spmm_f16_noalloc(const void *values, const uint32_t *meta, co
     if (e != cudaSuccess) return nfail(VNM_ERR_CUDA, "re-pack launch: %s", cudaGetErrorString(e));
 
     SpmmConfig cfg;
-    if (!spmm_select_config(V, N, M, 0, &cfg)) return nfail(VNM_ERR_UNSUPPORTED, "unsupported V");
+    if (spmm_select_config(V, N, M, ktiles, 0, &cfg) < 0.0f) return nfail(VNM_ERR_UNSUPPORTED, "unsupported V");
     EncodeTiledFn enc = get_encode_fn();
     if (!enc) return nfail(VNM_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
     CUtensorMap tmap_rows, tmap_tile;
@@ -146,6 +146,8 @@ extern "C" int vnm_spmm_f16_noalloc(const void *values, const uint32_t *meta, co
     p.B = (const __half *)B;
     p.ldb = ldb;
     p.tma_out = p.out32 = 0;
+    p.split_k = 1;
+    p.early = 0;
     p.hint_a = p.hint_b = L2_EVICT_NORMAL;
     p.group_m = mtiles;  // operands this small fit in L2 whole: row tiles fastest
     p.hybrid_rows = 0;

@@ -307,8 +307,8 @@ __global__ void __launch_bounds__(Traits<BN, NB>::NUM_THREADS, 1)
                 if (lane == 0) mbar_arrive(&acc_empty[grp]);
             };
             if (!p.tma_out) {
-                if (p.layout == 0) store_tile_mn<BN>(trow, q, (int64_t)mt * TILE_M, n0, p, release);
-                else store_tile_nm<BN>(trow, q, (int64_t)mt * TILE_M, n0, p, release);
+                if (p.layout == 0) store_tile<BN, false>(TileStoreMN(trow, q, (int64_t)mt * TILE_M, n0, p), release);
+                else store_tile<BN, false>(TileStoreNM(trow, q, (int64_t)mt * TILE_M, n0, p), release);
                 continue;
             }
             // [N,M] (+ bias) to several destinations (peers' buffers), or on request: parts of PART rows (n) x 128 columns (m) go
@@ -374,7 +374,7 @@ int g_num_sms = 0;
 
 // Tile configurations: V=128 -> one block per tile, BN 240 (two accumulators and the metadata fill tensor memory);
 // V=64 -> two blocks, BN 128; V=32 -> four blocks, BN 64 (NB * BN = 256: every B stage is 16 KiB).
-bool spmm_select_config(int V, int N, int M, int max_ctas, SpmmConfig *cfg)
+float spmm_select_config(int V, int N, int M, int ktiles, int max_ctas, SpmmConfig *cfg)
 {
     const int mtiles = (M + TILE_M - 1) / TILE_M;
     cfg->stages = Traits<240, 1>::PW;
@@ -386,13 +386,14 @@ bool spmm_select_config(int V, int N, int M, int max_ctas, SpmmConfig *cfg)
     } else if (V == 32) {
         cfg->bn = 64; cfg->nb = 4; cfg->part = Traits<64, 4>::PART; cfg->smem_bytes = Traits<64, 4>::SMEM_BYTES;
     } else {
-        return false;
+        return -1.0f;
     }
     const long long tiles = (long long)mtiles * ((N + cfg->bn - 1) / cfg->bn);
     int sms = g_num_sms > 0 ? g_num_sms : 148;
     if (max_ctas > 0 && max_ctas < sms) sms = max_ctas;  // the caller keeps some SMs free (e.g. for a collective that runs beside the product)
     cfg->grid = (int)(tiles < sms ? tiles : sms);
-    return true;
+    // start-up and last epilogue, then per wave of tiles a k-tile's 1430 clocks and what a tile change costs
+    return 5.5f + (float)((tiles + sms - 1) / sms) * (ktiles * 0.78f + 0.9f);
 }
 
 cudaError_t spmm_init_kernels()

@@ -6,18 +6,19 @@
 // with the 240 columns assembled from both halves.  Per k-tile a CTA therefore takes in 36 KiB of A and 32 KiB of B
 // instead of 36 + 64 KiB, which moves the mainloop from the SM's L2 intake limit to the tensor pipe.
 //
+// What bounds it: the shared-memory port.  Per k-tile a CTA's MMAs read 8 x (4 KiB of A + its 7.5 KiB half of B), the
+// metadata copies 4 KiB, and TMA writes 68 KiB: 164 KiB at 128 bytes a clock are 1312 clocks, against 960 of the tensor pipe.
+//
 // Cluster protocol (rank 0 = leader, rank 1 = peer); every load stays local to the CTA that issues it:
 //   * both CTAs run their own A producer, B producers and epilogue on their own shared / tensor memory;
 //   * the peer forwards "my A blocks of k-tile it landed" and "my half of stage j landed" to the leader with remote
 //     mbarrier arrivals on the leader's own a_full / b_full barriers (which expect two arrivals there: the leader's
-//     loads and the peer's message), so the leader's sequencer and MMA issuer wait on one barrier per hand-off,
-//     exactly as in the single-CTA kernel -- anything more on the issuing thread leaves the tensor pipe idle;
+//     loads and the peer's message), so the leader's MMA issuer waits on one barrier per hand-off;
 //   * only the leader issues tensor-core work: tcgen05.cp.cta_group::2 copies each CTA's metadata image into that
-//     CTA's tensor memory, tcgen05.mma.sp.cta_group::2 reads A and B from both CTAs' shared memory;
-//   * the leader's tcgen05.commit.cta_group::2 arrives on the stage-free / accumulator-full barriers of BOTH CTAs
-//     (two commits: the local barrier and the peer's barrier through its shared::cluster address; a spare thread
-//     forwarding the arrivals instead measured 1-2 % slower), and the peer's epilogue warps arrive remotely on the
-//     leader's accumulator-empty barrier.
+//     CTA's tensor memory, tcgen05.mma.sp.cta_group::2 reads A and B from both CTAs' shared memory.  Copies and MMAs come
+//     from one elected thread, which executes them in order (see vnm_spmm.cu);
+//   * the leader's tcgen05.commit.cta_group::2 arrives on the ring-free / accumulator-full barriers of BOTH CTAs, and the
+//     peer's epilogue warps arrive remotely on the leader's accumulator-empty barrier.
 // No copy with cluster multicast is used anywhere.  Every wait is bounded (status bit, drain, return), and the two CTAs
 // meet at a cluster barrier before tensor memory is freed, so neither leaves while the other may still touch it.
 #include "vnm_internal.h"
@@ -31,8 +32,6 @@ constexpr int BN = 240;          // output columns per pair tile
 constexpr int PART = 40;         // columns per epilogue part / TMA store
 constexpr int SA = 3;            // A ring: k-tiles (each RT blocks)
 constexpr int SB = 6;            // B ring: stages of 64 rows x 128 columns (this CTA's half of two K=32 blocks of the MMAs)
-constexpr int SF = 12;           // stage "free" barriers (twice the stages, so that a late waiter never sees a wrapped phase)
-constexpr int SR = 4;            // k-tile "ready" barriers
 constexpr int META_SETS = 3;     // metadata column sets in tensor memory (4 columns per row tile each)
 constexpr int KB_PER_STAGE = 2;                     // K=32 blocks per B stage: one 16 KiB TMA box (smaller boxes keep the copy engine less busy)
 constexpr int STAGES_PER_KT = 4 / KB_PER_STAGE;
@@ -47,18 +46,19 @@ constexpr int BAR_BYTES = 640;
 constexpr int SMEM_BYTES = A_RING_BYTES + B_RING_BYTES + OUT_RING_BYTES + BAR_BYTES + 1024;
 static_assert(A_RING_BYTES % 1024 == 0 && B_RING_BYTES % 1024 == 0, "swizzled staging needs 1024-byte alignment");
 static_assert(SMEM_BYTES <= 227 * 1024, "shared memory per CTA");
-constexpr int NUM_THREADS = 512;  // warps 0-3 single-thread roles, 4-7 B producers, 8-15 epilogue (2 x 4 warps)
-constexpr int EPI_WARP0 = 8;
-constexpr int NBP = 3;            // B producer warps (SB % NBP == 0: a ring slot always has the same owner)
+// Four single-thread roles and two epilogue groups of four warps: 384 threads may use 168 registers each, which holds an
+// accumulator row (120 packed words) without any re-allocation between warpgroups.  (With 512 threads and setmaxnreg the
+// MMAs of this kernel issued at 180-240 clocks instead of 120: 1700 clocks a k-tile, against 1380.)
+constexpr int NUM_THREADS = 384;
+constexpr int EPI_WARP0 = 4;
 constexpr int TMEM_COLS = 512;
 // tensor-memory columns: accumulator 0 at 0..239, metadata sets at 240 and 248, accumulator 1 at 256..495, metadata set at 496
 __device__ __forceinline__ uint32_t acc_col(int rt) { return (uint32_t)rt * 256u; }
 __device__ __forceinline__ uint32_t meta_col(int set) { return set == 0 ? 240u : (set == 1 ? 248u : 496u); }
-static_assert(SB % NBP == 0 && NBP <= 4, "B producers");
 constexpr int KT_RING = SB / STAGES_PER_KT;  // k-tiles the B ring holds
-static_assert(SB % STAGES_PER_KT == 0 && KT_RING == SA && KT_RING == META_SETS && SF == 2 * SB, "the rings and the metadata sets advance one k-tile at a time");
+static_assert(SB % STAGES_PER_KT == 0 && KT_RING == SA && KT_RING == META_SETS, "the rings and the metadata sets advance one k-tile at a time");
 static_assert(BN <= 240 && META_SETS == 3 && RT == 2 && BN % 16 == 0 && BN == 6 * PART, "tensor-memory column plan");
-static_assert((SA + SB + SF + SR + 4) * 8 + 16 <= BAR_BYTES, "barrier area too small");
+static_assert((2 * SA + 2 * SB + 4) * 8 + 16 <= BAR_BYTES, "barrier area too small");
 constexpr int HALF_N = BN / 2;   // columns of a B stage held by each CTA of the pair
 
 // ---- cluster helpers ----
@@ -93,11 +93,12 @@ __device__ __forceinline__ void tmem_dealloc2(uint32_t taddr, uint32_t ncols)
 {
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
-// arrives on the barrier at shared::cluster address `bar_addr` once every tcgen05 operation issued so far by this thread
-// has completed in both CTAs
-__device__ __forceinline__ void tc_commit2(uint32_t bar_addr)
+// arrives on the barrier at this shared-memory offset in both CTAs once every tcgen05 operation issued so far by this
+// thread has completed (in both CTAs)
+__device__ __forceinline__ void tc_commit2(uint64_t *bar)
 {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_addr) : "memory");
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)), "h"((uint16_t)3)
+                 : "memory");
 }
 // each CTA's shared-memory image (same offset in both) -> that CTA's tensor memory, 128 lanes x 128 bits
 __device__ __forceinline__ void tc_cp2_128x128b(uint32_t taddr, uint64_t sdesc)
@@ -116,15 +117,12 @@ __device__ __forceinline__ void tc_mma2_sp_f16(uint32_t d_tmem, uint64_t adesc, 
         : "memory");
 }
 
-// Warp roles (512 threads per CTA, as in the single-CTA kernel):
+// Warp roles:
 //   warp 0      A producer: two bulk copies per k-tile (this CTA's two row tiles).
-//   warp 1      leader: sequencer (waits for both CTAs' A blocks, copies both metadata images to tensor memory, waits
-//               for the four B stages of the k-tile, then flips the k-tile's "ready" barrier);
-//               peer: forwards "A blocks landed" to the leader.
-//   warp 3      tensor-memory owner in both CTAs; leader: MMA issuer (one wait, eight MMAs and two commits per k-tile);
-//               peer: forwards "B half landed" to the leader.
-//   warps 4..6  B producers: one 16 KiB TMA box per stage (64 rows of this CTA's 128-column half).
-//   warps 8..15 epilogue of this CTA's two accumulators.
+//   warp 1      B producer: one 16 KiB TMA box per stage (64 rows of this CTA's 128-column half).
+//   warp 2      peer: forwards "A blocks landed" and "B half landed" to the leader.
+//   warp 3      tensor-memory owner in both CTAs; leader: MMA issuer.
+//   warps 4..11 epilogue of this CTA's two accumulators.
 template <int R>
 __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const __grid_constant__ CUtensorMap tmap_tile, const __grid_constant__ CUtensorMap tmap_tile2,
                                                                            const __grid_constant__ CUtensorMap tmap_out, const __grid_constant__ OutMaps more_out,
@@ -138,12 +136,12 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
     uint8_t *out_ring = smem + A_RING_BYTES + B_RING_BYTES;
     uint64_t *a_full = reinterpret_cast<uint64_t *>(smem + A_RING_BYTES + B_RING_BYTES + OUT_RING_BYTES);
     uint64_t *b_full = a_full + SA;
-    uint64_t *b_free = b_full + SB;   // b_free[j % SF]: the MMAs that read B stage j have completed (arrives in both CTAs)
-    uint64_t *kready = b_free + SF;
+    uint64_t *a_free = b_full + SB;   // the MMAs that read this slot have completed (arrives in both CTAs)
+    uint64_t *b_free = a_free + SA;
     // accumulator hand-off.  R = 2: one barrier pair, both accumulators of a CTA belong to the same tile.  R = 1: a CTA has one
     // row tile, so its two accumulators alternate between consecutive tiles (barrier pair ti & 1) and the epilogue of one
     // tile runs beside the MMAs of the next.
-    uint64_t *acc_full_bar = kready + SR;      // [2]
+    uint64_t *acc_full_bar = b_free + SB;      // [2]
     uint64_t *acc_empty_bar = acc_full_bar + 2;  // [2]
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty_bar + 2);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
@@ -163,8 +161,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
         // in the leader a slot is full once its own loads have landed AND the peer has reported the same for its half
         for (int s = 0; s < SA; s++) mbar_init(&a_full[s], leader_cta ? 2 : 1);
         for (int s = 0; s < SB; s++) mbar_init(&b_full[s], leader_cta ? 2 : 1);
-        for (int s = 0; s < SF; s++) mbar_init(&b_free[s], 1);
-        for (int s = 0; s < SR; s++) mbar_init(&kready[s], 2);  // metadata copied to tensor memory + all operands landed
+        for (int s = 0; s < SA; s++) mbar_init(&a_free[s], 1);
+        for (int s = 0; s < SB; s++) mbar_init(&b_free[s], 1);
         for (int a = 0; a < 2; a++) {
             mbar_init(&acc_full_bar[a], 1);
             mbar_init(&acc_empty_bar[a], 2 * 4);  // R = 1: the four warps of one epilogue group in both CTAs
@@ -187,8 +185,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
 
     if (warp == 0) {
         // ---------------- A producer ----------------
-        setmaxnreg_dec<64>();
-        if (lane == 0) {
+        if (elect_one()) {
             int it = 0;
             bool alive = true;
             for (int tile = pair; alive && tile < total_tiles; tile += npairs) {
@@ -196,10 +193,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
                 tile_coords(tile, mquads, p.ntiles, p.group_m, &mq, &nt_unused);
                 for (int kt = 0; kt < p.ktiles; ++kt, ++it) {
                     const int s = it % SA;
-                    if (it >= SA) {
-                        const int jd = STAGES_PER_KT * (it - SA) + STAGES_PER_KT - 1;  // last B stage of the k-tile that used this slot
-                        if (!wait_one(&b_free[jd % SF], (uint32_t)(jd / SF) & 1u, abort_flag, p.status, DEV_TIMEOUT_PRODUCER)) { alive = false; break; }
-                    }
+                    if (!wait_quiet(&a_free[s], ((uint32_t)(it / SA) & 1u) ^ 1u, abort_flag, p.status, DEV_TIMEOUT_PRODUCER)) { alive = false; break; }
                     mbar_arrive_expect_tx(&a_full[s], R * AM_BLOCK_BYTES);
 #pragma unroll
                     for (int rt = 0; rt < R; rt++) {
@@ -232,182 +226,136 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
             }
         }
         __syncwarp();
-    } else if (warp >= 4 && warp < EPI_WARP0) {
-        // ---------------- B producers: warp 4 + w loads the stages j = w, w + NBP, ... of this CTA's half ----------------
-        setmaxnreg_dec<64>();
-        if (lane == 0 && warp - 4 < NBP) {
+    } else if (warp == 1) {
+        // ---------------- B producer: this CTA's half of every stage ----------------
+        if (elect_one()) {
             tma_prefetch_desc(&tmap_tile);
             tma_prefetch_desc(&tmap_tile2);
             const int per_tile = STAGES_PER_KT * p.ktiles;
-            int j = warp - 4;
-            int tile_i = j / per_tile, jl = j - tile_i * per_tile;
-            const int total_j = my_tiles * per_tile;
-            for (; j < total_j; j += NBP) {
-                const int tile = pair + tile_i * npairs;
+            int j = 0, s = 0;
+            uint32_t ph = 1;
+            bool alive = true;
+            for (int tile = pair; alive && tile < total_tiles; tile += npairs) {
                 int mq_unused, nt;
                 tile_coords(tile, mquads, p.ntiles, p.group_m, &mq_unused, &nt);
                 const int n0 = nt * BN + (int)crank * HALF_N;  // first column of this CTA's half
-                const int s = j % SB;
-                if (j >= SB) {
-                    const int jd = j - SB;
-                    if (!wait_one(&b_free[jd % SF], (uint32_t)(jd / SF) & 1u, abort_flag, p.status, DEV_TIMEOUT_PRODUCER)) break;
-                }
-                uint8_t *dst = b_ring + s * B_STAGE_BYTES;
-                if (p.gather_mode == GATHER_NONE) {  // ablation: no loads of B at all (timing floor; results are meaningless)
-                    mbar_arrive(&b_full[s]);
-                    jl += NBP;
-                    while (jl >= per_tile) { jl -= per_tile; ++tile_i; }
-                    continue;
-                }
-                // 64 rows x 128 columns come along per stage; the MMAs read the first 120 columns
-                mbar_arrive_expect_tx(&b_full[s], B_STAGE_BYTES);
-                if (p.b_nk) {
-                    tma_load_2d_hint(dst, &tmap_tile, jl * 64, n0, &b_full[s], p.hint_b);  // 128 rows (n) x 64 k, 128-byte swizzle
-                } else if (p.b_wide_ok && n0 + 128 <= p.N) {
-                    tma_load_4d_hint(dst, &tmap_tile, 0, jl * 64, 0, n0 / 8, &b_full[s], p.hint_b);  // {64 columns, 64 rows, 2 slices} from column n0
-                } else {  // ragged right edge: two boxes that clip (and zero-fill) at N
-                    for (int c = 0; c < 2; c++) tma_load_2d_hint(dst + c * B_CHUNK_BYTES, &tmap_tile2, n0 + c * 64, jl * 64, &b_full[s], p.hint_b);
-                }
-                if (p.l2_ahead > 0) {
-                    // this warp's stage a few of its own turns later, on its way into L2
-                    int jlp = jl + NBP * ((STAGES_PER_KT * p.l2_ahead + NBP - 1) / NBP), n0p = n0;
-                    bool ok = true;
-                    if (jlp >= per_tile) {
-                        jlp -= per_tile;
-                        ok = jlp < per_tile && tile + npairs < total_tiles;
-                        if (ok) {
-                            int ntp;
-                            tile_coords(tile + npairs, mquads, p.ntiles, p.group_m, &mq_unused, &ntp);
-                            n0p = ntp * BN + (int)crank * HALF_N;
+                const bool wide = p.b_wide_ok && n0 + 128 <= p.N;
+                for (int jl = 0; jl < per_tile; ++jl, ++j) {
+                    if (!wait_quiet(&b_free[s], ph, abort_flag, p.status, DEV_TIMEOUT_PRODUCER)) { alive = false; break; }
+                    uint8_t *dst = b_ring + s * B_STAGE_BYTES;
+                    if (p.gather_mode == GATHER_NONE) {  // ablation: no loads of B at all (timing floor; results are meaningless)
+                        mbar_arrive(&b_full[s]);
+                    } else {
+                        // 64 rows x 128 columns come along per stage; the MMAs read the first 120 columns
+                        mbar_arrive_expect_tx(&b_full[s], B_STAGE_BYTES);
+                        if (p.b_nk) {
+                            tma_load_2d_hint(dst, &tmap_tile, jl * 64, n0, &b_full[s], p.hint_b);  // 128 rows (n) x 64 k, 128-byte swizzle
+                        } else if (wide) {
+                            tma_load_4d_hint(dst, &tmap_tile, 0, jl * 64, 0, n0 / 8, &b_full[s], p.hint_b);  // {64 columns, 64 rows, 2 slices} from column n0
+                        } else {  // ragged right edge: two boxes that clip (and zero-fill) at N
+                            for (int c = 0; c < 2; c++) tma_load_2d_hint(dst + c * B_CHUNK_BYTES, &tmap_tile2, n0 + c * 64, jl * 64, &b_full[s], p.hint_b);
+                        }
+                        if (p.l2_ahead > 0) {
+                            // the same box of a later stage, on its way into L2
+                            int jlp = jl + STAGES_PER_KT * p.l2_ahead, n0p = n0;
+                            bool ok = true;
+                            if (jlp >= per_tile) {
+                                jlp -= per_tile;
+                                ok = jlp < per_tile && tile + npairs < total_tiles;
+                                if (ok) {
+                                    int ntp;
+                                    tile_coords(tile + npairs, mquads, p.ntiles, p.group_m, &mq_unused, &ntp);
+                                    n0p = ntp * BN + (int)crank * HALF_N;
+                                }
+                            }
+                            if (ok) {
+                                if (p.b_nk) tma_prefetch_2d(&tmap_tile, jlp * 64, n0p);
+                                else if (p.b_wide_ok && n0p + 128 <= p.N) tma_prefetch_4d(&tmap_tile, 0, jlp * 64, 0, n0p / 8);
+                                else for (int c = 0; c < 2; c++) tma_prefetch_2d(&tmap_tile2, n0p + c * 64, jlp * 64);
+                            }
                         }
                     }
-                    if (ok) {
-                        if (p.b_nk) tma_prefetch_2d(&tmap_tile, jlp * 64, n0p);
-                        else if (p.b_wide_ok && n0p + 128 <= p.N) tma_prefetch_4d(&tmap_tile, 0, jlp * 64, 0, n0p / 8);
-                        else for (int c = 0; c < 2; c++) tma_prefetch_2d(&tmap_tile2, n0p + c * 64, jlp * 64);
-                    }
+                    if (++s == SB) { s = 0; ph ^= 1; }
                 }
-                jl += NBP;
-                while (jl >= per_tile) { jl -= per_tile; ++tile_i; }
             }
             if (*abort_flag && p.gather_mode != GATHER_NONE) {
-                for (int k = j - NBP, n = 0; k >= 0 && n < SB / NBP; k -= NBP, ++n) drain_slot(&b_full[k % SB], (uint32_t)(k / SB) & 1u, p.status);
+                for (int k = j > SB ? j - SB : 0; k < j; ++k) drain_slot(&b_full[k % SB], (uint32_t)(k / SB) & 1u, p.status);
             }
         }
         __syncwarp();
-    } else if (warp == 1) {
-        setmaxnreg_dec<64>();
-        if (lane == 0 && leader_cta) {
-            // ---------------- sequencer (leader) ----------------
-            const uint64_t mdesc0 = make_smem_desc(smem_u32(a_ring) + A_IMG_BYTES, 0, 128, 0);
-            for (int it = 0; it < total_it; ++it) {
-                const int sa = it % SA;
-                if (it >= META_SETS) {  // column set it % META_SETS was last read by the MMAs of k-tile it - META_SETS
-                    const int jd = STAGES_PER_KT * (it - META_SETS) + STAGES_PER_KT - 1;
-                    if (!wait_one(&b_free[jd % SF], (uint32_t)(jd / SF) & 1u, abort_flag, p.status, DEV_TIMEOUT_MMA)) break;
-                }
-                if (!wait_one(&a_full[sa], (uint32_t)(it / SA) & 1u, abort_flag, p.status, DEV_TIMEOUT_MMA)) break;  // both CTAs' blocks
-                tc_fence_after();
-                const uint32_t mcol = tmem_base + meta_col(it % META_SETS);
-#pragma unroll
-                for (int rt = 0; rt < R; rt++)
-                    tc_cp2_128x128b(mcol + rt * 4, mdesc0 + ((uint32_t)(sa * A_STAGE_BYTES + rt * AM_BLOCK_BYTES) >> 4));
-                tc_commit2(smem_u32(&kready[it % SR]));  // first arrival: the metadata copies are done
-                // The B stages of the k-tile are waited for here, not by the MMA issuer: every probe of a barrier
-                // costs the issuing thread about as much as one MMA takes to execute, and the tensor pipe queues next to
-                // nothing, so a wait between two MMAs is a bubble in the pipe.
-                bool alive = true;
+    } else if (warp == 2) {
+        if (!leader_cta && elect_one()) {
+            // ---------------- peer: forward "A blocks landed" and "my half of the stage landed" ----------------
+            const uint32_t remote_a = mapa_shared(smem_u32(a_full), 0), remote_b = mapa_shared(smem_u32(b_full), 0);
+            int sa = 0;
+            uint32_t ph = 0;
+            bool alive = true;
+            for (int it = 0; alive && it < total_it; ++it) {
+                if (!wait_one(&a_full[sa], ph, abort_flag, p.status, DEV_TIMEOUT_MMA)) break;
+                mbar_arrive_cluster(remote_a + (uint32_t)sa * 8u);
 #pragma unroll
                 for (int st = 0; st < STAGES_PER_KT; st++) {
-                    const int j = STAGES_PER_KT * it + st;
-                    if (!wait_one(&b_full[j % SB], (uint32_t)(j / SB) & 1u, abort_flag, p.status, DEV_TIMEOUT_MMA)) { alive = false; break; }  // both halves
+                    const int sb = STAGES_PER_KT * sa + st;
+                    if (!wait_one(&b_full[sb], ph, abort_flag, p.status, DEV_TIMEOUT_MMA)) { alive = false; break; }
+                    mbar_arrive_cluster(remote_b + (uint32_t)sb * 8u);
                 }
-                if (!alive) break;
-                mbar_arrive(&kready[it % SR]);  // second arrival: every operand of the k-tile is in shared memory
-            }
-        } else if (lane == 0) {
-            // ---------------- peer: forward "A blocks landed" ----------------
-            const uint32_t remote0 = mapa_shared(smem_u32(a_full), 0);
-            for (int it = 0; it < total_it; ++it) {
-                const int sa = it % SA;
-                if (!wait_one(&a_full[sa], (uint32_t)(it / SA) & 1u, abort_flag, p.status, DEV_TIMEOUT_MMA)) break;
-                mbar_arrive_cluster(remote0 + sa * 8);
+                if (++sa == SA) { sa = 0; ph ^= 1; }
             }
         }
         __syncwarp();
     } else if (warp == 3) {
-        setmaxnreg_dec<64>();
-        if (lane == 0 && leader_cta) {
+        if (leader_cta && elect_one()) {
             // ---------------- MMA issuer (leader) ----------------
             const bool b_nk = p.b_nk != 0;
             const uint32_t idesc0 = make_idesc_f16(2 * TILE_M, BN, true, 0u, !b_nk);
             const uint64_t adesc0 = make_smem_desc(smem_u32(a_ring), 16, 1024, 2);
+            const uint64_t mdesc0 = make_smem_desc(smem_u32(a_ring) + A_IMG_BYTES, 0, 128, 0);
             // this CTA's half of a stage: N-major (two 64-column slices of 64 rows x 128 bytes, 128-byte swizzle; a K=32 block is
             // 32 rows = 4096 bytes further) or K-major (128 n-rows of 128 bytes = 64 k of which 120 rows are used, 128-byte swizzle,
             // 8-row groups 1024 bytes apart; a K=32 block is 64 bytes further inside the row)
             const uint64_t bdesc0 = b_nk ? make_smem_desc(smem_u32(b_ring), 16, 1024, 2) : make_smem_desc(smem_u32(b_ring), B_CHUNK_BYTES, 1024, 2);
             const uint32_t kb_step = b_nk ? 64u : 32u * 128u;  // bytes between the K=32 blocks of a stage
-            const uint32_t free_local = smem_u32(b_free), free_peer = mapa_shared(smem_u32(b_free), 1);
-            const uint32_t full_local = smem_u32(acc_full_bar), full_peer = mapa_shared(smem_u32(acc_full_bar), 1);
-            // The thread runs about one MMA ahead of the tensor pipe, so whatever it does between two MMAs must take less
-            // than one MMA (about 140 clocks).  A k-tile is therefore one wait, eight MMAs and two commits, and the wait for
-            // the NEXT k-tile sits in front of the last two MMAs, where the pipe still has work queued.
-            int it = 0, slot = 0;  // slot = it % KT_RING
-            bool alive = total_it > 0 && wait_one(&kready[0], 0u, abort_flag, p.status, DEV_TIMEOUT_MMA);
-            tc_fence_after();
+            int sa = 0;            // A slot and metadata set; the k-tile's B stages are slots STAGES_PER_KT * sa ...
+            uint32_t ph = 0;       // phase of all of them
+            bool alive = true;
             for (int ti = 0; alive && ti < my_tiles; ++ti) {
-                for (int kt = 0; alive && kt < p.ktiles; ++kt, ++it) {
-                    // accumulator set of this tile: R = 2 always set 0 (phase ti), R = 1 set ti & 1 (phase ti / 2)
-                    const int aset = R == 1 ? (ti & 1) : 0;
-                    const uint32_t aphase = R == 1 ? (uint32_t)(ti >> 1) & 1u : (uint32_t)ti & 1u;
-                    if (kt == 0) {
-                        if (!wait_one(&acc_empty_bar[aset], aphase ^ 1u, abort_flag, p.status, DEV_TIMEOUT_MMA)) { alive = false; break; }
+                // accumulator set of this tile: R = 2 always set 0 (phase ti), R = 1 set ti & 1 (phase ti / 2)
+                const int aset = R == 1 ? (ti & 1) : 0;
+                const uint32_t aphase = R == 1 ? (uint32_t)(ti >> 1) & 1u : (uint32_t)ti & 1u;
+                if (!wait_one(&acc_empty_bar[aset], aphase ^ 1u, abort_flag, p.status, DEV_TIMEOUT_MMA)) break;
+                for (int kt = 0; kt < p.ktiles; ++kt) {
+                    if (!wait_one(&a_full[sa], ph, abort_flag, p.status, DEV_TIMEOUT_MMA)) { alive = false; break; }  // both CTAs' blocks
+                    tc_fence_after();
+                    const uint32_t mcol = tmem_base + meta_col(sa);
+                    const uint32_t aoff = (uint32_t)(sa * A_STAGE_BYTES) >> 4;
+#pragma unroll
+                    for (int rt = 0; rt < R; rt++) tc_cp2_128x128b(mcol + rt * 4, mdesc0 + aoff + (uint32_t)((rt * AM_BLOCK_BYTES) >> 4));
+#pragma unroll
+                    for (int st = 0; st < STAGES_PER_KT; st++) {
+                        const int sb = STAGES_PER_KT * sa + st;
+                        if (!wait_one(&b_full[sb], ph, abort_flag, p.status, DEV_TIMEOUT_MMA)) { alive = false; break; }  // both halves
                         tc_fence_after();
-                    }
-                    const uint32_t mcol = tmem_base + meta_col(slot);
-                    const uint32_t aoff = (uint32_t)(slot * A_STAGE_BYTES) >> 4;
-                    const uint32_t boff0 = (uint32_t)(slot * STAGES_PER_KT * B_STAGE_BYTES) >> 4;
 #pragma unroll
-                    for (int kb = 0; kb < 4; kb++) {  // K=32 blocks of the k-tile, KB_PER_STAGE of them per B stage
-                        if (kb == 3 && it + 1 < total_it) {
-                            if (!wait_one(&kready[(it + 1) % SR], (uint32_t)((it + 1) / SR) & 1u, abort_flag, p.status, DEV_TIMEOUT_MMA)) { alive = false; break; }
-                            tc_fence_after();
-                        }
-                        const uint32_t boff = boff0 + (((uint32_t)(kb / KB_PER_STAGE) * B_STAGE_BYTES + (uint32_t)(kb % KB_PER_STAGE) * kb_step) >> 4);
+                        for (int k2 = 0; k2 < KB_PER_STAGE; k2++) {  // K=32 blocks of the stage
+                            const int kb = st * KB_PER_STAGE + k2;
+                            const uint32_t boff = ((uint32_t)sb * B_STAGE_BYTES + (uint32_t)k2 * kb_step) >> 4;
 #pragma unroll
-                        for (int rt = 0; rt < R; rt++)
-                            tc_mma2_sp_f16(tmem_base + acc_col(R == 1 ? aset : rt), adesc0 + aoff + (uint32_t)((rt * AM_BLOCK_BYTES + kb * 32) >> 4), bdesc0 + boff,
-                                           mcol + rt * 4 + (uint32_t)(kb & ~1), idesc0 | (uint32_t)(kb & 1), (kt | kb) != 0 ? 1u : 0u);
-                        if (kb % KB_PER_STAGE == KB_PER_STAGE - 1) {
-                            // the stage (and, after the last, the A blocks and the metadata set) may be refilled in both CTAs
-                            const int j = STAGES_PER_KT * it + kb / KB_PER_STAGE;
-                            tc_commit2(free_local + (uint32_t)(j % SF) * 8u);
-                            tc_commit2(free_peer + (uint32_t)(j % SF) * 8u);
+                            for (int rt = 0; rt < R; rt++)
+                                tc_mma2_sp_f16(tmem_base + acc_col(R == 1 ? aset : rt), adesc0 + aoff + (uint32_t)((rt * AM_BLOCK_BYTES + kb * 32) >> 4), bdesc0 + boff,
+                                               mcol + rt * 4 + (uint32_t)(kb & ~1), idesc0 | (uint32_t)(kb & 1), (kt | kb) != 0 ? 1u : 0u);
                         }
+                        tc_commit2(&b_free[sb]);
                     }
                     if (!alive) break;
-                    if (kt == p.ktiles - 1) {
-                        tc_commit2(full_local + (uint32_t)aset * 8u);
-                        tc_commit2(full_peer + (uint32_t)aset * 8u);
-                    }
-                    slot = slot + 1 == KT_RING ? 0 : slot + 1;
+                    tc_commit2(&a_free[sa]);
+                    if (kt == p.ktiles - 1) tc_commit2(&acc_full_bar[aset]);
+                    if (++sa == SA) { sa = 0; ph ^= 1; }
                 }
-            }
-        } else if (lane == 0) {
-            // ---------------- peer: forward "my half of stage j landed" ----------------
-            const uint32_t remote0 = mapa_shared(smem_u32(b_full), 0);
-            const int total_j = STAGES_PER_KT * total_it;
-            for (int j = 0; j < total_j; ++j) {
-                if (!wait_one(&b_full[j % SB], (uint32_t)(j / SB) & 1u, abort_flag, p.status, DEV_TIMEOUT_MMA)) break;
-                mbar_arrive_cluster(remote0 + (uint32_t)(j % SB) * 8u);
             }
         }
         __syncwarp();
-    } else if (warp == 2) {
-        setmaxnreg_dec<64>();  // idle warp of the first warpgroup
     } else {
         // ---------------- epilogue (both CTAs, own accumulators) ----------------
-        setmaxnreg_inc<192>();
         const int q = warp & 3;
         const int i = q * 32 + lane;
         const int arow = mma_row_to_actual(i);
@@ -427,6 +375,19 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
             {
                 const int rt = R == 1 ? 0 : grp;  // row tile of this CTA
                 const int mt = row_tile(mq, rt);
+                auto release = [&] {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster(empty_leader);  // the leader's MMA issuer waits for both CTAs' epilogues
+                };
+                if (p.n_out == 1) {
+                    // straight from tensor memory; with two row tiles per CTA the next tile's MMAs wait for both accumulators, so
+                    // they are read into registers whole before the first store
+                    const uint32_t tacc = tmem_base + ((uint32_t)(q * 32) << 16) + acc_col(grp);
+                    if (p.layout == 0) store_tile<BN, R == 2>(TileStoreMN(tacc, q, (int64_t)mt * TILE_M, n0, p), release);
+                    else store_tile<BN, R == 2>(TileStoreNM(tacc, q, (int64_t)mt * TILE_M, n0, p), release);
+                    continue;
+                }
                 const int64_t row = (int64_t)mt * TILE_M + arow;
                 const bool row_ok = mt < p.mtiles && row < p.M;
                 const bool has_bias = p.layout == 1 && p.bias != nullptr;
@@ -450,7 +411,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
                         pk[16 + jj] = *reinterpret_cast<uint32_t *>(&h1);
                     }
                 };
-                // one part -> staging buffer -> one TMA store (which clips at M and N).  In the CTA's last tile nothing hides the
+                // Several destinations: one part -> staging buffer -> one TMA store for each (which clips at M and N).  In the CTA's last tile nothing hides the
                 // stores behind later MMAs any more, and the operand rings are idle (every load has landed and every MMA that
                 // read them has completed, or this tile's accumulator would not be full): each part then gets a buffer of its
                 // own inside the rings, so no part waits for the previous store to release the staging buffer (final epilogue 9.6k ->
@@ -490,7 +451,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
                         bulk_commit_group();
                     }
                 };
-                constexpr int NPARTS = BN / PART, HELD = 5;
+                constexpr int NPARTS = BN / PART, HELD = R == 2 ? 5 : 1;  // R = 1: the next tile has the other accumulator
 #pragma unroll
                 for (int part = 0; part < NPARTS - HELD; part++) {
                     uint32_t pk[PART / 2];
@@ -500,9 +461,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
                 uint32_t held[HELD * (PART / 2)];
 #pragma unroll
                 for (int h = 0; h < HELD; h++) drain(NPARTS - HELD + h, held + h * (PART / 2));
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(empty_leader);  // the leader's MMA issuer waits for both CTAs' epilogues
+                release();
 #pragma unroll
                 for (int h = 0; h < HELD; h++) store_part(NPARTS - HELD + h, held + h * (PART / 2));
             }
@@ -549,30 +508,22 @@ cudaError_t spmm_dense_b_pair_init()
     return cudaSuccess;
 }
 
-// Pair tiles are 512 x 240 (two row tiles per CTA) or, where that would leave SM pairs without a tile, 256 x 240 (one
-// row tile per CTA: 34 KiB per CTA and k-tile, two alternating accumulators).  Returns false when the pair kernel should not be used for this problem
-// (row tiles do not group evenly, too few tiles to occupy the clusters, or clusters unavailable): the caller then
-// launches the single-CTA kernel.
-bool spmm_dense_b_pair_config(int M, int N, int K, int max_ctas, int force_rows, SpmmConfig *cfg)
+// Pair tiles are 512 x 240 (two row tiles per CTA) or 256 x 240 (one row tile per CTA, two alternating accumulators).  The
+// wide form reads every B stage once per 512 rows (0.66 us a k-tile for four row tiles against 0.47 for two) but drains both
+// accumulators between tiles, and it needs twice the rows for a full wave; row tiles that do not divide evenly are padded
+// (computed, never stored).  The smaller estimate wins.
+float spmm_dense_b_pair_config(int M, int N, int K, int max_ctas, int force_rows, SpmmConfig *cfg)
 {
-    if (g_pair_clusters <= 0) return false;
-    const int mtiles = (M + TILE_M - 1) / TILE_M;
-    (void)K;
+    if (g_pair_clusters <= 0) return -1.0f;
+    const int mtiles = (M + TILE_M - 1) / TILE_M, ktiles = (K + 127) / 128;
     const long long ntiles = (N + BN - 1) / BN;
     int clusters = g_pair_clusters;
     if (max_ctas > 0 && max_ctas / 2 < clusters) clusters = max_ctas / 2;
-    if (clusters < 1) return false;
-    const long long t2 = (long long)(mtiles / (2 * RT)) * ntiles, t1 = (long long)(mtiles / 2) * ntiles;
-    const bool ok2 = mtiles % (2 * RT) == 0 && t2 >= clusters;   // at least one full wave of 512-row tiles
-    const bool ok1 = mtiles % 2 == 0 && 4 * t1 >= 3 * clusters;   // most SM pairs get a 256-row tile
-    int rt = 0;
-    if (force_rows == 1 && ok1) rt = 1;
-    else if (force_rows == 2 && ok2) rt = RT;
-    // 512-row tiles read every B stage once per 512 rows and win wherever they fill the SM pairs (measured at K = 1024 .. 12288,
-    // although 256-row tiles alternate two accumulators and so run a tile's epilogue beside the next tile's MMAs)
-    else if (ok2) rt = RT;
-    else if (ok1) rt = 1;
-    if (rt == 0) return false;
+    if (clusters < 1) return -1.0f;
+    const long long t2 = (long long)((mtiles + 2 * RT - 1) / (2 * RT)) * ntiles, t1 = (long long)((mtiles + 1) / 2) * ntiles;
+    const float e2 = 6.0f + (float)((t2 + clusters - 1) / clusters) * (ktiles * 0.66f + 1.3f);
+    const float e1 = 6.0f + (float)((t1 + clusters - 1) / clusters) * (ktiles * 0.47f + 0.35f);
+    const int rt = force_rows == 1 ? 1 : force_rows == 2 && mtiles > 2 ? RT : e2 < e1 ? RT : 1;
     const long long tiles = rt == RT ? t2 : t1;
     cfg->bn = BN;
     cfg->part = PART;
@@ -581,7 +532,7 @@ bool spmm_dense_b_pair_config(int M, int N, int K, int max_ctas, int force_rows,
     cfg->smem_bytes = SMEM_BYTES;
     cfg->threads = NUM_THREADS;
     cfg->grid = 2 * (int)(tiles < clusters ? tiles : clusters);
-    return true;
+    return rt == RT ? e2 : e1;
 }
 
 cudaError_t launch_spmm_dense_b_pair(const SpmmConfig &cfg, const CUtensorMap &tmap_tile, const CUtensorMap &tmap_tile2, const CUtensorMap &tmap_out, const OutMaps &more_out,

@@ -1,0 +1,459 @@
+// SpMM kernel for few columns: C[M,N] = A * B for decoding steps and other products with too few 128 x 240 tiles to occupy the
+// GPU.  Both operand forms: the V:N:M form (rows of B gathered, NB = 128/V blocks) and the dense-B form (B as [K,N] or [N,K]
+// tiles shared by all blocks, NB = 1).
+//
+// Such products are bound by reading A once (a decoding step) or by latency (everything small), not by MMAs.  So a tile is
+// 128 rows x BN = 16, 32, 64 or 128 columns, two CTAs share an SM (one loads while the other starts or stores), and
+// when the row tiles do not fill the GPU a cluster of up to eight CTAs splits the k-tiles of one tile: the partial sums
+// travel through distributed shared memory, each CTA adds up and stores its share of the columns, always in rank order, so
+// results are the same on every call.
+//
+// One ring stage is a whole k-tile: the 18 KiB block of A (values and metadata, one bulk copy) and its rows of B.
+// Warps: 0..7 B producers (gather4 loads dealt to all of them; a warp needs about 65 clocks for each it issues), 8 A
+// producer, 9 tensor-memory owner and MMA issuer, 12..15 epilogue.  Every wait is bounded.
+#include "vnm_internal.h"
+
+#include <cstring>
+
+namespace vnm {
+
+namespace {
+
+template <int BN, int NB>
+struct Small {
+    static_assert(NB == 1 || NB == 2 || NB == 4, "128 rows hold 1, 2 or 4 vector blocks");
+    static constexpr int RB = BN >= 64 ? 128 : 2 * BN;        // bytes of a row of B in one slice (its swizzle span)
+    static constexpr int SWIZZLE = RB == 128 ? 2 : RB == 64 ? 4 : 6;   // descriptor code
+    static constexpr int CH = (BN + 63) / 64;                 // 64-column slices
+    static constexpr int B_CHUNK_BYTES = KT_ROWS * RB;        // one slice of a block: the k-tile's 128 rows
+    static constexpr int B_BLOCK_BYTES = CH * B_CHUNK_BYTES;
+    static constexpr int B_BYTES = NB * B_BLOCK_BYTES;
+    static constexpr int STAGE_BYTES = AM_BLOCK_BYTES + B_BYTES;
+    static constexpr int PW = 8;
+    static constexpr int GATHERS = NB * KT_GROUPS * CH;       // per k-tile
+    static constexpr int PER_WARP = GATHERS / PW;
+    static_assert(PER_WARP <= 32 && GATHERS % PW == 0, "gathers are dealt to the lanes of the producer warps");
+    static constexpr int STAGES = 104 * 1024 / STAGE_BYTES < 2 ? 2 : 104 * 1024 / STAGE_BYTES > 5 ? 5 : 104 * 1024 / STAGE_BYTES;
+    static constexpr int RED_BYTES = (BN + 8) * TILE_M * 4;   // split over K: this CTA's columns from every rank (8: its share is rounded up); in the idle rings
+    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 256 + 1024;
+    static_assert(SMEM_BYTES <= 227 * 1024 && (BN > 64 || RED_BYTES <= STAGES * STAGE_BYTES), "shared memory per CTA");
+    static constexpr int CTAS = 2 * (SMEM_BYTES + 1024) <= 227 * 1024 ? 2 : 1;   // resident per SM
+    static constexpr int A_WARP = PW, MMA_WARP = PW + 1, EPI_WARP0 = 12;
+    static constexpr int NUM_THREADS = 16 * 32;
+    static constexpr int META_COL = BN < 64 ? 64 : BN;        // the epilogue reads 64 columns at a time
+    static constexpr int META_SETS = 4;
+    static constexpr int TMEM_COLS = META_COL + 4 * META_SETS <= 128 ? 128 : 256;
+};
+
+__device__ __forceinline__ uint32_t cluster_ctarank()
+{
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ uint32_t mapa_shared(uint32_t saddr, uint32_t rank)
+{
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void st_cluster(uint32_t addr, uint32_t v) { asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
+
+template <int BN, int NB>
+__global__ void __launch_bounds__(Small<BN, NB>::NUM_THREADS, 2)
+    spmm_small_kernel(const __grid_constant__ CUtensorMap tmap_b, const SpmmParams p)
+{
+    using T = Small<BN, NB>;
+    constexpr int S = T::STAGES;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t *b_ring = smem;                                   // swizzled tiles first: 1024-byte alignment
+    uint8_t *a_ring = smem + S * T::B_BYTES;
+    uint64_t *full = reinterpret_cast<uint64_t *>(a_ring + S * AM_BLOCK_BYTES);
+    uint64_t *freed = full + S;
+    uint64_t *acc_full = freed + S;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_full + 1);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    float *red = reinterpret_cast<float *>(smem);
+    static_assert(T::B_BYTES % 1024 == 0 && (2 * S + 1) * 8 + 8 <= 256, "shared-memory plan");
+
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    const int split = p.split_k;
+    const uint32_t rank = split > 1 ? cluster_ctarank() : 0u;
+    const int tile = (int)blockIdx.x / split;
+    const int mt = tile / p.ntiles, nt = tile - mt * p.ntiles;
+    const int n0 = nt * BN;
+    const int k0 = (int)((int64_t)p.ktiles * rank / split), k1 = (int)((int64_t)p.ktiles * (rank + 1) / split);
+    const int mode = p.gather_mode;      // GATHER_TMA4, GATHER_CONTIG or GATHER_NONE
+    const bool b_nk = p.b_nk != 0;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < S; s++) {
+            mbar_init(&full[s], 1 + (mode == GATHER_TMA4 ? T::PW : 1));   // the A producer and each warp that loads B
+            mbar_init(&freed[s], 1);
+        }
+        mbar_init(acc_full, 1);
+        *abort_flag = 0;
+        fence_barrier_init();
+    }
+    if (warp == T::MMA_WARP) {
+        tmem_alloc(tmem_slot, T::TMEM_COLS);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    if (warp < T::PW) {
+        // ---------------- B producers ----------------
+        if (p.early) grid_dependency_wait();   // B is still being written; A, barriers and tensor memory do not depend on it
+        if (mode == GATHER_TMA4) {
+            const int q = warp * T::PER_WARP + lane;
+            const bool on = lane < T::PER_WARP;
+            const int gc = q % T::CH, gg = (q / T::CH) % KT_GROUPS, gb = on ? q / (T::CH * KT_GROUPS) : 0;
+            const int4 *rows = p.rows + ((size_t)(mt * NB + gb) * p.ktiles) * KT_GROUPS + gg;
+            if (lane == 0) tma_prefetch_desc(&tmap_b);
+            int4 r = make_int4(0, 0, 0, 0);
+            if (on && k0 < k1) r = __ldg(rows + (size_t)k0 * KT_GROUPS);
+            int s = 0;
+            uint32_t ph = 1;
+            int kt = k0;
+            for (; kt < k1; ++kt) {
+                const int4 cur = r;
+                if (on && kt + 1 < k1) r = __ldg(rows + (size_t)(kt + 1) * KT_GROUPS);
+                if (!__all_sync(0xffffffffu, wait_quiet(&freed[s], ph, abort_flag, p.status, DEV_TIMEOUT_PRODUCER))) break;
+                if (lane == 0) mbar_arrive_expect_tx(&full[s], T::PER_WARP * 4 * T::RB);
+                __syncwarp();
+                if (on) tma_gather4(b_ring + s * T::B_BYTES + gb * T::B_BLOCK_BYTES + gc * T::B_CHUNK_BYTES + gg * 4 * T::RB, &tmap_b, n0 + gc * 64, cur, &full[s]);
+                if (++s == S) { s = 0; ph ^= 1; }
+            }
+            if (*abort_flag && lane == 0)
+                for (int k = kt - k0 > S ? kt - k0 - S : 0; k < kt - k0; ++k) drain_slot(&full[k % S], (uint32_t)(k / S) & 1u, p.status);
+        } else if (warp == 0 && elect_one()) {
+            tma_prefetch_desc(&tmap_b);
+            int s = 0;
+            uint32_t ph = 1;
+            int kt = k0;
+            for (; kt < k1; ++kt) {
+                if (!wait_quiet(&freed[s], ph, abort_flag, p.status, DEV_TIMEOUT_PRODUCER)) break;
+                uint8_t *st = b_ring + s * T::B_BYTES;
+                if (mode == GATHER_NONE) {
+                    mbar_arrive(&full[s]);
+                } else if (b_nk) {           // two boxes of BN n-rows x 64 k (NB == 1)
+                    mbar_arrive_expect_tx(&full[s], 2 * BN * 128);
+                    for (int h = 0; h < 2; h++) tma_load_2d(st + h * BN * 128, &tmap_b, kt * 128 + h * 64, n0, &full[s]);
+                } else {                     // 128 consecutive rows; for NB > 1 every block reads the same ones
+                    mbar_arrive_expect_tx(&full[s], T::B_BYTES);
+                    for (int b = 0; b < NB; b++) {
+                        const int row = __ldg(&p.rows[((size_t)(mt * NB + b) * p.ktiles + kt) * KT_GROUPS].x);
+                        for (int c = 0; c < T::CH; c++) tma_load_2d(st + b * T::B_BLOCK_BYTES + c * T::B_CHUNK_BYTES, &tmap_b, n0 + c * 64, row, &full[s]);
+                    }
+                }
+                if (++s == S) { s = 0; ph ^= 1; }
+            }
+            if (*abort_flag && mode != GATHER_NONE)
+                for (int k = kt - k0 > S ? kt - k0 - S : 0; k < kt - k0; ++k) drain_slot(&full[k % S], (uint32_t)(k / S) & 1u, p.status);
+        }
+        __syncwarp();
+    } else if (warp == T::A_WARP) {
+        // ---------------- A producer ----------------
+        if (elect_one()) {
+            const uint8_t *src = p.am + (size_t)mt * p.ktiles * AM_BLOCK_BYTES;
+            int s = 0;
+            uint32_t ph = 1;
+            int kt = k0;
+            for (; kt < k1; ++kt) {
+                if (!wait_quiet(&freed[s], ph, abort_flag, p.status, DEV_TIMEOUT_PRODUCER)) break;
+                mbar_arrive_expect_tx(&full[s], AM_BLOCK_BYTES);
+                bulk_g2s(a_ring + s * AM_BLOCK_BYTES, src + (size_t)kt * AM_BLOCK_BYTES, AM_BLOCK_BYTES, &full[s]);
+                if (++s == S) { s = 0; ph ^= 1; }
+            }
+            if (*abort_flag)
+                for (int k = kt - k0 > S ? kt - k0 - S : 0; k < kt - k0; ++k) drain_slot(&full[k % S], (uint32_t)(k / S) & 1u, p.status);
+        }
+        __syncwarp();
+    } else if (warp == T::MMA_WARP) {
+        // ---------------- MMA issuer (see vnm_spmm.cu: one elected lane copies metadata and issues the MMAs behind it) ----------------
+        if (elect_one()) {
+            const uint32_t idesc0 = make_idesc_f16(TILE_M, BN, true, 0u, !b_nk);
+            const uint64_t adesc0 = make_smem_desc(smem_u32(a_ring), 16, 1024, 2);
+            const uint64_t mdesc0 = make_smem_desc(smem_u32(a_ring) + A_IMG_BYTES, 0, 128, 0);
+            // N-major: slices of 128 rows of RB bytes, a K=32 block is 32 rows further.  K-major: two boxes of BN rows of 128 bytes
+            // (64 k), a K=32 block is 64 bytes further inside a row.
+            const uint64_t bdesc0 = b_nk ? make_smem_desc(smem_u32(b_ring), 16, 1024, 2) : make_smem_desc(smem_u32(b_ring), T::B_CHUNK_BYTES, 8 * T::RB, T::SWIZZLE);
+            int s = 0;
+            uint32_t ph = 0;
+            for (int kt = k0; kt < k1; ++kt) {
+                if (!wait_one(&full[s], ph, abort_flag, p.status, DEV_TIMEOUT_MMA)) break;
+                tc_fence_after();
+                const uint32_t mcol = tmem_base + (uint32_t)(T::META_COL + ((kt - k0) % T::META_SETS) * 4);
+                const uint32_t aoff = (uint32_t)(s * AM_BLOCK_BYTES) >> 4, boff = (uint32_t)(s * T::B_BYTES) >> 4;
+                tc_cp_128x128b(mcol, mdesc0 + aoff);
+#pragma unroll
+                for (int kb = 0; kb < 4; kb++) {
+                    const uint32_t koff = b_nk ? (uint32_t)((kb >> 1) * BN * 128 + (kb & 1) * 64) : (uint32_t)(kb * 32 * T::RB);
+#pragma unroll
+                    for (int b = 0; b < NB; b++) {
+                        uint32_t mk[4] = {0u, 0u, 0u, 0u};  // bit set = output lane NOT written
+                        if (NB == 2) {
+                            mk[0] = mk[1] = (b == 0) ? 0u : 0xFFFFFFFFu;
+                            mk[2] = mk[3] = (b == 0) ? 0xFFFFFFFFu : 0u;
+                        } else if (NB == 4) {
+                            mk[0] = (b == 0) ? 0u : 0xFFFFFFFFu;
+                            mk[1] = (b == 1) ? 0u : 0xFFFFFFFFu;
+                            mk[2] = (b == 2) ? 0u : 0xFFFFFFFFu;
+                            mk[3] = (b == 3) ? 0u : 0xFFFFFFFFu;
+                        }
+                        tc_mma_sp_f16(tmem_base, adesc0 + aoff + (uint32_t)(kb * 32 >> 4), bdesc0 + boff + ((koff + (uint32_t)(b * T::B_BLOCK_BYTES)) >> 4),
+                                      mcol + (uint32_t)(kb & ~1), idesc0 | (uint32_t)(kb & 1), (kt != k0 || kb != 0) ? 1u : 0u, mk[0], mk[1], mk[2], mk[3]);
+                    }
+                }
+                tc_commit(&freed[s]);
+                if (++s == S) { s = 0; ph ^= 1; }
+            }
+            tc_commit(acc_full);   // on an abort, too: nothing of this thread is in flight when the CTA leaves
+        }
+        __syncwarp();
+    }
+
+    if (split == 1) {
+        if (warp >= T::EPI_WARP0) {
+            const int q = warp & 3;
+            if (wait_warp(acc_full, 0u, abort_flag, p.status, DEV_TIMEOUT_EPILOGUE) && *abort_flag == 0) {
+                tc_fence_after();
+                const uint32_t trow = tmem_base + ((uint32_t)(q * 32) << 16);
+                if (p.layout == 0) store_tile<BN, false>(TileStoreMN(trow, q, (int64_t)mt * TILE_M, n0, p), [] {});
+                else store_tile<BN, false>(TileStoreNM(trow, q, (int64_t)mt * TILE_M, n0, p), [] {});
+            }
+        }
+    } else if (BN <= 64) {
+        // ---------------- split over K: rank d adds up columns [d * share, (d + 1) * share) of all ranks ----------------
+        // A CTA whose waits ran out still takes part in the barriers; its sums are meaningless and the status word says so.
+        const int share = (BN + split - 1) / split;
+        if (warp >= T::EPI_WARP0) {
+            (void)wait_warp(acc_full, 0u, abort_flag, p.status, DEV_TIMEOUT_EPILOGUE);
+            tc_fence_after();
+        }
+        cluster_arrive();
+        cluster_wait();                  // every MMA of every rank is done: the rings are free
+        if (warp >= T::EPI_WARP0) {
+            const int q = warp & 3;
+            const uint32_t red0 = smem_u32(red) + (uint32_t)mma_row_to_actual(q * 32 + lane) * 4u;
+            for (int c0 = 0; c0 < BN; c0 += 8) {
+                uint32_t v[8];
+                tc_ld_32x32b_x8(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, v);
+                tc_wait_ld();
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    const int n = c0 + i, d = n / share;
+                    st_cluster(mapa_shared(red0, (uint32_t)d) + (uint32_t)(((int)rank * share + n - d * share) * TILE_M * 4), v[i]);
+                }
+            }
+        }
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();                  // all partial sums have arrived, and nobody writes here any more
+        const int first = (int)rank * share, count = first + share <= BN ? share : (BN > first ? BN - first : 0);
+        for (int e = threadIdx.x; e < count * (TILE_M / 2); e += T::NUM_THREADS) {
+            const int n = e / (TILE_M / 2), r2 = (e - n * (TILE_M / 2)) * 2;      // two neighbouring rows
+            float2 sum = make_float2(0.0f, 0.0f);
+            for (int d = 0; d < split; d++) {
+                const float2 x = *reinterpret_cast<const float2 *>(red + (d * share + n) * TILE_M + r2);
+                sum.x += x.x;
+                sum.y += x.y;
+            }
+            const int64_t row = (int64_t)mt * TILE_M + r2;
+            const int col = n0 + first + n;
+            if (row >= p.M || col >= p.N) continue;
+            __half2 h = __floats2half2_rn(sum.x, sum.y);
+            if (p.layout == 0) {
+                p.out[row * p.ldo + col] = __low2half(h);
+                p.out[(row + 1) * p.ldo + col] = __high2half(h);
+            } else {
+                if (p.bias) h = __hadd2(h, __halves2half2(p.bias[row], p.bias[row + 1]));
+                __half *d = p.out + (int64_t)col * p.ldo + row;
+                if ((p.ldo & 1) == 0 && ((uintptr_t)p.out & 3) == 0) {
+                    *reinterpret_cast<__half2 *>(d) = h;
+                } else {
+                    d[0] = __low2half(h);
+                    d[1] = __high2half(h);
+                }
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == T::MMA_WARP) {
+        tc_fence_after();
+        tmem_dealloc(tmem_base, T::TMEM_COLS);
+    }
+}
+
+int g_num_sms_small = 0;
+
+// Self-test of the bounded waits: two threads wait, through the same wait_one as the product kernels and with the
+// same limit, on a barrier that nothing ever signals.  The first to run out of time records its status bit and
+// raises the abort flag; the other sees the flag and leaves.  The kernel then returns normally.
+__global__ void wait_expiry_selftest_kernel(int *status)
+{
+    __shared__ uint64_t bar;
+    __shared__ int abort_word;
+    if (threadIdx.x == 0) {
+        mbar_init(&bar, 1);
+        abort_word = 0;
+        fence_barrier_init();
+    }
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) wait_one(&bar, 0u, &abort_word, status, DEV_TIMEOUT_EPILOGUE);
+    __syncthreads();
+}
+
+template <int BN, int NB>
+cudaError_t init_one()
+{
+    return cudaFuncSetAttribute(spmm_small_kernel<BN, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, Small<BN, NB>::SMEM_BYTES);
+}
+
+template <int BN, int NB>
+cudaError_t launch_one(const SpmmConfig &cfg, const CUtensorMap &tmap_b, const SpmmParams &p, cudaStream_t stream)
+{
+    using T = Small<BN, NB>;
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3((unsigned)cfg.grid, 1, 1);
+    lc.blockDim = dim3(T::NUM_THREADS, 1, 1);
+    lc.dynamicSmemBytes = (size_t)cfg.smem_bytes;
+    lc.stream = stream;
+    cudaLaunchAttribute attr[2];
+    lc.attrs = attr;
+    lc.numAttrs = 0;
+    if (p.split_k > 1) {
+        attr[lc.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[lc.numAttrs].val.clusterDim.x = (unsigned)p.split_k;
+        attr[lc.numAttrs].val.clusterDim.y = 1;
+        attr[lc.numAttrs++].val.clusterDim.z = 1;
+    }
+    if (p.early) {
+        attr[lc.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[lc.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    return cudaLaunchKernelEx(&lc, spmm_small_kernel<BN, NB>, tmap_b, p);
+}
+
+template <int BN, int NB>
+void fill(SpmmConfig *cfg)
+{
+    cfg->smem_bytes = Small<BN, NB>::SMEM_BYTES;
+    cfg->threads = Small<BN, NB>::NUM_THREADS;
+    cfg->resident = Small<BN, NB>::CTAS;
+}
+
+#define VNM_SMALL_DISPATCH(bn, nb, CALL)                                                                                  \
+    ((nb) == 1 ? ((bn) == 16 ? CALL(16, 1) : (bn) == 32 ? CALL(32, 1) : (bn) == 64 ? CALL(64, 1) : CALL(128, 1))           \
+     : (nb) == 2 ? ((bn) == 16 ? CALL(16, 2) : (bn) == 32 ? CALL(32, 2) : CALL(64, 2))                                       \
+                 : ((bn) == 16 ? CALL(16, 4) : (bn) == 32 ? CALL(32, 4) : CALL(64, 4)))
+
+}  // namespace
+
+cudaError_t launch_wait_expiry_selftest(int *status, cudaStream_t stream)
+{
+    wait_expiry_selftest_kernel<<<1, 64, 0, stream>>>(status);
+    return cudaGetLastError();
+}
+
+cudaError_t spmm_small_init()
+{
+    cudaError_t e;
+    if ((e = init_one<16, 1>()) != cudaSuccess || (e = init_one<32, 1>()) != cudaSuccess || (e = init_one<64, 1>()) != cudaSuccess ||
+        (e = init_one<128, 1>()) != cudaSuccess || (e = init_one<16, 2>()) != cudaSuccess || (e = init_one<32, 2>()) != cudaSuccess ||
+        (e = init_one<64, 2>()) != cudaSuccess || (e = init_one<16, 4>()) != cudaSuccess || (e = init_one<32, 4>()) != cudaSuccess ||
+        (e = init_one<64, 4>()) != cudaSuccess)
+        return e;
+    int dev = 0;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+    return cudaDeviceGetAttribute(&g_num_sms_small, cudaDevAttrMultiProcessorCount, dev);
+}
+
+// Tile width and split with the smallest estimated time (microseconds, returned).  The estimate is a fit to a sweep over
+// 1024 x 1024 .. 12288 x 12288, N = 8 .. 512, all widths and splits: a fixed part for launch, set-up, first loads and
+// epilogue; a k-tile's time in a CTA that has its SM to itself (latency of the ring for narrow tiles, the shared-memory port
+// for wide ones); a second CTA on an SM costs its set-up and shares the port; and A cannot be read faster than HBM delivers
+// it.  Widths of 16 and more CTAs than SMs lose more often than they win, which is what the fit expresses.  Only up to
+// SMALL_SPLIT_N columns are k-tiles split: beyond, the order of summation stays that of the other kernels, so that results do
+// not depend on how a caller cuts its columns.
+float spmm_small_config(int mtiles, int ktiles, int N, int nb, bool gather, SpmmConfig *cfg)
+{
+    const int sms = g_num_sms_small > 0 ? g_num_sms_small : 148;
+    static const int widths[4] = {16, 32, 64, 128};
+    static const float fixed[4] = {3.9f, 4.1f, 4.6f, 5.3f};
+    static const float dense_kt[4] = {0.185f, 0.19f, 0.25f, 0.43f}, gather_kt[4] = {0.32f, 0.33f, 0.36f, 0.53f};
+    const float hbm = 3.5f + (float)mtiles * ktiles * AM_BLOCK_BYTES / 5.6e6f;
+    float best = 1e30f;
+    for (int w = 0; w < 4; w++) {
+        const int bn = widths[w];
+        if ((bn == 128 && nb > 1) || (bn > 16 && bn >= 2 * N)) continue;
+        SpmmConfig c;
+        memset(&c, 0, sizeof(c));
+#define VNM_FILL(BN, NB) fill<BN, NB>(&c)
+        VNM_SMALL_DISPATCH(bn, nb, VNM_FILL);
+#undef VNM_FILL
+        const float kt_us = (gather ? gather_kt[w] : dense_kt[w]) * (nb == 4 ? 1.4f : nb == 2 ? 1.15f : 1.0f);
+        const long long tiles = (long long)mtiles * ((N + bn - 1) / bn);
+        for (int split = 1; split <= 8 && split <= ktiles; split++) {
+            const long long ctas = tiles * split, per = (ctas + sms - 1) / sms;
+            const int kts = (ktiles + split - 1) / split;
+            const int both = (int)(per < c.resident ? per : c.resident);      // CTAs that share an SM
+            float t = fixed[w] + (gather && nb > 1 ? 1.4f : 0.0f) + (split > 1 ? 0.3f + 0.006f * bn : 0.0f);
+            if (per <= c.resident) {
+                t += 2.2f * (both - 1) + kts * kt_us * (1.0f + 0.45f * (both - 1));
+            } else {   // several waves: the port is busy all the time and nothing is gained from the second CTA
+                t += (float)ctas / (float)(sms * c.resident) * (kts * kt_us * both * 1.25f + 3.0f);
+            }
+            t = t > hbm ? t : hbm + 0.01f * t;
+            if (t < best) {
+                best = t;
+                *cfg = c;
+                cfg->bn = bn;
+                cfg->nb = nb;
+                cfg->part = bn;
+                cfg->stages = 1;
+                cfg->split = split;
+                cfg->grid = (int)ctas;
+            }
+            if (N > SMALL_SPLIT_N) break;
+        }
+    }
+    return best;
+}
+
+// Tensor map of the dense operand for this kernel: rows of at most 64 columns, gathered four at a time or as boxes of 128
+// consecutive rows, or (b_nk) boxes of bn n-rows x 64 k.
+CUresult spmm_small_encode(EncodeTiledFn enc, CUtensorMap *map, const void *B, int64_t ldb, int K, int N, int b_nk, int gather_mode, int bn)
+{
+    cuuint32_t estr[2] = {1, 1};
+    cuuint64_t strides[1] = {(cuuint64_t)ldb * 2};
+    if (b_nk) {
+        cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)N};
+        cuuint32_t box[2] = {64, (cuuint32_t)bn};
+        return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(B), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    }
+    cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)K};
+    const cuuint32_t w = bn >= 64 ? 64u : (cuuint32_t)bn;
+    cuuint32_t box[2] = {w, gather_mode == GATHER_TMA4 ? 1u : 128u};
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(B), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               w == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : w == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+}
+
+cudaError_t launch_spmm_small(const SpmmConfig &cfg, const CUtensorMap &tmap_b, const SpmmParams &p, cudaStream_t stream)
+{
+#define VNM_LAUNCH(BN, NB) launch_one<BN, NB>(cfg, tmap_b, p, stream)
+    return VNM_SMALL_DISPATCH(cfg.bn, cfg.nb, VNM_LAUNCH);
+#undef VNM_LAUNCH
+}
+
+}  // namespace vnm
