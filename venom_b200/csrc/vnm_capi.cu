@@ -8,6 +8,7 @@
 #include <cstdlib>
 #include <cstdarg>
 #include <cstring>
+#include <initializer_list>
 #include <new>
 #include <string>
 
@@ -84,6 +85,28 @@ bool g_kernels_ready[kMaxDevices] = {};
 std::mutex g_init_mutex;
 int g_strategy = 0;  // VNM_STRATEGY_*
 
+// Device memory of the handles comes from one stream-ordered pool per device: cudaMalloc and cudaFree take 0.1 to 20 ms
+// each on a host with other tenants (the driver maps and unmaps under a lock), most of what preparing an operand costs.
+// The pool keeps at most POOL_KEEP_BYTES of freed memory for later handles and gives the rest back; the driver makes it safe
+// for several threads and streams.
+constexpr uint64_t POOL_KEEP_BYTES = 1ull << 30;
+cudaMemPool_t g_pools[kMaxDevices] = {};
+
+cudaError_t device_alloc(void **ptr, size_t bytes, int dev, cudaStream_t stream)
+{
+    return cudaMallocFromPoolAsync(ptr, bytes, g_pools[dev], stream);
+}
+
+// Like cudaFree: waits until nothing on the device can still use the memory.
+void device_free(std::initializer_list<void *> ptrs)
+{
+    bool any = false;
+    for (void *p : ptrs) any = any || p;
+    if (!any || cudaDeviceSynchronize() != cudaSuccess) return;   // a lost context has no memory to give back
+    for (void *p : ptrs)
+        if (p) cudaFreeAsync(p, nullptr);
+}
+
 // Opts every kernel instance into its shared-memory size on the current device (once per device).
 int ensure_kernels_ready(int *device_out)
 {
@@ -95,6 +118,13 @@ int ensure_kernels_ready(int *device_out)
         VNM_CUDA(spmm_init_kernels(), "cudaFuncSetAttribute(max dynamic shared memory)");
         VNM_CUDA(spmm_dense_b_pair_init(), "cudaFuncSetAttribute(max dynamic shared memory)");
         VNM_CUDA(spmm_small_init(), "cudaFuncSetAttribute(max dynamic shared memory)");
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        VNM_CUDA(cudaMemPoolCreate(&g_pools[dev], &props), "cudaMemPoolCreate");
+        uint64_t keep = POOL_KEEP_BYTES;
+        VNM_CUDA(cudaMemPoolSetAttribute(g_pools[dev], cudaMemPoolAttrReleaseThreshold, &keep), "cudaMemPoolSetAttribute");
         g_kernels_ready[dev] = true;
     }
     if (device_out) *device_out = dev;
@@ -250,8 +280,7 @@ int vnm_prepared_bytes(int M, int K, int V, int n, int m, int64_t *bytes)
     const int64_t Ksp = ksp_of(K, m);
     const bool dense_b = choose_dense_b(M, K, V, m, g_strategy);
     const int64_t mtiles = (M + TILE_M - 1) / TILE_M, ktiles = dense_b ? (K + 127) / 128 : (Ksp + KT_COMP - 1) / KT_COMP;
-    const int64_t nb = dense_b ? 1 : TILE_M / V;
-    if (bytes) *bytes = mtiles * ktiles * AM_BLOCK_BYTES + mtiles * nb * ktiles * KT_GROUPS * 16 + 256;
+    if (bytes) *bytes = mtiles * ktiles * AM_BLOCK_BYTES + (dense_b ? 0 : mtiles * (TILE_M / V) * ktiles * KT_GROUPS * 16) + 256;
     return VNM_OK;
 }
 
@@ -278,13 +307,18 @@ int vnm_prepare_as(const void *values, const uint32_t *meta, const uint32_t *col
     memset(h, 0, sizeof(*h));
     shape_handle(h, M, K, V, n, m, choose_dense_b(M, K, V, m, strategy));
     h->device = dev_now;
-    cudaError_t e = cudaMalloc(&h->am, (size_t)h->mtiles * h->ktiles * AM_BLOCK_BYTES);
-    if (e == cudaSuccess) e = cudaMalloc(&h->rows, (size_t)h->vblocks_padded * h->ktiles * KT_GROUPS * sizeof(int4));
-    if (e == cudaSuccess) e = cudaMalloc((void **)&h->status, sizeof(int));
-    if (e == cudaSuccess) e = cudaMemsetAsync(h->status, 0, sizeof(int), (cudaStream_t)stream);
+    // one block: value and metadata images | row table (gather form) | status word
+    const size_t am_bytes = (size_t)h->mtiles * h->ktiles * AM_BLOCK_BYTES;
+    const size_t rows_bytes = h->dense_b ? 0 : (size_t)h->vblocks_padded * h->ktiles * KT_GROUPS * sizeof(int4);
+    cudaError_t e = device_alloc(&h->am, am_bytes + rows_bytes + 256, dev_now, (cudaStream_t)stream);
+    if (e == cudaSuccess) {
+        h->rows = (uint8_t *)h->am + am_bytes;
+        h->status = (int *)((uint8_t *)h->am + am_bytes + rows_bytes);
+        e = cudaMemsetAsync(h->status, 0, sizeof(int), (cudaStream_t)stream);
+    }
     if (e == cudaSuccess) {
         if (h->dense_b)
-            e = launch_prepare_dense_b(values, meta, colloc, M, K, V, m, h->am, h->rows, h->mtiles, h->ktiles, (cudaStream_t)stream);
+            e = launch_prepare_dense_b(values, meta, colloc, M, K, V, m, h->am, h->mtiles, h->ktiles, (cudaStream_t)stream);
         else
             e = launch_prepare(values, meta, colloc, M, K, V, m, h->am, h->rows, h->mtiles, h->ktiles, h->vblocks_padded, (cudaStream_t)stream);
     }
@@ -299,12 +333,13 @@ int vnm_prepare_as(const void *values, const uint32_t *meta, const uint32_t *col
 int vnm_destroy(vnm_handle_t h)
 {
     if (!h) return VNM_OK;
-    cudaFree(h->am);
-    cudaFree(h->rows);
-    cudaFree(h->status);
-    cudaFree(h->stage_B);
-    cudaFree(h->stage_out);
-    cudaFree(h->stage_bias);
+    {
+        int now = -1;   // the memory belongs to the handle's device
+        const bool other = cudaGetDevice(&now) == cudaSuccess && now != h->device;
+        if (other) cudaSetDevice(h->device);
+        device_free({h->am, h->stage_B, h->stage_out, h->stage_bias});
+        if (other) cudaSetDevice(now);
+    }
     if (h->host_pipe_ready) {
         for (cudaEvent_t e : h->ev) cudaEventDestroy(e);
     }
@@ -719,13 +754,13 @@ int vnm_operand_form(vnm_handle_t h, int *dense_b)
     return VNM_OK;
 }
 
-static int grow(void **buf, size_t *cap, size_t need)
+static int grow(vnm_handle_t h, void **buf, size_t *cap, size_t need, cudaStream_t stream)
 {
     if (*cap >= need) return VNM_OK;
-    if (*buf) cudaFree(*buf);
+    device_free({*buf});
     *buf = nullptr; *cap = 0;
-    cudaError_t e = cudaMalloc(buf, need);
-    if (e != cudaSuccess) return fail_cuda(e, "staging cudaMalloc");
+    cudaError_t e = device_alloc(buf, need, h->device, stream);
+    if (e != cudaSuccess) return fail_cuda(e, "staging allocation");
     *cap = need;
     return VNM_OK;
 }
@@ -738,8 +773,8 @@ static int spmm_host_impl(vnm_handle_t h, const void *B_host, int N, const void 
     cudaStream_t s = (cudaStream_t)stream;
     const size_t b_bytes = (size_t)h->K * N * 2, o_bytes = (size_t)h->M * N * 2;
     int rc;
-    if ((rc = grow(&h->stage_B, &h->stage_B_bytes, b_bytes))) return rc;
-    if ((rc = grow(&h->stage_out, &h->stage_out_bytes, o_bytes))) return rc;
+    if ((rc = grow(h, &h->stage_B, &h->stage_B_bytes, b_bytes, s))) return rc;
+    if ((rc = grow(h, &h->stage_out, &h->stage_out_bytes, o_bytes, s))) return rc;
     if (!h->host_pipe_ready) {
         // One upload and one download stream per device for every handle: with a pair of streams per handle
         // the driver multiplexes them onto a few hardware queues and unrelated copies end up waiting for each other.
@@ -777,7 +812,7 @@ static int spmm_host_impl(vnm_handle_t h, const void *B_host, int N, const void 
     VNM_CUDA(cudaStreamWaitEvent(h->copy_in, ev_start, 0), "stream wait");
     VNM_CUDA(cudaStreamWaitEvent(h->copy_out, ev_start, 0), "stream wait");
     if (bias_host) {
-        if (!h->stage_bias) VNM_CUDA(cudaMalloc(&h->stage_bias, (size_t)h->M * 2), "bias cudaMalloc");
+        if (!h->stage_bias) VNM_CUDA(device_alloc(&h->stage_bias, (size_t)h->M * 2, h->device, h->copy_in), "bias allocation");
         VNM_CUDA(cudaMemcpyAsync(h->stage_bias, bias_host, (size_t)h->M * 2, cudaMemcpyHostToDevice, h->copy_in), "H2D copy of bias");
     }
     for (int c = 0, n0 = 0; c < chunks; n0 += widths[c], ++c) {

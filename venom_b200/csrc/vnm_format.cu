@@ -864,18 +864,6 @@ __global__ void __launch_bounds__(256) prepare_dense_b_kernel(const __half *__re
     }
 }
 
-// Row table of the dense-B form: stage j of a tile starts at original row 64*j.
-__global__ void __launch_bounds__(256) prepare_dense_b_rows_kernel(int K, int mtiles, int ktiles, int4 *__restrict__ rows)
-{
-    const int64_t per_tile = (int64_t)ktiles * KT_GROUPS;
-    const int64_t total = (int64_t)mtiles * per_tile;
-    for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t g = idx % per_tile;
-        const int64_t k = g * 4;
-        rows[idx] = k < K ? make_int4((int)k, (int)k + 1, (int)k + 2, (int)k + 3) : make_int4(K, K, K, K);
-    }
-}
-
 // ------------------------------------------------------------------------------------------------
 // Transpose of an activation, [N, K] -> [K, N] (fp16), for the gather form, which needs rows of B.  A block takes 64 n x 64 k:
 // a thread reads 16 bytes (8 k) of two neighbouring n, interleaves them into eight words (n, n + 1) and puts them into shared
@@ -930,26 +918,16 @@ cudaError_t launch_transpose(const void *src, int64_t ld_src, int N, int K, void
 }
 
 cudaError_t launch_prepare_dense_b(const void *values, const uint32_t *meta, const uint32_t *colloc, int M, int K, int V, int m,
-                                   void *am, void *rows, int mtiles, int ktiles, cudaStream_t stream)
+                                   void *am, int mtiles, int ktiles, cudaStream_t stream)
 {
     const int64_t Ksp = ksp_of(K, m);
     const int64_t cap = (int64_t)148 * 64;
-    {
-        const int64_t total = (int64_t)mtiles * ktiles * 512;
-        int64_t blocks = (total + 255) / 256;
-        if (blocks > cap) blocks = cap;
-        prepare_dense_b_kernel<<<(unsigned)blocks, 256, 0, stream>>>((const __half *)values, meta, colloc, M, K, V, m, Ksp, mtiles, ktiles,
-                                                                   (uint8_t *)am);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-    }
-    {
-        const int64_t total = (int64_t)mtiles * ktiles * KT_GROUPS;
-        int64_t blocks = (total + 255) / 256;
-        if (blocks > cap) blocks = cap;
-        prepare_dense_b_rows_kernel<<<(unsigned)blocks, 256, 0, stream>>>(K, mtiles, ktiles, (int4 *)rows);
-        return cudaGetLastError();
-    }
+    const int64_t total = (int64_t)mtiles * ktiles * 512;
+    int64_t blocks = (total + 255) / 256;
+    if (blocks > cap) blocks = cap;
+    prepare_dense_b_kernel<<<(unsigned)blocks, 256, 0, stream>>>((const __half *)values, meta, colloc, M, K, V, m, Ksp, mtiles, ktiles,
+                                                               (uint8_t *)am);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_prepare(const void *values, const uint32_t *meta, const uint32_t *colloc, int M, int K, int V, int m,

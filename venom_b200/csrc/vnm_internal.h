@@ -88,7 +88,7 @@ cudaError_t launch_prepare(const void *values, const uint32_t *meta, const uint3
                            void *rows, int mtiles, int ktiles, int vblocks_padded, cudaStream_t stream);
 
 cudaError_t launch_prepare_dense_b(const void *values, const uint32_t *meta, const uint32_t *colloc, int M, int K, int V, int m,
-                                   void *am, void *rows, int mtiles, int ktiles, cudaStream_t stream);
+                                   void *am, int mtiles, int ktiles, cudaStream_t stream);
 
 cudaError_t launch_transpose(const void *src, int64_t ld_src, int N, int K, void *dst, cudaStream_t stream);  // [N, K] -> [K, N], fp16
 

@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(Traits<BN, NB>::NUM_THREADS, 1)
         if (lane == 0) { tma_prefetch_desc(&tmap_rows); tma_prefetch_desc(&tmap_tile); }
         auto row_entry = [&](int b, int g) { return p.rows + ((size_t)(mt * NB + b) * p.ktiles) * KT_GROUPS + (size_t)jl * BS_GROUPS + g; };
         auto fetch = [&]() -> int4 {
-            if (gmode == GATHER_CONTIG) return box_on ? __ldg(row_entry(bb, 0)) : make_int4(0, 0, 0, 0);
+            if (gmode == GATHER_CONTIG) return make_int4(jl * BS_ROWS, 0, 0, 0);
             return on ? __ldg(row_entry(gb, gg)) : make_int4(0, 0, 0, 0);
         };
         int4 r = make_int4(0, 0, 0, 0);
@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(Traits<BN, NB>::NUM_THREADS, 1)
                 if (lane == 0) mbar_arrive_expect_tx(full, T::B_STAGE_BYTES / T::H);
                 __syncwarp();
                 if (on) tma_gather4(st + gb * T::B_BLOCK_BYTES + gc * T::B_CHUNK_BYTES + gg * 512, &tmap_rows, n0 + gc * 64, cur, full);
-            } else if (gmode == GATHER_CONTIG) {   // 32 consecutive rows starting at the first selected row of the stage
+            } else if (gmode == GATHER_CONTIG) {   // 32 consecutive rows (m == 4: all of them are selected)
                 if (lane == 0) mbar_arrive_expect_tx(full, T::B_STAGE_BYTES / T::H);
                 __syncwarp();
                 if (box_on) tma_load_2d(st + bb * T::B_BLOCK_BYTES + bc * T::B_CHUNK_BYTES, &tmap_tile, n0 + bc * 64, cur.x, full);

@@ -148,10 +148,8 @@ __global__ void __launch_bounds__(Small<BN, NB>::NUM_THREADS, 2)
                     for (int h = 0; h < 2; h++) tma_load_2d(st + h * BN * 128, &tmap_b, kt * 128 + h * 64, n0, &full[s]);
                 } else {                     // 128 consecutive rows; for NB > 1 every block reads the same ones
                     mbar_arrive_expect_tx(&full[s], T::B_BYTES);
-                    for (int b = 0; b < NB; b++) {
-                        const int row = __ldg(&p.rows[((size_t)(mt * NB + b) * p.ktiles + kt) * KT_GROUPS].x);
-                        for (int c = 0; c < T::CH; c++) tma_load_2d(st + b * T::B_BLOCK_BYTES + c * T::B_CHUNK_BYTES, &tmap_b, n0 + c * 64, row, &full[s]);
-                    }
+                    for (int b = 0; b < NB; b++)
+                        for (int c = 0; c < T::CH; c++) tma_load_2d(st + b * T::B_BLOCK_BYTES + c * T::B_CHUNK_BYTES, &tmap_b, n0 + c * 64, kt * KT_ROWS, &full[s]);
                 }
                 if (++s == S) { s = 0; ph ^= 1; }
             }
