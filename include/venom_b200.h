@@ -73,6 +73,14 @@ int vnm_compress_f16(const void *dense, int64_t ldd, const int32_t *mask, const 
 int vnm_prune_magnitude_f32(const float *w, int64_t ldw, int M, int K, int V, int n, int m,
                             int32_t *mask, int64_t ldm, uint32_t *colloc, void *stream);
 
+/* Pruner and compressor in one pass: the values, metadata and column-loc that vnm_prune_magnitude_f32 followed by
+ * vnm_compress_f16 (with its mask) give for the weights rounded to fp16, bit for bit, without the mask or the masked
+ * matrix ever being written.  w: fp16 or fp32 [M, K], leading dimension ldw.  A (row, group) of a block that keeps nothing counts
+ * as a violation, as there.  Needs K % m == 0 and m <= 64 (VNM_ERR_UNSUPPORTED otherwise). */
+enum { VNM_F32 = 0, VNM_F16 = 1 };
+int vnm_sparsify_magnitude(const void *w, int w_type, int64_t ldw, int M, int K, int V, int n, int m,
+                           void *values, uint32_t *meta, uint32_t *colloc, unsigned long long *violations, void *stream);
+
 /* V:N:M -> dense decompressor (CUDA).  dense [M, K] fp16, leading dimension ldd, fully overwritten.
  * Replaces: Format_sr_nm<T>::to_dense, src/format/format_sr_nm.cpp:327-417. */
 int vnm_decompress_f16(const void *values, const uint32_t *meta, const uint32_t *colloc,

@@ -38,6 +38,8 @@ def lib():
         L.vnm_decompress_f16.argtypes = [C.c_void_p] * 3 + [C.c_int] * 5 + [C.c_void_p, C.c_int64, C.c_void_p]
         L.vnm_prune_magnitude_f32.argtypes = [C.c_void_p, C.c_int64] + [C.c_int] * 5 + [C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p]
         L.vnm_prune_magnitude_f32.restype = C.c_int
+        L.vnm_sparsify_magnitude.argtypes = [C.c_void_p, C.c_int, C.c_int64] + [C.c_int] * 5 + [C.c_void_p] * 5
+        L.vnm_sparsify_magnitude.restype = C.c_int
         L.vnm_prepare.argtypes = [C.c_void_p] * 3 + [C.c_int] * 5 + [C.POINTER(C.c_void_p), C.c_void_p]
         L.vnm_prepare_as.argtypes = [C.c_void_p] * 3 + [C.c_int] * 6 + [C.POINTER(C.c_void_p), C.c_void_p]
         L.vnm_prepare_as.restype = C.c_int
@@ -174,6 +176,27 @@ def prune_magnitude(w, V, m, n=2):
     colloc = torch.empty(nc, dtype=torch.int32, device=w.device)
     _check(lib().vnm_prune_magnitude_f32(wf.data_ptr(), K, M, K, V, n, m, mask.data_ptr(), K, colloc.data_ptr(), _stream()))
     return mask, colloc
+
+
+def sparsify_magnitude(w, V, m, n=2):
+    """prune_magnitude and compress (with its mask) in one pass over the fp16 or fp32 weights w [M,K] (unit inner stride).
+    Returns (values fp16, meta int32, colloc int32, violations int), or None where the fused kernel does not apply
+    (K % m != 0, m > 64, other types).  Reading the violation count synchronises the stream."""
+    _need_cuda(w)
+    if w.dtype not in (torch.float16, torch.float32) or w.dim() != 2 or w.stride(1) != 1 or w.shape[1] % m or m > 64:
+        return None
+    M, K = w.shape
+    ksp, nv, nm, nc = sizes(M, K, V, m, n)
+    values = torch.empty(nv, dtype=torch.float16, device=w.device)
+    meta = torch.empty(nm, dtype=torch.int32, device=w.device)
+    colloc = torch.empty(nc, dtype=torch.int32, device=w.device)
+    viol = torch.zeros(1, dtype=torch.int64, device=w.device)
+    rc = lib().vnm_sparsify_magnitude(w.data_ptr(), 1 if w.dtype == torch.float16 else 0, w.stride(0), M, K, V, n, m, values.data_ptr(),
+                                      meta.data_ptr(), colloc.data_ptr(), viol.data_ptr(), _stream())
+    if rc == 3:      # VNM_ERR_UNSUPPORTED: the block does not fit
+        return None
+    _check(rc)
+    return values, meta, colloc, int(viol.item())
 
 
 def decompress(values, meta, colloc, M, K, V, m, n=2):

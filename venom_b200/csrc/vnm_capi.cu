@@ -261,6 +261,21 @@ int vnm_prune_magnitude_f32(const float *w, int64_t ldw, int M, int K, int V, in
     return VNM_OK;
 }
 
+int vnm_sparsify_magnitude(const void *w, int w_type, int64_t ldw, int M, int K, int V, int n, int m, void *values, uint32_t *meta, uint32_t *colloc,
+                           unsigned long long *violations, void *stream)
+{
+    int rc = check_format(M, K, V, n, m);
+    if (rc) return rc;
+    if (!w || !values || !meta || !colloc) return fail(VNM_ERR_BAD_ARG, "vnm_sparsify_magnitude: null pointer");
+    if (w_type != VNM_F32 && w_type != VNM_F16) return fail(VNM_ERR_BAD_ARG, "vnm_sparsify_magnitude: unknown weight type %d", w_type);
+    if (ldw < K) return fail(VNM_ERR_BAD_ARG, "vnm_sparsify_magnitude: ldw (%lld) < K (%d)", (long long)ldw, K);
+    if (((uintptr_t)values & 15) || ((uintptr_t)meta & 15) || ((uintptr_t)colloc & 15))
+        return fail(VNM_ERR_BAD_ARG, "vnm_sparsify_magnitude: values, metadata and colloc must be 16-byte aligned");
+    if (!sparsify_supported(K, V, m)) return fail(VNM_ERR_UNSUPPORTED, "vnm_sparsify_magnitude: needs K %% m == 0 and m <= 64 with a V x 4m block in shared memory (K %d, V %d, m %d)", K, V, m);
+    VNM_CUDA(launch_sparsify(w, w_type == VNM_F16, ldw, M, K, V, m, values, meta, colloc, violations, (cudaStream_t)stream), "sparsify launch");
+    return VNM_OK;
+}
+
 int vnm_decompress_f16(const void *values, const uint32_t *meta, const uint32_t *colloc, int M, int K, int V, int n, int m,
                        void *dense, int64_t ldd, void *stream)
 {

@@ -95,6 +95,11 @@ cudaError_t launch_transpose(const void *src, int64_t ld_src, int N, int K, void
 cudaError_t launch_prune(const float *w, int64_t ldw, int M, int K, int V, int m, int32_t *mask, int64_t ldm, uint32_t *colloc,
                          cudaStream_t stream);
 
+// Pruner and compressor in one pass over the weights (fp16 or fp32).
+bool sparsify_supported(int K, int V, int m);
+cudaError_t launch_sparsify(const void *w, bool half, int64_t ldw, int M, int K, int V, int m, void *values, uint32_t *meta, uint32_t *colloc,
+                            unsigned long long *violations, cudaStream_t stream);
+
 // Tile configuration of the gather kernel.
 float spmm_select_config(int V, int N, int M, int ktiles, int max_ctas, SpmmConfig *cfg);  // max_ctas: 0 = one per SM; returns an estimate in microseconds, < 0 for an unsupported V
 // Opt-in to large dynamic shared memory for every kernel instance on the CURRENT device (call once per device).

@@ -39,6 +39,18 @@ class SrNMTensor:
         self.values, self.metadata, self.violations = capi.compress(d, self.columns, tileM_, m_, n_, mask=mask)
         self._prepared = None
 
+    @classmethod
+    def from_arrays(cls, n_, m_, tileM_, shape, values, metadata, columns, violations):
+        """The tensor of arrays that are compressed already (on a CUDA device)."""
+        t = cls.__new__(cls)
+        t.n, t.m, t.tileM = n_, m_, tileM_
+        t.device = values.device
+        t.nrows, t.ncols = shape
+        t.nnz = values.numel()
+        t.values, t.metadata, t.columns, t.violations = values, metadata, columns, violations
+        t._prepared = None
+        return t
+
     def prepared(self):
         if self._prepared is None:
             self._prepared = capi.Prepared(self.values, self.metadata, self.columns, self.nrows, self.ncols, self.tileM, self.m, self.n)
@@ -62,7 +74,11 @@ class MagnitudeSparsifier:
 
     def __call__(self, tensor, device=None):
         device = tensor.device if device is None else device
-        mask, columns = nm_vector_mask_sparsify(tensor.to(device), self.n, self.m, self.tileM)
+        w = tensor.detach().to(device)
+        fused = capi.sparsify_magnitude(w, self.tileM, self.m, self.n)     # prunes and compresses in one pass
+        if fused is not None:
+            return SrNMTensor.from_arrays(self.n, self.m, self.tileM, tuple(tensor.shape), *fused)
+        mask, columns = nm_vector_mask_sparsify(w, self.n, self.m, self.tileM)
         dense = tensor.detach().to(device=device, dtype=torch.float16) * mask.to(torch.float16)
         return SrNMTensor(self.n, self.m, self.tileM, dense, mask, columns, device)
 
