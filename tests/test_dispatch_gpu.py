@@ -1,0 +1,98 @@
+"""The kernels and call paths that the dispatch picks by size, at the edges of their tiles, against a dense product of
+whole numbers (exact in every order of summation)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _operand(M, K, V, m, strategy, seed):
+    import torch
+    from venom_b200 import capi
+    from venom_b200.synth import random_vnm_dense
+    dense, cols, _ = random_vnm_dense(M, K, V, m, seed=seed, integer_values=True)
+    d = torch.from_numpy(dense).cuda()
+    c = torch.from_numpy(cols.view(np.int32)).cuda()
+    values, meta, bad = capi.compress(d, c, V, m)
+    assert bad == 0
+    return d.float(), values, meta, c, capi.Prepared(values, meta, c, M, K, V, m, strategy=strategy)
+
+
+def _ints(shape, seed):
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    return torch.randint(-4, 5, shape, generator=g, device="cuda").half()
+
+
+# Few columns: tile widths 16 .. 128 and their edges; k-tiles that split evenly, raggedly and not at all; ragged rows.
+@pytest.mark.parametrize("N", [8, 16, 24, 32, 40, 64, 72, 136])
+@pytest.mark.parametrize("cfg", [(128, 1024, 128, 16), (96, 520, 32, 8), (192, 2048, 64, 8), (704, 4480, 64, 32), (128, 512, 128, 4)])
+@pytest.mark.parametrize("form", ["gather", "dense_b"])
+def test_few_columns(N, cfg, form):
+    import torch
+    from venom_b200 import capi
+    M, K, V, m = cfg
+    d, _, _, _, prep = _operand(M, K, V, m, capi.STRATEGY_GATHER if form == "gather" else capi.STRATEGY_DENSE_B, seed=M + K)
+    B = _ints((K, N), N)
+    bias = _ints((M,), 3)
+    want = d @ B.float()
+    assert torch.equal(prep.spmm(B), want.half())
+    assert torch.equal(prep.spmm(B, bias=bias, layout=capi.VNM_LAYOUT_NM), (want.half() + bias[:, None]).T)
+    if form == "dense_b":
+        assert torch.equal(prep.spmm_nk(B.T.contiguous()), want.half().T)
+    assert prep.device_status() == 0
+
+
+# SM pairs: row tiles that do not fill the last pair (or group of four), fewer columns than a box, ragged columns.
+@pytest.mark.parametrize("rows", [3, 4])
+@pytest.mark.parametrize("cfg", [(128, 512, 128, 8, 248), (384, 264, 64, 8, 480), (640, 1152, 32, 16, 1000), (896, 1024, 64, 8, 72)])
+def test_odd_row_tiles_on_sm_pairs(cfg, rows):
+    import torch
+    from venom_b200 import capi
+    M, K, V, m, N = cfg
+    d, _, _, _, prep = _operand(M, K, V, m, capi.STRATEGY_DENSE_B, seed=M + N)
+    prep.set_pair_mode(rows)
+    B = _ints((K, N), N)
+    want = (d @ B.float()).half()
+    assert torch.equal(prep.spmm(B), want)
+    assert torch.equal(prep.spmm(B, layout=capi.VNM_LAYOUT_NM), want.T)
+    assert torch.equal(prep.spmm_nk(B.T.contiguous()), want.T)
+    assert prep.device_status() == 0
+
+
+# A layer reads its input as it lies ([tokens, features], any leading dimensions) in either form, and goes through the copying
+# path for one that it cannot read in place; edits of the arrays are seen by the next call.
+@pytest.mark.parametrize("cfg", [(256, 512, 128, 16, (3, 8)), (96, 520, 32, 8, (1368,)), (1024, 1024, 64, 8, (2, 4, 8)), (384, 640, 128, 16, (1000,)), (128, 120, 64, 10, (8,))])
+def test_layer_reads_its_input_in_place(cfg):
+    import torch
+    from venom_b200.nmv import SrnmSpmm
+    M, K, V, m, lead = cfg
+    d, values, meta, c, _ = _operand(M, K, V, m, None, seed=M + K)
+    layer = SrnmSpmm(torch.nn.Linear(K, M).half().cuda(), 2, m, V)
+    layer.values.data.copy_(values.reshape(-1))
+    layer.metadata, layer.columns = meta, c
+    layer.bias.data.copy_(_ints((M,), 5))
+    x = _ints(lead + (K,), 7)
+    want = ((x.reshape(-1, K).float() @ d.T).half() + layer.bias).reshape(lead + (M,))
+    assert torch.equal(layer(x), want)
+    wide = torch.zeros(lead + (K + 8,), dtype=torch.float16, device="cuda")
+    wide[..., 8:] = x
+    assert torch.equal(layer(wide[..., 8:]), want)
+    layer.values.data.mul_(2)
+    layer.values.add_(0)                       # an in-place edit that autograd counts
+    assert torch.equal(layer(x), (((want - layer.bias).float() * 2).half() + layer.bias))
+
+
+def test_product_reports_errors_as_before():
+    import torch
+    from venom_b200 import capi
+    _, _, _, _, prep = _operand(128, 256, 64, 8, None, seed=1)
+    for bad in (_ints((256, 12), 1), _ints((128, 16), 1), _ints((256, 16), 1).float(), _ints((16, 256), 1).T, _ints((256, 16), 1).cpu()):
+        with pytest.raises(capi.VenomError):
+            prep.spmm(bad)
+    with pytest.raises(capi.VenomError):
+        prep.spmm(_ints((256, 16), 1), bias=_ints((128,), 1))            # a bias needs layout NM
+    prep.close()
+    with pytest.raises(capi.VenomError):
+        prep.spmm(_ints((256, 16), 1))

@@ -207,6 +207,19 @@ def decompress(values, meta, colloc, M, K, V, m, n=2):
     return dense
 
 
+def _load_product():
+    """The extension's vnm_spmm_f16 call (checks, allocation and launch without the interpreter between them); None if the
+    extension has not been built -- the ctypes path below does the same."""
+    try:
+        from . import spatha_module
+        return spatha_module().product
+    except ImportError:
+        return None
+
+
+_product = None
+
+
 class Prepared:
     """Owns a vnm_handle_t: the kernel-private copy of one sparse operand."""
 
@@ -220,6 +233,9 @@ class Prepared:
             raise VenomError("values must be fp16, metadata and colloc 32-bit")
         self.M, self.K, self.V, self.m, self.n = M, K, V, m, n
         self.device = values.device
+        global _product
+        if _product is None:
+            _product = _load_product()
         self._h = C.c_void_p()
         if strategy is None:
             _check(lib().vnm_prepare(values.data_ptr(), meta.data_ptr(), colloc.data_ptr(), M, K, V, n, m,
@@ -241,6 +257,10 @@ class Prepared:
 
     def spmm(self, B, bias=None, layout=VNM_LAYOUT_MN, out=None):
         """B: [K,N] fp16 CUDA (unit inner stride).  Returns [M,N] (layout MN) or [N,M] (layout NM)."""
+        if out is None and _product is not None and isinstance(B, torch.Tensor):
+            out = _product(self._h.value or 0, B, bias, self.M, self.K, layout)
+            if out is not None:
+                return out
         _need_cuda(B, bias, out)
         if B.dtype != torch.float16 or B.dim() != 2 or B.shape[0] != self.K or B.stride(1) != 1:
             raise VenomError("B must be a [K,N] fp16 tensor with unit inner stride (K=%d)" % self.K)

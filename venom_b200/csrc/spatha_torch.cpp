@@ -40,6 +40,7 @@ struct Entry {
     // the operand re-packed per form (VNM_STRATEGY_GATHER, VNM_STRATEGY_DENSE_B), each when a call first wants it
     vnm_handle_t handle[2];
     int last_n, last_t, last_form;   // the form of the last shape of call
+    int64_t nv, nm, nc;              // sizes of the three arrays
     WeakStorage values, meta, idx;   // the storages the operand was re-packed from
     void release()
     {
@@ -79,6 +80,79 @@ void check(int rc, const char *what)
     TORCH_CHECK(rc == 0, what, " failed (", rc, "): ", vnm_last_error_string());
 }
 
+void check_sizes(const torch::Tensor &A_metadata, const torch::Tensor &A_indices, const torch::Tensor &A_values, int64_t nv, int64_t nm, int64_t nc)
+{
+    TORCH_CHECK(A_values.numel() == nv && A_metadata.numel() == nm && A_indices.numel() == nc, "spatha.spmm: array sizes do not match the format (values ",
+                nv, ", metadata ", nm, ", indices ", nc, ")");
+}
+
+// The handle that multiplies N columns: looked up in (or added to) the cache, in the form estimated to be the faster one
+// for this number of columns and the layout of the activation.  `dense_b` receives that form.
+vnm_handle_t operand_for(const torch::Tensor &A_metadata, const torch::Tensor &A_indices, const torch::Tensor &A_values, int M, int K, int V, int n, int m,
+                         int device, int N, bool in_place, cudaStream_t stream, int *dense_b)
+{
+    Key key{A_values.data_ptr(), A_metadata.data_ptr(), A_indices.data_ptr(), M, K, V, n, m, device,
+            (uint32_t)A_values._version(), (uint32_t)A_metadata._version(), (uint32_t)A_indices._version()};
+    std::lock_guard<std::mutex> lock(g_mutex);
+    auto it = g_cache.find(key);
+    if (it != g_cache.end() && !(same_storage(it->second.values, A_values) && same_storage(it->second.meta, A_metadata) &&
+                                 same_storage(it->second.idx, A_indices))) {
+        // same addresses, different (or freed) tensors: the cached copy belongs to an operand that is gone
+        it->second.release();
+        g_cache.erase(it);
+        it = g_cache.end();
+    }
+    if (it == g_cache.end()) {
+        int64_t ksp = 0, nv = 0, nm = 0, nc = 0;
+        check(vnm_sizes(M, K, V, n, m, &ksp, &nv, &nm, &nc), "vnm_sizes");
+        check_sizes(A_metadata, A_indices, A_values, nv, nm, nc);
+        sweep_dead_entries();
+        it = g_cache.emplace(key, Entry{{nullptr, nullptr}, -1, 0, 0, nv, nm, nc, weak_of(A_values), weak_of(A_metadata), weak_of(A_indices)}).first;
+    }
+    check_sizes(A_metadata, A_indices, A_values, it->second.nv, it->second.nm, it->second.nc);
+    // Dense-B form or gather form: by the estimate for this number of columns and the layout of the activation (a
+    // transposed [tokens, features] view is read in place by the dense-B form and transposed for the gather form).
+    Entry &e = it->second;
+    if (e.last_n != N || e.last_t != (int)in_place) {
+        int strategy = 0;
+        check(vnm_choose_form(M, K, V, n, m, N, in_place ? 1 : 0, &strategy), "vnm_choose_form");
+        e.last_form = strategy == VNM_STRATEGY_DENSE_B ? 1 : 0;
+        e.last_n = N;
+        e.last_t = in_place;
+    }
+    *dense_b = e.last_form;
+    vnm_handle_t &h = e.handle[e.last_form];
+    if (!h)
+        check(vnm_prepare_as(A_values.data_ptr(), (const uint32_t *)A_metadata.data_ptr(), (const uint32_t *)A_indices.data_ptr(), M, K, V, n, m,
+                             *dense_b ? VNM_STRATEGY_DENSE_B : VNM_STRATEGY_GATHER, &h, stream), "vnm_prepare_as");
+    return h;
+}
+
+void check_arrays(const torch::Tensor &A_metadata, const torch::Tensor &A_indices, const torch::Tensor &A_values, const torch::Tensor &rhs)
+{
+    TORCH_CHECK(A_values.is_cuda() && A_metadata.is_cuda() && A_indices.is_cuda() && rhs.is_cuda(), "spatha.spmm: CUDA tensors expected");
+    TORCH_CHECK(A_values.scalar_type() == torch::kFloat16 && rhs.scalar_type() == torch::kFloat16, "spatha.spmm: fp16 values / rhs expected");
+    TORCH_CHECK(A_metadata.scalar_type() == torch::kInt32 && A_indices.scalar_type() == torch::kInt32, "spatha.spmm: int32 metadata / indices expected");
+    TORCH_CHECK(A_values.is_contiguous() && A_metadata.is_contiguous() && A_indices.is_contiguous(), "spatha.spmm: contiguous sparse arrays expected");
+}
+
+// The bias as a pointer, null if there is none.
+const void *bias_pointer(const c10::optional<torch::Tensor> &bias, int M)
+{
+    if (!(bias.has_value() && bias->defined() && bias->numel() > 0)) return nullptr;
+    TORCH_CHECK(bias->is_cuda() && bias->scalar_type() == torch::kFloat16 && bias->numel() == M && bias->is_contiguous(), "spatha.spmm: bias must be fp16 [A_num_rows]");
+    return bias->data_ptr();
+}
+
+// out [N, M] = (A * B).T + bias for an activation that lies as [N, K] rows of stride `ld` (16-byte aligned).
+void product_nk(vnm_handle_t h, int dense_b, const torch::Tensor &act, int64_t ld, int K, int N, int M, const void *bias, torch::Tensor &out, cudaStream_t stream)
+{
+    torch::Tensor ws;
+    if (!dense_b) ws = torch::empty({K, N}, act.options());
+    check(vnm_spmm_f16_nk_ws(h, act.data_ptr(), ld, N, bias, out.data_ptr(), M, VNM_LAYOUT_NM, dense_b ? out.data_ptr() : ws.data_ptr(), stream),
+          "vnm_spmm_f16_nk");
+}
+
 }  // namespace
 
 torch::Tensor spmm(torch::Tensor A_metadata, torch::Tensor A_indices, torch::Tensor A_values, torch::Tensor rhs_matrix,
@@ -86,72 +160,72 @@ torch::Tensor spmm(torch::Tensor A_metadata, torch::Tensor A_indices, torch::Ten
                    int64_t vec_length, int64_t n, int64_t m, int64_t nnz, int64_t seed, int64_t mbrow, int64_t brow)
 {
     (void)seed;
-    TORCH_CHECK(A_values.is_cuda() && A_metadata.is_cuda() && A_indices.is_cuda() && rhs_matrix.is_cuda(), "spatha.spmm: CUDA tensors expected");
-    TORCH_CHECK(A_values.scalar_type() == torch::kFloat16 && rhs_matrix.scalar_type() == torch::kFloat16, "spatha.spmm: fp16 values / rhs expected");
-    TORCH_CHECK(A_metadata.scalar_type() == torch::kInt32 && A_indices.scalar_type() == torch::kInt32, "spatha.spmm: int32 metadata / indices expected");
+    check_arrays(A_metadata, A_indices, A_values, rhs_matrix);
     TORCH_CHECK(mbrow == 32 && brow == 4, "spatha.spmm: the storage format is defined for mbrow = 32, brow = 4");
-    TORCH_CHECK(A_values.is_contiguous() && A_metadata.is_contiguous() && A_indices.is_contiguous(), "spatha.spmm: contiguous sparse arrays expected");
     const int M = (int)A_num_rows, K = (int)A_num_cols, N = (int)B_num_cols, V = (int)vec_length;
     int64_t ksp = 0, nv = 0, nm = 0, nc = 0;
     check(vnm_sizes(M, K, V, (int)n, (int)m, &ksp, &nv, &nm, &nc), "vnm_sizes");
-    TORCH_CHECK(A_values.numel() == nv && A_metadata.numel() == nm && A_indices.numel() == nc, "spatha.spmm: array sizes do not match the format (values ",
-                nv, ", metadata ", nm, ", indices ", nc, ")");
     TORCH_CHECK(nnz == nv, "spatha.spmm: nnz must be A_num_rows * padded compressed columns (", nv, ")");
     TORCH_CHECK(rhs_matrix.dim() == 2 && rhs_matrix.size(0) == K && rhs_matrix.size(1) == N, "spatha.spmm: rhs_matrix must be [A_num_cols, B_num_cols]");
     // A transposed view of a [B_num_cols, A_num_cols] activation (what `flattened_input.T` is) is consumed as it lies;
     // any other non-contiguous rhs is copied like the reference does.
     const bool rhs_is_t_view = rhs_matrix.stride(0) == 1 && rhs_matrix.stride(1) >= K && N > 1;
-    const bool has_bias = bias.has_value() && bias->defined() && bias->numel() > 0;
-    if (has_bias) TORCH_CHECK(bias->is_cuda() && bias->scalar_type() == torch::kFloat16 && bias->numel() == M && bias->is_contiguous(), "spatha.spmm: bias must be fp16 [A_num_rows]");
+    const void *bias_ptr = bias_pointer(bias, M);
 
     c10::cuda::CUDAGuard guard(rhs_matrix.device());
     cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
-    Key key{A_values.data_ptr(), A_metadata.data_ptr(), A_indices.data_ptr(), M, K, V, (int)n, (int)m, (int)rhs_matrix.device().index(),
-            (uint32_t)A_values._version(), (uint32_t)A_metadata._version(), (uint32_t)A_indices._version()};
-    vnm_handle_t h = nullptr;
     int dense_b = 0;
     const bool in_place = rhs_is_t_view && rhs_matrix.stride(1) % 8 == 0 && (reinterpret_cast<uintptr_t>(rhs_matrix.data_ptr()) & 15) == 0;
-    {
-        std::lock_guard<std::mutex> lock(g_mutex);
-        auto it = g_cache.find(key);
-        if (it != g_cache.end() && !(same_storage(it->second.values, A_values) && same_storage(it->second.meta, A_metadata) &&
-                                     same_storage(it->second.idx, A_indices))) {
-            // same addresses, different (or freed) tensors: the cached copy belongs to an operand that is gone
-            it->second.release();
-            g_cache.erase(it);
-            it = g_cache.end();
-        }
-        if (it == g_cache.end()) {
-            sweep_dead_entries();
-            it = g_cache.emplace(key, Entry{{nullptr, nullptr}, -1, 0, 0, weak_of(A_values), weak_of(A_metadata), weak_of(A_indices)}).first;
-        }
-        // Dense-B form or gather form: by the estimate for this number of columns and the layout of the activation (a
-        // transposed [tokens, features] view is read in place by the dense-B form and transposed for the gather form).
-        Entry &e = it->second;
-        if (e.last_n != N || e.last_t != (int)in_place) {
-            int strategy = 0;
-            check(vnm_choose_form(M, K, V, (int)n, (int)m, N, in_place ? 1 : 0, &strategy), "vnm_choose_form");
-            e.last_form = strategy == VNM_STRATEGY_DENSE_B ? 1 : 0;
-            e.last_n = N;
-            e.last_t = in_place;
-        }
-        dense_b = e.last_form;
-        if (!e.handle[dense_b])
-            check(vnm_prepare_as(A_values.data_ptr(), (const uint32_t *)A_metadata.data_ptr(), (const uint32_t *)A_indices.data_ptr(), M, K, V,
-                                 (int)n, (int)m, dense_b ? VNM_STRATEGY_DENSE_B : VNM_STRATEGY_GATHER, &e.handle[dense_b], stream), "vnm_prepare_as");
-        h = e.handle[dense_b];
-    }
+    vnm_handle_t h = operand_for(A_metadata, A_indices, A_values, M, K, V, (int)n, (int)m, (int)rhs_matrix.device().index(), N, in_place, stream, &dense_b);
     auto out = torch::empty({N, M}, rhs_matrix.options());
-    const void *bias_ptr = has_bias ? bias->data_ptr() : nullptr;
     if (in_place) {
-        torch::Tensor ws;
-        if (!dense_b) ws = torch::empty({K, N}, rhs_matrix.options());
-        check(vnm_spmm_f16_nk_ws(h, rhs_matrix.data_ptr(), rhs_matrix.stride(1), N, bias_ptr, out.data_ptr(), M, VNM_LAYOUT_NM,
-                                 dense_b ? out.data_ptr() : ws.data_ptr(), stream), "vnm_spmm_f16_nk");
+        product_nk(h, dense_b, rhs_matrix, rhs_matrix.stride(1), K, N, M, bias_ptr, out, stream);
         return out;
     }
     torch::Tensor rhs = rhs_matrix.stride(1) == 1 ? rhs_matrix : rhs_matrix.contiguous();
     check(vnm_spmm_f16(h, rhs.data_ptr(), rhs.stride(0), N, bias_ptr, out.data_ptr(), M, VNM_LAYOUT_NM, stream), "vnm_spmm_f16");
+    return out;
+}
+
+// A layer's forward in one call: input [..., A_num_cols] -> [..., A_num_rows], as spmm() on the flattened input's transpose gives
+// it, without the views that call needs (each a trip through the dispatcher; at decoding sizes these and the interpreter's
+// share of the call took longer than the product: measured 12.2 us a call before, 6.3 after, for a kernel of 5 us).  An undefined
+// result (None) means: an input that is not read in place -- take spmm().
+c10::optional<torch::Tensor> linear(const torch::Tensor &input, const torch::Tensor &A_metadata, const torch::Tensor &A_indices, const torch::Tensor &A_values,
+                                    const c10::optional<torch::Tensor> &bias, int64_t A_num_rows, int64_t A_num_cols, int64_t vec_length, int64_t n, int64_t m)
+{
+    const int M = (int)A_num_rows, K = (int)A_num_cols;
+    const int64_t dims = input.dim();
+    if (dims < 2 || K <= 0 || K % 8 != 0 || input.size(-1) != K || !input.is_contiguous()) return c10::nullopt;
+    const int64_t N = input.numel() / K;
+    if (N <= 1 || N > INT32_MAX || (reinterpret_cast<uintptr_t>(input.data_ptr()) & 15) != 0) return c10::nullopt;
+    check_arrays(A_metadata, A_indices, A_values, input);
+    const void *bias_ptr = bias_pointer(bias, M);
+    c10::cuda::CUDAGuard guard(input.device());
+    cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
+    int dense_b = 0;
+    vnm_handle_t h = operand_for(A_metadata, A_indices, A_values, M, K, (int)vec_length, (int)n, (int)m, (int)input.device().index(), (int)N, true, stream, &dense_b);
+    c10::SmallVector<int64_t, 6> shape(input.sizes().begin(), input.sizes().end());
+    shape.back() = M;
+    auto out = torch::empty(shape, input.options());
+    product_nk(h, dense_b, input, K, K, (int)N, M, bias_ptr, out, stream);
+    return out;
+}
+
+// capi.Prepared.spmm's call of vnm_spmm_f16 with its allocation, without the interpreter's share (attribute reads, argument
+// boxing, and 3.4 us for torch.cuda.current_stream alone).  None: not the plain case, or an error that the caller's own path reports.
+c10::optional<torch::Tensor> product(int64_t handle, const torch::Tensor &B, const c10::optional<torch::Tensor> &bias, int64_t M, int64_t K, int64_t layout)
+{
+    if (!handle || !B.is_cuda() || B.scalar_type() != torch::kFloat16 || B.dim() != 2 || B.size(0) != K || B.stride(1) != 1) return c10::nullopt;
+    if (bias.has_value() && (!bias->defined() || !bias->is_cuda() || bias->scalar_type() != torch::kFloat16 || bias->numel() != M || !bias->is_contiguous()))
+        return c10::nullopt;
+    if ((layout != VNM_LAYOUT_MN && layout != VNM_LAYOUT_NM) || B.device().index() != c10::cuda::current_device()) return c10::nullopt;
+    const int64_t N = B.size(1);
+    if (N <= 0 || N > INT32_MAX) return c10::nullopt;
+    auto out = layout == VNM_LAYOUT_MN ? torch::empty({M, N}, B.options()) : torch::empty({N, M}, B.options());
+    if (vnm_spmm_f16(reinterpret_cast<vnm_handle_t>(handle), B.data_ptr(), B.stride(0), (int)N, bias.has_value() ? bias->data_ptr() : nullptr, out.data_ptr(),
+                     out.stride(0), (int)layout, c10::cuda::getCurrentCUDAStream().stream()) != 0)
+        return c10::nullopt;
     return out;
 }
 
@@ -174,6 +248,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, mod)
             pybind11::arg("A_values"), pybind11::arg("rhs_matrix"), pybind11::arg("bias"), pybind11::arg("A_num_rows"), pybind11::arg("A_num_cols"),
             pybind11::arg("B_num_cols"), pybind11::arg("vec_length"), pybind11::arg("n"), pybind11::arg("m"), pybind11::arg("nnz"),
             pybind11::arg("seed"), pybind11::arg("mbrow"), pybind11::arg("brow"));
+    mod.def("linear", &linear, "A layer's forward: [..., A_num_cols] -> [..., A_num_rows], or None", pybind11::call_guard<pybind11::gil_scoped_release>());
+    mod.def("product", &product, "vnm_spmm_f16 with its allocation, or None", pybind11::call_guard<pybind11::gil_scoped_release>());
     mod.def("clear_cache", &clear_cache, "Drop every cached prepared operand");
     mod.def("cache_size", &cache_size);
 }

@@ -160,17 +160,6 @@ struct vnm_prepared_s {
     void *am;
     void *rows;
     int *status;
-    // cached TMA descriptors of the last dense operand: single rows (for gather4) and 64-row tiles
-    const void *tm_B;
-    int64_t tm_ldb;
-    int tm_N;
-    int tm_nk;
-    int tm_kind;             // the kernel (and, for the small one, the tile width) that the cached maps belong to
-    bool tm_valid;
-    CUtensorMap tmap_rows;
-    CUtensorMap tmap_tile;
-    CUtensorMap tmap_tile2;  // dense-B kernel: 2-D map for the ragged right edge
-    bool tm_wide;            // tmap_tile is the 4-D one-box-per-stage map
     // device staging of the host-buffer entry point
     void *stage_B;
     size_t stage_B_bytes;
@@ -564,27 +553,28 @@ static int spmm_impl(vnm_handle_t h, const void *B, int64_t ldb, int N, int b_nk
     float us;
     if (!choose_kernel(h, N, n_more, &kernel, &cfg, &us)) return fail(VNM_ERR_UNSUPPORTED, "vnm_spmm_f16: no kernel for this operand and its switches");
     const bool pair = kernel == KERNEL_PAIR;
-    const int kind = kernel == KERNEL_SMALL ? 1000 * h->gather_mode + cfg.bn : -(int)kernel;
     EncodeTiledFn enc = get_encode_fn();
     if (!enc) return fail(VNM_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
 
-    if (!h->tm_valid || h->tm_B != B || h->tm_ldb != ldb || h->tm_N != N || h->tm_nk != b_nk || h->tm_kind != kind) {
+    // Tensor maps of this call's dense operand (0.1 us each to encode; kept nowhere, so that threads may share a handle):
+    // single rows (for gather4), tiles, and for the pair kernel 2-D tiles for the ragged right edge.
+    CUtensorMap tmap_rows, tmap_tile, tmap_tile2;
+    bool tm_wide = false;            // tmap_tile is the 4-D one-box-per-stage map
+    {
         cuuint32_t estr[2] = {1, 1};
         CUresult r;
         if (kernel == KERNEL_SMALL) {
-            r = spmm_small_encode(enc, &h->tmap_tile, B, ldb, h->K, N, b_nk, h->gather_mode, cfg.bn);
-            h->tm_wide = false;
+            r = spmm_small_encode(enc, &tmap_tile, B, ldb, h->K, N, b_nk, h->gather_mode, cfg.bn);
         } else if (b_nk) {
             cuuint64_t dims[2] = {(cuuint64_t)h->K, (cuuint64_t)N};
             cuuint64_t strides[1] = {(cuuint64_t)ldb * 2};
             // B given as [N, K] (K contiguous): a CTA of the pair loads its 128 n-rows, 64 k (two MMA K blocks, 128-byte rows) per box
             cuuint32_t box[2] = {64, 128};
-            r = enc(&h->tmap_tile, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(B), dims, strides, box, estr,
+            r = enc(&tmap_tile, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(B), dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-            h->tmap_rows = h->tmap_tile;
-            h->tmap_tile2 = h->tmap_tile;
-            h->tm_wide = false;
+            tmap_rows = tmap_tile;
+            tmap_tile2 = tmap_tile;
         } else {
             // B viewed as a 2-D tensor {N (contiguous), K}; one box = 64 columns (128 bytes) of one row
             // (gather4 picks four such rows) or of 32 consecutive rows (64 for the pair kernel), written with
@@ -593,15 +583,14 @@ static int spmm_impl(vnm_handle_t h, const void *B, int64_t ldb, int N, int b_nk
             cuuint64_t strides[1] = {(cuuint64_t)ldb * 2};
             cuuint32_t box_rows[2] = {64, 1};
             cuuint32_t box_tile[2] = {64, pair ? 64u : 32u};
-            r = enc(&h->tmap_rows, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(B), dims, strides, box_rows, estr,
+            r = enc(&tmap_rows, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(B), dims, strides, box_rows, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
             if (r == CUDA_SUCCESS)
-                r = enc(&h->tmap_tile, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(B), dims, strides, box_tile, estr,
+                r = enc(&tmap_tile, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(B), dims, strides, box_tile, estr,
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-            h->tmap_tile2 = h->tmap_tile;
-            h->tm_wide = false;
+            tmap_tile2 = tmap_tile;
             if (r == CUDA_SUCCESS && pair && N >= 128) {
                 // pair kernel: a CTA's half of a stage is {64 columns, 64 rows, 2 slices} starting at any multiple of 8 columns
                 // (pair tiles start at multiples of 240, the peer's half 120 columns further)
@@ -613,13 +602,12 @@ static int spmm_impl(vnm_handle_t h, const void *B, int64_t ldb, int N, int b_nk
                 if (enc(&wide, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<void *>(B), dims4, strides4, box4, estr4,
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS) {
-                    h->tmap_tile = wide;
-                    h->tm_wide = true;
+                    tmap_tile = wide;
+                    tm_wide = true;
                 }
             }
         }
         if (r != CUDA_SUCCESS) return fail(VNM_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
-        h->tm_B = B; h->tm_ldb = ldb; h->tm_N = N; h->tm_nk = b_nk; h->tm_kind = kind; h->tm_valid = true;
     }
 
     SpmmParams p;
@@ -661,7 +649,7 @@ static int spmm_impl(vnm_handle_t h, const void *B, int64_t ldb, int N, int b_nk
     }
     p.hybrid_rows = h->hybrid_rows;
     p.b_nk = b_nk;
-    p.b_wide_ok = h->tm_wide ? 1 : 0;
+    p.b_wide_ok = tm_wide ? 1 : 0;
     p.l2_ahead = h->l2_ahead;
     p.n_out = 1;
     p.tma_out = 1;
@@ -672,19 +660,19 @@ static int spmm_impl(vnm_handle_t h, const void *B, int64_t ldb, int N, int b_nk
         p.tma_out = 0;
         p.split_k = cfg.split;
         p.early = after_transpose ? 1 : 0;
-        VNM_CUDA(launch_spmm_small(cfg, h->tmap_tile, p, (cudaStream_t)stream), "spmm launch");
+        VNM_CUDA(launch_spmm_small(cfg, tmap_tile, p, (cudaStream_t)stream), "spmm launch");
     } else if (h->dense_b) {
-        // The result leaves through TMA stores: [M,N] as boxes of 40 columns x 128 rows, [N,M] as boxes of 128
-        // columns (m) x 40 rows (n).
+        // Several destinations leave through TMA stores: [M,N] as boxes of 40 columns x 128 rows, [N,M] as boxes of 128
+        // columns (m) x 40 rows (n); a single one needs no map.
         CUtensorMap tmap_out;
         OutMaps more;
-        memset(&more, 0, sizeof(more));
-        for (int d = 0; d <= n_more; d++) {
+        if (n_more > 0) memset(&more, 0, sizeof(more));
+        for (int d = 0; n_more > 0 && d <= n_more; d++) {
             CUresult r = encode_out_map(enc, d == 0 ? &tmap_out : &more.m[d - 1], d == 0 ? out : more_outs[d - 1], h->M, N, ldo, layout, cfg.part);
             if (r != CUDA_SUCCESS) return fail(VNM_ERR_CUDA, "cuTensorMapEncodeTiled (output %d) failed with CUresult %d", d, (int)r);
         }
         p.n_out = 1 + n_more;
-        VNM_CUDA(launch_spmm_dense_b_pair(cfg, h->tmap_tile, h->tmap_tile2, tmap_out, more, p, (cudaStream_t)stream), "spmm launch");
+        VNM_CUDA(launch_spmm_dense_b_pair(cfg, tmap_tile, tmap_tile2, tmap_out, more, p, (cudaStream_t)stream), "spmm launch");
     } else {
         // Gather form: the epilogue stores straight from tensor memory.  Only a [N,M] result with several destinations (or on
         // request) leaves through shared memory and TMA stores, boxes of 128 columns (m) x cfg.part rows (n).
@@ -703,7 +691,7 @@ static int spmm_impl(vnm_handle_t h, const void *B, int64_t ldb, int N, int b_nk
         } else if (n_more > 0) {
             return fail(VNM_ERR_UNSUPPORTED, "vnm_spmm_f16_multi: the register-store epilogue of the gather form writes one destination");
         }
-        VNM_CUDA(launch_spmm(cfg, h->tmap_rows, h->tmap_tile, tmap_out, more, p, (cudaStream_t)stream), "spmm launch");
+        VNM_CUDA(launch_spmm(cfg, tmap_rows, tmap_tile, tmap_out, more, p, (cudaStream_t)stream), "spmm launch");
     }
     return VNM_OK;
 }

@@ -399,11 +399,11 @@ float spmm_small_config(int mtiles, int ktiles, int N, int nb, bool gather, Spmm
         VNM_SMALL_DISPATCH(bn, nb, VNM_FILL);
 #undef VNM_FILL
         const float kt_us = (gather ? gather_kt[w] : dense_kt[w]) * (nb == 4 ? 1.4f : nb == 2 ? 1.15f : 1.0f);
-        const long long tiles = (long long)mtiles * ((N + bn - 1) / bn);
+        const int tiles = mtiles * ((N + bn - 1) / bn);
         for (int split = 1; split <= 8 && split <= ktiles; split++) {
-            const long long ctas = tiles * split, per = (ctas + sms - 1) / sms;
+            const int ctas = tiles * split, per = (ctas + sms - 1) / sms;
             const int kts = (ktiles + split - 1) / split;
-            const int both = (int)(per < c.resident ? per : c.resident);      // CTAs that share an SM
+            const int both = per < c.resident ? per : c.resident;      // CTAs that share an SM
             float t = fixed[w] + (gather && nb > 1 ? 1.4f : 0.0f) + (split > 1 ? 0.3f + 0.006f * bn : 0.0f);
             if (per <= c.resident) {
                 t += 2.2f * (both - 1) + kts * kt_us * (1.0f + 0.45f * (both - 1));
@@ -419,7 +419,7 @@ float spmm_small_config(int mtiles, int ktiles, int N, int nb, bool gather, Spmm
                 cfg->part = bn;
                 cfg->stages = 1;
                 cfg->split = split;
-                cfg->grid = (int)ctas;
+                cfg->grid = ctas;
             }
             if (N > SMALL_SPLIT_N) break;
         }
