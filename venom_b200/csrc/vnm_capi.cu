@@ -446,7 +446,7 @@ enum Kernel { KERNEL_GATHER, KERNEL_PAIR, KERNEL_SMALL };
 
 // Which kernel multiplies this operand with N columns, and its configuration: the one with the smallest estimate (in
 // microseconds, stored in *us).  False if none can.
-bool choose_kernel(vnm_handle_t h, int N, int n_more, Kernel *kernel, SpmmConfig *cfg, float *us)
+bool choose_kernel(vnm_handle_t h, int N, int b_nk, int n_more, Kernel *kernel, SpmmConfig *cfg, float *us)
 {
     memset(cfg, 0, sizeof(*cfg));
     float big = -1.0f;
@@ -454,7 +454,7 @@ bool choose_kernel(vnm_handle_t h, int N, int n_more, Kernel *kernel, SpmmConfig
         big = spmm_select_config(h->V, N, h->M, h->ktiles, h->max_ctas, cfg);
         *kernel = KERNEL_GATHER;
     } else {
-        if (h->pair_mode || n_more > 0) big = spmm_dense_b_pair_config(h->M, N, h->K, h->max_ctas, h->pair_rows, cfg);
+        if (h->pair_mode || n_more > 0) big = spmm_dense_b_pair_config(h->M, N, h->K, b_nk, h->max_ctas, h->pair_rows, n_more > 0, cfg);
         *kernel = KERNEL_PAIR;
     }
     *us = big;
@@ -469,7 +469,7 @@ bool choose_kernel(vnm_handle_t h, int N, int n_more, Kernel *kernel, SpmmConfig
             *us = small;
         }
     }
-    if (*us < 0.0f && h->dense_b) *us = spmm_dense_b_pair_config(h->M, N, h->K, h->max_ctas, h->pair_rows, cfg);   // one SM per tile is not to be had
+    if (*us < 0.0f && h->dense_b) *us = spmm_dense_b_pair_config(h->M, N, h->K, b_nk, h->max_ctas, h->pair_rows, n_more > 0, cfg);   // one SM per tile is not to be had
     return *us >= 0.0f;
 }
 
@@ -483,7 +483,7 @@ int vnm_spmm_config(vnm_handle_t h, int N, int *tile_m, int *tile_n, int *stages
     SpmmConfig cfg;
     Kernel kernel;
     float us;
-    if (!choose_kernel(h, N, 0, &kernel, &cfg, &us)) return fail(VNM_ERR_UNSUPPORTED, "no kernel for this operand and its switches");
+    if (!choose_kernel(h, N, 0, 0, &kernel, &cfg, &us)) return fail(VNM_ERR_UNSUPPORTED, "no kernel for this operand and its switches");
     if (tile_m) *tile_m = kernel == KERNEL_PAIR ? cfg.nb * TILE_M : TILE_M;  // pairs: 512 or 256
     if (tile_n) *tile_n = cfg.bn;
     if (stages) *stages = cfg.stages;
@@ -551,7 +551,7 @@ static int spmm_impl(vnm_handle_t h, const void *B, int64_t ldb, int N, int b_nk
     SpmmConfig cfg;
     Kernel kernel;
     float us;
-    if (!choose_kernel(h, N, n_more, &kernel, &cfg, &us)) return fail(VNM_ERR_UNSUPPORTED, "vnm_spmm_f16: no kernel for this operand and its switches");
+    if (!choose_kernel(h, N, b_nk, n_more, &kernel, &cfg, &us)) return fail(VNM_ERR_UNSUPPORTED, "vnm_spmm_f16: no kernel for this operand and its switches");
     const bool pair = kernel == KERNEL_PAIR;
     EncodeTiledFn enc = get_encode_fn();
     if (!enc) return fail(VNM_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
@@ -568,8 +568,8 @@ static int spmm_impl(vnm_handle_t h, const void *B, int64_t ldb, int N, int b_nk
         } else if (b_nk) {
             cuuint64_t dims[2] = {(cuuint64_t)h->K, (cuuint64_t)N};
             cuuint64_t strides[1] = {(cuuint64_t)ldb * 2};
-            // B given as [N, K] (K contiguous): a CTA of the pair loads its 128 n-rows, 64 k (two MMA K blocks, 128-byte rows) per box
-            cuuint32_t box[2] = {64, 128};
+            // B given as [N, K] (K contiguous): a CTA of the pair loads its half of the tile's n-rows, 64 k (two MMA K blocks, 128-byte rows) per box
+            cuuint32_t box[2] = {64, (cuuint32_t)cfg.bn / 2};
             r = enc(&tmap_tile, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(B), dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -593,7 +593,7 @@ static int spmm_impl(vnm_handle_t h, const void *B, int64_t ldb, int N, int b_nk
             tmap_tile2 = tmap_tile;
             if (r == CUDA_SUCCESS && pair && N >= 128) {
                 // pair kernel: a CTA's half of a stage is {64 columns, 64 rows, 2 slices} starting at any multiple of 8 columns
-                // (pair tiles start at multiples of 240, the peer's half 120 columns further)
+                // (pair tiles start at multiples of their width, the peer's half half a width further)
                 cuuint64_t dims4[4] = {64, (cuuint64_t)h->K, 2, (cuuint64_t)((N - 128) / 8 + 1)};
                 cuuint64_t strides4[3] = {(cuuint64_t)ldb * 2, 128, 16};
                 cuuint32_t box4[4] = {64, 64, 2, 1};
@@ -736,7 +736,7 @@ int vnm_choose_form(int M, int K, int V, int n, int m, int N, int b_nk, int *str
         shape_handle(&h, M, K, V, n, m, form == 1);
         Kernel kernel;
         SpmmConfig cfg;
-        if (!choose_kernel(&h, N, 0, &kernel, &cfg, &us[form])) us[form] = -1.0f;
+        if (!choose_kernel(&h, N, b_nk && form == 1, 0, &kernel, &cfg, &us[form])) us[form] = -1.0f;
     }
     if (us[0] >= 0.0f) us[0] += m == 4 ? 1e6f : 2.0f + 4.0f * (float)N * (float)K / 4.5e6f;
     *strategy = us[0] >= 0.0f && (us[1] < 0.0f || us[0] < us[1]) ? VNM_STRATEGY_GATHER : VNM_STRATEGY_DENSE_B;

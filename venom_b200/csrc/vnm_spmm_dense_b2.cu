@@ -28,38 +28,43 @@ namespace vnm {
 namespace {
 
 constexpr int RT = 2;            // row tiles (accumulators) per CTA; a pair tile has 2 * RT = 4 row tiles
-constexpr int BN = 240;          // output columns per pair tile
-constexpr int PART = 40;         // columns per epilogue part / TMA store
-constexpr int SA = 3;            // A ring: k-tiles (each RT blocks)
-constexpr int SB = 6;            // B ring: stages of 64 rows x 128 columns (this CTA's half of two K=32 blocks of the MMAs)
-constexpr int META_SETS = 3;     // metadata column sets in tensor memory (4 columns per row tile each)
+constexpr int PART = 40;         // columns per epilogue part / TMA store (several destinations, BN = 240)
 constexpr int KB_PER_STAGE = 2;                     // K=32 blocks per B stage: one 16 KiB TMA box (smaller boxes keep the copy engine less busy)
 constexpr int STAGES_PER_KT = 4 / KB_PER_STAGE;
 constexpr int B_CHUNK_BYTES = KB_PER_STAGE * 32 * 128;  // 64 rows x 64 columns
-constexpr int B_STAGE_BYTES = 2 * B_CHUNK_BYTES;    // 16 KiB: two 64-column slices of which 120 columns are used (or 128 n-rows of 64 k)
-constexpr int A_STAGE_BYTES = RT * AM_BLOCK_BYTES;  // 36 KiB
-constexpr int A_RING_BYTES = SA * A_STAGE_BYTES;
-constexpr int B_RING_BYTES = SB * B_STAGE_BYTES;
+constexpr int B_STAGE_BYTES = 2 * B_CHUNK_BYTES;    // 16 KiB: two 64-column slices of which BN / 2 columns are used (or BN / 2 n-rows of 64 k)
 constexpr int OUT_STAGE_BYTES = TILE_M * PART * 2;  // 128 rows x 40 fp16 columns, staging of one TMA store
-constexpr int OUT_RING_BYTES = RT * OUT_STAGE_BYTES;  // one staging buffer per accumulator
 constexpr int BAR_BYTES = 640;
-constexpr int SMEM_BYTES = A_RING_BYTES + B_RING_BYTES + OUT_RING_BYTES + BAR_BYTES + 1024;
-static_assert(A_RING_BYTES % 1024 == 0 && B_RING_BYTES % 1024 == 0, "swizzled staging needs 1024-byte alignment");
-static_assert(SMEM_BYTES <= 227 * 1024, "shared memory per CTA");
+// What depends on the row tiles per CTA.  The rings and the metadata sets advance one k-tile at a time; a k-tile is 68 KiB with
+// two row tiles, 50 KiB with one.
+template <int R>
+struct Plan {
+    static constexpr int SA = R == 1 ? 4 : 3;                          // A ring: k-tiles (each R blocks)
+    static constexpr int SB = SA * STAGES_PER_KT;                      // B ring: stages of 64 rows x 128 columns (this CTA's half of two K=32 blocks of the MMAs)
+    static constexpr int A_STAGE_BYTES = R * AM_BLOCK_BYTES;
+    static constexpr int A_RING_BYTES = SA * A_STAGE_BYTES;
+    static constexpr int B_RING_BYTES = SB * B_STAGE_BYTES;
+    static constexpr int OUT_RING_BYTES = RT * OUT_STAGE_BYTES;        // one staging buffer per accumulator
+    static constexpr int SMEM_BYTES = A_RING_BYTES + B_RING_BYTES + OUT_RING_BYTES + BAR_BYTES + 1024;
+    static_assert(A_STAGE_BYTES % 1024 == 0 && B_STAGE_BYTES % 1024 == 0, "swizzled staging needs 1024-byte alignment");
+    static_assert(SMEM_BYTES <= 227 * 1024, "shared memory per CTA");
+    static_assert((2 * SA + 2 * SB + 4) * 8 + 16 <= BAR_BYTES, "barrier area too small");
+};
 // Four single-thread roles and two epilogue groups of four warps: 384 threads may use 168 registers each, which holds an
 // accumulator row (120 packed words) without any re-allocation between warpgroups.  (With 512 threads and setmaxnreg the
 // MMAs of this kernel issued at 180-240 clocks instead of 120: 1700 clocks a k-tile, against 1380.)
 constexpr int NUM_THREADS = 384;
 constexpr int EPI_WARP0 = 4;
 constexpr int TMEM_COLS = 512;
-// tensor-memory columns: accumulator 0 at 0..239, metadata sets at 240 and 248, accumulator 1 at 256..495, metadata set at 496
+// tensor-memory columns: accumulator 0 from 0, accumulator 1 from 256 (at most 240 columns each); metadata sets of four columns a
+// row tile at 240..255 (and for a third set of two row tiles at 496)
 __device__ __forceinline__ uint32_t acc_col(int rt) { return (uint32_t)rt * 256u; }
-__device__ __forceinline__ uint32_t meta_col(int set) { return set == 0 ? 240u : (set == 1 ? 248u : 496u); }
-constexpr int KT_RING = SB / STAGES_PER_KT;  // k-tiles the B ring holds
-static_assert(SB % STAGES_PER_KT == 0 && KT_RING == SA && KT_RING == META_SETS, "the rings and the metadata sets advance one k-tile at a time");
-static_assert(BN <= 240 && META_SETS == 3 && RT == 2 && BN % 16 == 0 && BN == 6 * PART, "tensor-memory column plan");
-static_assert((2 * SA + 2 * SB + 4) * 8 + 16 <= BAR_BYTES, "barrier area too small");
-constexpr int HALF_N = BN / 2;   // columns of a B stage held by each CTA of the pair
+template <int R>
+__device__ __forceinline__ uint32_t meta_col(int set)
+{
+    if (R == 1) return 240u + 4u * (uint32_t)set;
+    return set == 2 ? 496u : 240u + 8u * (uint32_t)set;
+}
 
 // ---- cluster helpers ----
 __device__ __forceinline__ uint32_t cluster_ctarank()
@@ -123,12 +128,17 @@ __device__ __forceinline__ void tc_mma2_sp_f16(uint32_t d_tmem, uint64_t adesc, 
 //   warp 2      peer: forwards "A blocks landed" and "B half landed" to the leader.
 //   warp 3      tensor-memory owner in both CTAs; leader: MMA issuer.
 //   warps 4..11 epilogue of this CTA's two accumulators.
-template <int R>
+template <int R, int BN, bool MULTI>
 __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const __grid_constant__ CUtensorMap tmap_tile, const __grid_constant__ CUtensorMap tmap_tile2,
                                                                            const __grid_constant__ CUtensorMap tmap_out, const __grid_constant__ OutMaps more_out,
                                                                            const SpmmParams p)
 {
-    static_assert(R == 1 || R == RT, "row tiles per CTA");  // R = 1: pair tiles of 256 x 240 for problems with few row tiles
+    static_assert(R == 1 || R == RT, "row tiles per CTA");  // R = 1: pair tiles of 256 rows for problems with few row tiles
+    static_assert(BN <= 240 && BN % 16 == 0, "the tensor-memory column plan");
+    static_assert(!MULTI || BN == 6 * PART, "parts of a tile that leaves through TMA stores");
+    constexpr int SA = Plan<R>::SA, SB = Plan<R>::SB, A_STAGE_BYTES = Plan<R>::A_STAGE_BYTES, A_RING_BYTES = Plan<R>::A_RING_BYTES;
+    constexpr int B_RING_BYTES = Plan<R>::B_RING_BYTES, OUT_RING_BYTES = Plan<R>::OUT_RING_BYTES;
+    constexpr int HALF_N = BN / 2;   // columns of a B stage held by each CTA of the pair
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint8_t *a_ring = smem;
@@ -246,10 +256,10 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
                     if (p.gather_mode == GATHER_NONE) {  // ablation: no loads of B at all (timing floor; results are meaningless)
                         mbar_arrive(&b_full[s]);
                     } else {
-                        // 64 rows x 128 columns come along per stage; the MMAs read the first 120 columns
-                        mbar_arrive_expect_tx(&b_full[s], B_STAGE_BYTES);
+                        // 64 rows x 128 columns (the MMAs read the first BN / 2), or BN / 2 rows (n) x 64 k
+                        mbar_arrive_expect_tx(&b_full[s], p.b_nk ? HALF_N * 128 : B_STAGE_BYTES);
                         if (p.b_nk) {
-                            tma_load_2d_hint(dst, &tmap_tile, jl * 64, n0, &b_full[s], p.hint_b);  // 128 rows (n) x 64 k, 128-byte swizzle
+                            tma_load_2d_hint(dst, &tmap_tile, jl * 64, n0, &b_full[s], p.hint_b);  // 128-byte swizzle
                         } else if (wide) {
                             tma_load_4d_hint(dst, &tmap_tile, 0, jl * 64, 0, n0 / 8, &b_full[s], p.hint_b);  // {64 columns, 64 rows, 2 slices} from column n0
                         } else {  // ragged right edge: two boxes that clip (and zero-fill) at N
@@ -311,7 +321,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
             const uint64_t adesc0 = make_smem_desc(smem_u32(a_ring), 16, 1024, 2);
             const uint64_t mdesc0 = make_smem_desc(smem_u32(a_ring) + A_IMG_BYTES, 0, 128, 0);
             // this CTA's half of a stage: N-major (two 64-column slices of 64 rows x 128 bytes, 128-byte swizzle; a K=32 block is
-            // 32 rows = 4096 bytes further) or K-major (128 n-rows of 128 bytes = 64 k of which 120 rows are used, 128-byte swizzle,
+            // 32 rows = 4096 bytes further) or K-major (BN / 2 n-rows of 128 bytes = 64 k, 128-byte swizzle,
             // 8-row groups 1024 bytes apart; a K=32 block is 64 bytes further inside the row)
             const uint64_t bdesc0 = b_nk ? make_smem_desc(smem_u32(b_ring), 16, 1024, 2) : make_smem_desc(smem_u32(b_ring), B_CHUNK_BYTES, 1024, 2);
             const uint32_t kb_step = b_nk ? 64u : 32u * 128u;  // bytes between the K=32 blocks of a stage
@@ -326,7 +336,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
                 for (int kt = 0; kt < p.ktiles; ++kt) {
                     if (!wait_one(&a_full[sa], ph, abort_flag, p.status, DEV_TIMEOUT_MMA)) { alive = false; break; }  // both CTAs' blocks
                     tc_fence_after();
-                    const uint32_t mcol = tmem_base + meta_col(sa);
+                    const uint32_t mcol = tmem_base + meta_col<R>(sa);
                     const uint32_t aoff = (uint32_t)(sa * A_STAGE_BYTES) >> 4;
 #pragma unroll
                     for (int rt = 0; rt < R; rt++) tc_cp2_128x128b(mcol + rt * 4, mdesc0 + aoff + (uint32_t)((rt * AM_BLOCK_BYTES) >> 4));
@@ -380,14 +390,13 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
                     __syncwarp();
                     if (lane == 0) mbar_arrive_cluster(empty_leader);  // the leader's MMA issuer waits for both CTAs' epilogues
                 };
-                if (p.n_out == 1) {
+                if constexpr (!MULTI) {
                     // straight from tensor memory; with two row tiles per CTA the next tile's MMAs wait for both accumulators, so
                     // they are read into registers whole before the first store
                     const uint32_t tacc = tmem_base + ((uint32_t)(q * 32) << 16) + acc_col(grp);
                     if (p.layout == 0) store_tile<BN, R == 2>(TileStoreMN(tacc, q, (int64_t)mt * TILE_M, n0, p), release);
                     else store_tile<BN, R == 2>(TileStoreNM(tacc, q, (int64_t)mt * TILE_M, n0, p), release);
-                    continue;
-                }
+                } else {
                 const int64_t row = (int64_t)mt * TILE_M + arow;
                 const bool row_ok = mt < p.mtiles && row < p.M;
                 const bool has_bias = p.layout == 1 && p.bias != nullptr;
@@ -464,11 +473,12 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
                 release();
 #pragma unroll
                 for (int h = 0; h < HELD; h++) store_part(NPARTS - HELD + h, held + h * (PART / 2));
+                }
             }
         }
     }
 
-    if (warp >= EPI_WARP0 && ((warp - EPI_WARP0) & 3) == 0 && lane == 0) bulk_wait_group_read0();  // this thread's TMA stores have read shared memory (their global writes complete with the grid)
+    if (MULTI && warp >= EPI_WARP0 && ((warp - EPI_WARP0) & 3) == 0 && lane == 0) bulk_wait_group_read0();  // this thread's TMA stores have read shared memory (their global writes complete with the grid)
     tc_fence_before();
     __syncthreads();
     cluster_sync_all();  // the peer's shared and tensor memory stay alive until the leader's last MMA and commit are done
@@ -482,18 +492,22 @@ int g_pair_clusters = 0;  // co-resident clusters of two CTAs on this device (0 
 
 }  // namespace
 
+#define VNM_PAIR_INSTANCES(X) X(1, 192, false) X(1, 224, false) X(1, 240, false) X(1, 240, true) X(2, 192, false) X(2, 224, false) X(2, 240, false) X(2, 240, true)
+
 cudaError_t spmm_dense_b_pair_init()
 {
-    cudaError_t e = cudaFuncSetAttribute(spmm_dense_b_pair_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    if (e != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(spmm_dense_b_pair_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES)) != cudaSuccess) return e;
+    cudaError_t e;
+#define VNM_PAIR_ATTR(R, BN, MULTI) \
+    if ((e = cudaFuncSetAttribute(spmm_dense_b_pair_kernel<R, BN, MULTI>, cudaFuncAttributeMaxDynamicSharedMemorySize, Plan<R>::SMEM_BYTES)) != cudaSuccess) return e;
+    VNM_PAIR_INSTANCES(VNM_PAIR_ATTR)
+#undef VNM_PAIR_ATTR
     int dev = 0, sms = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3((unsigned)(sms & ~1), 1, 1);
     lc.blockDim = dim3(NUM_THREADS, 1, 1);
-    lc.dynamicSmemBytes = SMEM_BYTES;
+    lc.dynamicSmemBytes = Plan<1>::SMEM_BYTES;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
@@ -502,37 +516,47 @@ cudaError_t spmm_dense_b_pair_init()
     lc.attrs = attr;
     lc.numAttrs = 1;
     int clusters = 0;
-    e = cudaOccupancyMaxActiveClusters(&clusters, spmm_dense_b_pair_kernel<2>, &lc);
+    e = cudaOccupancyMaxActiveClusters(&clusters, spmm_dense_b_pair_kernel<1, 240, false>, &lc);
     if (e != cudaSuccess) { (void)cudaGetLastError(); clusters = 0; }
     g_pair_clusters = clusters;
     return cudaSuccess;
 }
 
-// Pair tiles are 512 x 240 (two row tiles per CTA) or 256 x 240 (one row tile per CTA, two alternating accumulators).  The
-// wide form reads every B stage once per 512 rows (0.66 us a k-tile for four row tiles against 0.47 for two) but drains both
-// accumulators between tiles, and it needs twice the rows for a full wave; row tiles that do not divide evenly are padded
-// (computed, never stored).  The smaller estimate wins.
-float spmm_dense_b_pair_config(int M, int N, int K, int max_ctas, int force_rows, SpmmConfig *cfg)
+// Pair tiles have 512 rows (two row tiles per CTA) or 256 (one row tile per CTA, two alternating accumulators) and 240, 224 or
+// 192 columns.  The tall form reads every B stage once per 512 rows but drains both accumulators between tiles, and it needs
+// twice the rows for a full wave; row tiles that do not divide evenly are padded (computed, never stored).  A [K,N] operand is
+// staged N-major, where halves of 120 columns, no multiple of 16, cost 0.73 us a k-tile against 0.54 (0.64 against 0.45 with
+// one row tile): it takes 224 columns.  Narrower tiles where they fill the last wave better.  The smallest estimate wins.
+float spmm_dense_b_pair_config(int M, int N, int K, int b_nk, int max_ctas, int force_rows, bool multi, SpmmConfig *cfg)
 {
     if (g_pair_clusters <= 0) return -1.0f;
     const int mtiles = (M + TILE_M - 1) / TILE_M, ktiles = (K + 127) / 128;
-    const long long ntiles = (N + BN - 1) / BN;
     int clusters = g_pair_clusters;
     if (max_ctas > 0 && max_ctas / 2 < clusters) clusters = max_ctas / 2;
     if (clusters < 1) return -1.0f;
-    const long long t2 = (long long)((mtiles + 2 * RT - 1) / (2 * RT)) * ntiles, t1 = (long long)((mtiles + 1) / 2) * ntiles;
-    const float e2 = 6.0f + (float)((t2 + clusters - 1) / clusters) * (ktiles * 0.66f + 1.3f);
-    const float e1 = 6.0f + (float)((t1 + clusters - 1) / clusters) * (ktiles * 0.47f + 0.35f);
-    const int rt = force_rows == 1 ? 1 : force_rows == 2 && mtiles > 2 ? RT : e2 < e1 ? RT : 1;
-    const long long tiles = rt == RT ? t2 : t1;
-    cfg->bn = BN;
+    static const int widths[3] = {240, 224, 192};
+    static const float tall_us[2][3] = {{0.73f, 0.51f, 0.49f}, {0.54f, 0.51f, 0.49f}}, low_us[2][3] = {{0.64f, 0.47f, 0.47f}, {0.45f, 0.45f, 0.45f}};
+    float best = 1e30f;
+    for (int w = 0; w < (multi ? 1 : 3); w++) {
+        const long long ntiles = (N + widths[w] - 1) / widths[w];
+        for (int rt = 1; rt <= RT; rt++) {
+            if ((force_rows == 1 && rt == RT) || (force_rows == 2 && mtiles > 2 && rt == 1)) continue;
+            const long long tiles = (long long)((mtiles + 2 * rt - 1) / (2 * rt)) * ntiles;
+            const float waves = (float)((tiles + clusters - 1) / clusters);
+            const float us = 6.0f + (rt == RT ? waves * (ktiles * tall_us[b_nk != 0][w] + 1.3f) : waves * (ktiles * low_us[b_nk != 0][w] + 0.35f));
+            if (us < best) {
+                best = us;
+                cfg->bn = widths[w];
+                cfg->nb = 2 * rt;  // row tiles per pair tile
+                cfg->smem_bytes = rt == RT ? Plan<2>::SMEM_BYTES : Plan<1>::SMEM_BYTES;
+                cfg->grid = 2 * (int)(tiles < clusters ? tiles : clusters);
+            }
+        }
+    }
     cfg->part = PART;
-    cfg->nb = 2 * rt;  // row tiles per pair tile
     cfg->stages = 2;
-    cfg->smem_bytes = SMEM_BYTES;
     cfg->threads = NUM_THREADS;
-    cfg->grid = 2 * (int)(tiles < clusters ? tiles : clusters);
-    return rt == RT ? e2 : e1;
+    return best;
 }
 
 cudaError_t launch_spmm_dense_b_pair(const SpmmConfig &cfg, const CUtensorMap &tmap_tile, const CUtensorMap &tmap_tile2, const CUtensorMap &tmap_out, const OutMaps &more_out,
@@ -541,7 +565,7 @@ cudaError_t launch_spmm_dense_b_pair(const SpmmConfig &cfg, const CUtensorMap &t
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3((unsigned)cfg.grid, 1, 1);
     lc.blockDim = dim3(NUM_THREADS, 1, 1);
-    lc.dynamicSmemBytes = SMEM_BYTES;
+    lc.dynamicSmemBytes = (size_t)cfg.smem_bytes;
     lc.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -550,8 +574,12 @@ cudaError_t launch_spmm_dense_b_pair(const SpmmConfig &cfg, const CUtensorMap &t
     attr[0].val.clusterDim.z = 1;
     lc.attrs = attr;
     lc.numAttrs = 1;
-    if (cfg.nb == 2) return cudaLaunchKernelEx(&lc, spmm_dense_b_pair_kernel<1>, tmap_tile, tmap_tile2, tmap_out, more_out, p);
-    return cudaLaunchKernelEx(&lc, spmm_dense_b_pair_kernel<2>, tmap_tile, tmap_tile2, tmap_out, more_out, p);
+    const bool multi = p.n_out > 1;
+#define VNM_PAIR_LAUNCH(R, BN, MULTI) \
+    if (cfg.nb == 2 * R && cfg.bn == BN && multi == MULTI) return cudaLaunchKernelEx(&lc, spmm_dense_b_pair_kernel<R, BN, MULTI>, tmap_tile, tmap_tile2, tmap_out, more_out, p);
+    VNM_PAIR_INSTANCES(VNM_PAIR_LAUNCH)
+#undef VNM_PAIR_LAUNCH
+    return cudaErrorInvalidValue;
 }
 
 }  // namespace vnm
