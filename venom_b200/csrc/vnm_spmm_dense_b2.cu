@@ -123,10 +123,12 @@ __device__ __forceinline__ void tc_mma2_sp_f16(uint32_t d_tmem, uint64_t adesc, 
 }
 
 // Warp roles:
-//   warp 0      A producer: two bulk copies per k-tile (this CTA's two row tiles).
-//   warp 1      B producer: one 16 KiB TMA box per stage (64 rows of this CTA's 128-column half).
-//   warp 2      peer: forwards "A blocks landed" and "B half landed" to the leader.
-//   warp 3      tensor-memory owner in both CTAs; leader: MMA issuer.
+//   warp 0      A producer: one bulk copy per k-tile and row tile.
+//   warps 1, 2  B producers, alternate stages: one TMA box each (64 k of this CTA's half of the columns).  One thread issues a
+//               stage in about 420 clocks (wait, expect, box): alone it held tiles of one row tile at 850 clocks a k-tile,
+//               against 480 of their MMAs; two of them: 35.1 -> 27.0 us at 1024 x 8192, N = 3072 ([N,K]).
+//   warp 3      tensor-memory owner in both CTAs; leader: MMA issuer; peer: forwards "A blocks landed" and "B half landed"
+//               to the leader.
 //   warps 4..11 epilogue of this CTA's two accumulators.
 template <int R, int BN, bool MULTI>
 __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const __grid_constant__ CUtensorMap tmap_tile, const __grid_constant__ CUtensorMap tmap_tile2,
@@ -236,13 +238,14 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
             }
         }
         __syncwarp();
-    } else if (warp == 1) {
+    } else if (warp == 1 || warp == 2) {
         // ---------------- B producer: this CTA's half of every stage ----------------
         if (elect_one()) {
             tma_prefetch_desc(&tmap_tile);
             tma_prefetch_desc(&tmap_tile2);
             const int per_tile = STAGES_PER_KT * p.ktiles;
-            int j = 0, s = 0;
+            const int half = warp - 1;   // stages of this parity
+            int j = half, s = half;
             uint32_t ph = 1;
             bool alive = true;
             for (int tile = pair; alive && tile < total_tiles; tile += npairs) {
@@ -250,7 +253,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
                 tile_coords(tile, mquads, p.ntiles, p.group_m, &mq_unused, &nt);
                 const int n0 = nt * BN + (int)crank * HALF_N;  // first column of this CTA's half
                 const bool wide = p.b_wide_ok && n0 + 128 <= p.N;
-                for (int jl = 0; jl < per_tile; ++jl, ++j) {
+                for (int jl = half; jl < per_tile; jl += 2, j += 2) {
                     if (!wait_quiet(&b_free[s], ph, abort_flag, p.status, DEV_TIMEOUT_PRODUCER)) { alive = false; break; }
                     uint8_t *dst = b_ring + s * B_STAGE_BYTES;
                     if (p.gather_mode == GATHER_NONE) {  // ablation: no loads of B at all (timing floor; results are meaningless)
@@ -285,15 +288,15 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
                             }
                         }
                     }
-                    if (++s == SB) { s = 0; ph ^= 1; }
+                    if ((s += 2) >= SB) { s = half; ph ^= 1; }
                 }
             }
             if (*abort_flag && p.gather_mode != GATHER_NONE) {
-                for (int k = j > SB ? j - SB : 0; k < j; ++k) drain_slot(&b_full[k % SB], (uint32_t)(k / SB) & 1u, p.status);
+                for (int k = j > SB ? j - SB : half; k < j; k += 2) drain_slot(&b_full[k % SB], (uint32_t)(k / SB) & 1u, p.status);
             }
         }
         __syncwarp();
-    } else if (warp == 2) {
+    } else if (warp == 3) {
         if (!leader_cta && elect_one()) {
             // ---------------- peer: forward "A blocks landed" and "my half of the stage landed" ----------------
             const uint32_t remote_a = mapa_shared(smem_u32(a_full), 0), remote_b = mapa_shared(smem_u32(b_full), 0);
@@ -312,8 +315,6 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
                 if (++sa == SA) { sa = 0; ph ^= 1; }
             }
         }
-        __syncwarp();
-    } else if (warp == 3) {
         if (leader_cta && elect_one()) {
             // ---------------- MMA issuer (leader) ----------------
             const bool b_nk = p.b_nk != 0;
