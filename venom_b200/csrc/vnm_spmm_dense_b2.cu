@@ -1,13 +1,12 @@
 // SpMM kernel for the dense-B operand form on PAIRS of SMs (thread-block clusters of two CTAs, tcgen05 cta_group::2).
 //
-// Same operand form and pipeline as vnm_spmm_dense_b.cu, but one B stage now feeds four 128-row tiles of A: the two
-// CTAs of a cluster each hold two row tiles (two accumulators of 240 tensor-memory columns) and HALF of every B
-// stage (32 rows x 120 of the 240 columns); one tcgen05.mma.sp.cta_group::2 multiplies 256 rows (128 from each CTA)
-// with the 240 columns assembled from both halves.  Per k-tile a CTA therefore takes in 36 KiB of A and 32 KiB of B
-// instead of 36 + 64 KiB, which moves the mainloop from the SM's L2 intake limit to the tensor pipe.
+// A pair tile is 512 rows x BN columns: each CTA holds two row tiles of 128 (two accumulators) and HALF of every B stage (64 k x
+// BN / 2 columns); one tcgen05.mma.sp.cta_group::2 multiplies 256 rows (128 from each CTA) with the BN columns assembled from both
+// halves.  Per k-tile of 128 a CTA takes in 36 KiB of A and 32 KiB of B.  With one row tile a CTA (256 rows): 18 + 32 KiB.
 //
-// What bounds it: the shared-memory port.  Per k-tile a CTA's MMAs read 8 x (4 KiB of A + its 7.5 KiB half of B), the
-// metadata copies 4 KiB, and TMA writes 68 KiB: 164 KiB at 128 bytes a clock are 1312 clocks, against 960 of the tensor pipe.
+// What bounds it: the tensor pipe inside a tile (8 MMAs x BN / 2 clocks a k-tile: 960 of 973 measured without loads, 991 with them,
+// BN = 240), and the stores of finished tiles between tiles (4096 x 1024, N = 16384: 50 us without stores, 68 with them,
+// floor 26), which leave in bursts and hold up the loads of the next tile.  One row tile a CTA: 480 clocks of MMAs, 490 to 600 with loads.
 //
 // Cluster protocol (rank 0 = leader, rank 1 = peer); every load stays local to the CTA that issues it:
 //   * both CTAs run their own A producer, B producers and epilogue on their own shared / tensor memory;
@@ -150,9 +149,9 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
     uint64_t *b_full = a_full + SA;
     uint64_t *a_free = b_full + SB;   // the MMAs that read this slot have completed (arrives in both CTAs)
     uint64_t *b_free = a_free + SA;
-    // accumulator hand-off.  R = 2: one barrier pair, both accumulators of a CTA belong to the same tile.  R = 1: a CTA has one
-    // row tile, so its two accumulators alternate between consecutive tiles (barrier pair ti & 1) and the epilogue of one
-    // tile runs beside the MMAs of the next.
+    // accumulator hand-off, a barrier pair for each.  R = 2: both accumulators of a CTA belong to the same tile.  R = 1: a CTA has
+    // one row tile, so its two accumulators alternate between consecutive tiles (ti & 1) and the epilogue of one tile runs
+    // beside the MMAs of the next.
     uint64_t *acc_full_bar = b_free + SB;      // [2]
     uint64_t *acc_empty_bar = acc_full_bar + 2;  // [2]
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty_bar + 2);
@@ -177,9 +176,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
         for (int s = 0; s < SB; s++) mbar_init(&b_free[s], 1);
         for (int a = 0; a < 2; a++) {
             mbar_init(&acc_full_bar[a], 1);
-            mbar_init(&acc_empty_bar[a], 2 * 4);  // R = 1: the four warps of one epilogue group in both CTAs
+            mbar_init(&acc_empty_bar[a], 2 * 4);  // the four warps of one epilogue group in both CTAs
         }
-        if (R == 2) mbar_init(&acc_empty_bar[0], 2 * 4 * R);  // every epilogue warp of both CTAs
         *abort_flag = 0;
         fence_barrier_init();
     }
@@ -330,36 +328,47 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
             uint32_t ph = 0;       // phase of all of them
             bool alive = true;
             for (int ti = 0; alive && ti < my_tiles; ++ti) {
-                // accumulator set of this tile: R = 2 always set 0 (phase ti), R = 1 set ti & 1 (phase ti / 2)
+                // accumulator set: R = 2 both (phase ti), R = 1 set ti & 1 (phase ti / 2)
                 const int aset = R == 1 ? (ti & 1) : 0;
                 const uint32_t aphase = R == 1 ? (uint32_t)(ti >> 1) & 1u : (uint32_t)ti & 1u;
-                if (!wait_one(&acc_empty_bar[aset], aphase ^ 1u, abort_flag, p.status, DEV_TIMEOUT_MMA)) break;
                 for (int kt = 0; kt < p.ktiles; ++kt) {
+                    if (kt == 0 && !wait_one(&acc_empty_bar[aset], aphase ^ 1u, abort_flag, p.status, DEV_TIMEOUT_MMA)) { alive = false; break; }
                     if (!wait_one(&a_full[sa], ph, abort_flag, p.status, DEV_TIMEOUT_MMA)) { alive = false; break; }  // both CTAs' blocks
                     tc_fence_after();
                     const uint32_t mcol = tmem_base + meta_col<R>(sa);
                     const uint32_t aoff = (uint32_t)(sa * A_STAGE_BYTES) >> 4;
 #pragma unroll
                     for (int rt = 0; rt < R; rt++) tc_cp2_128x128b(mcol + rt * 4, mdesc0 + aoff + (uint32_t)((rt * AM_BLOCK_BYTES) >> 4));
+                    // The k-tile's MMAs of one row tile, then those of the other: the first accumulator of a tile is full half a
+                    // k-tile before the second one, and its next tile may begin while the second one is still being read
+                    // (the hand-off of both at once kept the tensor pipe idle for 2600 clocks a tile).
 #pragma unroll
-                    for (int st = 0; st < STAGES_PER_KT; st++) {
-                        const int sb = STAGES_PER_KT * sa + st;
-                        if (!wait_one(&b_full[sb], ph, abort_flag, p.status, DEV_TIMEOUT_MMA)) { alive = false; break; }  // both halves
-                        tc_fence_after();
+                    for (int rt = 0; rt < R; rt++) {
+                        if (R == 2 && rt == 1 && kt == 0) {
+                            if (!wait_one(&acc_empty_bar[1], aphase ^ 1u, abort_flag, p.status, DEV_TIMEOUT_MMA)) { alive = false; break; }
+                            tc_fence_after();
+                        }
 #pragma unroll
-                        for (int k2 = 0; k2 < KB_PER_STAGE; k2++) {  // K=32 blocks of the stage
-                            const int kb = st * KB_PER_STAGE + k2;
-                            const uint32_t boff = ((uint32_t)sb * B_STAGE_BYTES + (uint32_t)k2 * kb_step) >> 4;
+                        for (int st = 0; st < STAGES_PER_KT; st++) {
+                            const int sb = STAGES_PER_KT * sa + st;
+                            if (rt == 0) {
+                                if (!wait_one(&b_full[sb], ph, abort_flag, p.status, DEV_TIMEOUT_MMA)) { alive = false; break; }  // both halves
+                                tc_fence_after();
+                            }
 #pragma unroll
-                            for (int rt = 0; rt < R; rt++)
+                            for (int k2 = 0; k2 < KB_PER_STAGE; k2++) {  // K=32 blocks of the stage
+                                const int kb = st * KB_PER_STAGE + k2;
+                                const uint32_t boff = ((uint32_t)sb * B_STAGE_BYTES + (uint32_t)k2 * kb_step) >> 4;
                                 tc_mma2_sp_f16(tmem_base + acc_col(R == 1 ? aset : rt), adesc0 + aoff + (uint32_t)((rt * AM_BLOCK_BYTES + kb * 32) >> 4), bdesc0 + boff,
                                                mcol + rt * 4 + (uint32_t)(kb & ~1), idesc0 | (uint32_t)(kb & 1), (kt | kb) != 0 ? 1u : 0u);
+                            }
+                            if (rt == R - 1) tc_commit2(&b_free[sb]);
                         }
-                        tc_commit2(&b_free[sb]);
+                        if (!alive) break;
+                        if (kt == p.ktiles - 1) tc_commit2(&acc_full_bar[R == 1 ? aset : rt]);
                     }
                     if (!alive) break;
                     tc_commit2(&a_free[sa]);
-                    if (kt == p.ktiles - 1) tc_commit2(&acc_full_bar[aset]);
                     if (++sa == SA) { sa = 0; ph ^= 1; }
                 }
             }
@@ -371,7 +380,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
         const int i = q * 32 + lane;
         const int arow = mma_row_to_actual(i);
         const int grp = (warp - EPI_WARP0) >> 2;  // R = 2: the accumulator (row tile) this group drains; R = 1: the tiles ti with ti & 1 == grp
-        const uint32_t empty_leader = mapa_shared(smem_u32(&acc_empty_bar[R == 1 ? grp : 0]), 0);
+        const uint32_t empty_leader = mapa_shared(smem_u32(&acc_empty_bar[grp]), 0);
         int ti = 0;
         for (int tile = pair; tile < total_tiles; tile += npairs, ++ti) {
             if (R == 1 && (ti & 1) != grp) continue;
@@ -379,7 +388,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
             tile_coords(tile, mquads, p.ntiles, p.group_m, &mq, &nt);
             const int n0 = nt * BN;
             // the four warps of a group leave the loop together (they meet at named barriers below)
-            const bool got = wait_warp(&acc_full_bar[R == 1 ? grp : 0], R == 1 ? (uint32_t)(ti >> 1) & 1u : (uint32_t)ti & 1u, abort_flag, p.status,
+            const bool got = wait_warp(&acc_full_bar[grp], R == 1 ? (uint32_t)(ti >> 1) & 1u : (uint32_t)ti & 1u, abort_flag, p.status,
                                        DEV_TIMEOUT_EPILOGUE);
             if (!named_barrier_and(1 + grp, 128, got)) break;
             tc_fence_after();
@@ -524,10 +533,11 @@ cudaError_t spmm_dense_b_pair_init()
 }
 
 // Pair tiles have 512 rows (two row tiles per CTA) or 256 (one row tile per CTA, two alternating accumulators) and 240, 224 or
-// 192 columns.  The tall form reads every B stage once per 512 rows but drains both accumulators between tiles, and it needs
-// twice the rows for a full wave; row tiles that do not divide evenly are padded (computed, never stored).  A [K,N] operand is
-// staged N-major, where halves of 120 columns, no multiple of 16, cost 0.73 us a k-tile against 0.54 (0.64 against 0.45 with
-// one row tile): it takes 224 columns.  Narrower tiles where they fill the last wave better.  The smallest estimate wins.
+// 192 columns.  The tall form reads every B stage once per 512 rows, but its accumulators are drained between tiles (3 to 4 us a
+// wave against 1.1 to 1.5) and it needs twice the rows for a full wave; row tiles that do not divide evenly are padded
+// (computed, never stored).  A [K,N] operand in tiles of 240 columns costs half as much again a k-tile: the peer's half, 240 bytes
+// further, starts inside a 32-byte sector.  The constants (us a k-tile and us a wave) are fitted to 18 shapes from 512 to 49152 rows, 512 to
+// 12288 k and 512 to 16384 columns; the smallest estimate wins.
 float spmm_dense_b_pair_config(int M, int N, int K, int b_nk, int max_ctas, int force_rows, bool multi, SpmmConfig *cfg)
 {
     if (g_pair_clusters <= 0) return -1.0f;
@@ -536,7 +546,8 @@ float spmm_dense_b_pair_config(int M, int N, int K, int b_nk, int max_ctas, int 
     if (max_ctas > 0 && max_ctas / 2 < clusters) clusters = max_ctas / 2;
     if (clusters < 1) return -1.0f;
     static const int widths[3] = {240, 224, 192};
-    static const float tall_us[2][3] = {{0.73f, 0.51f, 0.49f}, {0.54f, 0.51f, 0.49f}}, low_us[2][3] = {{0.64f, 0.47f, 0.47f}, {0.45f, 0.45f, 0.45f}};
+    static const float kt_us[2][2][3] = {{{0.635f, 0.365f, 0.376f}, {0.31f, 0.30f, 0.295f}}, {{0.72f, 0.505f, 0.48f}, {0.54f, 0.50f, 0.465f}}};   // [row tiles - 1][b_nk][width]
+    static const float wave_us[2][3] = {{1.2f, 1.45f, 1.1f}, {3.4f, 3.9f, 2.9f}}, start_us[2] = {5.2f, 4.7f};
     float best = 1e30f;
     for (int w = 0; w < (multi ? 1 : 3); w++) {
         const long long ntiles = (N + widths[w] - 1) / widths[w];
@@ -544,7 +555,7 @@ float spmm_dense_b_pair_config(int M, int N, int K, int b_nk, int max_ctas, int 
             if ((force_rows == 1 && rt == RT) || (force_rows == 2 && mtiles > 2 && rt == 1)) continue;
             const long long tiles = (long long)((mtiles + 2 * rt - 1) / (2 * rt)) * ntiles;
             const float waves = (float)((tiles + clusters - 1) / clusters);
-            const float us = 6.0f + (rt == RT ? waves * (ktiles * tall_us[b_nk != 0][w] + 1.3f) : waves * (ktiles * low_us[b_nk != 0][w] + 0.35f));
+            const float us = start_us[rt - 1] + waves * (ktiles * kt_us[rt - 1][b_nk != 0][w] + wave_us[rt - 1][w]);
             if (us < best) {
                 best = us;
                 cfg->bn = widths[w];
