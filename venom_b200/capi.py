@@ -137,6 +137,26 @@ def _need_cuda(*tensors):
             raise VenomError("expected CUDA tensors (there is no CPU path)")
 
 
+_ext = None
+
+
+def _native(name):
+    """A call of the extension that does what its caller here does (checks, allocation and launch without the interpreter
+    between them) for the plain case and returns None for anything else.  Without the extension: always None."""
+    global _ext
+    if _ext is None:
+        try:
+            from . import spatha_module
+            _ext = spatha_module()
+        except ImportError:
+            _ext = False
+    return getattr(_ext, name) if _ext else _never
+
+
+def _never(*args):
+    return None
+
+
 def sizes(M, K, V, m, n=2):
     """(Ksp, values_elems, meta_words, colloc_words) from the library."""
     out = [C.c_int64() for _ in range(4)]
@@ -148,6 +168,10 @@ def compress(dense, colloc, V, m, n=2, mask=None, count_violations=True):
     """dense: [M,K] fp16 CUDA (pruned); colloc: int32/uint32 CUDA.  Returns (values fp16, meta int32,
     violations int or None).  Reading the violation count synchronises the stream."""
     _need_cuda(dense, colloc, mask)
+    if mask is None:
+        done = _native("compress")(dense, colloc, V, m, n, bool(count_violations))
+        if done is not None:
+            return done
     if dense.dtype != torch.float16 or dense.dim() != 2 or dense.stride(1) != 1:
         raise VenomError("dense must be a 2-D fp16 tensor with unit inner stride")
     M, K = dense.shape
@@ -185,6 +209,9 @@ def sparsify_magnitude(w, V, m, n=2):
     _need_cuda(w)
     if w.dtype not in (torch.float16, torch.float32) or w.dim() != 2 or w.stride(1) != 1 or w.shape[1] % m or m > 64:
         return None
+    done = _native("sparsify")(w.detach(), V, m, n)
+    if done is not None:
+        return done
     M, K = w.shape
     ksp, nv, nm, nc = sizes(M, K, V, m, n)
     values = torch.empty(nv, dtype=torch.float16, device=w.device)
@@ -201,23 +228,13 @@ def sparsify_magnitude(w, V, m, n=2):
 
 def decompress(values, meta, colloc, M, K, V, m, n=2):
     _need_cuda(values, meta, colloc)
+    dense = _native("decompress")(values, meta, colloc, M, K, V, m, n)
+    if dense is not None:
+        return dense
     dense = torch.empty((M, K), dtype=torch.float16, device=values.device)
     _check(lib().vnm_decompress_f16(values.data_ptr(), meta.data_ptr(), colloc.data_ptr(), M, K, V, n, m,
                                     dense.data_ptr(), K, _stream()))
     return dense
-
-
-def _load_product():
-    """The extension's vnm_spmm_f16 call (checks, allocation and launch without the interpreter between them); None if the
-    extension has not been built -- the ctypes path below does the same."""
-    try:
-        from . import spatha_module
-        return spatha_module().product
-    except ImportError:
-        return None
-
-
-_product = None
 
 
 class Prepared:
@@ -233,9 +250,6 @@ class Prepared:
             raise VenomError("values must be fp16, metadata and colloc 32-bit")
         self.M, self.K, self.V, self.m, self.n = M, K, V, m, n
         self.device = values.device
-        global _product
-        if _product is None:
-            _product = _load_product()
         self._h = C.c_void_p()
         if strategy is None:
             _check(lib().vnm_prepare(values.data_ptr(), meta.data_ptr(), colloc.data_ptr(), M, K, V, n, m,
@@ -257,8 +271,8 @@ class Prepared:
 
     def spmm(self, B, bias=None, layout=VNM_LAYOUT_MN, out=None):
         """B: [K,N] fp16 CUDA (unit inner stride).  Returns [M,N] (layout MN) or [N,M] (layout NM)."""
-        if out is None and _product is not None and isinstance(B, torch.Tensor):
-            out = _product(self._h.value or 0, B, bias, self.M, self.K, layout)
+        if out is None and isinstance(B, torch.Tensor):
+            out = _native("product")(self._h.value or 0, B, bias, self.M, self.K, layout)
             if out is not None:
                 return out
         _need_cuda(B, bias, out)

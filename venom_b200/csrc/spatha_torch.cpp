@@ -229,6 +229,94 @@ c10::optional<torch::Tensor> product(int64_t handle, const torch::Tensor &B, con
     return out;
 }
 
+// The format conversions of capi with their allocations, without the interpreter's share.  None: not the plain case, or an error
+// that the caller's own path reports.
+
+// A page-locked word per thread that a violation count is copied to: a copy to pageable memory goes through a staging buffer.
+class HostWord {
+public:
+    ~HostWord() { if (p_) (void)cudaFreeHost(p_); }
+    unsigned long long *get()
+    {
+        if (!p_ && cudaHostAlloc(reinterpret_cast<void **>(&p_), sizeof(*p_), cudaHostAllocPortable) != cudaSuccess) { (void)cudaGetLastError(); p_ = nullptr; }
+        return p_;
+    }
+private:
+    unsigned long long *p_ = nullptr;
+};
+thread_local HostWord t_count;
+
+// Violations counted in `dev` by the work queued so far (waits for it); -1 if they cannot be read.
+int64_t read_count(const torch::Tensor &dev, cudaStream_t stream)
+{
+    unsigned long long *host = t_count.get();
+    if (!host || cudaMemcpyAsync(host, dev.data_ptr(), sizeof(*host), cudaMemcpyDeviceToHost, stream) != cudaSuccess || cudaStreamSynchronize(stream) != cudaSuccess) return -1;
+    return (int64_t)*host;
+}
+
+torch::Tensor new_count(const torch::Tensor &like, cudaStream_t stream)
+{
+    auto t = torch::empty({1}, like.options().dtype(torch::kInt64));
+    TORCH_CHECK(cudaMemsetAsync(t.data_ptr(), 0, 8, stream) == cudaSuccess, "cudaMemsetAsync failed");
+    return t;
+}
+
+bool on_current_device(const torch::Tensor &t) { return t.is_cuda() && t.device().index() == c10::cuda::current_device(); }
+
+using Compressed = std::tuple<torch::Tensor, torch::Tensor, c10::optional<int64_t>>;
+c10::optional<Compressed> compress(const torch::Tensor &dense, const torch::Tensor &colloc, int64_t V, int64_t m, int64_t n, bool count)
+{
+    if (!on_current_device(dense) || !on_current_device(colloc) || dense.scalar_type() != torch::kFloat16 || dense.dim() != 2 || dense.stride(1) != 1) return c10::nullopt;
+    const int64_t M = dense.size(0), K = dense.size(1);
+    int64_t ksp = 0, nv = 0, nm = 0, nc = 0;
+    if (M <= 0 || K <= 0 || M > INT32_MAX || K > INT32_MAX || vnm_sizes((int)M, (int)K, (int)V, (int)n, (int)m, &ksp, &nv, &nm, &nc) != 0) return c10::nullopt;
+    if (colloc.numel() != nc || colloc.element_size() != 4 || !colloc.is_contiguous()) return c10::nullopt;
+    cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
+    auto values = torch::empty({nv}, dense.options());
+    auto meta = torch::empty({nm}, dense.options().dtype(torch::kInt32));
+    torch::Tensor viol;
+    if (count) viol = new_count(dense, stream);
+    if (vnm_compress_f16(dense.data_ptr(), dense.stride(0), nullptr, (const uint32_t *)colloc.data_ptr(), (int)M, (int)K, (int)V, (int)n, (int)m, values.data_ptr(),
+                         (uint32_t *)meta.data_ptr(), count ? (unsigned long long *)viol.data_ptr() : nullptr, stream) != 0)
+        return c10::nullopt;
+    c10::optional<int64_t> bad;
+    if (count) {
+        bad = read_count(viol, stream);
+        if (*bad < 0) return c10::nullopt;
+    }
+    return Compressed(values, meta, bad);
+}
+
+using Sparsified = std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, int64_t>;
+c10::optional<Sparsified> sparsify(const torch::Tensor &w, int64_t V, int64_t m, int64_t n)
+{
+    const bool half = w.scalar_type() == torch::kFloat16;
+    if (!on_current_device(w) || (!half && w.scalar_type() != torch::kFloat32) || w.dim() != 2 || w.stride(1) != 1) return c10::nullopt;
+    const int64_t M = w.size(0), K = w.size(1);
+    int64_t ksp = 0, nv = 0, nm = 0, nc = 0;
+    if (M <= 0 || K <= 0 || M > INT32_MAX || K > INT32_MAX || vnm_sizes((int)M, (int)K, (int)V, (int)n, (int)m, &ksp, &nv, &nm, &nc) != 0) return c10::nullopt;
+    cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
+    const auto words = w.options().dtype(torch::kInt32);
+    auto values = torch::empty({nv}, w.options().dtype(torch::kFloat16));
+    auto meta = torch::empty({nm}, words), cols = torch::empty({nc}, words), viol = new_count(w, stream);
+    if (vnm_sparsify_magnitude(w.data_ptr(), half ? VNM_F16 : VNM_F32, w.stride(0), (int)M, (int)K, (int)V, (int)n, (int)m, values.data_ptr(), (uint32_t *)meta.data_ptr(),
+                               (uint32_t *)cols.data_ptr(), (unsigned long long *)viol.data_ptr(), stream) != 0)
+        return c10::nullopt;
+    const int64_t bad = read_count(viol, stream);
+    if (bad < 0) return c10::nullopt;
+    return Sparsified(values, meta, cols, bad);
+}
+
+c10::optional<torch::Tensor> decompress(const torch::Tensor &values, const torch::Tensor &meta, const torch::Tensor &colloc, int64_t M, int64_t K, int64_t V, int64_t m, int64_t n)
+{
+    if (!on_current_device(values) || !on_current_device(meta) || !on_current_device(colloc) || M <= 0 || K <= 0 || M > INT32_MAX || K > INT32_MAX) return c10::nullopt;
+    auto dense = torch::empty({M, K}, values.options().dtype(torch::kFloat16));
+    if (vnm_decompress_f16(values.data_ptr(), (const uint32_t *)meta.data_ptr(), (const uint32_t *)colloc.data_ptr(), (int)M, (int)K, (int)V, (int)n, (int)m, dense.data_ptr(),
+                           K, c10::cuda::getCurrentCUDAStream().stream()) != 0)
+        return c10::nullopt;
+    return dense;
+}
+
 void clear_cache()
 {
     std::lock_guard<std::mutex> lock(g_mutex);
@@ -250,6 +338,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, mod)
             pybind11::arg("seed"), pybind11::arg("mbrow"), pybind11::arg("brow"));
     mod.def("linear", &linear, "A layer's forward: [..., A_num_cols] -> [..., A_num_rows], or None", pybind11::call_guard<pybind11::gil_scoped_release>());
     mod.def("product", &product, "vnm_spmm_f16 with its allocation, or None", pybind11::call_guard<pybind11::gil_scoped_release>());
+    mod.def("compress", &compress, "vnm_compress_f16 with its allocations, or None", pybind11::call_guard<pybind11::gil_scoped_release>());
+    mod.def("sparsify", &sparsify, "vnm_sparsify_magnitude with its allocations, or None", pybind11::call_guard<pybind11::gil_scoped_release>());
+    mod.def("decompress", &decompress, "vnm_decompress_f16 with its allocation, or None", pybind11::call_guard<pybind11::gil_scoped_release>());
     mod.def("clear_cache", &clear_cache, "Drop every cached prepared operand");
     mod.def("cache_size", &cache_size);
 }
