@@ -941,6 +941,7 @@ __global__ void __launch_bounds__(256) prepare_dense_b_kernel(const __half *__re
 __global__ void __launch_bounds__(256) transpose_kernel(const __half *__restrict__ src, int64_t ld, int N, int K, __half *__restrict__ dst)
 {
     __shared__ uint32_t tile[64 * 33];
+    grid_dependency_wait();
     grid_launch_dependents();   // the product's set-up may begin
     const int k0 = blockIdx.x * 64, n0 = blockIdx.y * 64;
     {
@@ -981,8 +982,14 @@ __global__ void __launch_bounds__(256) transpose_kernel(const __half *__restrict
 cudaError_t launch_transpose(const void *src, int64_t ld_src, int N, int K, void *dst, cudaStream_t stream)
 {
     const dim3 grid((unsigned)((K + 63) / 64), (unsigned)((N + 63) / 64));
-    transpose_kernel<<<grid, 256, 0, stream>>>((const __half *)src, ld_src, N, K, (__half *)dst);
-    return cudaGetLastError();
+    cudaLaunchConfig_t lc = {};
+    cudaLaunchAttribute attr = early_launch();
+    lc.gridDim = grid;
+    lc.blockDim = dim3(256, 1, 1);
+    lc.stream = stream;
+    lc.attrs = &attr;
+    lc.numAttrs = 1;
+    return cudaLaunchKernelEx(&lc, transpose_kernel, (const __half *)src, ld_src, N, K, (__half *)dst);
 }
 
 cudaError_t launch_prepare_dense_b(const void *values, const uint32_t *meta, const uint32_t *colloc, int M, int K, int V, int m,

@@ -38,7 +38,7 @@ struct SpmmParams {
     int l2_ahead;         // pair kernel: k-tiles by which L2 prefetches run ahead of the loads into shared memory (0 = none)
     int out32;            // gather kernel, layout MN: 32-bit stores (ablation)
     int tma_out;          // gather kernel, layout NM: the result leaves through shared memory and TMA stores (tmap_out / OutMaps valid), else from registers
-    int early;            // small kernel: launched before the kernel that writes B has finished (programmatic dependent launch)
+    int early;            // small kernel: the kernel ahead only transposes B; all else may be read before it has finished
     int split_k;          // small kernel: CTAs of a cluster that share one tile's k-tiles
     int n_out;            // destinations of every output tile stored through TMA (1 = `out` only; more: the OutMaps argument, e.g. peers' buffers)
 };
@@ -122,6 +122,19 @@ cudaError_t spmm_dense_b_pair_init();
 float spmm_dense_b_pair_config(int M, int N, int K, int b_nk, int max_ctas, int force_rows, bool multi, SpmmConfig *cfg);  // < 0: not for this problem, else an estimate in microseconds; force_rows: 0 auto, 1 / 2 row tiles per CTA
 cudaError_t launch_spmm_dense_b_pair(const SpmmConfig &cfg, const CUtensorMap &tmap_tile, const CUtensorMap &tmap_tile2, const CUtensorMap &tmap_out, const OutMaps &more_out,
                                      const SpmmParams &p, cudaStream_t stream);
+
+// Every product (and the transpose ahead of one) is launched with this attribute: it may be scheduled once all blocks of the kernel
+// ahead of it in the stream have called grid_launch_dependents() or left, sets up its barriers beside that kernel's last blocks,
+// and waits for its end in grid_dependency_wait() before it touches memory that others use.  Tensor memory is allocated after that
+// wait and dependents are let in only after the allocation: a block that waits for another kernel holds none of what that kernel's
+// blocks may still be waiting for.
+inline cudaLaunchAttribute early_launch()
+{
+    cudaLaunchAttribute a = {};
+    a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    a.val.programmaticStreamSerializationAllowed = 1;
+    return a;
+}
 
 #if defined(__CUDACC__)
 // Programmatic dependent launch: waits until the kernels this launch depends on have finished; lets dependents start.

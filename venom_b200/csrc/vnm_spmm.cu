@@ -106,6 +106,7 @@ __global__ void __launch_bounds__(Traits<BN, NB>::NUM_THREADS, 1)
         *abort_flag = 0;
         fence_barrier_init();
     }
+    grid_dependency_wait();
     if (warp == T::MMA_WARP) {
         tmem_alloc(tmem_slot, T::TMEM_COLS);
         tmem_relinquish();
@@ -114,6 +115,7 @@ __global__ void __launch_bounds__(Traits<BN, NB>::NUM_THREADS, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    grid_launch_dependents();
 
     if (warp < T::PW) {
         // ---------------- B producers ----------------
@@ -364,8 +366,15 @@ cudaError_t launch_one(const SpmmConfig &cfg, const CUtensorMap &tmap_rows, cons
                        const OutMaps &more_out, const SpmmParams &p, cudaStream_t stream)
 {
     using T = Traits<BN, NB>;
-    spmm_kernel<BN, NB><<<(unsigned)cfg.grid, T::NUM_THREADS, T::SMEM_BYTES, stream>>>(tmap_rows, tmap_tile, tmap_out, more_out, p);
-    return cudaGetLastError();
+    cudaLaunchConfig_t lc = {};
+    cudaLaunchAttribute attr = early_launch();
+    lc.gridDim = dim3((unsigned)cfg.grid, 1, 1);
+    lc.blockDim = dim3(T::NUM_THREADS, 1, 1);
+    lc.dynamicSmemBytes = T::SMEM_BYTES;
+    lc.stream = stream;
+    lc.attrs = &attr;
+    lc.numAttrs = 1;
+    return cudaLaunchKernelEx(&lc, spmm_kernel<BN, NB>, tmap_rows, tmap_tile, tmap_out, more_out, p);
 }
 
 int g_num_sms = 0;

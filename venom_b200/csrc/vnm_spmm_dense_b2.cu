@@ -181,6 +181,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
         *abort_flag = 0;
         fence_barrier_init();
     }
+    grid_dependency_wait();
     if (warp == 3) {
         tmem_alloc2(tmem_slot, TMEM_COLS);
         tmem_relinquish2();
@@ -190,6 +191,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
     cluster_sync_all();  // both CTAs' barriers exist before anyone arrives on them remotely
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    grid_launch_dependents();
     // row tile of accumulator rt of this CTA in pair tile (mq, *)
     auto row_tile = [&](int mq, int rt) { return mq * 2 * R + (int)crank * R + rt; };
 
@@ -579,13 +581,14 @@ cudaError_t launch_spmm_dense_b_pair(const SpmmConfig &cfg, const CUtensorMap &t
     lc.blockDim = dim3(NUM_THREADS, 1, 1);
     lc.dynamicSmemBytes = (size_t)cfg.smem_bytes;
     lc.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     lc.attrs = attr;
-    lc.numAttrs = 1;
+    attr[1] = early_launch();
+    lc.numAttrs = 2;
     const bool multi = p.n_out > 1;
 #define VNM_PAIR_LAUNCH(R, BN, MULTI) \
     if (cfg.nb == 2 * R && cfg.bn == BN && multi == MULTI) return cudaLaunchKernelEx(&lc, spmm_dense_b_pair_kernel<R, BN, MULTI>, tmap_tile, tmap_tile2, tmap_out, more_out, p);

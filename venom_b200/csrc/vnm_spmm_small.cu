@@ -99,6 +99,7 @@ __global__ void __launch_bounds__(Small<BN, NB>::NUM_THREADS, 2)
         *abort_flag = 0;
         fence_barrier_init();
     }
+    if (!p.early) grid_dependency_wait();
     if (warp == T::MMA_WARP) {
         tmem_alloc(tmem_slot, T::TMEM_COLS);
         tmem_relinquish();
@@ -107,6 +108,7 @@ __global__ void __launch_bounds__(Small<BN, NB>::NUM_THREADS, 2)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    grid_launch_dependents();
 
     if (warp < T::PW) {
         // ---------------- B producers ----------------
@@ -334,10 +336,7 @@ cudaError_t launch_one(const SpmmConfig &cfg, const CUtensorMap &tmap_b, const S
         attr[lc.numAttrs].val.clusterDim.y = 1;
         attr[lc.numAttrs++].val.clusterDim.z = 1;
     }
-    if (p.early) {
-        attr[lc.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[lc.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
-    }
+    attr[lc.numAttrs++] = early_launch();
     return cudaLaunchKernelEx(&lc, spmm_small_kernel<BN, NB>, tmap_b, p);
 }
 
