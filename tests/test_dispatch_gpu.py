@@ -96,3 +96,19 @@ def test_product_reports_errors_as_before():
     prep.close()
     with pytest.raises(capi.VenomError):
         prep.spmm(_ints((256, 16), 1))
+
+
+# Decompressor: pieces of 8 and of 4 columns, a last piece block that ends inside a row, a ragged last group and last tile, rows
+# aligned to 8 bytes only.
+@pytest.mark.parametrize("cfg", [(64, 96, 32, 16), (32, 1000, 32, 8), (32, 1032, 32, 16), (64, 100, 32, 20), (32, 84, 32, 12), (32, 4104, 32, 24), (128, 2304, 64, 32), (64, 4100, 64, 4)])
+def test_decompress_pieces(cfg):
+    import torch
+    from venom_b200 import capi
+    from venom_b200.synth import random_vnm_dense
+    M, K, V, m = cfg
+    dense, cols, _ = random_vnm_dense(M, K, V, m, seed=K)
+    d = torch.from_numpy(dense).cuda()
+    c = torch.from_numpy(cols.view(np.int32)).cuda()
+    values, meta, bad = capi.compress(d, c, V, m)
+    assert bad == 0
+    assert torch.equal(capi.decompress(values, meta, c, M, K, V, m), d)

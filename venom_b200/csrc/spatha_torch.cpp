@@ -12,6 +12,7 @@
 //     dead, its device copy is released and the operand is re-packed.  In-place edits bump the tensors'
 //     version counters, which are part of the key.
 #include <torch/extension.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
@@ -73,6 +74,12 @@ void sweep_dead_entries()
             ++it;
         }
     }
+}
+
+// torch::empty on the device of `like`, without the dispatcher (0.4 us a call)
+torch::Tensor device_empty(at::IntArrayRef shape, c10::ScalarType type, const torch::Tensor &like)
+{
+    return at::detail::empty_cuda(shape, type, like.device(), c10::nullopt);
 }
 
 void check(int rc, const char *what)
@@ -148,7 +155,7 @@ const void *bias_pointer(const c10::optional<torch::Tensor> &bias, int M)
 void product_nk(vnm_handle_t h, int dense_b, const torch::Tensor &act, int64_t ld, int K, int N, int M, const void *bias, torch::Tensor &out, cudaStream_t stream)
 {
     torch::Tensor ws;
-    if (!dense_b) ws = torch::empty({K, N}, act.options());
+    if (!dense_b) ws = device_empty({K, N}, torch::kFloat16, act);
     check(vnm_spmm_f16_nk_ws(h, act.data_ptr(), ld, N, bias, out.data_ptr(), M, VNM_LAYOUT_NM, dense_b ? out.data_ptr() : ws.data_ptr(), stream),
           "vnm_spmm_f16_nk");
 }
@@ -177,7 +184,7 @@ torch::Tensor spmm(torch::Tensor A_metadata, torch::Tensor A_indices, torch::Ten
     int dense_b = 0;
     const bool in_place = rhs_is_t_view && rhs_matrix.stride(1) % 8 == 0 && (reinterpret_cast<uintptr_t>(rhs_matrix.data_ptr()) & 15) == 0;
     vnm_handle_t h = operand_for(A_metadata, A_indices, A_values, M, K, V, (int)n, (int)m, (int)rhs_matrix.device().index(), N, in_place, stream, &dense_b);
-    auto out = torch::empty({N, M}, rhs_matrix.options());
+    auto out = device_empty({N, M}, torch::kFloat16, rhs_matrix);
     if (in_place) {
         product_nk(h, dense_b, rhs_matrix, rhs_matrix.stride(1), K, N, M, bias_ptr, out, stream);
         return out;
@@ -207,7 +214,7 @@ c10::optional<torch::Tensor> linear(const torch::Tensor &input, const torch::Ten
     vnm_handle_t h = operand_for(A_metadata, A_indices, A_values, M, K, (int)vec_length, (int)n, (int)m, (int)input.device().index(), (int)N, true, stream, &dense_b);
     c10::SmallVector<int64_t, 6> shape(input.sizes().begin(), input.sizes().end());
     shape.back() = M;
-    auto out = torch::empty(shape, input.options());
+    auto out = device_empty(shape, torch::kFloat16, input);
     product_nk(h, dense_b, input, K, K, (int)N, M, bias_ptr, out, stream);
     return out;
 }
@@ -222,7 +229,7 @@ c10::optional<torch::Tensor> product(int64_t handle, const torch::Tensor &B, con
     if ((layout != VNM_LAYOUT_MN && layout != VNM_LAYOUT_NM) || B.device().index() != c10::cuda::current_device()) return c10::nullopt;
     const int64_t N = B.size(1);
     if (N <= 0 || N > INT32_MAX) return c10::nullopt;
-    auto out = layout == VNM_LAYOUT_MN ? torch::empty({M, N}, B.options()) : torch::empty({N, M}, B.options());
+    auto out = layout == VNM_LAYOUT_MN ? device_empty({M, N}, torch::kFloat16, B) : device_empty({N, M}, torch::kFloat16, B);
     if (vnm_spmm_f16(reinterpret_cast<vnm_handle_t>(handle), B.data_ptr(), B.stride(0), (int)N, bias.has_value() ? bias->data_ptr() : nullptr, out.data_ptr(),
                      out.stride(0), (int)layout, c10::cuda::getCurrentCUDAStream().stream()) != 0)
         return c10::nullopt;
@@ -256,7 +263,7 @@ int64_t read_count(const torch::Tensor &dev, cudaStream_t stream)
 
 torch::Tensor new_count(const torch::Tensor &like, cudaStream_t stream)
 {
-    auto t = torch::empty({1}, like.options().dtype(torch::kInt64));
+    auto t = device_empty({1}, torch::kInt64, like);
     TORCH_CHECK(cudaMemsetAsync(t.data_ptr(), 0, 8, stream) == cudaSuccess, "cudaMemsetAsync failed");
     return t;
 }
@@ -272,8 +279,8 @@ c10::optional<Compressed> compress(const torch::Tensor &dense, const torch::Tens
     if (M <= 0 || K <= 0 || M > INT32_MAX || K > INT32_MAX || vnm_sizes((int)M, (int)K, (int)V, (int)n, (int)m, &ksp, &nv, &nm, &nc) != 0) return c10::nullopt;
     if (colloc.numel() != nc || colloc.element_size() != 4 || !colloc.is_contiguous()) return c10::nullopt;
     cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
-    auto values = torch::empty({nv}, dense.options());
-    auto meta = torch::empty({nm}, dense.options().dtype(torch::kInt32));
+    auto values = device_empty({nv}, torch::kFloat16, dense);
+    auto meta = device_empty({nm}, torch::kInt32, dense);
     torch::Tensor viol;
     if (count) viol = new_count(dense, stream);
     if (vnm_compress_f16(dense.data_ptr(), dense.stride(0), nullptr, (const uint32_t *)colloc.data_ptr(), (int)M, (int)K, (int)V, (int)n, (int)m, values.data_ptr(),
@@ -296,9 +303,8 @@ c10::optional<Sparsified> sparsify(const torch::Tensor &w, int64_t V, int64_t m,
     int64_t ksp = 0, nv = 0, nm = 0, nc = 0;
     if (M <= 0 || K <= 0 || M > INT32_MAX || K > INT32_MAX || vnm_sizes((int)M, (int)K, (int)V, (int)n, (int)m, &ksp, &nv, &nm, &nc) != 0) return c10::nullopt;
     cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
-    const auto words = w.options().dtype(torch::kInt32);
-    auto values = torch::empty({nv}, w.options().dtype(torch::kFloat16));
-    auto meta = torch::empty({nm}, words), cols = torch::empty({nc}, words), viol = new_count(w, stream);
+    auto values = device_empty({nv}, torch::kFloat16, w);
+    auto meta = device_empty({nm}, torch::kInt32, w), cols = device_empty({nc}, torch::kInt32, w), viol = new_count(w, stream);
     if (vnm_sparsify_magnitude(w.data_ptr(), half ? VNM_F16 : VNM_F32, w.stride(0), (int)M, (int)K, (int)V, (int)n, (int)m, values.data_ptr(), (uint32_t *)meta.data_ptr(),
                                (uint32_t *)cols.data_ptr(), (unsigned long long *)viol.data_ptr(), stream) != 0)
         return c10::nullopt;
@@ -310,7 +316,7 @@ c10::optional<Sparsified> sparsify(const torch::Tensor &w, int64_t V, int64_t m,
 c10::optional<torch::Tensor> decompress(const torch::Tensor &values, const torch::Tensor &meta, const torch::Tensor &colloc, int64_t M, int64_t K, int64_t V, int64_t m, int64_t n)
 {
     if (!on_current_device(values) || !on_current_device(meta) || !on_current_device(colloc) || M <= 0 || K <= 0 || M > INT32_MAX || K > INT32_MAX) return c10::nullopt;
-    auto dense = torch::empty({M, K}, values.options().dtype(torch::kFloat16));
+    auto dense = device_empty({M, K}, torch::kFloat16, values);
     if (vnm_decompress_f16(values.data_ptr(), (const uint32_t *)meta.data_ptr(), (const uint32_t *)colloc.data_ptr(), (int)M, (int)K, (int)V, (int)n, (int)m, dense.data_ptr(),
                            K, c10::cuda::getCurrentCUDAStream().stream()) != 0)
         return c10::nullopt;

@@ -112,6 +112,9 @@ def sparse_dense_mul_dispatch(sparse_values, sparse_indices, sparse_metadata, de
     return spatha_module().spmm(sparse_metadata, sparse_indices, sparse_values, dense_, bias, nrows_sp, ncols_sp, ncols_d, v, n, m, nnz, 0, 32, 4)
 
 
+_linear = None     # the extension's call, looked up once
+
+
 class SrnmSpmm(torch.nn.Module):
     """Drop-in replacement of torch.nn.Linear whose weight is stored in V:N:M form."""
 
@@ -130,7 +133,10 @@ class SrnmSpmm(torch.nn.Module):
         p = self._parameters
         bias = p["bias"] if "bias" in p else self.bias
         values = p["values"] if "values" in p else self.values
-        out = spatha_module().linear(input, self.metadata, self.columns, values, bias, self.nrows_sp, self.ncols_sp, self.v, self.n, self.m)
+        global _linear
+        if _linear is None:
+            _linear = spatha_module().linear
+        out = _linear(input, self.metadata, self.columns, values, bias, self.nrows_sp, self.ncols_sp, self.v, self.n, self.m)
         if out is not None:
             return out
         flat = torch.flatten(input, start_dim=0, end_dim=-2)
