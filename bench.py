@@ -466,7 +466,7 @@ def main():
     form = "dense-B" if prep.dense_b_form() else "gather"
     kcfg = prep.config(ns)
     kernel_name = ("vnm::spmm_dense_b_pair_kernel (clusters of two CTAs, tcgen05 cta_group::2)" if (form == "dense-B" and kcfg["stages"] == 2) else
-                   "vnm::spmm_dense_b_kernel" if form == "dense-B" else "vnm::spmm_kernel")
+                   "vnm::spmm_small_kernel" if kcfg["stages"] == 1 else "vnm::spmm_kernel")
 
     if args.kernel_only:
         if rank == 0:

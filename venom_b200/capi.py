@@ -363,7 +363,7 @@ class Prepared:
         _check(lib().vnm_set_gather_split(self._h, tma_rows))
 
     def set_pair_mode(self, mode):
-        """Dense-B form: 1 = two-SM (cta_group::2) kernel where it applies (default), 0 = single-SM kernel only,
+        """Dense-B form: 1 = two-SM (cta_group::2) kernel where it applies (default), 0 = one SM per tile where possible,
         2 = pairs without L2 hints, 3 / 4 = pairs with one / two row tiles per CTA forced where the shape allows."""
         _check(lib().vnm_set_pair_mode(self._h, mode))
 

@@ -469,7 +469,7 @@ bool choose_kernel(vnm_handle_t h, int N, int b_nk, int n_more, Kernel *kernel, 
             *us = small;
         }
     }
-    if (*us < 0.0f && h->dense_b) *us = spmm_dense_b_pair_config(h->M, N, h->K, b_nk, h->max_ctas, h->pair_rows, n_more > 0, cfg);   // one SM per tile is not to be had
+    if (*us < 0.0f && h->dense_b) *us = spmm_dense_b_pair_config(h->M, N, h->K, b_nk, h->max_ctas, h->pair_rows, n_more > 0, cfg);   // switched off, but nothing else takes it
     return *us >= 0.0f;
 }
 
@@ -629,7 +629,7 @@ static int spmm_impl(vnm_handle_t h, const void *B, int64_t ldb, int N, int b_nk
         // keeps either `g` row groups of A (18 KiB per row tile and k-tile) or `q` column panels of B (K x tile-N fp16)
         // within about 32 MB while the other operand streams past; the cheaper of the two in bytes re-read from HBM wins:
         //   row bands: A once + B once per band;   column bands: B once + A once per band.
-        const int64_t rows_per_group = h->dense_b ? (int64_t)cfg.nb * TILE_M : TILE_M;   // dense-B: 256 / 128 (one SM per tile) or 512 (pairs); gather: 128
+        const int64_t rows_per_group = h->dense_b ? (int64_t)cfg.nb * TILE_M : TILE_M;   // pairs: 256 or 512; gather: 128
         const int64_t row_groups = (h->M + rows_per_group - 1) / rows_per_group;
         const int64_t bytes_per_group = (rows_per_group / TILE_M) * (int64_t)h->ktiles * AM_BLOCK_BYTES;
         const int64_t bytes_per_panel = (int64_t)h->K * cfg.bn * 2;
@@ -641,7 +641,7 @@ static int spmm_impl(vnm_handle_t h, const void *B, int64_t ldb, int N, int b_nk
         const double a_total = (double)row_groups * bytes_per_group, b_total = (double)p.ntiles * bytes_per_panel;
         const double cost_rows = a_total + b_total * (double)((row_groups + g - 1) / g);
         const double cost_cols = b_total + a_total * (double)((p.ntiles + q - 1) / q);
-        const bool col_bands = pair && cost_cols < cost_rows;   // the one-SM and gather kernels keep row bands
+        const bool col_bands = pair && cost_cols < cost_rows;   // the gather kernel keeps row bands
         p.group_m = col_bands ? -(int)q : (int)g;
         p.hint_a = col_bands ? L2_EVICT_NORMAL : L2_EVICT_LAST;
         p.hint_b = col_bands ? L2_EVICT_LAST : L2_EVICT_NORMAL;
