@@ -227,11 +227,6 @@ __device__ __forceinline__ bool named_barrier_and(uint32_t id, uint32_t threads,
         : "memory");
     return r != 0;
 }
-// 8-byte asynchronous copy global -> shared (8-byte aligned on both sides), grouped with commit / wait.
-__device__ __forceinline__ void cp_async_8(uint32_t saddr, const void *gsrc)
-{
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(saddr), "l"(gsrc) : "memory");
-}
 // 16-byte asynchronous copy global -> shared that bypasses L1; src_bytes = 16 copies, 0 writes zeros (src is not read).
 __device__ __forceinline__ void cp_async_16_zfill(uint32_t saddr, const void *gsrc, uint32_t src_bytes)
 {
@@ -244,12 +239,6 @@ __device__ __forceinline__ void cp_async_mbar_arrive_noinc(uint64_t *bar)
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int kPending>
-__device__ __forceinline__ void cp_async_wait()
-{
-    asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory");
-}
 // Register re-allocation between warpgroups (all four warps of a warpgroup must execute the same one).
 template <int kRegs>
 __device__ __forceinline__ void setmaxnreg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegs)); }

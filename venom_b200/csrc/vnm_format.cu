@@ -5,239 +5,112 @@
 namespace vnm {
 
 // ------------------------------------------------------------------------------------------------
-// Compressor, general form (any alignment, any m).  One thread owns one metadata word = (row pair 2p,2p+1) x (tile t of four groups):
-// it scans 2 x 4 groups x 4 column-loc candidates of the pruned dense matrix in ascending order,
-// emits the first two kept entries of every (row, group) as values + 2-bit positions, and writes one
-// 32-bit metadata word plus four 8-byte value pieces.  Threads of a warp walk consecutive tiles of
-// the same row pair, so the dense reads of a warp cover 32*4*m consecutive columns of two rows.
+// Compressor, general form (any m, alignment and K, with or without a mask).  A thread owns one group of the 16 rows of a value
+// strip; neighbouring lanes own neighbouring groups.  Of every row it loads the four candidate entries only (two bytes each; the
+// lanes of a warp cover a contiguous piece of the row, so a sector is fetched once and only if a candidate lies in it), four rows
+// at a time, and keeps the first two in ascending order.  The kept pairs of four consecutive rows are one 16-byte piece of the
+// reference's value order [sub-block][group][row][slot]; the four lanes of a tile OR their metadata nibbles with shuffles and write
+// the strip's 32 bytes of the tile's metadata.  Bound by the sectors fetched (HBM); staging whole rows in shared memory
+// instead (the kernel before this one) took 113 us at 12288 x 12280, m = 20, 93 at m = 32, and 398 with a mask at m = 16.
 // Follows Format_sr_nm<T>::to_sparse_sr_nm (format_sr_nm.cpp:441-536): candidates with an original
 // column >= K contribute a (position 0, value 0) slot for j < 2 only (:486-500).
 // ------------------------------------------------------------------------------------------------
+constexpr int GATHER_THREADS = 128;
 template <bool kHasMask>
-__global__ void __launch_bounds__(256) compress_kernel(const __half *__restrict__ dense, int64_t ldd, const int32_t *__restrict__ mask,
-                                                       const uint32_t *__restrict__ colloc, int M, int K, int V, int m, int64_t Ksp,
-                                                       __half *__restrict__ values, uint32_t *__restrict__ meta,
-                                                       unsigned long long *violations)
+__global__ void __launch_bounds__(GATHER_THREADS) compress_gather_kernel(const __half *__restrict__ dense, int64_t ldd, const int32_t *__restrict__ mask,
+                                                                         const uint32_t *__restrict__ colloc, int K, int V, int m, int64_t Ksp, uint32_t spans,
+                                                                         uint32_t items, int wide, uint32_t *__restrict__ values, uint32_t *__restrict__ meta,
+                                                                         unsigned long long *violations)
 {
+    const int lane = threadIdx.x & 31, gi = lane & 3;
     const int64_t tiles = Ksp / 8;
-    const int64_t total = (int64_t)(M / 2) * tiles;
     unsigned int bad = 0;
-    for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t rp = idx / tiles;
-        const int64_t t = idx - rp * tiles;
-        uint32_t word = 0;
-        const int64_t r0 = rp * 2;
-        const uint4 *c4p = reinterpret_cast<const uint4 *>(colloc + (r0 / V) * (Ksp / 2) * 4 + t * 16);
-        // values of rows r0, r0+1 for group gi are 4 consecutive halves at vbase + gi*8
-        const int64_t vbase = (r0 / 16) * 16 * Ksp + t * 128 + ((r0 % 16) / 4) * 32 + (r0 % 4) * 2;
+    for (uint32_t item = blockIdx.x; item < items; item += gridDim.x) {
+        const uint32_t strip = item / spans;
+        const int64_t G = (int64_t)(item - strip * spans) * GATHER_THREADS + threadIdx.x;
+        const bool on = G < Ksp / 2;              // whole tiles: the four lanes of one agree
+        const int64_t T = on ? G >> 2 : 0;
+        const int64_t r0 = (int64_t)strip * 16;
+        uint32_t cand[4] = {0, 0, 0, 0};
+        if (on) {
+            const uint4 c4 = __ldg(reinterpret_cast<const uint4 *>(colloc + (r0 / V) * (Ksp / 2) * 4) + G);
+            cand[0] = c4.x; cand[1] = c4.y; cand[2] = c4.z; cand[3] = c4.w;
+        }
+        const int64_t col0 = G * m;
+        // a column offset outside its group: nothing of the group is read, its slots are zero and every row counts as a violation
+        const bool corrupt = cand[0] >= (uint32_t)m || cand[1] >= (uint32_t)m || cand[2] >= (uint32_t)m || cand[3] >= (uint32_t)m;
+        bool inside[4];
 #pragma unroll
-        for (int gi = 0; gi < 4; gi++) {
-            const uint4 c4 = __ldg(c4p + gi);
-            const uint32_t cand[4] = {c4.x, c4.y, c4.z, c4.w};
-            const int64_t g = t * 4 + gi;
-            unsigned short out[4] = {0, 0, 0, 0};
+        for (int j = 0; j < 4; j++) inside[j] = on && !corrupt && col0 + (int64_t)cand[j] < K;
+        uint32_t words[8];
+        const __half *row = dense + r0 * ldd + col0;
+        const int32_t *mrow = kHasMask ? mask + r0 * ldd + col0 : nullptr;
+        uint32_t *vdst = values + (r0 * Ksp + T * 128) / 2 + gi * 4;
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const __half *drow = dense + (r0 + h) * ldd;
-                const int32_t *mrow = kHasMask ? mask + (r0 + h) * ldd : nullptr;
+        for (int sb = 0; sb < 4; sb++) {
+            unsigned short x[4][4];
+            int32_t keep[4][4];
+#pragma unroll
+            for (int r = 0; r < 4; r++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const int64_t at = (int64_t)(sb * 4 + r) * ldd + cand[j];
+                    x[r][j] = inside[j] ? __ldg(reinterpret_cast<const unsigned short *>(row) + at) : (unsigned short)0;
+                    if (kHasMask) keep[r][j] = inside[j] ? __ldg(mrow + at) : 0;
+                }
+            uint32_t out[4];
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                uint32_t two = 0, nib = 0;
                 int pos = 0;
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
-                    const int64_t col = g * m + (int64_t)cand[j];
-                    if (cand[j] >= (uint32_t)m) {
-                        pos = 3;  // a column offset outside its group (corrupt column-loc): counted as a violation, never read
-                    } else if (col < K) {
-                        const unsigned short bits = __half_as_ushort(drow[col]);
-                        const bool keep = kHasMask ? (mrow[col] != 0) : ((bits & 0x7FFFu) != 0);  // value != +-0
-                        if (keep) {
+                    if (inside[j]) {
+                        if (kHasMask ? keep[r][j] != 0 : (x[r][j] & 0x7FFFu) != 0) {  // value != +-0
                             if (pos < 2) {
-                                out[h * 2 + pos] = bits;
-                                word |= (uint32_t)j << (h * 16 + gi * 4 + pos * 2);
+                                two |= (uint32_t)x[r][j] << (16 * pos);
+                                nib |= (uint32_t)j << (2 * pos);
                             }
                             pos++;
                         }
                     } else if (j < 2) {
-                        pos++;  // slot (position 0, value 0): nothing to OR in
+                        pos++;   // slot (position 0, value 0): nothing to OR in
                     }
                 }
-                bad += (pos != 2);
+                bad += on && (corrupt || pos != 2);
+                out[r] = two;
+                // word of rows (2i, 2i + 1) of the strip: 16 bits a row, four a group
+                if (r & 1) words[sb * 2 + (r >> 1)] |= nib << (16 + 4 * gi);
+                else words[sb * 2 + (r >> 1)] = nib << (4 * gi);
             }
-            uint2 pk;
-            pk.x = (uint32_t)out[0] | ((uint32_t)out[1] << 16);
-            pk.y = (uint32_t)out[2] | ((uint32_t)out[3] << 16);
-            *reinterpret_cast<uint2 *>(values + vbase + gi * 8) = pk;
-        }
-        meta[(r0 / 32) * 16 * tiles + t * 16 + (r0 % 32) / 2] = word;
-    }
-    if (violations != nullptr) {
-        for (int o = 16; o > 0; o >>= 1) bad += __shfl_xor_sync(0xffffffffu, bad, o);
-        if ((threadIdx.x & 31) == 0 && bad) atomicAdd(violations, (unsigned long long)bad);
-    }
-}
-
-// ------------------------------------------------------------------------------------------------
-// Tiled compressor (the one normally used).  A CTA takes 32 rows (inside one V-block, so one column-loc
-// row) x TS tiles of four groups = TS*4*m consecutive columns:
-//   1. the 32 dense row segments come in with coalesced 8-byte asynchronous copies into one of two
-//      shared-memory buffers (row pitch an odd number of words, so 32 lanes reading one column of 32 rows
-//      hit 32 banks), one chunk ahead of the work; in mask mode the int32 mask is folded into one bit per
-//      element;
-//   2. lane = row, warp = tile: the same selection as compress_kernel, results staged in shared memory in
-//      the reference's value order (128 halves per 16 rows x tile) and metadata order (16 words per
-//      32 rows x tile);
-//   3. both stagings are contiguous in global memory (TS*256 bytes per 16 rows, TS*64 bytes of metadata)
-//      and leave with 16-byte stores.
-// Needs 8-byte aligned dense and mask rows and an even m; launch_compress falls back to compress_kernel
-// otherwise.
-// ------------------------------------------------------------------------------------------------
-template <bool kHasMask>
-__global__ void __launch_bounds__(256) compress_tiled_kernel(const __half *__restrict__ dense, int64_t ldd, const int32_t *__restrict__ mask,
-                                                             const uint32_t *__restrict__ colloc, int M, int K, int V, int m, int64_t Ksp, int TS,
-                                                             uint32_t *__restrict__ values, uint32_t *__restrict__ meta,
-                                                             unsigned long long *violations)
-{
-    extern __shared__ __align__(16) uint8_t csm[];
-    const int span = TS * 4 * m;                 // columns per chunk, even
-    const int pitch = span + 4;                  // halves; 8-byte aligned rows, pitch / 2 = 2 mod 32: rows r and r+16 share banks
-    const int mpitch = ((span / 2 + 7) & ~7) + 4;  // mask bytes per row (two bits per byte); mpitch / 4 is odd
-    uint32_t *val_s = reinterpret_cast<uint32_t *>(csm);                 // [2][TS][64]
-    uint32_t *meta_s = val_s + 2 * TS * 64;                              // [TS][16]
-    unsigned short *in_s = reinterpret_cast<unsigned short *>(meta_s + TS * 16);  // [2 buffers][32][pitch]
-    uint8_t *mk_s = reinterpret_cast<uint8_t *>(in_s + 2 * 32 * pitch);  // [32][mpitch]
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t tiles = Ksp / 8;
-    const int spans = (int)((tiles + TS - 1) / TS);
-    const int64_t chunks = (int64_t)(M / 32) * spans;
-    unsigned int bad = 0;
-
-    // Asynchronous 8-byte copies bring the 32 row segments of a chunk into one of two buffers: a warp takes
-    // rows warp, warp+8, ..., its lanes consecutive pieces, so global reads are coalesced and shared-memory
-    // writes hit consecutive banks.  The chunk after the current one is in flight while this one is worked on.
-    auto fetch = [&](int64_t ch, int buf) {
-        const int64_t rc = ch / spans;
-        const int64_t c0 = (ch - rc * spans) * TS * 4 * m;
-        const int valid = (int)(c0 >= K ? 0 : (K - c0 < span ? K - c0 : span));
-        const int nq = (valid + 3) / 4;  // 8-byte pieces per row holding existing columns
-        for (int r = warp; r < 32; r += 8) {
-            const __half *drow = dense + (rc * 32 + r) * ldd + c0;
-            unsigned short *srow = in_s + (buf * 32 + r) * pitch;
-            const uint32_t sbase = smem_u32(srow);
-#pragma unroll 4
-            for (int q = lane; q < nq; q += 32) {
-                if (4 * q + 4 <= valid) {
-                    cp_async_8(sbase + q * 8, reinterpret_cast<const uint2 *>(drow) + q);
-                } else {  // ragged end of the matrix
-                    for (int c = 4 * q; c < valid; c++) srow[c] = __half_as_ushort(drow[c]);
-                }
-            }
-        }
-        cp_async_commit();
-    };
-
-    int buf = 0;
-    if ((int64_t)blockIdx.x < chunks) fetch(blockIdx.x, 0);
-    for (int64_t ch = blockIdx.x; ch < chunks; ch += gridDim.x, buf ^= 1) {
-        const int64_t rc = ch / spans;
-        const int sp = (int)(ch - rc * spans);
-        const int64_t R0 = rc * 32;
-        const int64_t t0 = (int64_t)sp * TS;
-        const int tcount = (int)(tiles - t0 < TS ? tiles - t0 : TS);
-        const int64_t c0 = t0 * 4 * m;
-        if (ch + gridDim.x < chunks) {
-            fetch(ch + gridDim.x, buf ^ 1);
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
-        }
-        if (kHasMask) {  // the int32 mask, folded into one bit per element
-            const int valid = (int)(c0 >= K ? 0 : (K - c0 < span ? K - c0 : span));
-            const int nw = (valid + 1) / 2;
-            for (int r = warp; r < 32; r += 8) {
-                const int32_t *mrow = mask + (R0 + r) * ldd + c0;
-                for (int w = lane; w < nw; w += 32) {
-                    uint32_t mb;
-                    if (2 * w + 1 < valid) {
-                        const int2 mm = __ldg(reinterpret_cast<const int2 *>(mrow) + w);
-                        mb = (mm.x != 0) | ((mm.y != 0) << 1);
-                    } else {
-                        mb = mrow[2 * w] != 0;
-                    }
-                    mk_s[r * mpitch + w] = (uint8_t)mb;
-                }
-            }
-        }
-        __syncthreads();
-        // ---- lane = row, warp = tile
-        const uint32_t *crow = colloc + (R0 / V) * (Ksp / 2) * 4;
-        const unsigned short *my_in = in_s + (buf * 32 + lane) * pitch;
-        const uint8_t *my_mk = mk_s + lane * mpitch;
-        const int validc = (int)(c0 >= K ? 0 : (K - c0 < span ? K - c0 : span));
-        for (int tl = warp; tl < tcount; tl += 8) {
-            uint32_t hw = 0;
-            uint32_t *vdst = val_s + ((lane >> 4) * TS + tl) * 64 + ((lane & 15) >> 2) * 16 + (lane & 3);
-            const uint4 *c4p = reinterpret_cast<const uint4 *>(crow + (t0 + tl) * 16);
-#pragma unroll
-            for (int gi = 0; gi < 4; gi++) {
-                const uint4 c4 = __ldg(c4p + gi);
-                const int cand[4] = {(int)c4.x, (int)c4.y, (int)c4.z, (int)c4.w};
-                const int lg = (tl * 4 + gi) * m;  // first column of the group, relative to the chunk
-                uint32_t out = 0;
-                int pos = 0;
-                if (max(max(c4.x, c4.y), max(c4.z, c4.w)) >= (uint32_t)m) {
-                    pos = 3;  // a column offset outside its group (corrupt column-loc): counted as a violation, nothing is read
-                } else if (lg + m <= validc) {  // the whole group exists (same for every lane)
-#pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        const int lc = lg + cand[j];
-                        const uint32_t bits = my_in[lc];
-                        const bool keep = kHasMask ? ((my_mk[lc >> 1] >> (lc & 1)) & 1) != 0 : (bits & 0x7FFFu) != 0;
-                        if (keep) {
-                            if (pos < 2) {
-                                out |= bits << (16 * pos);
-                                hw |= (uint32_t)j << (gi * 4 + pos * 2);
-                            }
-                            pos++;
-                        }
-                    }
+            if (on) {
+                if (wide) {
+                    *reinterpret_cast<uint4 *>(vdst + sb * 16) = make_uint4(out[0], out[1], out[2], out[3]);
                 } else {
 #pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        const int lc = lg + cand[j];
-                        if (lc < validc) {
-                            const uint32_t bits = my_in[lc];
-                            const bool keep = kHasMask ? ((my_mk[lc >> 1] >> (lc & 1)) & 1) != 0 : (bits & 0x7FFFu) != 0;
-                            if (keep) {
-                                if (pos < 2) {
-                                    out |= bits << (16 * pos);
-                                    hw |= (uint32_t)j << (gi * 4 + pos * 2);
-                                }
-                                pos++;
-                            }
-                        } else if (j < 2) {
-                            pos++;  // slot (position 0, value 0) of a column past K
-                        }
-                    }
+                    for (int r = 0; r < 4; r++) vdst[sb * 16 + r] = out[r];
                 }
-                bad += (pos != 2);
-                vdst[gi * 4] = out;
             }
-            const uint32_t other = __shfl_xor_sync(0xffffffffu, hw, 1);
-            if ((lane & 1) == 0) meta_s[tl * 16 + (lane >> 1)] = hw | (other << 16);
         }
-        __syncthreads();
-        // ---- staged values and metadata -> global memory
-        const int vq = tcount * 16;  // 16-byte pieces per 16-row group
-        for (int i = threadIdx.x; i < 2 * vq; i += 256) {
-            const int rg = i >= vq ? 1 : 0;
-            const int k = i - rg * vq;
-            uint4 *dst = reinterpret_cast<uint4 *>(values + ((R0 / 16 + rg) * 16 * Ksp + t0 * 128) / 2);
-            dst[k] = reinterpret_cast<const uint4 *>(val_s + rg * TS * 64)[k];
+#pragma unroll
+        for (int w = 0; w < 8; w++) {
+            words[w] |= __shfl_xor_sync(0xffffffffu, words[w], 1);
+            words[w] |= __shfl_xor_sync(0xffffffffu, words[w], 2);
         }
-        uint4 *mdst = reinterpret_cast<uint4 *>(meta + (R0 / 32) * 16 * tiles + t0 * 16);
-        for (int i = threadIdx.x; i < tcount * 4; i += 256) mdst[i] = reinterpret_cast<const uint4 *>(meta_s)[i];
+        if (on) {
+            uint32_t *mdst = meta + (int64_t)(strip >> 1) * 16 * tiles + T * 16 + (strip & 1u) * 8 + gi * 2;
+            const uint32_t lo = gi == 0 ? words[0] : gi == 1 ? words[2] : gi == 2 ? words[4] : words[6];
+            const uint32_t hi = gi == 0 ? words[1] : gi == 1 ? words[3] : gi == 2 ? words[5] : words[7];
+            if (wide) {
+                *reinterpret_cast<uint2 *>(mdst) = make_uint2(lo, hi);
+            } else {
+                mdst[0] = lo;
+                mdst[1] = hi;
+            }
+        }
     }
     if (violations != nullptr) {
-        for (int o = 16; o > 0; o >>= 1) bad += __shfl_xor_sync(0xffffffffu, bad, o);
+        bad = __reduce_add_sync(0xffffffffu, bad);
         if (lane == 0 && bad) atomicAdd(violations, (unsigned long long)bad);
     }
 }
@@ -448,38 +321,16 @@ cudaError_t launch_compress(const void *dense, int64_t ldd, const int32_t *mask,
             return cudaGetLastError();
         }
     }
-    const bool aligned = ldd % 4 == 0 && ((uintptr_t)dense & 7) == 0 && ((uintptr_t)mask & 7) == 0 && ((uintptr_t)meta & 15) == 0 &&
-                         m <= 128 && M % 32 == 0 && V % 32 == 0;
-    if (aligned) {
-        const int TS = m >= 128 ? 1 : (m <= 8 ? 16 : 128 / m);  // at most 512 columns per chunk
-        const int span = TS * 4 * m;
-        const size_t smem = (size_t)(2 * TS * 64 + TS * 16) * 4 + (size_t)2 * 32 * (span + 4) * 2 + (mask ? (size_t)32 * (((span / 2 + 7) & ~7) + 4) : 0);
-        const int64_t chunks = (int64_t)(M / 32) * ((Ksp / 8 + TS - 1) / TS);
-        int64_t blocks = chunks < (int64_t)148 * 3 ? chunks : (int64_t)148 * 3;
-        // up to ~83 KiB: two input buffers, the output staging and the mask bits
-        cudaError_t e = mask ? cudaFuncSetAttribute(compress_tiled_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024)
-                             : cudaFuncSetAttribute(compress_tiled_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-        if (e != cudaSuccess) return e;
-        if (blocks < 1) blocks = 1;
-        if (mask)
-            compress_tiled_kernel<true><<<(unsigned)blocks, threads, smem, stream>>>((const __half *)dense, ldd, mask, colloc, M, K, V, m, Ksp, TS,
-                                                                                   (uint32_t *)values, meta, violations);
-        else
-            compress_tiled_kernel<false><<<(unsigned)blocks, threads, smem, stream>>>((const __half *)dense, ldd, mask, colloc, M, K, V, m, Ksp, TS,
-                                                                                    (uint32_t *)values, meta, violations);
-        return cudaGetLastError();
-    }
-    const int64_t total = (int64_t)(M / 2) * (Ksp / 8);
-    int64_t blocks = (total + threads - 1) / threads;
-    const int64_t cap = (int64_t)148 * 64;
-    if (blocks > cap) blocks = cap;
-    if (blocks < 1) blocks = 1;
+    const int64_t spans = (Ksp / 2 + GATHER_THREADS - 1) / GATHER_THREADS, items = (int64_t)(M / 16) * spans;
+    if (items >= ((int64_t)1 << 32)) return cudaErrorInvalidValue;
+    const unsigned blocks = (unsigned)(items < (1 << 20) ? items : (1 << 20));
+    const int wide = ((uintptr_t)values & 15) == 0 && ((uintptr_t)meta & 7) == 0;
     if (mask)
-        compress_kernel<true><<<(unsigned)blocks, threads, 0, stream>>>((const __half *)dense, ldd, mask, colloc, M, K, V, m, Ksp,
-                                                                       (__half *)values, meta, violations);
+        compress_gather_kernel<true><<<blocks, GATHER_THREADS, 0, stream>>>((const __half *)dense, ldd, mask, colloc, K, V, m, Ksp, (uint32_t)spans, (uint32_t)items, wide,
+                                                                            (uint32_t *)values, meta, violations);
     else
-        compress_kernel<false><<<(unsigned)blocks, threads, 0, stream>>>((const __half *)dense, ldd, mask, colloc, M, K, V, m, Ksp,
-                                                                        (__half *)values, meta, violations);
+        compress_gather_kernel<false><<<blocks, GATHER_THREADS, 0, stream>>>((const __half *)dense, ldd, mask, colloc, K, V, m, Ksp, (uint32_t)spans, (uint32_t)items, wide,
+                                                                             (uint32_t *)values, meta, violations);
     return cudaGetLastError();
 }
 
@@ -509,7 +360,7 @@ __global__ void __launch_bounds__(256) decompress_kernel(const __half *__restric
 }
 
 // ------------------------------------------------------------------------------------------------
-// Tiled decompressor (the one normally used): the mirror image of compress_tiled_kernel.  A CTA takes 32 rows x
+// Tiled decompressor (m not a multiple of four, or rows aligned to two bytes only):  A CTA takes 32 rows x
 // TS tiles: the values (TS * 256 contiguous bytes per 16 rows) and metadata (TS * 64 bytes) come in with 16-byte
 // loads, lane = row / warp = tile scatters the two values of every (row, group) into a zeroed shared-memory image
 // of the 32 dense row segments (slot 0 first, like the general kernel), and the image leaves with 8-byte stores.
@@ -583,87 +434,12 @@ __global__ void __launch_bounds__(256) decompress_tiled_kernel(const uint32_t *_
 }
 
 // ------------------------------------------------------------------------------------------------
-// Decompressor, register form: the mirror image of compress_direct_kernel (used for m in {4, 8}, whole
-// tiles, V % 16 == 0, aligned rows).  Lanes lie along the row; a thread owns one group (two for m = 4) of the 16 rows of
-// a strip.  For four consecutive rows its kept pairs are one 16-byte piece of the value array and its metadata nibbles
-// sit in the tile's two metadata words of those rows; it rebuilds the m halves of the group in registers (zeros, slot 0,
-// then slot 1, so a padded slot overwrites as in the reference's loop order) and stores them with 16-byte stores: a
-// warp writes 512 contiguous bytes of a row (1 KiB for m = 16).  Every output element is written exactly once.
-// ------------------------------------------------------------------------------------------------
-template <int M_>
-__global__ void __launch_bounds__(256) decompress_direct_kernel(const uint32_t *__restrict__ values, const uint32_t *__restrict__ meta,
-                                                                const uint32_t *__restrict__ colloc, int V, int tiles, uint32_t spans,
-                                                                uint32_t items, __half *__restrict__ dense, int64_t ldd)
-{
-    constexpr int NW = M_ / 2;             // 32-bit words per group
-    constexpr int GPT = M_ == 4 ? 2 : 1;   // groups per thread
-    constexpr int TW = GPT * NW;           // words per thread and row
-    constexpr int TL = 4 / GPT;            // lanes per tile
-    constexpr int TPW = 32 / TL;           // tiles per warp
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int g0 = (lane % TL) * GPT;
-    const int64_t Ksp = (int64_t)tiles * 8;
-    for (uint32_t item = blockIdx.x; item < items; item += gridDim.x) {
-        const uint32_t strip = item / spans;
-        const int T = (int)(item - strip * spans) * (8 * TPW) + warp * TPW + lane / TL;
-        if (T >= tiles) continue;   // no exchange between lanes: threads past the last tile have nothing to do
-        const int64_t G = (int64_t)T * 4 + g0;
-        // the candidates of a group as four bytes of one word: candidate `sel` is one byte permute away
-        uint32_t candpack[GPT];
-        {
-            const uint4 *c4p = reinterpret_cast<const uint4 *>(colloc + ((int64_t)(strip * 16u / (uint32_t)V) * (Ksp / 2) + G) * 4);
-#pragma unroll
-            for (int j = 0; j < GPT; j++) {
-                const uint4 c4 = __ldg(c4p + j);
-                candpack[j] = (c4.x & 0xFFu) | ((c4.y & 0xFFu) << 8) | ((c4.z & 0xFFu) << 16) | ((c4.w & 0xFFu) << 24);
-            }
-        }
-        const uint4 *vsrc = reinterpret_cast<const uint4 *>(values) + ((int64_t)strip * 16 * Ksp + (int64_t)T * 128) / 8 + g0;
-        const uint4 *msrc = reinterpret_cast<const uint4 *>(meta + (int64_t)(strip >> 1) * 16 * tiles + (int64_t)T * 16 + (strip & 1u) * 8);
-        uint4 vals[4][GPT];
-#pragma unroll
-        for (int sb = 0; sb < 4; sb++)
-#pragma unroll
-            for (int j = 0; j < GPT; j++) vals[sb][j] = __ldg(vsrc + sb * 4 + j);
-        const uint4 ma = __ldg(msrc), mb = __ldg(msrc + 1);
-        const uint32_t mw[8] = {ma.x, ma.y, ma.z, ma.w, mb.x, mb.y, mb.z, mb.w};   // word 2*sb + (r >> 1): rows r, r+1 of sub-block sb
-        __half *drow0 = dense + (int64_t)strip * 16 * ldd + G * M_;
-#pragma unroll
-        for (int sb = 0; sb < 4; sb++) {
-#pragma unroll
-            for (int r = 0; r < 4; r++) {
-                const uint32_t hw = mw[sb * 2 + (r >> 1)] >> ((r & 1) * 16);
-                uint32_t w[TW];
-#pragma unroll
-                for (int j = 0; j < GPT; j++) {
-                    const uint32_t two = r == 0 ? vals[sb][j].x : r == 1 ? vals[sb][j].y : r == 2 ? vals[sb][j].z : vals[sb][j].w;
-                    const uint32_t nib = hw >> ((g0 + j) * 4);
-                    const uint32_t p0 = __byte_perm(candpack[j], 0u, 0x4440u | (nib & 3u));          // column of slot 0 inside the group
-                    const uint32_t p1 = __byte_perm(candpack[j], 0u, 0x4440u | ((nib >> 2) & 3u));   // column of slot 1
-                    const uint32_t lo0 = two & 0xFFFFu, hi0 = two << 16;          // slot 0 as a low / high half
-                    const uint32_t lo1 = two >> 16, hi1 = two & 0xFFFF0000u;      // slot 1
-#pragma unroll
-                    for (int k = 0; k < NW; k++) {
-                        uint32_t x = 0;
-                        if ((p0 >> 1) == (uint32_t)k) x = (p0 & 1u) ? hi0 : lo0;
-                        if ((p1 >> 1) == (uint32_t)k) x = (p1 & 1u) ? ((x & 0xFFFFu) | hi1) : ((x & 0xFFFF0000u) | lo1);
-                        w[j * NW + k] = x;
-                    }
-                }
-                uint4 *dst = reinterpret_cast<uint4 *>(drow0 + (int64_t)(sb * 4 + r) * ldd);
-#pragma unroll
-                for (int i = 0; i < TW / 4; i++) dst[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
-            }
-        }
-    }
-}
-
-// ------------------------------------------------------------------------------------------------
 // Decompressor, piece form, for m a multiple of 8 (PW = 8) or of 4 (PW = 4) and rows aligned to PW halves: lanes lie along the
 // OUTPUT row.  A thread owns PW consecutive columns, all of one group, of the 16 rows of a strip; the m / PW threads of a group
 // load the same values and metadata (one sector for all of them) and each keeps the slots that fall into its columns.
 // Every store instruction of a warp writes 512 contiguous bytes (256 for PW = 4).  Bound by HBM writes: 12288 x 12288, m = 16
-// takes 60 us (floor 54); through the tiled kernel (shared-memory scatter, two barriers a chunk) it took 78.
+// takes 60 us (floor 54); through the tiled kernel (shared-memory scatter, two barriers a chunk) it took 78.  A thread per group instead of
+// a piece (m = 8: the same; m = 4: two groups) in one resident wave took 76 us at m = 8 and 96 at m = 4, against 68 and 84.
 // ------------------------------------------------------------------------------------------------
 template <int PW>
 __global__ void __launch_bounds__(256) decompress_piece_kernel(const uint32_t *__restrict__ values, const uint32_t *__restrict__ meta,
@@ -713,43 +489,11 @@ __global__ void __launch_bounds__(256) decompress_piece_kernel(const uint32_t *_
     }
 }
 
-template <int M_>
-static int decompress_direct_wave()
-{
-    static int cached[64] = {0};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64) dev = 0;
-    if (cached[dev] == 0) {
-        int per_sm = 0, sms = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, decompress_direct_kernel<M_>, 256, 0);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cached[dev] = (per_sm > 0 && sms > 0) ? per_sm * sms : 148 * 4;
-    }
-    return cached[dev];
-}
-
 cudaError_t launch_decompress(const void *values, const uint32_t *meta, const uint32_t *colloc, int M, int K, int V, int m,
                               void *dense, int64_t ldd, cudaStream_t stream)
 {
     const int64_t Ksp = ksp_of(K, m);
     const bool arrays_aligned = M % 16 == 0 && V % 16 == 0 && ((uintptr_t)values & 15) == 0 && ((uintptr_t)colloc & 15) == 0 && ((uintptr_t)meta & 15) == 0;
-    // register form: whole tiles, 16-byte aligned rows and arrays
-    if ((m == 4 || m == 8) && K % (4 * m) == 0 && Ksp == (int64_t)K / m * 2 && M % 16 == 0 && V % 16 == 0 && ldd % 8 == 0 &&
-        ((uintptr_t)dense & 15) == 0 && ((uintptr_t)values & 15) == 0 && ((uintptr_t)colloc & 15) == 0 && ((uintptr_t)meta & 15) == 0) {
-        const int tiles = (int)(Ksp / 8);
-        const int tiles_per_item = m == 4 ? 8 * 16 : 8 * 8;   // 8 warps x tiles per warp
-        const int64_t spans = (tiles + tiles_per_item - 1) / tiles_per_item, items = (int64_t)(M / 16) * spans;
-        if (items < ((int64_t)1 << 31)) {
-            const int wave = m == 4 ? decompress_direct_wave<4>() : decompress_direct_wave<8>();
-            const unsigned blocks = items < wave ? (unsigned)items : (unsigned)wave;
-            if (m == 4)
-                decompress_direct_kernel<4><<<blocks, 256, 0, stream>>>((const uint32_t *)values, meta, colloc, V, tiles, (uint32_t)spans, (uint32_t)items, (__half *)dense, ldd);
-            else
-                decompress_direct_kernel<8><<<blocks, 256, 0, stream>>>((const uint32_t *)values, meta, colloc, V, tiles, (uint32_t)spans, (uint32_t)items, (__half *)dense, ldd);
-            return cudaGetLastError();
-        }
-    }
     // piece form: a piece never straddles groups or the end of a row
     const int pw = m % 8 == 0 && K % 8 == 0 && ldd % 8 == 0 && ((uintptr_t)dense & 15) == 0 ? 8 : m % 4 == 0 && K % 4 == 0 && ldd % 4 == 0 && ((uintptr_t)dense & 7) == 0 ? 4 : 0;
     if (arrays_aligned && pw && m <= 256) {
