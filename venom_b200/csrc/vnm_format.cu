@@ -607,7 +607,9 @@ __global__ void __launch_bounds__(256) prepare_rows_kernel(const uint32_t *__res
 // missing slots are filled with explicit zeros.  The product can then read B as ordinary 64-row tiles
 // that every vector block shares (no per-block gather, no lane masks), at the price of m/4 times the MMA
 // work.  Same block format as prepare_am_kernel, but a k-tile now covers 128 ORIGINAL columns.
-// One thread handles one (row pair, 16 original columns): two 16-byte value chunks and one metadata word.
+// One thread handles one (row pair, 16 original columns): two 16-byte value chunks and one metadata word.  The column-loc, the values and
+// the metadata of a group are loaded once for both rows and all of its chunks in the slab (loading them per row, chunk and slot took
+// 436 us at 12288 x 12288, 128:2:8, against 165 now).
 // ------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) prepare_dense_b_kernel(const __half *__restrict__ values, const uint32_t *__restrict__ meta,
                                                               const uint32_t *__restrict__ colloc, int M, int K, int V, int m, int64_t Ksp,
@@ -617,35 +619,44 @@ __global__ void __launch_bounds__(256) prepare_dense_b_kernel(const __half *__re
     for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (int64_t)gridDim.x * blockDim.x) {
         const int q = (int)(idx & 7);          // 16-column slab of the 128-column k-tile
         const int pr = (int)((idx >> 3) & 63);  // row pair inside the 128-row tile
-        const int64_t blk = idx >> 9;
-        const int mt = (int)(blk / ktiles);
-        const int kt = (int)(blk - (int64_t)mt * ktiles);
-        uint8_t *block = am + blk * AM_BLOCK_BYTES;
+        const uint32_t blk = (uint32_t)(idx >> 9);
+        const int mt = (int)(blk / (uint32_t)ktiles);
+        const int kt = (int)(blk - (uint32_t)mt * (uint32_t)ktiles);
+        uint8_t *block = am + (size_t)blk * AM_BLOCK_BYTES;
         uint32_t word = 0;
         const int i0 = actual_to_mma_row(2 * pr);  // MMA row of the even row; the odd row sits 8 rows further
+        const int64_t r0 = (int64_t)mt * TILE_M + 2 * pr;
+        unsigned short v8[2][8] = {{0, 0, 0, 0, 0, 0, 0, 0}, {0, 0, 0, 0, 0, 0, 0, 0}};
+        int cb = kt * 128 + q * 16;                // first original column of the chunk
+        int g = cb / m, o0 = cb - g * m;
+        uint4 c4 = make_uint4(0, 0, 0, 0);
+        uint2 two = make_uint2(0, 0);              // slots 0 and 1 of the even row, of the odd row
+        uint32_t w = 0;
+        bool fresh = true;                         // the group's words are still to be loaded
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int64_t r = (int64_t)mt * TILE_M + 2 * pr + h;
-            unsigned short v8[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-            uint32_t nib16 = 0;
+        for (int c = 0; c < 4; c++) {
+            const bool in = r0 < M && cb < K;
+            if (in && fresh) {
+                c4 = __ldg(reinterpret_cast<const uint4 *>(colloc + (r0 / V) * (Ksp / 2) * 4) + g);
+                const uint32_t *v = reinterpret_cast<const uint32_t *>(values + values_index(r0, g, 0, Ksp));   // 4-byte aligned at least
+                two = make_uint2(__ldg(v), __ldg(v + 1));
+                w = __ldg(meta + meta_index(r0, g, Ksp));
+            }
 #pragma unroll
-            for (int c = 0; c < 4; c++) {
-                const int64_t cb = (int64_t)kt * 128 + q * 16 + c * 4;  // first original column of the chunk
+            for (int h = 0; h < 2; h++) {
                 int npos = 0;
                 uint32_t pos[2] = {0, 1};
                 unsigned short val[2] = {0, 0};
-                if (r < M && cb < K) {
-                    const int64_t g = cb / m;
-                    const int o0 = (int)(cb - g * m);
-                    const uint32_t w = meta[meta_index(r, g, Ksp)];
-                    const uint32_t *c4 = colloc + (r / V) * (Ksp / 2) * 4 + g * 4;
+                if (in) {
+                    const uint32_t nib = w >> meta_shift(r0 + h, g, 0), v2 = h ? two.y : two.x;
 #pragma unroll
                     for (int sl = 0; sl < 2; sl++) {
-                        const uint32_t sel = (w >> meta_shift(r, g, sl)) & 3u;
-                        const int off = (int)c4[sel] - o0;
-                        if (off >= 0 && off < 4 && npos < 2 && cb + off < K) {
-                            pos[npos] = (uint32_t)off;
-                            val[npos] = __half_as_ushort(values[values_index(r, g, sl, Ksp)]);
+                        const uint32_t sel = (nib >> (2 * sl)) & 3u;
+                        const int off = (int)(sel == 0 ? c4.x : sel == 1 ? c4.y : sel == 2 ? c4.z : c4.w) - o0;
+                        if (off >= 0 && off < 4 && cb + off < K) {
+                            const unsigned short x = (unsigned short)(v2 >> (16 * sl));
+                            if (npos == 0) { pos[0] = (uint32_t)off; val[0] = x; }
+                            else { pos[1] = (uint32_t)off; val[1] = x; }
                             npos++;
                         }
                     }
@@ -653,22 +664,26 @@ __global__ void __launch_bounds__(256) prepare_dense_b_kernel(const __half *__re
                 if (npos == 1) {  // partner slot with an explicit zero, positions kept ascending
                     if (pos[0] == 3) { pos[1] = 3; pos[0] = 2; val[1] = val[0]; val[0] = 0; }
                     else { pos[1] = pos[0] + 1; val[1] = 0; }
-                } else if (npos == 0) {
-                    pos[0] = 0; pos[1] = 1;
-                } else if (pos[0] == pos[1]) {  // duplicate offsets only arise from padded slots (zero values)
+                } else if (npos == 2 && pos[0] == pos[1]) {  // duplicate offsets only arise from padded slots (zero values)
                     if (pos[0] == 3) pos[0] = 2; else pos[1] = pos[0] + 1;
                 }
-                v8[2 * c] = val[0];
-                v8[2 * c + 1] = val[1];
-                nib16 |= (pos[0] | (pos[1] << 2)) << (4 * c);
+                v8[h][2 * c] = val[0];
+                v8[h][2 * c + 1] = val[1];
+                word |= (pos[0] | (pos[1] << 2)) << (4 * c + 16 * h);
             }
-            word |= nib16 << (16 * h);
+            cb += 4;
+            o0 += 4;
+            fresh = o0 == m;
+            if (fresh) { o0 = 0; g++; }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
             const int i = i0 + 8 * h;
             uint4 o;
-            o.x = (uint32_t)v8[0] | ((uint32_t)v8[1] << 16);
-            o.y = (uint32_t)v8[2] | ((uint32_t)v8[3] << 16);
-            o.z = (uint32_t)v8[4] | ((uint32_t)v8[5] << 16);
-            o.w = (uint32_t)v8[6] | ((uint32_t)v8[7] << 16);
+            o.x = (uint32_t)v8[h][0] | ((uint32_t)v8[h][1] << 16);
+            o.y = (uint32_t)v8[h][2] | ((uint32_t)v8[h][3] << 16);
+            o.z = (uint32_t)v8[h][4] | ((uint32_t)v8[h][5] << 16);
+            o.w = (uint32_t)v8[h][6] | ((uint32_t)v8[h][7] << 16);
             *reinterpret_cast<uint4 *>(block + i * 128 + ((q ^ (i & 7)) << 4)) = o;
         }
         const int lane = (i0 & 7) + 8 * (q & 1) + 16 * (i0 >> 4);
