@@ -112,3 +112,19 @@ def test_decompress_pieces(cfg):
     values, meta, bad = capi.compress(d, c, V, m)
     assert bad == 0
     assert torch.equal(capi.decompress(values, meta, c, M, K, V, m), d)
+
+
+# A [tokens, features] activation of more rows than 65535 blocks of 64, which the gather form transposes first.
+def test_gather_form_takes_millions_of_tokens():
+    import torch
+    from venom_b200 import capi
+    M, K, V, m = 32, 32, 32, 16
+    N = 65535 * 64 + 8
+    d, _, _, _, prep = _operand(M, K, V, m, capi.STRATEGY_GATHER, seed=9)
+    x = _ints((N, K), 4)
+    out = torch.empty((N, M), dtype=torch.float16, device="cuda")
+    workspace = torch.empty((K, N), dtype=torch.float16, device="cuda")
+    rc = capi.lib().vnm_spmm_f16_nk_ws(prep._h, x.data_ptr(), K, N, None, out.data_ptr(), M, capi.VNM_LAYOUT_NM, workspace.data_ptr(), capi._stream())
+    assert rc == 0, capi.lib().vnm_last_error_string()
+    assert torch.equal(out, (x.float() @ d.T).half())
+    assert prep.device_status() == 0
