@@ -87,7 +87,8 @@ int vnm_decompress_f16(const void *values, const uint32_t *meta, const uint32_t 
                        int M, int K, int V, int n, int m, void *dense, int64_t ldd, void *stream);
 
 /* Re-pack reference-format arrays into the kernel-private layout and return a handle that owns only
- * that private copy (the inputs may be freed once `stream` has drained).
+ * that private copy (the inputs may be freed once `stream` has drained).  Prepare before a stream capture: on a stream that is being
+ * captured the call fails with VNM_ERR_CUDA, except in the relaxed mode, where the copy is filled by each replay of the graph.
  * Replaces: BlockwiseSpMatrix<half>::init_sparse + transform_and_sync_device,
  * include/spatha/block_sparse/spmm/blockwise_format.h:248-283,327-373, and
  * Format_sr_nm<T>::transform_and_sync_device, src/format/format_sr_nm.cpp:239-285. */

@@ -128,3 +128,87 @@ def test_gather_form_takes_millions_of_tokens():
     assert rc == 0, capi.lib().vnm_last_error_string()
     assert torch.equal(out, (x.float() @ d.T).half())
     assert prep.device_status() == 0
+
+
+def _two_forms(M, K, V, m):
+    """Token counts for which a layer wants its weight in different forms."""
+    import ctypes as C
+    from venom_b200 import capi
+    form, first = C.c_int(), {}
+    for n in (4096, 2048, 1024, 512, 256, 128, 64, 32, 16, 8):
+        assert capi.lib().vnm_choose_form(M, K, V, 2, m, n, 1, C.byref(form)) == 0
+        first.setdefault(form.value, n)
+    assert len(first) == 2, first
+    return first[capi.STRATEGY_GATHER], first[capi.STRATEGY_DENSE_B]
+
+
+def _layer_of(values, meta, c, M, K, V, m):
+    import torch
+    from venom_b200.nmv import SrnmSpmm
+    layer = SrnmSpmm(torch.nn.Linear(K, M, bias=False).half().cuda(), 2, m, V)
+    layer.values = torch.nn.Parameter(values.reshape(-1), requires_grad=False)
+    layer.metadata, layer.columns = meta, c
+    return layer
+
+
+# A graph captured at a token count that wants a form the weight is not held in yet: it uses the other one, and calls outside
+# of it, before and after its replays, are not disturbed.
+@pytest.mark.parametrize("warm", [0, 1])
+def test_layer_captured_before_its_form_exists(warm):
+    import torch
+    M, K, V, m = 1024, 4096, 128, 16
+    ns = _two_forms(M, K, V, m)
+    d, values, meta, c, _ = _operand(M, K, V, m, None, seed=21)
+    layer = _layer_of(values, meta, c, M, K, V, m)
+    xs = [_ints((n, K), n) for n in ns]
+    want = [(x.float() @ d.T).half() for x in xs]
+    assert torch.equal(layer(xs[warm]), want[warm])
+    x = xs[1 - warm].clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = layer(x)
+    assert torch.equal(layer(xs[1 - warm]), want[1 - warm])
+    graph.replay()
+    assert torch.equal(y, want[1 - warm])
+    x.mul_(2)
+    graph.replay()
+    assert torch.equal(y, (xs[1 - warm].float() * 2 @ d.T).half())
+    assert torch.equal(layer(xs[warm]), want[warm])
+
+
+# vnm_prepare on a stream that is being captured: refused in the global mode, allowed in the relaxed one, where the copy is filled by
+# every replay and outlives the graph.
+def test_prepare_under_capture():
+    import ctypes as C
+    import torch
+    from venom_b200 import capi
+    M, K, V, m, N = 256, 512, 64, 8, 64
+    d, values, meta, c, _ = _operand(M, K, V, m, None, seed=5)
+    B = _ints((K, N), 2)
+    want = (d @ B.float()).half()
+    out = torch.zeros((M, N), dtype=torch.float16, device="cuda")
+    torch.cuda.synchronize()
+    rt, L = C.CDLL("libcudart.so.12"), capi.lib()
+    s = C.c_void_p(torch.cuda.Stream().cuda_stream)
+    graph, run, h = C.c_void_p(), C.c_void_p(), C.c_void_p()
+    assert rt.cudaStreamBeginCapture(s, 0) == 0
+    assert L.vnm_prepare(values.data_ptr(), meta.data_ptr(), c.data_ptr(), M, K, V, 2, m, C.byref(h), s) == 2
+    assert rt.cudaStreamEndCapture(s, C.byref(graph)) != 0
+    rt.cudaGetLastError()
+    assert rt.cudaStreamBeginCapture(s, 2) == 0
+    assert L.vnm_prepare(values.data_ptr(), meta.data_ptr(), c.data_ptr(), M, K, V, 2, m, C.byref(h), s) == 0
+    assert L.vnm_spmm_f16(h, B.data_ptr(), N, N, None, out.data_ptr(), N, 0, s) == 0
+    assert rt.cudaStreamEndCapture(s, C.byref(graph)) == 0
+    assert rt.cudaGraphInstantiate(C.byref(run), graph, C.c_ulonglong(0)) == 0
+    for _ in range(2):
+        out.zero_()
+        torch.cuda.synchronize()
+        assert rt.cudaGraphLaunch(run, s) == 0 and rt.cudaStreamSynchronize(s) == 0
+        assert torch.equal(out, want)
+    assert rt.cudaGraphExecDestroy(run) == 0 and rt.cudaGraphDestroy(graph) == 0
+    out.zero_()
+    torch.cuda.synchronize()
+    assert L.vnm_spmm_f16(h, B.data_ptr(), N, N, None, out.data_ptr(), N, 0, None) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
+    assert L.vnm_destroy(h) == 0

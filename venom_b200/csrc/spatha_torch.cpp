@@ -13,6 +13,7 @@
 //     version counters, which are part of the key.
 #include <torch/extension.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -131,7 +132,9 @@ vnm_handle_t operand_for(const torch::Tensor &A_metadata, const torch::Tensor &A
         e.last_t = in_place;
     }
     *dense_b = e.last_form;
-    vnm_handle_t &h = e.handle[e.last_form];
+    // A graph that is being captured uses the form that is there: re-packing is work for outside of it.
+    if (!e.handle[*dense_b] && e.handle[1 - *dense_b] && c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) *dense_b = 1 - *dense_b;
+    vnm_handle_t &h = e.handle[*dense_b];
     if (!h)
         check(vnm_prepare_as(A_values.data_ptr(), (const uint32_t *)A_metadata.data_ptr(), (const uint32_t *)A_indices.data_ptr(), M, K, V, n, m,
                              *dense_b ? VNM_STRATEGY_DENSE_B : VNM_STRATEGY_GATHER, &h, stream), "vnm_prepare_as");

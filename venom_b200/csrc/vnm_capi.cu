@@ -92,19 +92,38 @@ int g_strategy = 0;  // VNM_STRATEGY_*
 constexpr uint64_t POOL_KEEP_BYTES = 1ull << 30;
 cudaMemPool_t g_pools[kMaxDevices] = {};
 
-cudaError_t device_alloc(void **ptr, size_t bytes, int dev, cudaStream_t stream)
+struct DeviceBuffer {
+    void *ptr;
+    bool pooled;   // from the device's pool, else from cudaMalloc
+};
+
+bool is_capturing(cudaStream_t stream)
 {
-    return cudaMallocFromPoolAsync(ptr, bytes, g_pools[dev], stream);
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    const cudaError_t e = cudaStreamIsCapturing(stream, &status);
+    if (e != cudaSuccess) (void)cudaGetLastError();   // the legacy stream beside a capture
+    return e != cudaSuccess || status != cudaStreamCaptureStatusNone;
+}
+
+// An allocation from the pool on a stream that is being captured would become a node of the graph: memory that exists only once
+// the graph runs, and only until it is destroyed.  Handles are used outside of graphs and outlive them, so there the memory comes from
+// cudaMalloc, which a capture in the relaxed mode allows and one in the other modes refuses.
+cudaError_t device_alloc(DeviceBuffer *buf, size_t bytes, int dev, cudaStream_t stream)
+{
+    buf->pooled = !is_capturing(stream);
+    const cudaError_t e = buf->pooled ? cudaMallocFromPoolAsync(&buf->ptr, bytes, g_pools[dev], stream) : cudaMalloc(&buf->ptr, bytes);
+    if (e != cudaSuccess) buf->ptr = nullptr;
+    return e;
 }
 
 // Like cudaFree: waits until nothing on the device can still use the memory.
-void device_free(std::initializer_list<void *> ptrs)
+void device_free(std::initializer_list<DeviceBuffer> bufs)
 {
     bool any = false;
-    for (void *p : ptrs) any = any || p;
+    for (const DeviceBuffer &b : bufs) any = any || b.ptr;
     if (!any || cudaDeviceSynchronize() != cudaSuccess) return;   // a lost context has no memory to give back
-    for (void *p : ptrs)
-        if (p) cudaFreeAsync(p, nullptr);
+    for (const DeviceBuffer &b : bufs)
+        if (b.ptr) (void)(b.pooled ? cudaFreeAsync(b.ptr, nullptr) : cudaFree(b.ptr));
 }
 
 // Opts every kernel instance into its shared-memory size on the current device (once per device).
@@ -157,15 +176,16 @@ struct vnm_prepared_s {
     int64_t Ksp;
     int mtiles, ktiles, nb, vblocks_padded;
     int device;
+    DeviceBuffer packed;   // the private copy: am, rows and status lie in it
     void *am;
     void *rows;
     int *status;
     // device staging of the host-buffer entry point
-    void *stage_B;
+    DeviceBuffer stage_B;
     size_t stage_B_bytes;
-    void *stage_out;
+    DeviceBuffer stage_out;
     size_t stage_out_bytes;
-    void *stage_bias;
+    DeviceBuffer stage_bias;
     cudaStream_t copy_in, copy_out;   // host-buffer entry point: the device's two copy streams (shared by all handles)
     cudaEvent_t ev[2 * HOST_CHUNKS_MAX + 2];
     bool host_pipe_ready;
@@ -314,8 +334,9 @@ int vnm_prepare_as(const void *values, const uint32_t *meta, const uint32_t *col
     // one block: value and metadata images | row table (gather form) | status word
     const size_t am_bytes = (size_t)h->mtiles * h->ktiles * AM_BLOCK_BYTES;
     const size_t rows_bytes = h->dense_b ? 0 : (size_t)h->vblocks_padded * h->ktiles * KT_GROUPS * sizeof(int4);
-    cudaError_t e = device_alloc(&h->am, am_bytes + rows_bytes + 256, dev_now, (cudaStream_t)stream);
+    cudaError_t e = device_alloc(&h->packed, am_bytes + rows_bytes + 256, dev_now, (cudaStream_t)stream);
     if (e == cudaSuccess) {
+        h->am = h->packed.ptr;
         h->rows = (uint8_t *)h->am + am_bytes;
         h->status = (int *)((uint8_t *)h->am + am_bytes + rows_bytes);
         e = cudaMemsetAsync(h->status, 0, sizeof(int), (cudaStream_t)stream);
@@ -327,6 +348,7 @@ int vnm_prepare_as(const void *values, const uint32_t *meta, const uint32_t *col
             e = launch_prepare(values, meta, colloc, M, K, V, m, h->am, h->rows, h->mtiles, h->ktiles, h->vblocks_padded, (cudaStream_t)stream);
     }
     if (e != cudaSuccess) {
+        (void)cudaGetLastError();
         vnm_destroy(h);
         return fail_cuda(e, "vnm_prepare");
     }
@@ -341,7 +363,7 @@ int vnm_destroy(vnm_handle_t h)
         int now = -1;   // the memory belongs to the handle's device
         const bool other = cudaGetDevice(&now) == cudaSuccess && now != h->device;
         if (other) cudaSetDevice(h->device);
-        device_free({h->am, h->stage_B, h->stage_out, h->stage_bias});
+        device_free({h->packed, h->stage_B, h->stage_out, h->stage_bias});
         if (other) cudaSetDevice(now);
     }
     if (h->host_pipe_ready) {
@@ -757,11 +779,11 @@ int vnm_operand_form(vnm_handle_t h, int *dense_b)
     return VNM_OK;
 }
 
-static int grow(vnm_handle_t h, void **buf, size_t *cap, size_t need, cudaStream_t stream)
+static int grow(vnm_handle_t h, DeviceBuffer *buf, size_t *cap, size_t need, cudaStream_t stream)
 {
     if (*cap >= need) return VNM_OK;
     device_free({*buf});
-    *buf = nullptr; *cap = 0;
+    buf->ptr = nullptr; *cap = 0;
     cudaError_t e = device_alloc(buf, need, h->device, stream);
     if (e != cudaSuccess) return fail_cuda(e, "staging allocation");
     *cap = need;
@@ -815,18 +837,18 @@ static int spmm_host_impl(vnm_handle_t h, const void *B_host, int N, const void 
     VNM_CUDA(cudaStreamWaitEvent(h->copy_in, ev_start, 0), "stream wait");
     VNM_CUDA(cudaStreamWaitEvent(h->copy_out, ev_start, 0), "stream wait");
     if (bias_host) {
-        if (!h->stage_bias) VNM_CUDA(device_alloc(&h->stage_bias, (size_t)h->M * 2, h->device, h->copy_in), "bias allocation");
-        VNM_CUDA(cudaMemcpyAsync(h->stage_bias, bias_host, (size_t)h->M * 2, cudaMemcpyHostToDevice, h->copy_in), "H2D copy of bias");
+        if (!h->stage_bias.ptr) VNM_CUDA(device_alloc(&h->stage_bias, (size_t)h->M * 2, h->device, h->copy_in), "bias allocation");
+        VNM_CUDA(cudaMemcpyAsync(h->stage_bias.ptr, bias_host, (size_t)h->M * 2, cudaMemcpyHostToDevice, h->copy_in), "H2D copy of bias");
     }
     for (int c = 0, n0 = 0; c < chunks; n0 += widths[c], ++c) {
         const int w = widths[c];
-        uint8_t *dB = (uint8_t *)h->stage_B + (size_t)h->K * n0 * 2;
-        uint8_t *dO = (uint8_t *)h->stage_out + (size_t)h->M * n0 * 2;
+        uint8_t *dB = (uint8_t *)h->stage_B.ptr + (size_t)h->K * n0 * 2;
+        uint8_t *dO = (uint8_t *)h->stage_out.ptr + (size_t)h->M * n0 * 2;
         VNM_CUDA(cudaMemcpy2DAsync(dB, (size_t)w * 2, (const uint8_t *)B_host + (size_t)n0 * 2, (size_t)N * 2, (size_t)w * 2, h->K,
                                    cudaMemcpyHostToDevice, h->copy_in), "H2D copy of B");
         VNM_CUDA(cudaEventRecord(h->ev[2 * c], h->copy_in), "event record");
         VNM_CUDA(cudaStreamWaitEvent(s, h->ev[2 * c], 0), "stream wait");
-        rc = vnm_spmm_f16(h, dB, w, w, bias_host ? h->stage_bias : nullptr, dO, layout == VNM_LAYOUT_MN ? w : h->M, layout, stream);
+        rc = vnm_spmm_f16(h, dB, w, w, bias_host ? h->stage_bias.ptr : nullptr, dO, layout == VNM_LAYOUT_MN ? w : h->M, layout, stream);
         if (rc) break;
         VNM_CUDA(cudaEventRecord(h->ev[2 * c + 1], s), "event record");
         VNM_CUDA(cudaStreamWaitEvent(h->copy_out, h->ev[2 * c + 1], 0), "stream wait");
