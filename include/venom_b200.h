@@ -97,8 +97,9 @@ int vnm_prepare(const void *values, const uint32_t *meta, const uint32_t *colloc
 int vnm_prepared_bytes(int M, int K, int V, int n, int m, int64_t *bytes);
 int vnm_destroy(vnm_handle_t handle);
 
-/* Threading: a handle caches the tensor maps of the last dense operand and owns the host-buffer staging, so two
- * host threads must not call into the SAME handle at the same time (different handles are independent).  A handle
+/* Threading: products of one handle may be queued from several host threads and on several streams at a time; one on another
+ * stream than vnm_prepare's waits for the private copy.  The host-buffer entry points own their staging and the setters change the
+ * handle: those must not run beside any other call on the SAME handle (different handles are independent).  A handle
  * belongs to the device that was current in vnm_prepare; calls with another device current return VNM_ERR_BAD_ARG. */
 
 /* out = A_vnm * B (+ bias), fp16 in, fp32 accumulate, fp16 out.

@@ -212,3 +212,51 @@ def test_prepare_under_capture():
     torch.cuda.synchronize()
     assert torch.equal(out, want)
     assert L.vnm_destroy(h) == 0
+
+
+# An operand that is still being re-packed behind other work of one stream: a product on another stream, plain or captured, waits.
+@pytest.mark.parametrize("captured", [False, True])
+@pytest.mark.parametrize("form", ["gather", "dense_b"])
+def test_product_waits_for_an_operand_packed_on_another_stream(form, captured):
+    import torch
+    from venom_b200 import capi
+    M, K, V, m, N = 256, 1024, 64, 8, 200
+    d, values, meta, c, _ = _operand(M, K, V, m, None, seed=13)
+    B = _ints((K, N), 6)
+    want = (d @ B.float()).half()
+    busy, other = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(busy):
+        torch.cuda._sleep(50_000_000)
+        prep = capi.Prepared(values, meta, c, M, K, V, m, strategy=capi.STRATEGY_GATHER if form == "gather" else capi.STRATEGY_DENSE_B)
+    if captured:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.stream(other):
+            graph.capture_begin()            # not torch.cuda.graph, which waits for the device first
+            out = prep.spmm(B)
+            graph.capture_end()
+            graph.replay()
+    else:
+        with torch.cuda.stream(other):
+            out = prep.spmm(B)
+    other.synchronize()
+    assert torch.equal(out, want)
+    assert prep.device_status() == 0
+
+
+def test_layer_called_on_two_streams():
+    import torch
+    M, K, V, m = 1024, 4096, 128, 16
+    d, values, meta, c, _ = _operand(M, K, V, m, None, seed=17)
+    layer = _layer_of(values, meta, c, M, K, V, m)
+    xs = [_ints((n, K), n) for n in _two_forms(M, K, V, m)]
+    want = [(x.float() @ d.T).half() for x in xs]
+    busy = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for x, w in zip(xs, want):
+        with torch.cuda.stream(busy):
+            torch.cuda._sleep(50_000_000)
+            a = layer(x)             # re-packs the weight into the form that this token count wants
+        assert torch.equal(layer(x), w)
+        busy.synchronize()
+        assert torch.equal(a, w)

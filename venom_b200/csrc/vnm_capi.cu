@@ -177,6 +177,8 @@ struct vnm_prepared_s {
     int mtiles, ktiles, nb, vblocks_padded;
     int device;
     DeviceBuffer packed;   // the private copy: am, rows and status lie in it
+    cudaEvent_t ready;     // the copy is complete (null if it is written inside a graph)
+    int ready_seen;        // ... and has been seen to be
     void *am;
     void *rows;
     int *status;
@@ -203,6 +205,29 @@ struct vnm_prepared_s {
 };
 
 namespace {
+
+// The private copy is written by vnm_prepare's stream; a product on any stream comes after it.  Once the copy has been seen complete
+// (usually at the second product) this costs one load.
+cudaError_t wait_ready(vnm_prepared_s *h, cudaStream_t stream)
+{
+    if (__atomic_load_n(&h->ready_seen, __ATOMIC_ACQUIRE)) return cudaSuccess;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // a query is not an operation that a capture must not miss
+    (void)cudaThreadExchangeStreamCaptureMode(&mode);
+    cudaError_t e = cudaEventQuery(h->ready);
+    bool seen = e == cudaSuccess;
+    if (e == cudaErrorNotReady) {
+        (void)cudaGetLastError();
+        if (is_capturing(stream)) {   // what a graph depends on has to be part of it, or over
+            e = cudaEventSynchronize(h->ready);
+            seen = e == cudaSuccess;
+        } else {
+            e = cudaStreamWaitEvent(stream, h->ready, 0);
+        }
+    }
+    (void)cudaThreadExchangeStreamCaptureMode(&mode);
+    if (seen) __atomic_store_n(&h->ready_seen, 1, __ATOMIC_RELEASE);
+    return e;
+}
 
 // Fills in what follows from the shape and the operand form.
 void shape_handle(vnm_prepared_s *h, int M, int K, int V, int n, int m, bool dense_b)
@@ -347,6 +372,12 @@ int vnm_prepare_as(const void *values, const uint32_t *meta, const uint32_t *col
         else
             e = launch_prepare(values, meta, colloc, M, K, V, m, h->am, h->rows, h->mtiles, h->ktiles, h->vblocks_padded, (cudaStream_t)stream);
     }
+    if (!h->packed.pooled) {
+        h->ready_seen = 1;   // written inside a graph, which orders the products in it
+    } else {
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ready, cudaEventDisableTiming);
+        if (e == cudaSuccess) e = cudaEventRecord(h->ready, (cudaStream_t)stream);
+    }
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
         vnm_destroy(h);
@@ -366,6 +397,7 @@ int vnm_destroy(vnm_handle_t h)
         device_free({h->packed, h->stage_B, h->stage_out, h->stage_bias});
         if (other) cudaSetDevice(now);
     }
+    if (h->ready) cudaEventDestroy(h->ready);
     if (h->host_pipe_ready) {
         for (cudaEvent_t e : h->ev) cudaEventDestroy(e);
     }
@@ -570,6 +602,7 @@ static int spmm_impl(vnm_handle_t h, const void *B, int64_t ldb, int N, int b_nk
     } else {
         return fail(VNM_ERR_BAD_ARG, "vnm_spmm_f16: unknown layout %d", layout);
     }
+    VNM_CUDA(wait_ready(h, (cudaStream_t)stream), "wait for the prepared operand");
     SpmmConfig cfg;
     Kernel kernel;
     float us;
@@ -902,6 +935,7 @@ int vnm_device_status(vnm_handle_t h, int *status, void *stream)
     if (!h || !status) return fail(VNM_ERR_BAD_ARG, "vnm_device_status: null pointer");
     cudaStream_t s = (cudaStream_t)stream;
     int v = 0;
+    VNM_CUDA(wait_ready(h, s), "wait for the prepared operand");   // which clears the word first
     VNM_CUDA(cudaMemcpyAsync(&v, h->status, sizeof(int), cudaMemcpyDeviceToHost, s), "status copy");
     VNM_CUDA(cudaStreamSynchronize(s), "stream synchronize");
     if (v != 0) VNM_CUDA(cudaMemsetAsync(h->status, 0, sizeof(int), s), "status clear");
