@@ -260,3 +260,59 @@ def test_layer_called_on_two_streams():
         assert torch.equal(layer(x), w)
         busy.synchronize()
         assert torch.equal(a, w)
+
+
+# A layer holds its weight in each form that a token count has wanted, or in the one that it was given.
+@pytest.mark.parametrize("form", [0, 1, 2])
+def test_layer_holds_the_form_it_is_given(form):
+    import torch
+    from venom_b200 import spatha_module
+    ext = spatha_module()
+    M, K, V, m = 1024, 4096, 128, 16
+    d, values, meta, c, _ = _operand(M, K, V, m, None, seed=23)
+    layer = _layer_of(values, meta, c, M, K, V, m)
+    layer.form = form
+    ext.clear_cache()
+    for n in _two_forms(M, K, V, m):
+        x = _ints((n, K), n)
+        want = (x.float() @ d.T).half()
+        assert torch.equal(layer(x), want)
+        wide = torch.zeros((n, K + 8), dtype=torch.float16, device="cuda")
+        wide[:, :K] = x
+        assert torch.equal(layer(wide[:, :K]), want)                  # through spmm(), a transposed view
+        b = x.T.contiguous()
+        assert torch.equal(ext.spmm(meta, c, layer.values, b, None, M, K, n, V, 2, m, values.numel(), 0, 32, 4, form), want)
+    assert ext.cache_size() == 1 and ext.cached_copies() == (2 if form == 0 else 1)
+    with pytest.raises(RuntimeError, match="form"):
+        ext.linear(x, meta, c, layer.values, None, M, K, V, 2, m, 3)
+
+
+def test_layer_without_a_dense_b_form():
+    import torch
+    M, K, V, m = 128, 280, 64, 10
+    d, values, meta, c, _ = _operand(M, K, V, m, None, seed=3)
+    layer = _layer_of(values, meta, c, M, K, V, m)
+    layer.form = 2
+    x = _ints((16, K), 1)
+    assert torch.equal(layer(x), (x.float() @ d.T).half())
+
+
+# A form that does not fit the device (193 GB) is an error of its own call only.
+def test_form_that_does_not_fit():
+    import torch
+    from venom_b200 import capi, spatha_module
+    M, K, V, m, N = 262144, 655360, 128, 256, 8
+    ksp, nv, nm, nc = capi.sizes(M, K, V, m)
+    values = torch.zeros(nv, dtype=torch.float16, device="cuda")
+    meta = torch.full((nm,), 0x44444444, dtype=torch.int32, device="cuda")
+    cols = torch.tensor([0, 1, 2, 3], dtype=torch.int32, device="cuda").repeat(nc // 4)
+    x = torch.ones((N, K), dtype=torch.float16, device="cuda")
+    for form in (2, 1, 2):
+        call = lambda: spatha_module().linear(x, meta, cols, values, None, M, K, V, 2, m, form)
+        if form == 2:
+            with pytest.raises(RuntimeError, match="out of memory"):
+                call()
+        else:
+            assert not call().any()
+    assert torch.ones(4, device="cuda").sum().item() == 4             # no error left behind
+    spatha_module().clear_cache()

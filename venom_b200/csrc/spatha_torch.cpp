@@ -10,7 +10,8 @@
 //     prepared operand is cached.  An entry is tied to the three tensors' storages through weak references:
 //     once any of them has been freed (even if a new tensor later lands on the same address) the entry is
 //     dead, its device copy is released and the operand is re-packed.  In-place edits bump the tensors'
-//     version counters, which are part of the key.
+//     version counters, which are part of the key (the copies of earlier versions go with the tensors, or with clear_cache()).
+//   * an operand is held in each form (gather, dense-B) that a call has wanted, at most two copies; `form` holds it in one.
 #include <torch/extension.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGraphsC10Utils.h>
@@ -42,7 +43,7 @@ struct Key {
 using WeakStorage = c10::weak_intrusive_ptr<c10::StorageImpl>;
 
 struct Entry {
-    // the operand re-packed per form (VNM_STRATEGY_GATHER, VNM_STRATEGY_DENSE_B), each when a call first wants it
+    // the operand re-packed per form (0: gather, 1: dense-B), each when a call first wants it
     vnm_handle_t handle[2];
     int last_n, last_t, last_form;   // the form of the last shape of call
     int64_t nv, nm, nc;              // sizes of the three arrays
@@ -97,11 +98,12 @@ void check_sizes(const torch::Tensor &A_metadata, const torch::Tensor &A_indices
                 nv, ", metadata ", nm, ", indices ", nc, ")");
 }
 
-// The handle that multiplies N columns: looked up in (or added to) the cache, in the form estimated to be the faster one
-// for this number of columns and the layout of the activation.  `dense_b` receives that form.
+// The handle that multiplies N columns: looked up in (or added to) the cache, in the form `form` (VNM_STRATEGY_*), or for AUTO in
+// the one estimated to be the faster for this number of columns and the layout of the activation.  `dense_b` receives that form.
 vnm_handle_t operand_for(const torch::Tensor &A_metadata, const torch::Tensor &A_indices, const torch::Tensor &A_values, int M, int K, int V, int n, int m,
-                         int device, int N, bool in_place, cudaStream_t stream, int *dense_b)
+                         int device, int N, bool in_place, int form, cudaStream_t stream, int *dense_b)
 {
+    TORCH_CHECK(form == VNM_STRATEGY_AUTO || form == VNM_STRATEGY_GATHER || form == VNM_STRATEGY_DENSE_B, "spatha.spmm: unknown form ", form);
     Key key{A_values.data_ptr(), A_metadata.data_ptr(), A_indices.data_ptr(), M, K, V, n, m, device,
             (uint32_t)A_values._version(), (uint32_t)A_metadata._version(), (uint32_t)A_indices._version()};
     std::lock_guard<std::mutex> lock(g_mutex);
@@ -124,21 +126,27 @@ vnm_handle_t operand_for(const torch::Tensor &A_metadata, const torch::Tensor &A
     // Dense-B form or gather form: by the estimate for this number of columns and the layout of the activation (a
     // transposed [tokens, features] view is read in place by the dense-B form and transposed for the gather form).
     Entry &e = it->second;
-    if (e.last_n != N || e.last_t != (int)in_place) {
-        int strategy = 0;
-        check(vnm_choose_form(M, K, V, n, m, N, in_place ? 1 : 0, &strategy), "vnm_choose_form");
-        e.last_form = strategy == VNM_STRATEGY_DENSE_B ? 1 : 0;
-        e.last_n = N;
-        e.last_t = in_place;
+    if (form != VNM_STRATEGY_AUTO) {
+        *dense_b = form == VNM_STRATEGY_DENSE_B && m % 4 == 0 && K % m == 0;   // else there is only the gather form
+    } else {
+        if (e.last_n != N || e.last_t != (int)in_place) {
+            int strategy = 0;
+            check(vnm_choose_form(M, K, V, n, m, N, in_place ? 1 : 0, &strategy), "vnm_choose_form");
+            e.last_form = strategy == VNM_STRATEGY_DENSE_B ? 1 : 0;
+            e.last_n = N;
+            e.last_t = in_place;
+        }
+        *dense_b = e.last_form;
+        // A graph that is being captured uses the form that is there: re-packing is work for outside of it.
+        if (!e.handle[*dense_b] && e.handle[1 - *dense_b] && c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) *dense_b = 1 - *dense_b;
     }
-    *dense_b = e.last_form;
-    // A graph that is being captured uses the form that is there: re-packing is work for outside of it.
-    if (!e.handle[*dense_b] && e.handle[1 - *dense_b] && c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) *dense_b = 1 - *dense_b;
-    vnm_handle_t &h = e.handle[*dense_b];
-    if (!h)
-        check(vnm_prepare_as(A_values.data_ptr(), (const uint32_t *)A_metadata.data_ptr(), (const uint32_t *)A_indices.data_ptr(), M, K, V, n, m,
-                             *dense_b ? VNM_STRATEGY_DENSE_B : VNM_STRATEGY_GATHER, &h, stream), "vnm_prepare_as");
-    return h;
+    if (!e.handle[*dense_b]) {
+        const int rc = vnm_prepare_as(A_values.data_ptr(), (const uint32_t *)A_metadata.data_ptr(), (const uint32_t *)A_indices.data_ptr(), M, K, V, n, m,
+                                      *dense_b ? VNM_STRATEGY_DENSE_B : VNM_STRATEGY_GATHER, &e.handle[*dense_b], stream);
+        if (rc == VNM_ERR_CUDA && form == VNM_STRATEGY_AUTO && e.handle[1 - *dense_b]) e.last_form = *dense_b = 1 - *dense_b;   // no memory for a second form
+        else check(rc, "vnm_prepare_as");
+    }
+    return e.handle[*dense_b];
 }
 
 void check_arrays(const torch::Tensor &A_metadata, const torch::Tensor &A_indices, const torch::Tensor &A_values, const torch::Tensor &rhs)
@@ -170,7 +178,7 @@ void product_nk(vnm_handle_t h, int dense_b, const torch::Tensor &act, int64_t l
 
 torch::Tensor spmm(torch::Tensor A_metadata, torch::Tensor A_indices, torch::Tensor A_values, torch::Tensor rhs_matrix,
                    c10::optional<torch::Tensor> bias, int64_t A_num_rows, int64_t A_num_cols, int64_t B_num_cols,
-                   int64_t vec_length, int64_t n, int64_t m, int64_t nnz, int64_t seed, int64_t mbrow, int64_t brow)
+                   int64_t vec_length, int64_t n, int64_t m, int64_t nnz, int64_t seed, int64_t mbrow, int64_t brow, int64_t form)
 {
     (void)seed;
     check_arrays(A_metadata, A_indices, A_values, rhs_matrix);
@@ -189,7 +197,7 @@ torch::Tensor spmm(torch::Tensor A_metadata, torch::Tensor A_indices, torch::Ten
     cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
     int dense_b = 0;
     const bool in_place = rhs_is_t_view && rhs_matrix.stride(1) % 8 == 0 && (reinterpret_cast<uintptr_t>(rhs_matrix.data_ptr()) & 15) == 0;
-    vnm_handle_t h = operand_for(A_metadata, A_indices, A_values, M, K, V, (int)n, (int)m, (int)rhs_matrix.device().index(), N, in_place, stream, &dense_b);
+    vnm_handle_t h = operand_for(A_metadata, A_indices, A_values, M, K, V, (int)n, (int)m, (int)rhs_matrix.device().index(), N, in_place, (int)form, stream, &dense_b);
     auto out = device_empty({N, M}, torch::kFloat16, rhs_matrix);
     if (in_place) {
         product_nk(h, dense_b, rhs_matrix, rhs_matrix.stride(1), K, N, M, bias_ptr, out, stream);
@@ -205,7 +213,7 @@ torch::Tensor spmm(torch::Tensor A_metadata, torch::Tensor A_indices, torch::Ten
 // share of the call took longer than the product: measured 12.2 us a call before, 6.3 after, for a kernel of 5 us).  An undefined
 // result (None) means: an input that is not read in place -- take spmm().
 c10::optional<torch::Tensor> linear(const torch::Tensor &input, const torch::Tensor &A_metadata, const torch::Tensor &A_indices, const torch::Tensor &A_values,
-                                    const c10::optional<torch::Tensor> &bias, int64_t A_num_rows, int64_t A_num_cols, int64_t vec_length, int64_t n, int64_t m)
+                                    const c10::optional<torch::Tensor> &bias, int64_t A_num_rows, int64_t A_num_cols, int64_t vec_length, int64_t n, int64_t m, int64_t form)
 {
     const int M = (int)A_num_rows, K = (int)A_num_cols;
     const int64_t dims = input.dim();
@@ -217,7 +225,7 @@ c10::optional<torch::Tensor> linear(const torch::Tensor &input, const torch::Ten
     c10::cuda::CUDAGuard guard(input.device());
     cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
     int dense_b = 0;
-    vnm_handle_t h = operand_for(A_metadata, A_indices, A_values, M, K, (int)vec_length, (int)n, (int)m, (int)input.device().index(), (int)N, true, stream, &dense_b);
+    vnm_handle_t h = operand_for(A_metadata, A_indices, A_values, M, K, (int)vec_length, (int)n, (int)m, (int)input.device().index(), (int)N, true, (int)form, stream, &dense_b);
     c10::SmallVector<int64_t, 6> shape(input.sizes().begin(), input.sizes().end());
     shape.back() = M;
     auto out = device_empty(shape, torch::kFloat16, input);
@@ -342,6 +350,15 @@ int64_t cache_size()
     return (int64_t)g_cache.size();
 }
 
+int64_t cached_copies()
+{
+    std::lock_guard<std::mutex> lock(g_mutex);
+    int64_t n = 0;
+    for (const auto &kv : g_cache)
+        for (vnm_handle_t h : kv.second.handle) n += h != nullptr;
+    return n;
+}
+
 // linear() and product() as plain C functions of the module: pybind11's conversion of their arguments took 0.4 us a call.
 namespace {
 
@@ -366,15 +383,15 @@ PyObject *wrapped(c10::optional<torch::Tensor> &t)
 PyObject *py_linear(PyObject *, PyObject *const *args, Py_ssize_t n)
 {
     HANDLE_TH_ERRORS
-    TORCH_CHECK_TYPE(n == 10, "linear(input, A_metadata, A_indices, A_values, bias, A_num_rows, A_num_cols, vec_length, n, m)");
+    TORCH_CHECK_TYPE(n == 10 || n == 11, "linear(input, A_metadata, A_indices, A_values, bias, A_num_rows, A_num_cols, vec_length, n, m, form=0)");
     const at::Tensor &input = tensor_of(args[0]), &meta = tensor_of(args[1]), &idx = tensor_of(args[2]), &values = tensor_of(args[3]);
     const c10::optional<torch::Tensor> bias = tensor_or_none(args[4]);
-    int64_t v[5];
-    for (int i = 0; i < 5; i++) v[i] = THPUtils_unpackLong(args[5 + i]);
+    int64_t v[6] = {0, 0, 0, 0, 0, VNM_STRATEGY_AUTO};
+    for (int i = 0; i < (int)n - 5; i++) v[i] = THPUtils_unpackLong(args[5 + i]);
     c10::optional<torch::Tensor> out;
     {
         pybind11::gil_scoped_release no_gil;
-        out = linear(input, meta, idx, values, bias, v[0], v[1], v[2], v[3], v[4]);
+        out = linear(input, meta, idx, values, bias, v[0], v[1], v[2], v[3], v[4], v[5]);
     }
     return wrapped(out);
     END_HANDLE_TH_ERRORS
@@ -410,11 +427,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, mod)
     mod.def("spmm", &spmm, "V:N:M sparse x dense product (returns [B_num_cols, A_num_rows])", pybind11::arg("A_metadata"), pybind11::arg("A_indices"),
             pybind11::arg("A_values"), pybind11::arg("rhs_matrix"), pybind11::arg("bias"), pybind11::arg("A_num_rows"), pybind11::arg("A_num_cols"),
             pybind11::arg("B_num_cols"), pybind11::arg("vec_length"), pybind11::arg("n"), pybind11::arg("m"), pybind11::arg("nnz"),
-            pybind11::arg("seed"), pybind11::arg("mbrow"), pybind11::arg("brow"));
+            pybind11::arg("seed"), pybind11::arg("mbrow"), pybind11::arg("brow"), pybind11::arg("form") = (int64_t)VNM_STRATEGY_AUTO);
     if (PyModule_AddFunctions(mod.ptr(), fast_calls) != 0) throw pybind11::error_already_set();
     mod.def("compress", &compress, "vnm_compress_f16 with its allocations, or None", pybind11::call_guard<pybind11::gil_scoped_release>());
     mod.def("sparsify", &sparsify, "vnm_sparsify_magnitude with its allocations, or None", pybind11::call_guard<pybind11::gil_scoped_release>());
     mod.def("decompress", &decompress, "vnm_decompress_f16 with its allocation, or None", pybind11::call_guard<pybind11::gil_scoped_release>());
     mod.def("clear_cache", &clear_cache, "Drop every cached prepared operand");
-    mod.def("cache_size", &cache_size);
+    mod.def("cache_size", &cache_size, "Cached operands");
+    mod.def("cached_copies", &cached_copies, "Device copies they hold: one or two (gather form, dense-B form) each");
 }

@@ -104,23 +104,31 @@ class NMVectorSparsifier:
         return SrNMTensor(self.n, self.m, self.tileM, dense, mask, columns, device)
 
 
-def sparse_dense_mul_dispatch(sparse_values, sparse_indices, sparse_metadata, dense, nrows_sp, ncols_sp, ncols_d, m, n, v, nnz, bias):
-    """Same call as the reference helper: returns [ncols_d, nrows_sp] = (A @ dense).T + bias."""
+def sparse_dense_mul_dispatch(sparse_values, sparse_indices, sparse_metadata, dense, nrows_sp, ncols_sp, ncols_d, m, n, v, nnz, bias, form=capi.STRATEGY_AUTO):
+    """Same call as the reference helper: returns [ncols_d, nrows_sp] = (A @ dense).T + bias.  form: see SrnmSpmm."""
     # the reference materialises `dense.contiguous()` here; the op accepts the transposed view itself and
     # copies only when it has to
     dense_ = dense
-    return spatha_module().spmm(sparse_metadata, sparse_indices, sparse_values, dense_, bias, nrows_sp, ncols_sp, ncols_d, v, n, m, nnz, 0, 32, 4)
+    return spatha_module().spmm(sparse_metadata, sparse_indices, sparse_values, dense_, bias, nrows_sp, ncols_sp, ncols_d, v, n, m, nnz, 0, 32, 4, form)
 
 
 _linear = None     # the extension's call, looked up once
 
 
 class SrnmSpmm(torch.nn.Module):
-    """Drop-in replacement of torch.nn.Linear whose weight is stored in V:N:M form."""
+    """Drop-in replacement of torch.nn.Linear whose weight is stored in V:N:M form.
 
-    def __init__(self, original, n=2, m=8, v=64, sparsifier=None):
+    form: the kernel-private copy of the weight that the layer holds on the device beside the arrays.  The default,
+    capi.STRATEGY_AUTO, takes for every number of tokens the form estimated to be faster and keeps each form that has been
+    wanted: at most 1.125 bytes (dense-B) plus 4.5 / m bytes (gather) a weight element.  capi.STRATEGY_GATHER and
+    capi.STRATEGY_DENSE_B hold that one form only, whatever is faster."""
+
+    form = capi.STRATEGY_AUTO    # layers that were pickled without one
+
+    def __init__(self, original, n=2, m=8, v=64, sparsifier=None, form=capi.STRATEGY_AUTO):
         super().__init__()
         self.n, self.m, self.v = n, m, v
+        self.form = form
         self.bias = original.bias
         w = (sparsifier or NMVectorSparsifier(n, m, v))(original.weight)
         self.values = torch.nn.Parameter(w.values, requires_grad=False)
@@ -136,25 +144,25 @@ class SrnmSpmm(torch.nn.Module):
         global _linear
         if _linear is None:
             _linear = spatha_module().linear
-        out = _linear(input, self.metadata, self.columns, values, bias, self.nrows_sp, self.ncols_sp, self.v, self.n, self.m)
+        out = _linear(input, self.metadata, self.columns, values, bias, self.nrows_sp, self.ncols_sp, self.v, self.n, self.m, self.form)
         if out is not None:
             return out
         flat = torch.flatten(input, start_dim=0, end_dim=-2)
         ncols_d = flat.shape[0]
         out = sparse_dense_mul_dispatch(values, self.columns, self.metadata, flat.T, self.nrows_sp, self.ncols_sp, ncols_d,
-                                        self.m, self.n, self.v, self.nnz, bias)
+                                        self.m, self.n, self.v, self.nnz, bias, self.form)
         return out.reshape((*input.shape[0:-1], -1))
 
 
-def linear_to_spmm(mod, n=2, m=8, v=64, skip=()):
+def linear_to_spmm(mod, n=2, m=8, v=64, skip=(), form=capi.STRATEGY_AUTO):
     """Replaces every torch.nn.Linear below `mod` by SrnmSpmm (end2end/bert_pytorch.py:155-167)."""
     if isinstance(mod, torch.nn.Linear):
-        return SrnmSpmm(mod, n, m, v)
+        return SrnmSpmm(mod, n, m, v, form=form)
     for name, child in mod.named_children():
         if isinstance(child, SrnmSpmm) or name in skip:
             continue
         if isinstance(child, torch.nn.Linear):
-            setattr(mod, name, SrnmSpmm(child, n, m, v))
+            setattr(mod, name, SrnmSpmm(child, n, m, v, form=form))
         elif child is not mod:
-            linear_to_spmm(child, n, m, v, skip)
+            linear_to_spmm(child, n, m, v, skip, form)
     return mod
