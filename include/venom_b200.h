@@ -205,7 +205,8 @@ int vnm_selftest_wait_expiry(vnm_handle_t handle, void *stream);
  * indirection exactly like the reference's compile-time IDEAL_KERNEL experiment
  * (include/spatha/block_sparse/spmm/blockwise_kernel.h:328-642, row = nz_block_idx % 4 at :536);
  * 2 = B is not loaded at all (timing floor; results are meaningless).
- * Producer warps: 4 and 8 are accepted for compatibility; sixteen warps issue the gather loads whatever is set. */
+ * Producer warps: how many warps of the gather kernel issue those loads, 16 (default), 8 or 4; fewer than 16 also keep the product
+ * in that kernel where another one would be chosen.  Identical bits for more than 64 columns. */
 int vnm_set_gather_mode(vnm_handle_t handle, int mode);
 /* Gather mode 3 only: of the 64 gathered rows of every stage, `tma_rows` (0, 16, 32 or 48) are fetched by TMA
  * tile::gather4 and the others by the per-thread copies, so that both paths into the SM are busy at once. */

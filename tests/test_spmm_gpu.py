@@ -210,8 +210,8 @@ def test_spmm_baseline_shapes_sampled_rows(capi, oracle, shape):
 
 
 def test_gather_modes_agree_when_every_row_is_selected(capi, oracle):
-    """m == 4: the 64-row tile loads (default) and the gather4 loads must give identical bits; both
-    producer-warp counts too."""
+    """m == 4: the 64-row tile loads (default) and the gather4 loads must give identical bits, in the kernel that the
+    size chooses and in the gather kernel with each number of producer warps."""
     import torch
     M, K, V, m, N = 256, 1024, 128, 4, 512
     capi.set_strategy(capi.STRATEGY_GATHER)          # the gather-mode switch belongs to the V:N:M form
@@ -222,10 +222,40 @@ def test_gather_modes_agree_when_every_row_is_selected(capi, oracle):
     a = prep.spmm(Bd)
     prep.set_gather_mode(0)
     b = prep.spmm(Bd)
-    prep.set_producer_warps(4)
-    c = prep.spmm(Bd)
+    assert torch.equal(a, b)
+    assert prep.config(N)["stages"] == 1                 # the kernel for few tiles
+    prep.set_epilogue(2)                                 # keeps the product in the gather kernel
+    for warps in (16, 8, 4):
+        prep.set_producer_warps(warps)
+        assert prep.config(N)["stages"] == warps         # the gather kernel, with that many
+        for mode in (0, 1, 3):
+            prep.set_gather_mode(mode)
+            assert torch.equal(prep.spmm(Bd), a), (warps, mode)
     assert prep.device_status() == 0
-    assert torch.equal(a, b) and torch.equal(a, c)
+    with pytest.raises(capi.VenomError):
+        prep.set_producer_warps(6)
+    prep.set_epilogue(0)
+    prep.set_gather_mode(0)
+    assert prep.config(N)["stages"] == 4                 # fewer warps alone keep it there, too
+
+
+@pytest.mark.parametrize("shape", [(256, 2048, 128, 16, 1000), (320, 1200, 64, 20, 520), (2048, 2048, 32, 32, 4096), (128, 128, 32, 8, 72)])
+def test_fewer_producer_warps_give_identical_bits(capi, oracle, shape):
+    """Two and four pairs of producer warps go round the ring of nine stages in other steps than eight: stages of one tile and
+    of many, tiles that a pair skips."""
+    import torch
+    M, K, V, m, N = shape
+    capi.set_strategy(capi.STRATEGY_GATHER)
+    try:
+        prep, Bd, _ = _setup(capi, oracle, M, K, V, m, N, seed=5 * M + K, ints=False)
+    finally:
+        capi.set_strategy(capi.STRATEGY_AUTO)
+    want = prep.spmm(Bd)
+    for warps in (4, 8):
+        prep.set_producer_warps(warps)
+        assert prep.config(N)["stages"] == warps
+        assert torch.equal(prep.spmm(Bd), want)
+    assert prep.device_status() == 0
 
 
 @pytest.mark.parametrize("shape", [(256, 1024, 128, 8, 512), (256, 2048, 64, 16, 384), (128, 1024, 32, 8, 72), (96, 520, 32, 10, 200),

@@ -356,6 +356,7 @@ class Prepared:
         _check(lib().vnm_set_gather_mode(self._h, mode))
 
     def set_producer_warps(self, warps):
+        """Gather kernel: warps that load the selected rows of B, 16 (default), 8 or 4 (ablation)."""
         _check(lib().vnm_set_producer_warps(self._h, warps))
 
     def set_gather_split(self, tma_rows):

@@ -197,6 +197,7 @@ struct vnm_prepared_s {
     int gather_mode;
     int dense_b;       // 1: A re-expressed as 2:4 over all K columns, B read as plain tiles
     int out32;         // ablation: 32-bit epilogue stores (gather form, layout MN)
+    int producer_warps;  // gather kernel: warps that load B (ablation: fewer than GATHER_PRODUCER_WARPS)
     int hybrid_rows;   // gather form: rows of every 64-row stage fetched by TMA gather4 beside the per-thread copies
     int nm_tma_always; // gather kernel: 1 = the [N,M] result leaves through TMA stores even for a single destination (ablation)
     int l2_ahead;      // pair kernel: k-tiles of L2 prefetch ahead of the shared-memory loads (0 = none)
@@ -252,6 +253,7 @@ void shape_handle(vnm_prepared_s *h, int M, int K, int V, int n, int m, bool den
         h->gather_mode = (m == 4) ? GATHER_CONTIG : GATHER_TMA4;  // with m == 4 every row of B is selected
     }
     h->vblocks_padded = h->mtiles * h->nb;
+    h->producer_warps = GATHER_PRODUCER_WARPS;
     h->pair_mode = 1;
     h->l2_hints = 1;
 }
@@ -495,8 +497,9 @@ int vnm_set_max_ctas(vnm_handle_t h, int max_ctas)
 int vnm_set_producer_warps(vnm_handle_t h, int warps)
 {
     if (!h) return fail(VNM_ERR_BAD_ARG, "null handle");
-    if (warps != 4 && warps != 8) return fail(VNM_ERR_BAD_ARG, "producer warps must be 4 or 8 (got %d)", warps);
-    return VNM_OK;   // the kernel's sixteen producer warps are part of its layout
+    if (warps != 4 && warps != 8 && warps != GATHER_PRODUCER_WARPS) return fail(VNM_ERR_BAD_ARG, "producer warps must be 4, 8 or 16 (got %d)", warps);
+    h->producer_warps = warps;
+    return VNM_OK;
 }
 
 }  // extern "C"
@@ -513,6 +516,7 @@ bool choose_kernel(vnm_handle_t h, int N, int b_nk, int n_more, Kernel *kernel, 
     float big = -1.0f;
     if (!h->dense_b) {
         big = spmm_select_config(h->V, N, h->M, h->ktiles, h->max_ctas, cfg);
+        cfg->stages = h->producer_warps;
         *kernel = KERNEL_GATHER;
     } else {
         if (h->pair_mode || n_more > 0) big = spmm_dense_b_pair_config(h->M, N, h->K, b_nk, h->max_ctas, h->pair_rows, n_more > 0, cfg);
@@ -520,7 +524,7 @@ bool choose_kernel(vnm_handle_t h, int N, int b_nk, int n_more, Kernel *kernel, 
     }
     *us = big;
     // The small kernel has one destination, no cap on its CTAs (it is not persistent) and none of the other kernels' ablations.
-    if (n_more == 0 && h->max_ctas == 0 && !h->nm_tma_always && !h->out32 && h->pair_rows == 0 && h->gather_mode != GATHER_CPASYNC) {
+    if (n_more == 0 && h->max_ctas == 0 && !h->nm_tma_always && !h->out32 && h->producer_warps == GATHER_PRODUCER_WARPS && h->pair_rows == 0 && h->gather_mode != GATHER_CPASYNC) {
         SpmmConfig small_cfg;
         const float small = spmm_small_config(h->mtiles, h->ktiles, N, h->nb, h->gather_mode == GATHER_TMA4, &small_cfg);
         // up to SMALL_SPLIT_N columns it alone is used: its split makes the order of summation its own
@@ -709,7 +713,8 @@ static int spmm_impl(vnm_handle_t h, const void *B, int64_t ldb, int N, int b_nk
         p.hint_b = col_bands ? L2_EVICT_LAST : L2_EVICT_NORMAL;
         if (h->l2_hints == 0) p.hint_a = p.hint_b = L2_EVICT_NORMAL;
     }
-    p.hybrid_rows = h->hybrid_rows;
+    p.producer_pairs = (int16_t)(h->producer_warps / 2);
+    p.hybrid_rows = (int16_t)h->hybrid_rows;
     p.b_nk = b_nk;
     p.b_wide_ok = tm_wide ? 1 : 0;
     p.l2_ahead = h->l2_ahead;

@@ -15,6 +15,7 @@ enum : int {
     DEV_TIMEOUT_DRAIN = 8      // drain of in-flight copies after an abort gave up
 };
 
+// 160 bytes: four more cost the small kernel's launches 0.5 us each (5.5 -> 6.0 us a call at 1024 x 1024, 8 columns).
 struct SpmmParams {
     const uint8_t *am;    // [mtiles][ktiles][AM_BLOCK_BYTES] value + metadata images
     const int4 *rows;     // [vblocks_padded][ktiles*32] absolute B rows
@@ -30,7 +31,8 @@ struct SpmmParams {
     int total_tiles;      // mtiles * ntiles
     const __half *B;      // gather kernel, GATHER_CPASYNC: the dense operand [K, N] itself (row pieces are copied by address)
     int64_t ldb;
-    int hybrid_rows;      // gather kernel, GATHER_CPASYNC: of 64 rows of a block, those fetched by TMA gather4 beside the copies (0, 16, 32, 48)
+    int16_t producer_pairs;   // gather kernel: pairs of warps that load B, 8 except for an ablation
+    int16_t hybrid_rows;  // gather kernel, GATHER_CPASYNC: of 64 rows of a block, those fetched by TMA gather4 beside the copies (0, 16, 32, 48)
     int group_m;          // band of the tile order (tile_coords): > 0 row groups per band, < 0 column tiles per band
     uint64_t hint_a, hint_b;  // pair kernel: L2 eviction-priority policies of the A and B loads (L2_EVICT_*)
     int b_nk;             // dense-B form only: the dense operand is given as [N, K] row-major (K contiguous)
@@ -42,6 +44,7 @@ struct SpmmParams {
     int split_k;          // small kernel: CTAs of a cluster that share one tile's k-tiles
     int n_out;            // destinations of every output tile stored through TMA (1 = `out` only; more: the OutMaps argument, e.g. peers' buffers)
 };
+static_assert(sizeof(SpmmParams) <= 160, "see above");
 
 // Destinations 2 .. MAX_OUTS of a product whose every output tile is stored to several buffers of one geometry
 // (a rank's own result buffer and the same rows of its peers' buffers): tensor maps like the first output map.
@@ -101,6 +104,7 @@ cudaError_t launch_sparsify(const void *w, bool half, int64_t ldw, int M, int K,
                             unsigned long long *violations, cudaStream_t stream);
 
 // Tile configuration of the gather kernel.
+constexpr int GATHER_PRODUCER_WARPS = 16;
 float spmm_select_config(int V, int N, int M, int ktiles, int max_ctas, SpmmConfig *cfg);  // max_ctas: 0 = one per SM; returns an estimate in microseconds, < 0 for an unsupported V
 // Opt-in to large dynamic shared memory for every kernel instance on the CURRENT device (call once per device).
 cudaError_t spmm_init_kernels();

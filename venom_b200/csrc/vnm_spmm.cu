@@ -14,6 +14,7 @@
 //                 numbers per instruction, precomputed by the prepare step).  A warp needs about 65 clocks for each gather4
 //                 it issues, whatever the others do, so the intake of an SM is a matter of how many warps issue at
 //                 once: 1 warp 8 B/clk, 6 warps 41, 12 warps 57, 24 warps 67 (B in L2; plain 8 KiB tile loads reach 73).
+//                 (vnm_set_producer_warps, an ablation, leaves only the first two or four pairs at work.)
 //   warp 16       A producer (one lane).
 //   warp 17       tensor-memory owner and MMA issuer.  It waits for the operands itself, copies a k-tile's metadata to
 //                 tensor memory (tcgen05.cp) and issues the MMAs right behind it: copies and MMAs of one thread execute
@@ -47,7 +48,7 @@ struct Traits {
     static_assert(GATHERS == 32, "a stage is dealt to the 2 x 16 lanes of a producer pair");
     static constexpr int SA = 3, SB = 9;
     static constexpr int H = 2;                  // producer warps that share a stage
-    static constexpr int PW = 16;                // producer warps
+    static constexpr int PW = GATHER_PRODUCER_WARPS;
     static constexpr int NG = PW / H;
     static constexpr int A_WARP = PW, MMA_WARP = PW + 1, EPI_WARP0 = PW + 4;
     static constexpr int NUM_WARPS = EPI_WARP0 + 8;
@@ -117,8 +118,9 @@ __global__ void __launch_bounds__(Traits<BN, NB>::NUM_THREADS, 1)
     const uint32_t tmem_base = *tmem_slot;
     grid_launch_dependents();
 
-    if (warp < T::PW) {
+    if (warp < T::H * p.producer_pairs) {
         // ---------------- B producers ----------------
+        const int ng = p.producer_pairs;
         const int part = warp % T::H;
         int j = warp / T::H, s = j, wrap = 0;         // stage, its ring slot, times the ring has gone round
         static_assert(T::NG <= SB, "a pair's first stage has its own slot");
@@ -187,7 +189,7 @@ __global__ void __launch_bounds__(Traits<BN, NB>::NUM_THREADS, 1)
                 cp_async_mbar_arrive_noinc(full);   // arrives once this lane's copies have landed
             }
             ++issued;
-            j += T::NG; jl += T::NG; s += T::NG;
+            j += ng; jl += ng; s += ng;
             if (s >= SB) { s -= SB; ++wrap; }
             if (jl >= per_tile) {
                 do { jl -= per_tile; ++tile_i; } while (jl >= per_tile);
@@ -196,9 +198,9 @@ __global__ void __launch_bounds__(Traits<BN, NB>::NUM_THREADS, 1)
             if (j < total_j) r = fetch();
         }
         if (gmode == GATHER_CPASYNC) cp_async_wait_all();
-        if (*abort_flag && lane == 0 && gmode != GATHER_NONE) {   // this warp's copies still in flight: its last two stages at most
-            for (int back = 1; back <= 2 && back <= issued; back++) {
-                const int jj = j - back * T::NG;
+        if (*abort_flag && lane == 0 && gmode != GATHER_NONE) {   // this warp's copies still in flight: its stages of the last round of the ring
+            for (int back = 1; back <= (SB + ng - 1) / ng && back <= issued; back++) {
+                const int jj = j - back * ng;
                 drain_slot(&b_full[jj % SB], (uint32_t)(jj / SB) & 1u, p.status);
             }
         }
