@@ -193,14 +193,6 @@ __device__ __forceinline__ void tma_load_2d(void *smem_dst, const void *tmap, in
                  "l"(tmap), "r"(col), "r"(row), "r"(smem_u32(bar))
                  : "memory");
 }
-// TMA tile load of a 4-D box at (c0, c1, c2, c3), c0 innermost.
-__device__ __forceinline__ void tma_load_4d(void *smem_dst, const void *tmap, int c0, int c1, int c2, int c3, uint64_t *bar)
-{
-    asm volatile("cp.async.bulk.tensor.4d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(
-                     smem_u32(smem_dst)),
-                 "l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(bar))
-                 : "memory");
-}
 // TMA tile store shared -> global of a 2-D box at (col, row); completion is tracked by bulk groups.
 __device__ __forceinline__ void tma_store_2d(const void *tmap, const void *smem_src, int col, int row)
 {
@@ -211,7 +203,6 @@ __device__ __forceinline__ void tma_store_2d(const void *tmap, const void *smem_
 __device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // Waits until the bulk groups of this thread have finished READING shared memory (the source may be reused).
 __device__ __forceinline__ void bulk_wait_group_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_group0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void named_barrier_sync(uint32_t id, uint32_t threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 // Named barrier that also returns the AND of `pred` over its participants.
 __device__ __forceinline__ bool named_barrier_and(uint32_t id, uint32_t threads, bool pred)
@@ -239,11 +230,6 @@ __device__ __forceinline__ void cp_async_mbar_arrive_noinc(uint64_t *bar)
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-// Register re-allocation between warpgroups (all four warps of a warpgroup must execute the same one).
-template <int kRegs>
-__device__ __forceinline__ void setmaxnreg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegs)); }
-template <int kRegs>
-__device__ __forceinline__ void setmaxnreg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegs)); }
 __device__ __forceinline__ void tma_prefetch_desc(const void *tmap)
 {
     asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory");
@@ -306,17 +292,6 @@ __device__ __forceinline__ void tc_mma_sp_f16(uint32_t d_tmem, uint64_t adesc, u
         "setp.ne.b32 p, %5, 0;\n\t"
         "tcgen05.mma.sp.cta_group::1.kind::f16 [%0], %1, %2, [%3], %4, {%6, %7, %8, %9}, p;\n\t}" ::"r"(d_tmem),
         "l"(adesc), "l"(bdesc), "r"(meta_tmem), "r"(idesc), "r"(accumulate), "r"(m0), "r"(m1), "r"(m2), "r"(m3)
-        : "memory");
-}
-// Dense counterpart (used by the self-test of the descriptors).
-__device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate,
-                                           uint32_t m0, uint32_t m1, uint32_t m2, uint32_t m3)
-{
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}" ::"r"(d_tmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(m0), "r"(m1), "r"(m2), "r"(m3)
         : "memory");
 }
 // 32 lanes x 32 consecutive 32-bit columns -> 32 registers per thread (thread t = lane base + t).
