@@ -35,15 +35,15 @@ constexpr int B_STAGE_BYTES = 2 * B_CHUNK_BYTES;    // 16 KiB: two 64-column sli
 constexpr int OUT_STAGE_BYTES = TILE_M * PART * 2;  // 128 rows x 40 fp16 columns, staging of one TMA store
 constexpr int BAR_BYTES = 640;
 // What depends on the row tiles per CTA.  The rings and the metadata sets advance one k-tile at a time; a k-tile is 68 KiB with
-// two row tiles, 50 KiB with one.
-template <int R>
+// two row tiles, 50 KiB with one.  Only results with several destinations pass through staging buffers.
+template <int R, bool MULTI>
 struct Plan {
     static constexpr int SA = R == 1 ? 4 : 3;                          // A ring: k-tiles (each R blocks)
     static constexpr int SB = SA * STAGES_PER_KT;                      // B ring: stages of 64 rows x 128 columns (this CTA's half of two K=32 blocks of the MMAs)
     static constexpr int A_STAGE_BYTES = R * AM_BLOCK_BYTES;
     static constexpr int A_RING_BYTES = SA * A_STAGE_BYTES;
     static constexpr int B_RING_BYTES = SB * B_STAGE_BYTES;
-    static constexpr int OUT_RING_BYTES = RT * OUT_STAGE_BYTES;        // one staging buffer per accumulator
+    static constexpr int OUT_RING_BYTES = MULTI ? RT * OUT_STAGE_BYTES : 0;   // one staging buffer per accumulator
     static constexpr int SMEM_BYTES = A_RING_BYTES + B_RING_BYTES + OUT_RING_BYTES + BAR_BYTES + 1024;
     static_assert(A_STAGE_BYTES % 1024 == 0 && B_STAGE_BYTES % 1024 == 0, "swizzled staging needs 1024-byte alignment");
     static_assert(SMEM_BYTES <= 227 * 1024, "shared memory per CTA");
@@ -137,8 +137,9 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
     static_assert(R == 1 || R == RT, "row tiles per CTA");  // R = 1: pair tiles of 256 rows for problems with few row tiles
     static_assert(BN <= 240 && BN % 16 == 0, "the tensor-memory column plan");
     static_assert(!MULTI || BN == 6 * PART, "parts of a tile that leaves through TMA stores");
-    constexpr int SA = Plan<R>::SA, SB = Plan<R>::SB, A_STAGE_BYTES = Plan<R>::A_STAGE_BYTES, A_RING_BYTES = Plan<R>::A_RING_BYTES;
-    constexpr int B_RING_BYTES = Plan<R>::B_RING_BYTES, OUT_RING_BYTES = Plan<R>::OUT_RING_BYTES;
+    using P = Plan<R, MULTI>;
+    constexpr int SA = P::SA, SB = P::SB, A_STAGE_BYTES = P::A_STAGE_BYTES, A_RING_BYTES = P::A_RING_BYTES;
+    constexpr int B_RING_BYTES = P::B_RING_BYTES, OUT_RING_BYTES = P::OUT_RING_BYTES;
     constexpr int HALF_N = BN / 2;   // columns of a B stage held by each CTA of the pair
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -510,7 +511,7 @@ cudaError_t spmm_dense_b_pair_init()
 {
     cudaError_t e;
 #define VNM_PAIR_ATTR(R, BN, MULTI) \
-    if ((e = cudaFuncSetAttribute(spmm_dense_b_pair_kernel<R, BN, MULTI>, cudaFuncAttributeMaxDynamicSharedMemorySize, Plan<R>::SMEM_BYTES)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(spmm_dense_b_pair_kernel<R, BN, MULTI>, cudaFuncAttributeMaxDynamicSharedMemorySize, Plan<R, MULTI>::SMEM_BYTES)) != cudaSuccess) return e;
     VNM_PAIR_INSTANCES(VNM_PAIR_ATTR)
 #undef VNM_PAIR_ATTR
     int dev = 0, sms = 0;
@@ -519,7 +520,7 @@ cudaError_t spmm_dense_b_pair_init()
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3((unsigned)(sms & ~1), 1, 1);
     lc.blockDim = dim3(NUM_THREADS, 1, 1);
-    lc.dynamicSmemBytes = Plan<1>::SMEM_BYTES;
+    lc.dynamicSmemBytes = Plan<1, false>::SMEM_BYTES;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
@@ -562,7 +563,7 @@ float spmm_dense_b_pair_config(int M, int N, int K, int b_nk, int max_ctas, int 
                 best = us;
                 cfg->bn = widths[w];
                 cfg->nb = 2 * rt;  // row tiles per pair tile
-                cfg->smem_bytes = rt == RT ? Plan<2>::SMEM_BYTES : Plan<1>::SMEM_BYTES;
+                cfg->smem_bytes = rt == RT ? (multi ? Plan<2, true>::SMEM_BYTES : Plan<2, false>::SMEM_BYTES) : (multi ? Plan<1, true>::SMEM_BYTES : Plan<1, false>::SMEM_BYTES);
                 cfg->grid = 2 * (int)(tiles < clusters ? tiles : clusters);
             }
         }
