@@ -221,7 +221,7 @@ int vnm_set_gather_split(vnm_handle_t handle, int tma_rows);
 int vnm_set_epilogue(vnm_handle_t handle, int mode);
 
 /* How vnm_prepare lays the sparse operand out for the kernel (process-wide, applies to later calls):
- *   AUTO     pick per (V, m) from measurements on B200 (default);
+ *   AUTO     pick per (V, m, rows) from measurements on B200 (default), the same for every number of columns;
  *   GATHER   the V:N:M form: only the four selected rows of B per group are gathered per vector block;
  *   DENSE_B  the pattern re-expressed as plain 2:4 over all K columns (needs m % 4 == 0 and K % m == 0):
  *            B is read as ordinary tiles shared by all vector blocks, at m/4 times the MMA work.
@@ -234,7 +234,7 @@ int vnm_prepare_as(const void *values, const uint32_t *meta, const uint32_t *col
                    int M, int K, int V, int n, int m, int strategy, vnm_handle_t *handle, void *stream);
 int vnm_set_producer_warps(vnm_handle_t handle, int warps);
 /* Dense-B form only: 1 (default) = products with enough tiles run on pairs of SMs (thread-block clusters of two CTAs, tcgen05
- * cta_group::2: each CTA loads half of every B stage), 0 = one SM per tile wherever the result has a single destination,
+ * cta_group::2: each CTA loads half of every B stage), 0 = the kernel for few tiles (one SM a tile) wherever the result has a single destination,
  * 2 = pairs without the L2 eviction-priority hints that ask the banded operand to stay cached,
  * 3 / 4 = pairs with one / two row tiles per CTA forced (default: whichever has the smaller estimate; with one, the two
  * accumulators alternate between consecutive tiles).  Ablation switches; all give identical bits for more than 64 columns. */
@@ -242,7 +242,7 @@ int vnm_set_pair_mode(vnm_handle_t handle, int mode);
 /* Host-buffer entry points: number of equal column slices of the upload / product / download pipeline (1 .. 32; slices
  * are multiples of 256 columns and at least 1024 wide; 0 = the default, 8). */
 int vnm_set_host_slices(vnm_handle_t handle, int slices);
-/* Two-SM kernel: the producers also send L2-only prefetches (cp.async.bulk.prefetch) for the operands of the k-tile
+/* Pair kernel (ablation): the producers also send L2-only prefetches (cp.async.bulk.prefetch) for the operands of the k-tile
  * `ktiles_ahead` further on (0 .. 32; 0 = none), beyond the three k-tiles the shared-memory rings hold.  Never changes a
  * result. */
 int vnm_set_l2_prefetch(vnm_handle_t handle, int ktiles_ahead);

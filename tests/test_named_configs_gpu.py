@@ -139,9 +139,9 @@ PAIR_CASES = [(1024, 1024, 64, 8, 17000), (2048, 512, 128, 4, 9000), (512, 4096,
 
 
 @pytest.mark.parametrize("shape", PAIR_CASES, ids=lambda p: "%dx%d_V%d_2:%d_N%d" % p)
-def test_two_sm_kernel_matches_single_sm_kernel_and_oracle(capi, oracle, shape):
-    """Dense-B form on pairs of SMs (cta_group::2, each CTA loading half of every B stage) against the single-SM kernel:
-    same MMAs in the same order, so the bits must be identical -- [M,N], [N,M] + bias, and the [N,K] dense operand --
+def test_pair_kernel_matches_few_tile_kernel_and_oracle(capi, oracle, shape):
+    """Dense-B form on pairs of SMs (cta_group::2, each CTA loading half of every B stage) against the kernel for few tiles
+    (one SM a tile, forced here): same order of summation, so the bits must be identical -- [M,N], [N,M] + bias, and the [N,K] dense operand --
     with a ragged last column tile; and against the CPU oracle on sampled rows."""
     import torch
     M, K, V, m, N = shape
@@ -177,8 +177,8 @@ def test_two_sm_kernel_matches_single_sm_kernel_and_oracle(capi, oracle, shape):
                          ids=lambda p: "%dx%d_V%d_2:%d_N%d" % p)
 def test_product_stored_to_several_destinations(capi, shape):
     """vnm_spmm_f16_multi: every output tile is stored to each destination (the store side of the peer-store gathered
-    product, here with all destinations on one GPU).  Both dense-B kernels, both layouts; every copy must carry the bits
-    of the single-destination product, and memory outside the destinations' rows must stay untouched."""
+    product, here with all destinations on one GPU).  The pair kernel, both layouts; every copy must carry the bits
+    of the single-destination product of the pair kernel and of the kernel for few tiles (pair mode 0), and memory outside the destinations' rows must stay untouched."""
     import torch
     M, K, V, m, N = shape
     dense, colloc, values, meta, B = _operands(capi, M, K, V, m, N, seed=5 * M + K + N)

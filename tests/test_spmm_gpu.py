@@ -261,7 +261,7 @@ def test_fewer_producer_warps_give_identical_bits(capi, oracle, shape):
 @pytest.mark.parametrize("shape", [(256, 1024, 128, 8, 512), (256, 2048, 64, 16, 384), (128, 1024, 32, 8, 72), (96, 520, 32, 10, 200),
                                    (2048, 2048, 128, 16, 4096)])
 def test_gather_paths_give_identical_bits(capi, oracle, shape):
-    """The selected rows of B reach shared memory by per-thread cp.async copies (default), by TMA gather4, or by any
+    """The selected rows of B reach shared memory by TMA gather4 (default), by per-thread cp.async copies, or by any
     split of the two; the MMAs and their order do not change, so every variant must produce the same bits."""
     import torch
     M, K, V, m, N = shape

@@ -241,7 +241,9 @@ class Prepared:
     """Owns a vnm_handle_t: the kernel-private copy of one sparse operand."""
 
     def __init__(self, values, meta, colloc, M, K, V, m, n=2, strategy=None):
-        """strategy: None = the process-wide setting (set_strategy), else STRATEGY_AUTO / _GATHER / _DENSE_B."""
+        """strategy: None = the process-wide setting (set_strategy), else STRATEGY_AUTO / _GATHER / _DENSE_B.  The operand is held in
+        that one form whatever number of columns it is multiplied with; at few columns, where reading it is what takes the time, the
+        gather form has 4 / m of the dense-B form's bytes."""
         _need_cuda(values, meta, colloc)
         ksp, nv, nm, nc = sizes(M, K, V, m, n)
         if values.numel() != nv or meta.numel() != nm or colloc.numel() != nc:
@@ -364,7 +366,7 @@ class Prepared:
         _check(lib().vnm_set_gather_split(self._h, tma_rows))
 
     def set_pair_mode(self, mode):
-        """Dense-B form: 1 = two-SM (cta_group::2) kernel where it applies (default), 0 = one SM per tile where possible,
+        """Dense-B form: 1 = pair (cta_group::2) kernel where it applies (default), 0 = the kernel for few tiles (one SM a tile) where possible,
         2 = pairs without L2 hints, 3 / 4 = pairs with one / two row tiles per CTA forced where the shape allows."""
         _check(lib().vnm_set_pair_mode(self._h, mode))
 
@@ -373,7 +375,7 @@ class Prepared:
         _check(lib().vnm_set_host_slices(self._h, slices))
 
     def set_l2_prefetch(self, ktiles_ahead):
-        """Two-SM kernel: L2-only prefetches this many k-tiles ahead of the loads into shared memory (0 = none)."""
+        """Pair kernel: L2-only prefetches this many k-tiles ahead of the loads into shared memory (0 = none)."""
         _check(lib().vnm_set_l2_prefetch(self._h, ktiles_ahead))
 
     def set_epilogue(self, mode):

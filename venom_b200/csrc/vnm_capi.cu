@@ -150,12 +150,21 @@ int ensure_kernels_ready(int *device_out)
     return VNM_OK;
 }
 
-// Gather form vs dense-B form (see vnm_set_strategy in the header).  The gather form multiplies only what the pattern
-// keeps but gathers, and multiplies with masked MMAs, once per vector block of a row tile; the dense-B form costs m/4 times
-// the MMA work and shares B between all blocks.  Measured on B200 (4096 x 4096, N = 16384): V = 128 from m = 16 on 125 us
-// against 240, at m = 8 207 against 245 (and 15.7 against 20.2 ms at 49152 x 12288 x 32768, where the power cap decides and
-// the zeros of the dense-B form cost what they weigh) unless there are only a few row tiles; V = 64 from m = 32 on; V = 32
-// beyond m = 32.
+// Gather form vs dense-B form where the number of columns is not known (see vnm_set_strategy in the header).  The gather form multiplies
+// only what the pattern keeps but gathers, and multiplies with masked MMAs, once per vector block of a row tile; the dense-B form costs
+// m/4 times the MMA work and shares B between all blocks.  Measured on B200, [K,N] to [M,N], new inputs from call to call, each form
+// by itself until the clock is steady (both run into the power limit: the dense-B form at 1040 to 1500 MHz, the gather form at 1500
+// to 1700), us gather / dense-B:
+//   V = 128, m = 8, 1024 rows and more: 100 / 110 at 12288 x 4096, N = 2048;  250 / 258 at 4096 x 4096 and 76.5 / 75.3 at 1024 x 4096, N =
+//     16384;  1057 / 1125 at 12288 x 12288, N = 8192;  16.2 / 18.2 ms at 49152 x 12288, N = 32768; from 0.64 of the dense-B time (512 columns) to
+//     1.05 (1024 x 1024, N = 8192) over 54 sizes.  Calls of the two forms in turn show the opposite (1128 / 949 and 4554 / 3890 at 12288 and
+//     49152 x 12288, N = 8192), because each then runs at the clock that the other one left behind; after a pause, at the full clock,
+//     913 / 971 and 3580 / 3926, but 69 / 62 at 1024 x 4096, N = 16384.
+//   V = 128, m = 8, fewer rows: the line at 1024 is older than these figures, which have the gather form at 0.55 to 1.19 there (11.7 / 18.5
+//     at 128 x 4096, 24.6 / 26.2 at 512 x 4096, 11.6 / 9.8 at 768 x 512, N = 8192).
+//   4096 x 4096, N = 16384 (at N = 2048 and at 12288 x 12288 the ratios are the same or smaller):  m = 4 420 / 266;  V = 128: m = 16 147 / 248;
+//     V = 64: m = 8 388 / 252, m = 16 215 / 246, m = 32 127 / 243;  V = 32: m = 16 397 / 246, m = 32 220 / 243, m = 64 131 / 240.  The
+//     lines that leave V = 64, m = 16 and V = 32, m = 32 to the dense-B form are older than these figures, too.
 bool choose_dense_b(int M, int K, int V, int m, int strategy)
 {
     const bool possible = (m % 4 == 0) && (K % m == 0);
@@ -203,7 +212,7 @@ struct vnm_prepared_s {
     int l2_ahead;      // pair kernel: k-tiles of L2 prefetch ahead of the shared-memory loads (0 = none)
     int pair_rows;     // pair kernel: 0 = row tiles per CTA chosen per problem, 1 / 2 = forced where possible (ablation)
     int l2_hints;      // pair kernel: 1 = ask L2 to keep the banded operand (default), 0 = no eviction-priority hints
-    int pair_mode;     // dense-B form: 1 = use the two-SM (cta_group::2) kernel where it applies (default), 0 = never
+    int pair_mode;     // dense-B form: 1 = use the pair (cta_group::2) kernel where it applies (default), 0 = only for several destinations
     int max_ctas;      // 0 = one persistent CTA per SM, else the cap set by vnm_set_max_ctas
 };
 

@@ -121,7 +121,7 @@ float spmm_small_config(int mtiles, int ktiles, int N, int nb, bool gather, Spmm
 CUresult spmm_small_encode(EncodeTiledFn enc, CUtensorMap *map, const void *B, int64_t ldb, int K, int N, int b_nk, int gather_mode, int bn);
 cudaError_t launch_spmm_small(const SpmmConfig &cfg, const CUtensorMap &tmap_b, const SpmmParams &p, cudaStream_t stream);
 
-// Dense-B form on pairs of SMs (clusters of two CTAs, tcgen05 cta_group::2): 512 x 240 pair tiles (vnm_spmm_dense_b2.cu).
+// Dense-B form on pairs of SMs (clusters of two CTAs, tcgen05 cta_group::2): pair tiles of 512 or 256 rows (vnm_spmm_dense_b2.cu).
 cudaError_t spmm_dense_b_pair_init();
 float spmm_dense_b_pair_config(int M, int N, int K, int b_nk, int max_ctas, int force_rows, bool multi, SpmmConfig *cfg);  // < 0: not for this problem, else an estimate in microseconds; force_rows: 0 auto, 1 / 2 row tiles per CTA
 cudaError_t launch_spmm_dense_b_pair(const SpmmConfig &cfg, const CUtensorMap &tmap_tile, const CUtensorMap &tmap_tile2, const CUtensorMap &tmap_out, const OutMaps &more_out,

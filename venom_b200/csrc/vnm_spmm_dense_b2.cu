@@ -4,9 +4,11 @@
 // BN / 2 columns); one tcgen05.mma.sp.cta_group::2 multiplies 256 rows (128 from each CTA) with the BN columns assembled from both
 // halves.  Per k-tile of 128 a CTA takes in 36 KiB of A and 32 KiB of B.  With one row tile a CTA (256 rows): 18 + 32 KiB.
 //
-// What bounds it: the tensor pipe inside a tile (8 MMAs x BN / 2 clocks a k-tile: 960 of 973 measured without loads, 991 with them,
-// BN = 240), and the stores of finished tiles between tiles (4096 x 1024, N = 16384: 50 us without stores, 68 with them,
-// floor 26), which leave in bursts and hold up the loads of the next tile.  One row tile a CTA: 480 clocks of MMAs, 490 to 600 with loads.
+// What bounds it: the tensor pipe inside a tile of 512 rows (8 MMAs x BN / 2 clocks a k-tile: 960 of 973 measured without loads, 991 with
+// them, BN = 240); in a tile of 256 rows the intake (48 to 50 KiB for 480 clocks of MMAs, 490 to 600 with loads); and the stores of finished tiles,
+// which leave in bursts and hold up the loads of the next tile.  4096 x 1024, N = 16384, [N,K] to [N,M], at 1965 MHz: 256 x 240 tiles
+// (what the estimate takes) 72.5 us, 52.1 without stores, MMAs 29, floor 26; 512 x 224 tiles 68.0, without stores 65.0.
+// Many such calls run into the power limit: 1430 MHz, 83 us.
 //
 // Cluster protocol (rank 0 = leader, rank 1 = peer); every load stays local to the CTA that issues it:
 //   * both CTAs run their own A producer, B producers and epilogue on their own shared / tensor memory;
@@ -539,8 +541,13 @@ cudaError_t spmm_dense_b_pair_init()
 // 192 columns.  The tall form reads every B stage once per 512 rows, but its accumulators are drained between tiles (3 to 4 us a
 // wave against 1.1 to 1.5) and it needs twice the rows for a full wave; row tiles that do not divide evenly are padded
 // (computed, never stored).  A [K,N] operand in tiles of 240 columns costs half as much again a k-tile: the peer's half, 240 bytes
-// further, starts inside a 32-byte sector.  The constants (us a k-tile and us a wave) are fitted to 18 shapes from 512 to 49152 rows, 512 to
-// 12288 k and 512 to 16384 columns; the smallest estimate wins.
+// further, starts inside a 32-byte sector.  The constants are us a k-tile and us a wave, fitted to 18 shapes from 512 to 49152 rows, 512 to
+// 12288 k and 512 to 16384 columns; the smallest estimate wins.  They are a ranking more than a time: calls at the full clock (1965
+// MHz) on inputs that change from call to call take 1.08 to 1.48 of them (seven shapes, both layouts, all six tiles: 0.94 to
+// 1.48), least with [K,N] and many waves, most with a single wave that reads everything from HBM.  Of those 14 problems the tile
+// chosen is the fastest or within 1 % of it for 11; it is 512 x 192 instead of 256 x 240 (20.0 us instead of 15.9) for [K,N] 2976 x
+// 2040, N = 1368, and 256 x 240 instead of 512 x 224 for [N,K] 4096 x 1024 (72.5, 68.0) and 1024 x 1024 (25.2, 22.8), N = 16384, where
+// the stores of a wave outweigh its few k-tiles.
 float spmm_dense_b_pair_config(int M, int N, int K, int b_nk, int max_ctas, int force_rows, bool multi, SpmmConfig *cfg)
 {
     if (g_pair_clusters <= 0) return -1.0f;
