@@ -217,28 +217,35 @@ def test_prepare_under_capture():
 # An operand that is still being re-packed behind other work of one stream: a product on another stream, plain or captured, waits.
 @pytest.mark.parametrize("captured", [False, True])
 @pytest.mark.parametrize("form", ["gather", "dense_b"])
-def test_product_waits_for_an_operand_packed_on_another_stream(form, captured):
+@pytest.mark.parametrize("lies", ["kn", "nk"])     # nk in gather form: a transpose, and a product that starts beside it
+def test_product_waits_for_an_operand_packed_on_another_stream(form, captured, lies):
     import torch
     from venom_b200 import capi
-    M, K, V, m, N = 256, 1024, 64, 8, 200
+    M, K, V, m, N = 256, 1024, 64, 8, 64
     d, values, meta, c, _ = _operand(M, K, V, m, None, seed=13)
     B = _ints((K, N), 6)
+    Bt = B.T.contiguous()
     want = (d @ B.float()).half()
+    workspace, out = torch.empty((K, N), dtype=torch.float16, device="cuda"), torch.zeros((M, N), dtype=torch.float16, device="cuda")
     busy, other = torch.cuda.Stream(), torch.cuda.Stream()
     torch.cuda.synchronize()
+
+    def product():
+        if lies == "kn":
+            return prep.spmm(B, out=out)
+        assert capi.lib().vnm_spmm_f16_nk_ws(prep._h, Bt.data_ptr(), K, N, None, out.data_ptr(), N, capi.VNM_LAYOUT_MN, workspace.data_ptr(), capi._stream()) == 0
     with torch.cuda.stream(busy):
         torch.cuda._sleep(50_000_000)
         prep = capi.Prepared(values, meta, c, M, K, V, m, strategy=capi.STRATEGY_GATHER if form == "gather" else capi.STRATEGY_DENSE_B)
-    if captured:
-        graph = torch.cuda.CUDAGraph()
-        with torch.cuda.stream(other):
+    with torch.cuda.stream(other):
+        if captured:
+            graph = torch.cuda.CUDAGraph()
             graph.capture_begin()            # not torch.cuda.graph, which waits for the device first
-            out = prep.spmm(B)
+            product()
             graph.capture_end()
             graph.replay()
-    else:
-        with torch.cuda.stream(other):
-            out = prep.spmm(B)
+        else:
+            product()
     other.synchronize()
     assert torch.equal(out, want)
     assert prep.device_status() == 0

@@ -622,7 +622,7 @@ static int spmm_impl(vnm_handle_t h, const void *B, int64_t ldb, int N, int b_nk
     } else {
         return fail(VNM_ERR_BAD_ARG, "vnm_spmm_f16: unknown layout %d", layout);
     }
-    VNM_CUDA(wait_ready(h, (cudaStream_t)stream), "wait for the prepared operand");
+    if (!after_transpose) VNM_CUDA(wait_ready(h, (cudaStream_t)stream), "wait for the prepared operand");
     SpmmConfig cfg;
     Kernel kernel;
     float us;
@@ -790,6 +790,8 @@ int vnm_spmm_f16_nk_ws(vnm_handle_t h, const void *Bt, int64_t ldbt, int N, cons
     if (ldbt < h->K || ldbt % 8 != 0 || ((uintptr_t)Bt & 15) || ((uintptr_t)workspace & 15))
         return fail(VNM_ERR_BAD_ARG, "vnm_spmm_f16_nk_ws: ldbt (%lld) must be >= K and a multiple of 8, Bt and workspace 16-byte aligned", (long long)ldbt);
     if (h->dense_b) return spmm_impl(h, Bt, ldbt, N, 1, bias, out, ldo, layout, stream);
+    // ahead of the transpose: the product may read the operand before the transpose has ended
+    VNM_CUDA(wait_ready(h, (cudaStream_t)stream), "wait for the prepared operand");
     VNM_CUDA(launch_transpose(Bt, ldbt, N, h->K, workspace, (cudaStream_t)stream), "transpose launch");
     return spmm_impl(h, workspace, N, N, 0, bias, out, ldo, layout, stream, nullptr, 0, true);
 }
