@@ -132,8 +132,8 @@ def test_bert_encoder_harness_small(spatha):
 
 
 def test_transposed_view_prepares_dense_b_form_at_high_sparsity(spatha, oracle):
-    """At 128:2:32 the automatic choice is the gather form; an activation that arrives as a transposed view
-    makes the op prepare the dense-B form instead (read in place).  Both must agree with the oracle."""
+    """At 128:2:32 an operand of [K,N] products is held in gather form; for an activation that arrives as a transposed view the op
+    asks the estimate, which takes the dense-B form (read in place) at this size.  Both must agree with the oracle."""
     import torch
     from venom_b200 import capi
     from venom_b200.synth import random_dense_b, random_vnm_dense

@@ -695,16 +695,16 @@ __global__ void __launch_bounds__(256) prepare_dense_b_kernel(const __half *__re
 // Transpose of an activation, [N, K] -> [K, N] (fp16), for the gather form, which needs rows of B.  A block takes 64 n x 64 k:
 // a thread reads 16 bytes (8 k) of two neighbouring n, interleaves them into eight words (n, n + 1) and puts them into shared
 // memory as [k][n pair] (pitch 33 words); then eight threads write the 128 bytes of one k.  Bound by HBM / L2: both
-// sides move 128 contiguous bytes a row.  The blocks are numbered along k first in one dimension of the grid, which holds 2^31 - 1 of
-// them: as the grid's second dimension (65535) the n blocks ended at 4194240 rows.
+// sides move 128 contiguous bytes a row.  The n blocks are the grid's second dimension and, beyond its 65535 (4194240 rows), the third.
 // ------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) transpose_kernel(const __half *__restrict__ src, int64_t ld, int N, int K, __half *__restrict__ dst)
 {
     __shared__ uint32_t tile[64 * 33];
+    const unsigned first = (blockIdx.y + blockIdx.z * gridDim.y) * 64u;
+    const int k0 = blockIdx.x * 64, n0 = (int)first;
     grid_dependency_wait();
     grid_launch_dependents();   // the product's set-up may begin
-    const unsigned kblocks = ((unsigned)K + 63u) / 64u, nb = blockIdx.x / kblocks;
-    const int k0 = (int)(blockIdx.x - nb * kblocks) * 64, n0 = (int)nb * 64;
+    if (first >= (unsigned)N) return;   // the whole block
     {
         const int c = threadIdx.x & 7, np = threadIdx.x >> 3;   // 8 k at k0 + 8 c of rows n0 + 2 np, + 1 (N is even: both exist or neither)
         const int k = k0 + 8 * c, n = n0 + 2 * np;
@@ -742,11 +742,10 @@ __global__ void __launch_bounds__(256) transpose_kernel(const __half *__restrict
 
 cudaError_t launch_transpose(const void *src, int64_t ld_src, int N, int K, void *dst, cudaStream_t stream)
 {
-    const int64_t blocks = (((int64_t)K + 63) / 64) * (((int64_t)N + 63) / 64);
-    if (blocks > INT32_MAX) return cudaErrorInvalidValue;   // more than 8.7e12 elements
+    const unsigned kblocks = ((unsigned)K + 63u) / 64u, nblocks = ((unsigned)N + 63u) / 64u, rows = nblocks < 65535u ? nblocks : 65535u;
     cudaLaunchConfig_t lc = {};
     cudaLaunchAttribute attr = early_launch();
-    lc.gridDim = dim3((unsigned)blocks, 1, 1);
+    lc.gridDim = dim3(kblocks, rows, (nblocks + rows - 1) / rows);
     lc.blockDim = dim3(256, 1, 1);
     lc.stream = stream;
     lc.attrs = &attr;
