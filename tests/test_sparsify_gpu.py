@@ -5,8 +5,10 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-# (M, K, V, m): one quadruple; padded tiles; m not a multiple of four; m = 8, 16, 32 (compiled sizes); V above 128
-SHAPES = [(64, 64, 32, 4), (128, 96, 32, 16), (128, 160, 64, 20), (64, 70, 32, 7), (192, 72, 64, 8), (128, 48, 128, 16), (64, 96, 32, 32), (256, 64, 256, 16)]
+# (M, K, V, m): one quadruple; padded tiles; m not a multiple of four; m = 8, 16, 32 (compiled sizes); V above 128; the smallest m that scores;
+# the last m of the task lists and the first beyond; enough blocks for the small CTAs
+SHAPES = [(64, 64, 32, 4), (128, 96, 32, 16), (128, 160, 64, 20), (64, 70, 32, 7), (192, 72, 64, 8), (128, 48, 128, 16), (64, 96, 32, 32), (256, 64, 256, 16),
+          (64, 45, 32, 5), (64, 62, 64, 31), (32, 66, 32, 33), (2048, 640, 32, 8)]
 
 
 def _weights(kind, M, K, V, m, seed):
@@ -14,6 +16,8 @@ def _weights(kind, M, K, V, m, seed):
     w = rng.normal(0, 0.02, (M, K)).astype(np.float16)
     if kind == "ties":                 # few distinct magnitudes: candidate lists overflow into the exhaustive search
         w = (np.round(w.astype(np.float32) * 100) / 100).astype(np.float16)
+    elif kind == "near":               # many candidates that the integer scores cannot tell apart
+        w = (0.02 * (1 + 1e-3 * rng.normal(size=(M, K)))).astype(np.float16)
     elif kind == "zeros":              # blocks that keep nothing, rows with fewer than two entries
         w[:V] = 0
         w[V:, :m] = 0
@@ -22,7 +26,7 @@ def _weights(kind, M, K, V, m, seed):
 
 
 @pytest.mark.parametrize("shape", SHAPES)
-@pytest.mark.parametrize("kind", ["normal", "ties", "zeros"])
+@pytest.mark.parametrize("kind", ["normal", "ties", "near", "zeros"])
 @pytest.mark.parametrize("half", [True, False])
 def test_sparsify_equals_prune_then_compress(oracle, shape, kind, half):
     import torch
