@@ -44,6 +44,36 @@ def test_few_columns(N, cfg, form):
     assert prep.device_status() == 0
 
 
+# Gather kernel: a last wave of at most half of the SMs has its tiles cut in two, a fuller one has not.  Column tiles that end inside
+# the first and the second half; more tiles than one a SM, so that whole and half tiles follow one another on it.
+@pytest.mark.parametrize("N", [96, 200, 256 + 72])
+@pytest.mark.parametrize("rest", ["few", "one", "half", "more"])
+@pytest.mark.parametrize("cfg", [(128, 16), (64, 16), (32, 8)])
+def test_last_tiles_cut_in_two(cfg, rest, N):
+    import torch
+    from venom_b200 import capi
+    from venom_b200.synth import random_vnm_dense_cuda
+    V, m = cfg
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    bn = {128: 256, 64: 128, 32: 64}[V]
+    ntiles = -(-N // bn)
+    want_tiles = {"few": 5, "one": sms + 1, "half": sms + sms // 2, "more": sms + sms // 2 + 3}[rest]
+    M, K = 128 * -(-want_tiles // ntiles), 320
+    dense, cols = random_vnm_dense_cuda(M, K, V, m, seed=M + N)
+    dense = torch.sign(dense) * torch.ceil(dense.abs() * 3)
+    values, meta, bad = capi.compress(dense, cols, V, m)
+    assert bad == 0
+    prep = capi.Prepared(values, meta, cols, M, K, V, m, strategy=capi.STRATEGY_GATHER)
+    prep.set_pair_mode(3)   # not the kernel for few tiles
+    B, bias = _ints((K, N), N), _ints((M,), 3)
+    want = (dense.float() @ B.float()).half()
+    for mode in (0, 2):     # stores from tensor memory, through shared memory
+        prep.set_epilogue(mode)
+        assert torch.equal(prep.spmm(B), want)
+        assert torch.equal(prep.spmm(B, bias=bias, layout=capi.VNM_LAYOUT_NM), (want + bias[:, None]).T)
+    assert prep.device_status() == 0
+
+
 # SM pairs: row tiles that do not fill the last pair (or group of four), fewer columns than a box, ragged columns.
 @pytest.mark.parametrize("rows", [3, 4])
 @pytest.mark.parametrize("cfg", [(128, 512, 128, 8, 248), (384, 264, 64, 8, 480), (640, 1152, 32, 16, 1000), (896, 1024, 64, 8, 72)])

@@ -524,7 +524,7 @@ bool choose_kernel(vnm_handle_t h, int N, int b_nk, int n_more, Kernel *kernel, 
     memset(cfg, 0, sizeof(*cfg));
     float big = -1.0f;
     if (!h->dense_b) {
-        big = spmm_select_config(h->V, N, h->M, h->ktiles, h->max_ctas, cfg);
+        big = spmm_select_config(h->V, N, h->M, h->ktiles, h->max_ctas, h->gather_mode == GATHER_TMA4, cfg);
         cfg->stages = h->producer_warps;
         *kernel = KERNEL_GATHER;
     } else {
@@ -696,7 +696,7 @@ static int spmm_impl(vnm_handle_t h, const void *B, int64_t ldb, int N, int b_nk
     p.layout = layout;
     p.status = h->status;
     p.gather_mode = h->gather_mode;
-    p.total_tiles = p.mtiles * p.ntiles;
+    p.total_tiles = kernel == KERNEL_GATHER ? cfg.tiles : p.mtiles * p.ntiles;
     p.B = (const __half *)B;
     p.ldb = ldb;
     {

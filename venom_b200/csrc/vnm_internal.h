@@ -28,7 +28,7 @@ struct SpmmParams {
     int layout;           // 0 = [M,N], 1 = [N,M] + bias
     int *status;          // device status word
     int gather_mode;      // GATHER_* below
-    int total_tiles;      // mtiles * ntiles
+    int total_tiles;      // mtiles * ntiles; gather kernel: tiles and halves of tiles
     const __half *B;      // gather kernel, GATHER_CPASYNC: the dense operand [K, N] itself (row pieces are copied by address)
     int64_t ldb;
     int16_t producer_pairs;   // gather kernel: pairs of warps that load B, 8 except for an ablation
@@ -72,6 +72,8 @@ struct SpmmConfig {
     int grid;    // CTAs (persistent ones, except in the small kernel)
     int split;   // small kernel: CTAs that share a tile's k-tiles
     int resident;  // small kernel: CTAs per SM
+    int tiles;     // gather kernel: tiles of the launch, halves counted
+    int cut_from;  // gather kernel: first of the tiles that are cut in two (`tiles`: none)
 };
 
 // Host-side helpers shared by the translation units that implement C-ABI entry points (defined in vnm_capi.cu).
@@ -105,7 +107,7 @@ cudaError_t launch_sparsify(const void *w, bool half, int64_t ldw, int M, int K,
 
 // Tile configuration of the gather kernel.
 constexpr int GATHER_PRODUCER_WARPS = 16;
-float spmm_select_config(int V, int N, int M, int ktiles, int max_ctas, SpmmConfig *cfg);  // max_ctas: 0 = one per SM; returns an estimate in microseconds, < 0 for an unsupported V
+float spmm_select_config(int V, int N, int M, int ktiles, int max_ctas, bool may_cut, SpmmConfig *cfg);  // max_ctas: 0 = one per SM; may_cut: the last tiles, in two; returns an estimate in microseconds, < 0 for an unsupported V
 // Opt-in to large dynamic shared memory for every kernel instance on the CURRENT device (call once per device).
 cudaError_t spmm_init_kernels();
 cudaError_t launch_spmm(const SpmmConfig &cfg, const CUtensorMap &tmap_rows, const CUtensorMap &tmap_tile, const CUtensorMap &tmap_out,

@@ -23,8 +23,16 @@
 //                 with the loads of B switched off, against four MMAs of 152.)  The whole warp runs the loop and one elected
 //                 lane issues, so that descriptors stay in uniform registers.
 //   warps 18, 19  idle (the epilogue starts at a multiple of four warps: tensor-memory lane quadrants)
-//   last eight    epilogue, two groups of four warps.  Consecutive tiles alternate between two accumulators, one for each
-//                 group, so that a tile is drained and stored beside the MMAs of the next.
+//   last eight    epilogue, two groups of four warps.  V = 128: each group drains half of the columns of the one accumulator.  V = 64
+//                 and 32: consecutive tiles alternate between two accumulators, one for each group.
+// V = 128: tiles of 256 columns fill whole gathers (64 columns each).  Two accumulators and the metadata would leave room for 240, of
+// whose fourth gather a quarter goes unused, and the gather is the bound: 79 KiB a k-tile in about 1400 clocks, the MMAs take 640.  With one
+// accumulator the MMAs stop while a tile is drained, which costs nothing as long as the rings (2.25 k-tiles) take in what arrives meanwhile.
+// [K,N] to [M,N], us, many calls (in brackets after a pause, 1965 MHz), 240 columns and two accumulators against 256 and one, without cut tiles:
+//   12288 x 12288, m = 16, N = 2048: 143.0 (128.2), 131.7 (121.1);  4096 x 4096, N = 16384, m = 8: 241.0 (213.1), 217.0 (192.7), m = 16: 141.5 (124.9),
+//   128.5 (113.5);  4096 x 512, m = 16 (one k-tile), N = 16384: 48.6 (50.0), 43.1 (44.3);  49152 x 12288, m = 8, N = 32768: 16040 (13880), 15444 (13304).
+// A tenth B stage in the place of the staging buffers: 0.5 to 1 % faster up to 0.2 ms, slower at the largest.  A fourth A stage or L2 prefetches
+// of A six k-tiles ahead: no change, 1 to 2 % slower.
 // For NB > 1 each MMA runs on all 128 rows of the value tile with the output lanes of the other blocks disabled.
 // Every wait is bounded: on expiry the kernel records a status bit, drains and returns.
 #include "vnm_internal.h"
@@ -44,8 +52,11 @@ struct Traits {
     static constexpr int B_CHUNK_BYTES = BS_ROWS * 128;       // one slice: 32 rows x 128 B
     static constexpr int B_BLOCK_BYTES = CH * B_CHUNK_BYTES;
     static constexpr int B_STAGE_BYTES = NB * B_BLOCK_BYTES;
+    static constexpr bool CAN_CUT = CH > 1;                   // the last tiles of a launch may be cut in two
     static constexpr int GATHERS = NB * BS_GROUPS * CH;       // gather4 instructions per B stage (always 32)
     static_assert(GATHERS == 32, "a stage is dealt to the 2 x 16 lanes of a producer pair");
+    // 256 columns: one accumulator, which the two epilogue groups drain half and half.  Fewer: two that alternate between tiles.
+    static constexpr int ACCS = BN == 256 ? 1 : 2;
     static constexpr int SA = 3, SB = 9;
     static constexpr int H = 2;                  // producer warps that share a stage
     static constexpr int PW = GATHER_PRODUCER_WARPS;
@@ -53,29 +64,28 @@ struct Traits {
     static constexpr int A_WARP = PW, MMA_WARP = PW + 1, EPI_WARP0 = PW + 4;
     static constexpr int NUM_WARPS = EPI_WARP0 + 8;
     static constexpr int NUM_THREADS = NUM_WARPS * 32;
-    static constexpr int PART = BN == 240 ? 40 : 32;          // columns per part of the epilogue that stores through TMA
-    static constexpr int PARTS = BN / PART;
-    static_assert(BN % PART == 0 && BN % 16 == 0, "epilogue parts");
+    static constexpr int DRAIN = ACCS == 1 ? BN / 2 : BN;     // columns of a tile that an epilogue group drains
+    static constexpr int PART = 32;                           // columns per part of the epilogue that stores through TMA
+    static_assert(BN % 64 == 0 && DRAIN % 64 == 0, "whole slices and epilogue chunks");
     static constexpr int A_RING_BYTES = SA * AM_BLOCK_BYTES;
     static constexpr int B_RING_BYTES = SB * B_STAGE_BYTES;
     static constexpr int OUT_STAGE_BYTES = TILE_M * PART * 2;
     static constexpr int BAR_BYTES = 512;
-    static constexpr int SMEM_BYTES = A_RING_BYTES + B_RING_BYTES + 2 * OUT_STAGE_BYTES + BAR_BYTES + 1024;  // + alignment slack
+    static constexpr int OUT_RING_BYTES = 2 * OUT_STAGE_BYTES;
+    static constexpr int SMEM_BYTES = A_RING_BYTES + B_RING_BYTES + OUT_RING_BYTES + BAR_BYTES + 1024;  // + alignment slack
     static_assert(SMEM_BYTES <= 227 * 1024, "shared memory per CTA");
     static_assert((2 * SA + 2 * SB + 4) * 8 + 16 <= BAR_BYTES, "barrier area too small");
     static_assert(A_RING_BYTES % 1024 == 0 && B_STAGE_BYTES % 1024 == 0 && OUT_STAGE_BYTES % 1024 == 0, "swizzled tiles need aligned rings");
-    // tensor memory: two accumulators, three alternating metadata sets of four columns behind the first
-    static constexpr int ACC_STRIDE = BN == 240 ? 256 : BN;
-    static constexpr int META_COL = BN == 240 ? 240 : 2 * BN;
+    // tensor memory: the accumulators, three alternating metadata sets of four columns behind them
+    static constexpr int META_COL = ACCS * BN;
     static constexpr int META_SETS = 3;
-    static_assert(META_COL + META_SETS * 4 <= (BN == 240 ? 256 : 512), "tensor-memory column plan");
-    static constexpr int TMEM_COLS = (BN == 240 || 2 * BN + 12 > 256) ? 512 : 256;
+    static constexpr int TMEM_COLS = META_COL + META_SETS * 4 > 256 ? 512 : 256;
 };
 
 template <int BN, int NB>
 __global__ void __launch_bounds__(Traits<BN, NB>::NUM_THREADS, 1)
     spmm_kernel(const __grid_constant__ CUtensorMap tmap_rows, const __grid_constant__ CUtensorMap tmap_tile, const __grid_constant__ CUtensorMap tmap_out,
-                const __grid_constant__ OutMaps more_out, const SpmmParams p)
+                const __grid_constant__ OutMaps more_out, const SpmmParams p, const int cut_from)
 {
     using T = Traits<BN, NB>;
     constexpr int SA = T::SA, SB = T::SB;
@@ -84,11 +94,11 @@ __global__ void __launch_bounds__(Traits<BN, NB>::NUM_THREADS, 1)
     uint8_t *a_ring = smem;
     uint8_t *b_ring = a_ring + T::A_RING_BYTES;
     uint8_t *out_ring = b_ring + T::B_RING_BYTES;
-    uint64_t *a_full = reinterpret_cast<uint64_t *>(out_ring + 2 * T::OUT_STAGE_BYTES);
+    uint64_t *a_full = reinterpret_cast<uint64_t *>(out_ring + T::OUT_RING_BYTES);
     uint64_t *a_free = a_full + SA;
     uint64_t *b_full = a_free + SA;
     uint64_t *b_free = b_full + SB;
-    uint64_t *acc_full = b_free + SB;      // [2]
+    uint64_t *acc_full = b_free + SB;      // [2], one of which is used if there is one accumulator
     uint64_t *acc_empty = acc_full + 2;    // [2]
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty + 2);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
@@ -103,7 +113,7 @@ __global__ void __launch_bounds__(Traits<BN, NB>::NUM_THREADS, 1)
         // each warp of a producer pair arrives once with its byte count (TMA modes) or once per lane behind its copies
         const uint32_t per_warp = gmode == GATHER_CPASYNC ? 32 + (p.hybrid_rows ? 1 : 0) : 1;
         for (int s = 0; s < SB; s++) { mbar_init(&b_full[s], T::H * per_warp); mbar_init(&b_free[s], 1); }
-        for (int a = 0; a < 2; a++) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 4); }
+        for (int a = 0; a < 2; a++) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], T::ACCS == 1 ? 8 : 4); }
         *abort_flag = 0;
         fence_barrier_init();
     }
@@ -118,6 +128,19 @@ __global__ void __launch_bounds__(Traits<BN, NB>::NUM_THREADS, 1)
     const uint32_t tmem_base = *tmem_slot;
     grid_launch_dependents();
 
+    // tile of the launch -> row tile, first column, slices of 64 columns.  From `cut_from` on two numbers are the halves of one tile.
+    auto locate_tile = [&](int tile, int *mt, int *n0, int *slices) {
+        int nt, half = 0;
+        *slices = T::CH;
+        if (T::CAN_CUT && tile >= cut_from) {
+            half = (tile - cut_from) & 1;
+            tile = cut_from + ((tile - cut_from) >> 1);
+            *slices = T::CH / 2;
+        }
+        tile_coords(tile, p.mtiles, p.ntiles, p.group_m, mt, &nt);
+        *n0 = nt * BN + half * (BN / 2);
+    };
+
     if (warp < T::H * p.producer_pairs) {
         // ---------------- B producers ----------------
         const int ng = p.producer_pairs;
@@ -127,8 +150,8 @@ __global__ void __launch_bounds__(Traits<BN, NB>::NUM_THREADS, 1)
         const int per_tile = STAGES_PER_KT * p.ktiles;
         const int total_j = my_tiles * per_tile;
         int tile_i = j / per_tile, jl = j - tile_i * per_tile;
-        int mt = 0, nt = 0;
-        auto locate = [&] { tile_coords((int)blockIdx.x + tile_i * (int)gridDim.x, p.mtiles, p.ntiles, p.group_m, &mt, &nt); };
+        int mt = 0, n0 = 0, slices = T::CH;
+        auto locate = [&] { locate_tile((int)blockIdx.x + tile_i * (int)gridDim.x, &mt, &n0, &slices); };
         // this lane's fixed share of a stage: block, group, 64-column slice (gather4), or one whole slice (plain tiles)
         const int q = part * (T::GATHERS / T::H) + lane;
         const bool on = lane < T::GATHERS / T::H;
@@ -148,15 +171,14 @@ __global__ void __launch_bounds__(Traits<BN, NB>::NUM_THREADS, 1)
         if (j < total_j) { locate(); r = fetch(); }
         int issued = 0;
         while (j < total_j) {
-            const int n0 = nt * BN;
             const int4 cur = r;
             uint8_t *st = b_ring + s * T::B_STAGE_BYTES;
             uint64_t *full = &b_full[s];
             if (!__all_sync(0xffffffffu, wait_quiet(&b_free[s], (uint32_t)(wrap & 1) ^ 1u, abort_flag, p.status, DEV_TIMEOUT_PRODUCER))) break;
             if (gmode == GATHER_TMA4) {
-                if (lane == 0) mbar_arrive_expect_tx(full, T::B_STAGE_BYTES / T::H);
+                if (lane == 0) mbar_arrive_expect_tx(full, T::CAN_CUT ? T::B_STAGE_BYTES / T::H / T::CH * slices : T::B_STAGE_BYTES / T::H);
                 __syncwarp();
-                if (on) tma_gather4(st + gb * T::B_BLOCK_BYTES + gc * T::B_CHUNK_BYTES + gg * 512, &tmap_rows, n0 + gc * 64, cur, full);
+                if (on && (!T::CAN_CUT || gc < slices)) tma_gather4(st + gb * T::B_BLOCK_BYTES + gc * T::B_CHUNK_BYTES + gg * 512, &tmap_rows, n0 + gc * 64, cur, full);
             } else if (gmode == GATHER_CONTIG) {   // 32 consecutive rows (m == 4: all of them are selected)
                 if (lane == 0) mbar_arrive_expect_tx(full, T::B_STAGE_BYTES / T::H);
                 __syncwarp();
@@ -212,8 +234,8 @@ __global__ void __launch_bounds__(Traits<BN, NB>::NUM_THREADS, 1)
             uint32_t ph = 1;
             bool alive = true;
             for (int tile = blockIdx.x; alive && tile < p.total_tiles; tile += gridDim.x) {
-                int mt, nt_unused;
-                tile_coords(tile, p.mtiles, p.ntiles, p.group_m, &mt, &nt_unused);
+                int mt, n0_unused, slices_unused;
+                locate_tile(tile, &mt, &n0_unused, &slices_unused);
                 const uint8_t *src = p.am + (size_t)mt * p.ktiles * AM_BLOCK_BYTES;
                 for (int kt = 0; kt < p.ktiles; ++kt, ++it) {
                     if (!wait_quiet(&a_free[s], ph, abort_flag, p.status, DEV_TIMEOUT_PRODUCER)) { alive = false; break; }
@@ -233,7 +255,8 @@ __global__ void __launch_bounds__(Traits<BN, NB>::NUM_THREADS, 1)
         // registers, otherwise every MMA costs 161 clocks to issue, more than it takes to execute).  The tensor pipe queues
         // about two MMAs, so the wait for a stage sits directly in front of its MMAs, where it hides behind the previous stage's.
         if (elect_one()) {
-            const uint32_t idesc0 = make_idesc_f16(TILE_M, BN, true, 0u, true);
+            const uint32_t idesc_full = make_idesc_f16(TILE_M, BN, true, 0u, true);
+            const uint32_t idesc_cut = T::CAN_CUT ? make_idesc_f16(TILE_M, BN / 2, true, 0u, true) : idesc_full;
             // descriptor templates: only the start-address field (low 14 bits, in 16-byte units) varies
             const uint64_t adesc0 = make_smem_desc(smem_u32(a_ring), 16, 1024, 2);
             const uint64_t mdesc0 = make_smem_desc(smem_u32(a_ring) + A_IMG_BYTES, 0, 128, 0);
@@ -242,10 +265,11 @@ __global__ void __launch_bounds__(Traits<BN, NB>::NUM_THREADS, 1)
             uint32_t pa = 0, pb = 0;
             bool alive = true;
             for (int ti = 0; alive && ti < my_tiles; ++ti) {
-                const int aset = ti & 1;
-                const uint32_t acc = tmem_base + (uint32_t)(aset * T::ACC_STRIDE);
+                const int aset = T::ACCS == 1 ? 0 : ti & 1;
+                const uint32_t acc = tmem_base + (uint32_t)(aset * BN);
+                const uint32_t idesc0 = (int)blockIdx.x + ti * (int)gridDim.x >= cut_from ? idesc_cut : idesc_full;
                 // the epilogue must have read this accumulator's previous tile
-                if (!wait_one(&acc_empty[aset], ((uint32_t)(ti >> 1) & 1u) ^ 1u, abort_flag, p.status, DEV_TIMEOUT_MMA)) break;
+                if (!wait_one(&acc_empty[aset], ((uint32_t)(T::ACCS == 1 ? ti : ti >> 1) & 1u) ^ 1u, abort_flag, p.status, DEV_TIMEOUT_MMA)) break;
                 for (int kt = 0; kt < p.ktiles; ++kt) {
                     if (!wait_one(&a_full[sa], pa, abort_flag, p.status, DEV_TIMEOUT_MMA)) { alive = false; break; }
                     tc_fence_after();
@@ -296,23 +320,34 @@ __global__ void __launch_bounds__(Traits<BN, NB>::NUM_THREADS, 1)
         const int arow = mma_row_to_actual(q * 32 + lane);
         const bool leader = ((warp - T::EPI_WARP0) & 3) == 0 && lane == 0;
         uint8_t *stg = out_ring + grp * T::OUT_STAGE_BYTES;
-        const uint32_t trow = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(grp * T::ACC_STRIDE);
-        for (int ti = grp; ti < my_tiles; ti += 2) {
-            int mt, nt;
-            tile_coords((int)blockIdx.x + ti * (int)gridDim.x, p.mtiles, p.ntiles, p.group_m, &mt, &nt);
-            const int n0 = nt * BN;
+        const uint32_t trow = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(T::ACCS == 1 ? 0 : grp * BN);
+        for (int ti = T::ACCS == 1 ? 0 : grp; ti < my_tiles; ti += T::ACCS) {
+            const int tile = (int)blockIdx.x + ti * (int)gridDim.x;
+            int mt, n0, slices;
+            locate_tile(tile, &mt, &n0, &slices);
+            const int aset = T::ACCS == 1 ? 0 : grp;
             // the four warps of a group leave the loop together (they meet at named barriers below)
-            const bool got = wait_warp(&acc_full[grp], (uint32_t)(ti >> 1) & 1u, abort_flag, p.status, DEV_TIMEOUT_EPILOGUE);
+            const bool got = wait_warp(&acc_full[aset], (uint32_t)(T::ACCS == 1 ? ti : ti >> 1) & 1u, abort_flag, p.status, DEV_TIMEOUT_EPILOGUE);
             if (!named_barrier_and(1 + grp, 128, got)) break;
             tc_fence_after();
             auto release = [&] {
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&acc_empty[grp]);
+                if (lane == 0) mbar_arrive(&acc_empty[aset]);
             };
+            // This group's columns.  With one accumulator the MMAs of the next tile wait until the last column has been read, but the loads
+            // go on: the rings hold what arrives in that time, and the MMAs are more than twice as fast as the loads.
+            const int mine = T::DRAIN / T::CH * slices, first = T::ACCS == 1 ? grp * mine : 0;
+            const uint32_t tacc = trow + (uint32_t)first;
+            n0 += first;
             if (!p.tma_out) {
-                if (p.layout == 0) store_tile<BN, false>(TileStoreMN(trow, q, (int64_t)mt * TILE_M, n0, p), release);
-                else store_tile<BN, false>(TileStoreNM(trow, q, (int64_t)mt * TILE_M, n0, p), release);
+                if (mine == T::DRAIN) {
+                    if (p.layout == 0) store_tile<T::DRAIN, false>(TileStoreMN(tacc, q, (int64_t)mt * TILE_M, n0, p), release);
+                    else store_tile<T::DRAIN, false>(TileStoreNM(tacc, q, (int64_t)mt * TILE_M, n0, p), release);
+                } else if (T::CAN_CUT) {   // half a tile
+                    if (p.layout == 0) store_tile<64, false>(TileStoreMN(tacc, q, (int64_t)mt * TILE_M, n0, p), release);
+                    else store_tile<64, false>(TileStoreNM(tacc, q, (int64_t)mt * TILE_M, n0, p), release);
+                }
                 continue;
             }
             // [N,M] (+ bias) to several destinations (peers' buffers), or on request: parts of PART rows (n) x 128 columns (m) go
@@ -321,12 +356,12 @@ __global__ void __launch_bounds__(Traits<BN, NB>::NUM_THREADS, 1)
             const bool has_bias = p.bias != nullptr;
             const __half bias = (has_bias && row < p.M) ? p.bias[row] : __ushort_as_half((unsigned short)0);
 #pragma unroll 1
-            for (int part = 0; part < T::PARTS; part++) {
+            for (int part = 0; part < mine / PART; part++) {
                 uint32_t v[PART / 8][8];
 #pragma unroll
-                for (int i = 0; i < PART / 8; i++) tc_ld_32x32b_x8(trow + (uint32_t)(part * PART + 8 * i), v[i]);
+                for (int i = 0; i < PART / 8; i++) tc_ld_32x32b_x8(tacc + (uint32_t)(part * PART + 8 * i), v[i]);
                 tc_wait_ld();
-                if (part == T::PARTS - 1) release();
+                if (part == mine / PART - 1) release();
                 if (leader) bulk_wait_group_read0();   // the previous store has finished reading the staging buffer
                 named_barrier_sync(1 + grp, 128);
                 __half *col = reinterpret_cast<__half *>(stg) + arow;
@@ -376,42 +411,55 @@ cudaError_t launch_one(const SpmmConfig &cfg, const CUtensorMap &tmap_rows, cons
     lc.stream = stream;
     lc.attrs = &attr;
     lc.numAttrs = 1;
-    return cudaLaunchKernelEx(&lc, spmm_kernel<BN, NB>, tmap_rows, tmap_tile, tmap_out, more_out, p);
+    return cudaLaunchKernelEx(&lc, spmm_kernel<BN, NB>, tmap_rows, tmap_tile, tmap_out, more_out, p, cfg.cut_from);
 }
 
 int g_num_sms = 0;
 
 }  // namespace
 
-// Tile configurations: V=128 -> one block per tile, BN 240 (two accumulators and the metadata fill tensor memory);
-// V=64 -> two blocks, BN 128; V=32 -> four blocks, BN 64 (NB * BN = 256: every B stage is 16 KiB).
-float spmm_select_config(int V, int N, int M, int ktiles, int max_ctas, SpmmConfig *cfg)
+// A last wave that fills at most half of the SMs has its tiles cut in two (V = 128 and 64, gather4 only: the ablations load whole stages).  Half a
+// tile takes 0.65 of the time of a whole one, bound by the latency of its half-filled stages; quarters take as long as halves.  [K,N] to
+// [M,N], us, many calls (after a pause), whole and cut:  12288 x 12288, V = 128, m = 16, N = 2048 (28 tiles beyond five waves) 131.7 (121.1), 129.3 (116.7);
+// 4096 x 12288, m = 8, N = 4096 (68 beyond three) 165.9 (152.8), 160.5 (144.1);  12288 x 12288, V = 64, m = 32, N = 2048 (56 beyond ten) 114.6
+// (110.9), 113.0 (108.7).  More than half (124 beyond 13 waves, 4096 x 4096, m = 8, N = 16384), which makes two waves of halves: 217.0, 221.2.
+//
+// The estimate, in us: start-up and last epilogue, then per wave a k-tile's 1430 clocks and what a tile change costs.  It is 0.97 to 1.03 of a call
+// after a pause from 8 k-tiles a tile and 3 waves on.
+//
+// Tile configurations: V=128 -> one block per tile, BN 256; V=64 -> two blocks, BN 128; V=32 -> four blocks, BN 64 (NB * BN = 256:
+// every B stage is 16 KiB).
+float spmm_select_config(int V, int N, int M, int ktiles, int max_ctas, bool may_cut, SpmmConfig *cfg)
 {
     const int mtiles = (M + TILE_M - 1) / TILE_M;
-    cfg->stages = Traits<240, 1>::PW;
-    cfg->threads = Traits<240, 1>::NUM_THREADS;
+    cfg->stages = Traits<256, 1>::PW;
+    cfg->threads = Traits<256, 1>::NUM_THREADS;
+    cfg->part = Traits<256, 1>::PART;
     if (V == 128) {
-        cfg->bn = 240; cfg->nb = 1; cfg->part = Traits<240, 1>::PART; cfg->smem_bytes = Traits<240, 1>::SMEM_BYTES;
+        cfg->bn = 256; cfg->nb = 1; cfg->smem_bytes = Traits<256, 1>::SMEM_BYTES;
     } else if (V == 64) {
-        cfg->bn = 128; cfg->nb = 2; cfg->part = Traits<128, 2>::PART; cfg->smem_bytes = Traits<128, 2>::SMEM_BYTES;
+        cfg->bn = 128; cfg->nb = 2; cfg->smem_bytes = Traits<128, 2>::SMEM_BYTES;
     } else if (V == 32) {
-        cfg->bn = 64; cfg->nb = 4; cfg->part = Traits<64, 4>::PART; cfg->smem_bytes = Traits<64, 4>::SMEM_BYTES;
+        cfg->bn = 64; cfg->nb = 4; cfg->smem_bytes = Traits<64, 4>::SMEM_BYTES;
     } else {
         return -1.0f;
     }
     const long long tiles = (long long)mtiles * ((N + cfg->bn - 1) / cfg->bn);
     int sms = g_num_sms > 0 ? g_num_sms : 148;
     if (max_ctas > 0 && max_ctas < sms) sms = max_ctas;  // the caller keeps some SMs free (e.g. for a collective that runs beside the product)
-    cfg->grid = (int)(tiles < sms ? tiles : sms);
-    // start-up and last epilogue, then per wave of tiles a k-tile's 1430 clocks and what a tile change costs: 887 us at 12288 x 12288, m = 8,
-    // N = 8192, where a call after a pause takes 913 and one of many, at the clock that the power limit leaves, 1057
-    return 5.5f + (float)((tiles + sms - 1) / sms) * (ktiles * 0.78f + 0.9f);
+    const long long waves = tiles / sms;
+    const int rest = (int)(tiles - waves * sms);
+    const bool cut = may_cut && cfg->bn > 64 && rest > 0 && 2 * rest <= sms;
+    cfg->tiles = (int)tiles + (cut ? rest : 0);
+    cfg->cut_from = cut ? (int)(waves * sms) : cfg->tiles;
+    cfg->grid = cfg->tiles < sms ? cfg->tiles : sms;
+    return 5.5f + ((float)waves + (rest == 0 ? 0.0f : cut ? 0.65f : 1.0f)) * (ktiles * 0.74f + 2.0f);
 }
 
 cudaError_t spmm_init_kernels()
 {
     cudaError_t e;
-    if ((e = set_attr<240, 1>()) != cudaSuccess) return e;
+    if ((e = set_attr<256, 1>()) != cudaSuccess) return e;
     if ((e = set_attr<128, 2>()) != cudaSuccess) return e;
     if ((e = set_attr<64, 4>()) != cudaSuccess) return e;
     int dev = 0;
@@ -422,7 +470,7 @@ cudaError_t spmm_init_kernels()
 cudaError_t launch_spmm(const SpmmConfig &cfg, const CUtensorMap &tmap_rows, const CUtensorMap &tmap_tile, const CUtensorMap &tmap_out,
                         const OutMaps &more_out, const SpmmParams &p, cudaStream_t stream)
 {
-    if (cfg.nb == 1) return launch_one<240, 1>(cfg, tmap_rows, tmap_tile, tmap_out, more_out, p, stream);
+    if (cfg.nb == 1) return launch_one<256, 1>(cfg, tmap_rows, tmap_tile, tmap_out, more_out, p, stream);
     if (cfg.nb == 2) return launch_one<128, 2>(cfg, tmap_rows, tmap_tile, tmap_out, more_out, p, stream);
     if (cfg.nb == 4) return launch_one<64, 4>(cfg, tmap_rows, tmap_tile, tmap_out, more_out, p, stream);
     return cudaErrorInvalidValue;
