@@ -722,7 +722,7 @@ static int spmm_impl(vnm_handle_t h, const void *B, int64_t ldb, int N, int b_nk
         p.hint_b = col_bands ? L2_EVICT_LAST : L2_EVICT_NORMAL;
         if (h->l2_hints == 0) p.hint_a = p.hint_b = L2_EVICT_NORMAL;
     }
-    p.producer_pairs = (int16_t)(h->producer_warps / 2);
+    p.producer_warps = (int16_t)h->producer_warps;
     p.hybrid_rows = (int16_t)h->hybrid_rows;
     p.b_nk = b_nk;
     p.b_wide_ok = tm_wide ? 1 : 0;

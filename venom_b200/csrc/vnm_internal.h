@@ -31,7 +31,7 @@ struct SpmmParams {
     int total_tiles;      // mtiles * ntiles; gather kernel: tiles and halves of tiles
     const __half *B;      // gather kernel, GATHER_CPASYNC: the dense operand [K, N] itself (row pieces are copied by address)
     int64_t ldb;
-    int16_t producer_pairs;   // gather kernel: pairs of warps that load B, 8 except for an ablation
+    int16_t producer_warps;   // gather kernel: how much of the warps that load B is at work, in 16ths: 16 except for an ablation
     int16_t hybrid_rows;  // gather kernel, GATHER_CPASYNC: of 64 rows of a block, those fetched by TMA gather4 beside the copies (0, 16, 32, 48)
     int group_m;          // band of the tile order (tile_coords): > 0 row groups per band, < 0 column tiles per band
     uint64_t hint_a, hint_b;  // pair kernel: L2 eviction-priority policies of the A and B loads (L2_EVICT_*)
@@ -106,7 +106,7 @@ cudaError_t launch_sparsify(const void *w, bool half, int64_t ldw, int M, int K,
                             unsigned long long *violations, cudaStream_t stream);
 
 // Tile configuration of the gather kernel.
-constexpr int GATHER_PRODUCER_WARPS = 16;
+constexpr int GATHER_PRODUCER_WARPS = 16;   // all of them, in the units of vnm_set_producer_warps
 float spmm_select_config(int V, int N, int M, int ktiles, int max_ctas, bool may_cut, SpmmConfig *cfg);  // max_ctas: 0 = one per SM; may_cut: the last tiles, in two; returns an estimate in microseconds, < 0 for an unsupported V
 // Opt-in to large dynamic shared memory for every kernel instance on the CURRENT device (call once per device).
 cudaError_t spmm_init_kernels();
@@ -379,12 +379,22 @@ __device__ __forceinline__ void store_tile(const Store &st, Release release)
         uint32_t pk[CHUNKS][32];
 #pragma unroll
         for (int k = 0; k < CHUNKS; k++) {
-            uint32_t v0[32], v1[32];   // both groups in flight before the wait: the next tile's MMAs wait for this
-            tc_ld_16x256b(st.taddr + (uint32_t)(64 * k), v0);
-            tc_ld_16x256b(st.taddr + (16u << 16) + (uint32_t)(64 * k), v1);
-            tc_wait_ld();
-            Store::pack(v0, pk[k]);
-            Store::pack(v1, pk[k] + 16);
+            if (BN > 128 || k == 0) {
+                uint32_t v0[32], v1[32];   // both groups in flight before the wait: the next tile's MMAs wait for this
+                tc_ld_16x256b(st.taddr + (uint32_t)(64 * k), v0);
+                tc_ld_16x256b(st.taddr + (16u << 16) + (uint32_t)(64 * k), v1);
+                tc_wait_ld();
+                Store::pack(v0, pk[k]);
+                Store::pack(v1, pk[k] + 16);
+            } else {                       // kernels of fewer registers: one after the other
+#pragma unroll
+                for (int g = 0; g < 2; g++) {
+                    uint32_t v[32];
+                    tc_ld_16x256b(st.taddr + ((uint32_t)(16 * g) << 16) + (uint32_t)(64 * k), v);
+                    tc_wait_ld();
+                    Store::pack(v, pk[k] + 16 * g);
+                }
+            }
         }
         release();
 #pragma unroll

@@ -150,7 +150,7 @@ extern "C" int vnm_spmm_f16_noalloc(const void *values, const uint32_t *meta, co
     p.early = 0;
     p.hint_a = p.hint_b = L2_EVICT_NORMAL;
     p.group_m = mtiles;  // operands this small fit in L2 whole: row tiles fastest
-    p.producer_pairs = GATHER_PRODUCER_WARPS / 2;
+    p.producer_warps = GATHER_PRODUCER_WARPS;
     p.hybrid_rows = 0;
     p.b_nk = 0;
     p.b_wide_ok = 0;

@@ -11,10 +11,14 @@
 //           N-major, 128-byte swizzle.
 // Warp roles:
 //   warps 0..15   B producers in eight pairs; pair j % 8 fills stage j, 16 TMA gather4 loads a warp (four absolute row
-//                 numbers per instruction, precomputed by the prepare step).  A warp needs about 65 clocks for each gather4
-//                 it issues, whatever the others do, so the intake of an SM is a matter of how many warps issue at
-//                 once: 1 warp 8 B/clk, 6 warps 41, 12 warps 57, 24 warps 67 (B in L2; plain 8 KiB tile loads reach 73).
-//                 (vnm_set_producer_warps, an ablation, leaves only the first two or four pairs at work.)
+//                 numbers per instruction, precomputed by the prepare step).  One elected lane issues them, with the row numbers of its
+//                 groups in its registers: 42 clocks a gather4.  (With a gather4 a lane, the warp goes through its lanes at 109 clocks
+//                 each when all sixteen are at it, and the slots of the ring were waiting for that: 128.4 us at 12288 x 12288, 128:2:16, N = 2048,
+//                 [K,N] to [M,N], many calls, against 117.2; 4096 x 4096, 128:2:8, N = 16384 218 and 197; 12288 x 12288, 64:2:32, N = 2048 113 and 106.)
+//                 At V = 32 a warp has 16 groups of one gather4 each, too many for every lane to hold: there each lane holds and issues one
+//                 (105 us at 4096 x 4096, 32:2:32, N = 8192; four warps a stage with eight groups each 111).  The row numbers are asked for
+//                 before the wait for the slot, which takes longer.  (vnm_set_producer_warps, an ablation, leaves a quarter or half of the
+//                 pairs at work.)
 //   warp 16       A producer (one lane).
 //   warp 17       tensor-memory owner and MMA issuer.  It waits for the operands itself, copies a k-tile's metadata to
 //                 tensor memory (tcgen05.cp) and issues the MMAs right behind it: copies and MMAs of one thread execute
@@ -26,9 +30,13 @@
 //   last eight    epilogue, two groups of four warps.  V = 128: each group drains half of the columns of the one accumulator.  V = 64
 //                 and 32: consecutive tiles alternate between two accumulators, one for each group.
 // V = 128: tiles of 256 columns fill whole gathers (64 columns each).  Two accumulators and the metadata would leave room for 240, of
-// whose fourth gather a quarter goes unused, and the gather is the bound: 79 KiB a k-tile in about 1400 clocks, the MMAs take 640.  With one
-// accumulator the MMAs stop while a tile is drained, which costs nothing as long as the rings (2.25 k-tiles) take in what arrives meanwhile.
-// [K,N] to [M,N], us, many calls (in brackets after a pause, 1965 MHz), 240 columns and two accumulators against 256 and one, without cut tiles:
+// whose fourth gather a quarter goes unused.  With one accumulator the MMAs stop while a tile is drained (2800 clocks from the last MMA to the
+// next one: 440 until the epilogue sees it, the rest to read and store half of its columns and read the others), and the rings (2.25 k-tiles)
+// take in what arrives meanwhile.  Holding all columns in registers first needs more of them than 832 threads have.
+// What bounds a k-tile now: 640 clocks of MMAs, whose operands and the 82 KiB of loads share the port of shared memory (900 without the
+// loads of B, 1130 with them on 18 SMs, 1340 on all).
+// [K,N] to [M,N], us, many calls (in brackets after a pause, 1965 MHz), 240 columns and two accumulators against 256 and one, without cut tiles
+// and with a gather4 a lane:
 //   12288 x 12288, m = 16, N = 2048: 143.0 (128.2), 131.7 (121.1);  4096 x 4096, N = 16384, m = 8: 241.0 (213.1), 217.0 (192.7), m = 16: 141.5 (124.9),
 //   128.5 (113.5);  4096 x 512, m = 16 (one k-tile), N = 16384: 48.6 (50.0), 43.1 (44.3);  49152 x 12288, m = 8, N = 32768: 16040 (13880), 15444 (13304).
 // A tenth B stage in the place of the staging buffers: 0.5 to 1 % faster up to 0.2 ms, slower at the largest.  A fourth A stage or L2 prefetches
@@ -54,13 +62,15 @@ struct Traits {
     static constexpr int B_STAGE_BYTES = NB * B_BLOCK_BYTES;
     static constexpr bool CAN_CUT = CH > 1;                   // the last tiles of a launch may be cut in two
     static constexpr int GATHERS = NB * BS_GROUPS * CH;       // gather4 instructions per B stage (always 32)
-    static_assert(GATHERS == 32, "a stage is dealt to the 2 x 16 lanes of a producer pair");
     // 256 columns: one accumulator, which the two epilogue groups drain half and half.  Fewer: two that alternate between tiles.
     static constexpr int ACCS = BN == 256 ? 1 : 2;
     static constexpr int SA = 3, SB = 9;
     static constexpr int H = 2;                  // producer warps that share a stage
-    static constexpr int PW = GATHER_PRODUCER_WARPS;
+    static constexpr int PW = 16;
     static constexpr int NG = PW / H;
+    static constexpr int GROUPS = NB * BS_GROUPS / H;         // groups of a stage that a warp gathers, CH instructions each
+    static constexpr bool BY_LANE = NB == 4;                  // sixteen groups: a lane holds the rows of each (else every lane those of all)
+    static_assert(GATHERS == 32 && (!BY_LANE || (GROUPS <= 32 && CH == 1)), "a stage is dealt to the warps by groups");
     static constexpr int A_WARP = PW, MMA_WARP = PW + 1, EPI_WARP0 = PW + 4;
     static constexpr int NUM_WARPS = EPI_WARP0 + 8;
     static constexpr int NUM_THREADS = NUM_WARPS * 32;
@@ -141,89 +151,112 @@ __global__ void __launch_bounds__(Traits<BN, NB>::NUM_THREADS, 1)
         *n0 = nt * BN + half * (BN / 2);
     };
 
-    if (warp < T::H * p.producer_pairs) {
-        // ---------------- B producers ----------------
-        const int ng = p.producer_pairs;
-        const int part = warp % T::H;
-        int j = warp / T::H, s = j, wrap = 0;         // stage, its ring slot, times the ring has gone round
-        static_assert(T::NG <= SB, "a pair's first stage has its own slot");
+    const int ng = T::NG * p.producer_warps / GATHER_PRODUCER_WARPS > 0 ? T::NG * p.producer_warps / GATHER_PRODUCER_WARPS : 1;   // groups of H warps at work
+    if (warp < T::H * ng) {
+        // ---------------- B producers: the groups of H warps take the stages in turn ----------------
+        constexpr int G = T::GROUPS, HELD = T::BY_LANE ? 1 : G;
+        const int part = warp % T::H, first = warp / T::H;
         const int per_tile = STAGES_PER_KT * p.ktiles;
-        const int total_j = my_tiles * per_tile;
-        int tile_i = j / per_tile, jl = j - tile_i * per_tile;
-        int mt = 0, n0 = 0, slices = T::CH;
-        auto locate = [&] { locate_tile((int)blockIdx.x + tile_i * (int)gridDim.x, &mt, &n0, &slices); };
-        // this lane's fixed share of a stage: block, group, 64-column slice (gather4), or one whole slice (plain tiles)
-        const int q = part * (T::GATHERS / T::H) + lane;
-        const bool on = lane < T::GATHERS / T::H;
-        const int gc = q % T::CH, gg = (q / T::CH) % BS_GROUPS, gb = on ? q / (T::CH * BS_GROUPS) : 0;
-        constexpr int BOXES = NB * T::CH;             // plain tiles: boxes per stage
-        static_assert(BOXES % T::H == 0, "boxes are dealt to the pair");
+        // this warp's groups of a stage are part * G ..; group q is group q % BS_GROUPS of vector block q / BS_GROUPS
+        const int mine = part * G + (T::BY_LANE ? lane % G : 0);
+        constexpr int BOXES = NB * T::CH;             // plain tiles: boxes per stage, a lane each
+        static_assert(BOXES % T::H == 0, "boxes are dealt to the warps");
         const bool box_on = lane < BOXES / T::H;
         const int bc = (part * (BOXES / T::H) + lane) % T::CH, bb = box_on ? (part * (BOXES / T::H) + lane) / T::CH : 0;
-        const int HG = gmode == GATHER_CPASYNC ? p.hybrid_rows / 8 : BS_GROUPS;   // groups of a block that go through gather4
         if (lane == 0) { tma_prefetch_desc(&tmap_rows); tma_prefetch_desc(&tmap_tile); }
-        auto row_entry = [&](int b, int g) { return p.rows + ((size_t)(mt * NB + b) * p.ktiles) * KT_GROUPS + (size_t)jl * BS_GROUPS + g; };
-        auto fetch = [&]() -> int4 {
-            if (gmode == GATHER_CONTIG) return make_int4(jl * BS_ROWS, 0, 0, 0);
-            return on ? __ldg(row_entry(gb, gg)) : make_int4(0, 0, 0, 0);
+        int tile_i = first / per_tile, jl = first - tile_i * per_tile, s = first;
+        static_assert(T::NG <= SB, "a group's first stage has its own slot");
+        uint32_t parity = 1;
+        int n0 = 0, slices = T::CH;
+        const int4 *entry = nullptr;                  // the row numbers of group `mine` in stage jl
+        auto locate = [&] {
+            int mt;
+            locate_tile((int)blockIdx.x + tile_i * (int)gridDim.x, &mt, &n0, &slices);
+            entry = p.rows + ((size_t)(mt * NB + mine / BS_GROUPS) * p.ktiles) * KT_GROUPS + (size_t)jl * BS_GROUPS + mine % BS_GROUPS;
         };
-        int4 r = make_int4(0, 0, 0, 0);
-        if (j < total_j) { locate(); r = fetch(); }
+        if (tile_i < my_tiles) locate();
         int issued = 0;
-        while (j < total_j) {
-            const int4 cur = r;
+        while (tile_i < my_tiles) {
+            int4 rows[HELD];                          // on their way while the warp waits for the slot
+            if (gmode == GATHER_TMA4 || gmode == GATHER_CPASYNC) {
+#pragma unroll
+                for (int g = 0; g < HELD; g++) rows[g] = __ldg(entry + g);   // one block's
+            }
+            const int n = n0, cols = slices, k_row = jl * BS_ROWS;
             uint8_t *st = b_ring + s * T::B_STAGE_BYTES;
-            uint64_t *full = &b_full[s];
-            if (!__all_sync(0xffffffffu, wait_quiet(&b_free[s], (uint32_t)(wrap & 1) ^ 1u, abort_flag, p.status, DEV_TIMEOUT_PRODUCER))) break;
+            uint64_t *full = &b_full[s], *free = &b_free[s];
+            const uint32_t cur_parity = parity;
+            jl += ng;
+            s += ng;
+            entry += ng * BS_GROUPS;
+            if (s >= SB) { s -= SB; parity ^= 1; }
+            if (jl >= per_tile) {
+                do { jl -= per_tile; ++tile_i; } while (jl >= per_tile);
+                if (tile_i < my_tiles) locate();
+            }
+            if (!__all_sync(0xffffffffu, wait_quiet(free, cur_parity, abort_flag, p.status, DEV_TIMEOUT_PRODUCER))) break;
+            auto slot = [&](int q) { return st + q / BS_GROUPS * T::B_BLOCK_BYTES + q % BS_GROUPS * 512; };   // of a group, first slice
             if (gmode == GATHER_TMA4) {
-                if (lane == 0) mbar_arrive_expect_tx(full, T::CAN_CUT ? T::B_STAGE_BYTES / T::H / T::CH * slices : T::B_STAGE_BYTES / T::H);
-                __syncwarp();
-                if (on && (!T::CAN_CUT || gc < slices)) tma_gather4(st + gb * T::B_BLOCK_BYTES + gc * T::B_CHUNK_BYTES + gg * 512, &tmap_rows, n0 + gc * 64, cur, full);
+                if constexpr (T::BY_LANE) {
+                    if (lane == 0) mbar_arrive_expect_tx(full, G * 512);
+                    __syncwarp();
+                    if (lane < G) tma_gather4(slot(mine), &tmap_rows, n, rows[0], full);
+                } else if (elect_one()) {
+                    mbar_arrive_expect_tx(full, G * 512 * cols);
+                    uint8_t *dst = slot(mine);
+#pragma unroll
+                    for (int g = 0; g < G; g++) {
+#pragma unroll
+                        for (int c = 0; c < T::CH; c++)
+                            if (c < T::CH / 2 || cols == T::CH) tma_gather4(dst + c * T::B_CHUNK_BYTES + g * 512, &tmap_rows, n + c * 64, rows[g], full);
+                    }
+                }
             } else if (gmode == GATHER_CONTIG) {   // 32 consecutive rows (m == 4: all of them are selected)
                 if (lane == 0) mbar_arrive_expect_tx(full, T::B_STAGE_BYTES / T::H);
                 __syncwarp();
-                if (box_on) tma_load_2d(st + bb * T::B_BLOCK_BYTES + bc * T::B_CHUNK_BYTES, &tmap_tile, n0 + bc * 64, cur.x, full);
+                if (box_on) tma_load_2d(st + bb * T::B_BLOCK_BYTES + bc * T::B_CHUNK_BYTES, &tmap_tile, n + bc * 64, k_row, full);
             } else if (gmode == GATHER_NONE) {     // ablation: no loads of B (timing floor; results are meaningless)
                 if (lane == 0) mbar_arrive(full);
             } else {
                 // ablation: per-thread 16-byte asynchronous copies driven by the row table, optionally beside gather4 loads of
-                // the first HG groups of every block.  A warp copies the groups it would otherwise have gathered.
-                if (HG > 0) {
-                    int mine = 0;
-                    for (int i = 0; i < T::GATHERS / T::H; i++) mine += ((part * (T::GATHERS / T::H) + i) / T::CH) % BS_GROUPS < HG;
-                    if (lane == 0) mbar_arrive_expect_tx(full, (uint32_t)mine * 512);
+                // the first `by_tma` groups of every block
+                const int by_tma = p.hybrid_rows / 8;
+                if (by_tma > 0) {
+                    int here = 0;
+                    for (int g = 0; g < G; g++) here += (part * G + g) % BS_GROUPS < by_tma;
+                    if (lane == 0) mbar_arrive_expect_tx(full, here * 512 * T::CH);
                     __syncwarp();
-                    if (on && gg < HG) tma_gather4(st + gb * T::B_BLOCK_BYTES + gc * T::B_CHUNK_BYTES + gg * 512, &tmap_rows, n0 + gc * 64, cur, full);
                 }
-                for (int i = 0; i < T::GATHERS / T::H; i++) {
-                    const int4 rr = make_int4(__shfl_sync(0xffffffffu, cur.x, i), __shfl_sync(0xffffffffu, cur.y, i), __shfl_sync(0xffffffffu, cur.z, i),
-                                              __shfl_sync(0xffffffffu, cur.w, i));
-                    const int qi = part * (T::GATHERS / T::H) + i;
-                    const int c = qi % T::CH, g = (qi / T::CH) % BS_GROUPS, b = qi / (T::CH * BS_GROUPS);
-                    if (g < HG) continue;
-                    const int row_in = lane >> 3, piece = lane & 7;       // four rows x eight 16-byte pieces
-                    const int row = row_in == 0 ? rr.x : row_in == 1 ? rr.y : row_in == 2 ? rr.z : rr.w;
-                    const int rs = g * 4 + row_in, col = n0 + c * 64 + piece * 8;
-                    const bool ok = col < p.N && row < p.K;               // N % 8 == 0: a piece lies entirely inside or outside
-                    cp_async_16_zfill(smem_u32(st) + (uint32_t)(b * T::B_BLOCK_BYTES + c * T::B_CHUNK_BYTES + rs * 128 + ((piece ^ (rs & 7)) << 4)),
-                                      ok ? p.B + (size_t)row * p.ldb + col : p.B, ok ? 16u : 0u);
+#pragma unroll
+                for (int g = 0; g < G; g++) {
+                    const int q = part * G + g;
+                    int4 rr = rows[T::BY_LANE ? 0 : g];
+                    if (T::BY_LANE)
+                        rr = make_int4(__shfl_sync(0xffffffffu, rr.x, g), __shfl_sync(0xffffffffu, rr.y, g), __shfl_sync(0xffffffffu, rr.z, g),
+                                       __shfl_sync(0xffffffffu, rr.w, g));
+#pragma unroll
+                    for (int c = 0; c < T::CH; c++) {
+                        if (q % BS_GROUPS < by_tma) {
+                            if (lane == 0) tma_gather4(slot(q) + c * T::B_CHUNK_BYTES, &tmap_rows, n + c * 64, rr, full);
+                            continue;
+                        }
+                        const int row_in = lane >> 3, piece = lane & 7;       // four rows x eight 16-byte pieces
+                        const int row = row_in == 0 ? rr.x : row_in == 1 ? rr.y : row_in == 2 ? rr.z : rr.w;
+                        const int rs = q % BS_GROUPS * 4 + row_in, col = n + c * 64 + piece * 8;
+                        const bool ok = col < p.N && row < p.K;               // N % 8 == 0: a piece lies entirely inside or outside
+                        cp_async_16_zfill(smem_u32(st) + (uint32_t)(q / BS_GROUPS * T::B_BLOCK_BYTES + c * T::B_CHUNK_BYTES + rs * 128 + ((piece ^ (rs & 7)) << 4)),
+                                          ok ? p.B + (size_t)row * p.ldb + col : p.B, ok ? 16u : 0u);
+                    }
                 }
                 cp_async_mbar_arrive_noinc(full);   // arrives once this lane's copies have landed
             }
             ++issued;
-            j += ng; jl += ng; s += ng;
-            if (s >= SB) { s -= SB; ++wrap; }
-            if (jl >= per_tile) {
-                do { jl -= per_tile; ++tile_i; } while (jl >= per_tile);
-                if (j < total_j) locate();
-            }
-            if (j < total_j) r = fetch();
         }
         if (gmode == GATHER_CPASYNC) cp_async_wait_all();
         if (*abort_flag && lane == 0 && gmode != GATHER_NONE) {   // this warp's copies still in flight: its stages of the last round of the ring
             for (int back = 1; back <= (SB + ng - 1) / ng && back <= issued; back++) {
-                const int jj = j - back * ng;
-                drain_slot(&b_full[jj % SB], (uint32_t)(jj / SB) & 1u, p.status);
+                const int j = first + (issued - back) * ng;
+                drain_slot(&b_full[j % SB], (uint32_t)(j / SB) & 1u, p.status);
             }
         }
         __syncwarp();
@@ -271,10 +304,10 @@ __global__ void __launch_bounds__(Traits<BN, NB>::NUM_THREADS, 1)
                 // the epilogue must have read this accumulator's previous tile
                 if (!wait_one(&acc_empty[aset], ((uint32_t)(T::ACCS == 1 ? ti : ti >> 1) & 1u) ^ 1u, abort_flag, p.status, DEV_TIMEOUT_MMA)) break;
                 for (int kt = 0; kt < p.ktiles; ++kt) {
-                    if (!wait_one(&a_full[sa], pa, abort_flag, p.status, DEV_TIMEOUT_MMA)) { alive = false; break; }
-                    tc_fence_after();
                     const uint32_t mcol = tmem_base + (uint32_t)(T::META_COL + set * 4);
                     const uint32_t aoff = (uint32_t)(sa * AM_BLOCK_BYTES) >> 4;
+                    if (!wait_one(&a_full[sa], pa, abort_flag, p.status, DEV_TIMEOUT_MMA)) { alive = false; break; }
+                    tc_fence_after();
                     // metadata image: 128 rows x 16 bytes, 8-row core matrices stored back to back
                     tc_cp_128x128b(mcol, mdesc0 + aoff);
 #pragma unroll
@@ -328,7 +361,7 @@ __global__ void __launch_bounds__(Traits<BN, NB>::NUM_THREADS, 1)
             const int aset = T::ACCS == 1 ? 0 : grp;
             // the four warps of a group leave the loop together (they meet at named barriers below)
             const bool got = wait_warp(&acc_full[aset], (uint32_t)(T::ACCS == 1 ? ti : ti >> 1) & 1u, abort_flag, p.status, DEV_TIMEOUT_EPILOGUE);
-            if (!named_barrier_and(1 + grp, 128, got)) break;
+            if (p.tma_out ? !named_barrier_and(1 + grp, 128, got) : !got) break;
             tc_fence_after();
             auto release = [&] {
                 tc_fence_before();
@@ -424,7 +457,7 @@ int g_num_sms = 0;
 // 4096 x 12288, m = 8, N = 4096 (68 beyond three) 165.9 (152.8), 160.5 (144.1);  12288 x 12288, V = 64, m = 32, N = 2048 (56 beyond ten) 114.6
 // (110.9), 113.0 (108.7).  More than half (124 beyond 13 waves, 4096 x 4096, m = 8, N = 16384), which makes two waves of halves: 217.0, 221.2.
 //
-// The estimate, in us: start-up and last epilogue, then per wave a k-tile's 1430 clocks and what a tile change costs.  It is 0.97 to 1.03 of a call
+// The estimate, in us: start-up and last epilogue, then per wave a k-tile's 1330 clocks and what a tile change costs.  It is 0.97 to 1.03 of a call
 // after a pause from 8 k-tiles a tile and 3 waves on.
 //
 // Tile configurations: V=128 -> one block per tile, BN 256; V=64 -> two blocks, BN 128; V=32 -> four blocks, BN 64 (NB * BN = 256:
@@ -432,7 +465,7 @@ int g_num_sms = 0;
 float spmm_select_config(int V, int N, int M, int ktiles, int max_ctas, bool may_cut, SpmmConfig *cfg)
 {
     const int mtiles = (M + TILE_M - 1) / TILE_M;
-    cfg->stages = Traits<256, 1>::PW;
+    cfg->stages = GATHER_PRODUCER_WARPS;
     cfg->threads = Traits<256, 1>::NUM_THREADS;
     cfg->part = Traits<256, 1>::PART;
     if (V == 128) {
@@ -453,7 +486,7 @@ float spmm_select_config(int V, int N, int M, int ktiles, int max_ctas, bool may
     cfg->tiles = (int)tiles + (cut ? rest : 0);
     cfg->cut_from = cut ? (int)(waves * sms) : cfg->tiles;
     cfg->grid = cfg->tiles < sms ? cfg->tiles : sms;
-    return 5.5f + ((float)waves + (rest == 0 ? 0.0f : cut ? 0.65f : 1.0f)) * (ktiles * 0.74f + 2.0f);
+    return 5.5f + ((float)waves + (rest == 0 ? 0.0f : cut ? 0.65f : 1.0f)) * (V == 128 ? ktiles * 0.675f + 1.5f : ktiles * 0.6f + 1.2f);
 }
 
 cudaError_t spmm_init_kernels()
