@@ -44,6 +44,34 @@ def test_few_columns(N, cfg, form):
     assert prep.device_status() == 0
 
 
+# SM pairs, 256 rows a tile: every width, columns that end inside a tile; one tile a cluster, whose columns both epilogue groups share,
+# and two or three, the last of which they share; ragged rows.
+@pytest.mark.parametrize("tiles", [1, 2, 3])
+@pytest.mark.parametrize("N", [176, 192, 216, 240, 248, 504])
+def test_pair_tiles_shared_by_both_epilogue_groups(N, tiles):
+    import torch
+    from venom_b200 import capi
+    from venom_b200.synth import random_vnm_dense_cuda
+    pairs = torch.cuda.get_device_properties(0).multi_processor_count // 2
+    M, K, V, m = (256 * 3 if tiles == 1 else 256 * (pairs * (tiles - 1) + 2)) - 96, 264, 32, 8
+    dense, cols = random_vnm_dense_cuda(M, K, V, m, seed=M + N)
+    dense = torch.sign(dense) * torch.ceil(dense.abs() * 3)
+    values, meta, bad = capi.compress(dense, cols, V, m)
+    assert bad == 0
+    prep = capi.Prepared(values, meta, cols, M, K, V, m, strategy=capi.STRATEGY_DENSE_B)
+    prep.set_pair_mode(3)   # 256 rows a tile, not the kernel for few tiles
+    assert prep.config(N)["tile_m"] == 256
+    if N in (248, 504):
+        assert prep.config(N)["tile_n"] == 256
+    B, bias = _ints((K, N), N), _ints((M,), 3)
+    want = (dense.float() @ B.float()).half()
+    assert torch.equal(prep.spmm(B), want)
+    assert torch.equal(prep.spmm(B, bias=bias, layout=capi.VNM_LAYOUT_NM), (want + bias[:, None]).T)
+    assert torch.equal(prep.spmm_nk(B.T.contiguous(), bias=bias), (want + bias[:, None]).T)
+    assert torch.equal(prep.spmm_nk(B.T.contiguous(), layout=capi.VNM_LAYOUT_MN), want)
+    assert prep.device_status() == 0
+
+
 # Gather kernel: a last wave of at most half of the SMs has its tiles cut in two, a fuller one has not.  Column tiles that end inside
 # the first and the second half; more tiles than one a SM, so that whole and half tiles follow one another on it.
 @pytest.mark.parametrize("N", [96, 200, 256 + 72])

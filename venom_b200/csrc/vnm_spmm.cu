@@ -486,7 +486,7 @@ float spmm_select_config(int V, int N, int M, int ktiles, int max_ctas, bool may
     cfg->tiles = (int)tiles + (cut ? rest : 0);
     cfg->cut_from = cut ? (int)(waves * sms) : cfg->tiles;
     cfg->grid = cfg->tiles < sms ? cfg->tiles : sms;
-    return 5.5f + ((float)waves + (rest == 0 ? 0.0f : cut ? 0.65f : 1.0f)) * (V == 128 ? ktiles * 0.675f + 1.5f : ktiles * 0.6f + 1.2f);
+    return 5.5f + ((float)waves + (rest == 0 ? 0.0f : cut ? 0.65f : 1.0f)) * (V == 128 ? ktiles * 0.76f + 1.7f : ktiles * 0.68f + 1.35f);
 }
 
 cudaError_t spmm_init_kernels()

@@ -6,9 +6,10 @@
 //
 // What bounds it: the tensor pipe inside a tile of 512 rows (8 MMAs x BN / 2 clocks a k-tile: 960 of 973 measured without loads, 991 with
 // them, BN = 240); in a tile of 256 rows the intake (48 to 50 KiB for 480 clocks of MMAs, 490 to 600 with loads); and the stores of finished tiles,
-// which leave in bursts and hold up the loads of the next tile.  4096 x 1024, N = 16384, [N,K] to [N,M], at 1965 MHz: 256 x 240 tiles
-// (what the estimate takes) 72.5 us, 52.1 without stores, MMAs 29, floor 26; 512 x 224 tiles 68.0, without stores 65.0.
-// Many such calls run into the power limit: 1430 MHz, 83 us.
+// which leave in bursts and hold up the loads of the next tile.  4096 x 1024, N = 16384, [N,K] to [N,M], many calls at the clock that the power
+// limit leaves: 512 x 240 tiles 76.7 us (after a pause, at 1965 MHz, 68.2), 256 x 240 80.3 (71.2); MMAs 29, floor 26.
+// The last tile of a pair of 256 rows is drained by both epilogue groups, and no group waits for its slowest warp before it starts
+// (2976 x 2040, N = 1368, [N,K], one wave: 15.3 -> 14.0 us).
 //
 // Cluster protocol (rank 0 = leader, rank 1 = peer); every load stays local to the CTA that issues it:
 //   * both CTAs run their own A producer, B producers and epilogue on their own shared / tensor memory;
@@ -23,6 +24,8 @@
 // No copy with cluster multicast is used anywhere.  Every wait is bounded (status bit, drain, return), and the two CTAs
 // meet at a cluster barrier before tensor memory is freed, so neither leaves while the other may still touch it.
 #include "vnm_internal.h"
+
+#include <type_traits>
 
 namespace vnm {
 
@@ -60,9 +63,10 @@ constexpr int TMEM_COLS = 512;
 // tensor-memory columns: accumulator 0 from 0, accumulator 1 from 256 (at most 240 columns each); metadata sets of four columns a
 // row tile at 240..255 (and for a third set of two row tiles at 496)
 __device__ __forceinline__ uint32_t acc_col(int rt) { return (uint32_t)rt * 256u; }
-template <int R>
+template <int R, int BN>
 __device__ __forceinline__ uint32_t meta_col(int set)
 {
+    if (BN == 256) return 256u + 4u * (uint32_t)set;
     if (R == 1) return 240u + 4u * (uint32_t)set;
     return set == 2 ? 496u : 240u + 8u * (uint32_t)set;
 }
@@ -137,7 +141,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
                                                                            const SpmmParams p)
 {
     static_assert(R == 1 || R == RT, "row tiles per CTA");  // R = 1: pair tiles of 256 rows for problems with few row tiles
-    static_assert(BN <= 240 && BN % 16 == 0, "the tensor-memory column plan");
+    constexpr bool ONE = BN == 256;                         // one accumulator: a tile's MMAs wait for the drain of the one before
+    static_assert((BN <= 240 && BN % 16 == 0) || (ONE && R == 1 && !MULTI), "the tensor-memory column plan");
     static_assert(!MULTI || BN == 6 * PART, "parts of a tile that leaves through TMA stores");
     using P = Plan<R, MULTI>;
     constexpr int SA = P::SA, SB = P::SB, A_STAGE_BYTES = P::A_STAGE_BYTES, A_RING_BYTES = P::A_RING_BYTES;
@@ -179,7 +184,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
         for (int s = 0; s < SB; s++) mbar_init(&b_free[s], 1);
         for (int a = 0; a < 2; a++) {
             mbar_init(&acc_full_bar[a], 1);
-            mbar_init(&acc_empty_bar[a], 2 * 4);  // the four warps of one epilogue group in both CTAs
+            mbar_init(&acc_empty_bar[a], ONE ? 2 * 8 : 2 * 4);  // the four warps of one epilogue group (of both) in both CTAs
         }
         *abort_flag = 0;
         fence_barrier_init();
@@ -334,13 +339,13 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
             bool alive = true;
             for (int ti = 0; alive && ti < my_tiles; ++ti) {
                 // accumulator set: R = 2 both (phase ti), R = 1 set ti & 1 (phase ti / 2)
-                const int aset = R == 1 ? (ti & 1) : 0;
-                const uint32_t aphase = R == 1 ? (uint32_t)(ti >> 1) & 1u : (uint32_t)ti & 1u;
+                const int aset = R == 1 && !ONE ? (ti & 1) : 0;
+                const uint32_t aphase = R == 1 && !ONE ? (uint32_t)(ti >> 1) & 1u : (uint32_t)ti & 1u;
                 for (int kt = 0; kt < p.ktiles; ++kt) {
                     if (kt == 0 && !wait_one(&acc_empty_bar[aset], aphase ^ 1u, abort_flag, p.status, DEV_TIMEOUT_MMA)) { alive = false; break; }
                     if (!wait_one(&a_full[sa], ph, abort_flag, p.status, DEV_TIMEOUT_MMA)) { alive = false; break; }  // both CTAs' blocks
                     tc_fence_after();
-                    const uint32_t mcol = tmem_base + meta_col<R>(sa);
+                    const uint32_t mcol = tmem_base + meta_col<R, BN>(sa);
                     const uint32_t aoff = (uint32_t)(sa * A_STAGE_BYTES) >> 4;
 #pragma unroll
                     for (int rt = 0; rt < R; rt++) tc_cp2_128x128b(mcol + rt * 4, mdesc0 + aoff + (uint32_t)((rt * AM_BLOCK_BYTES) >> 4));
@@ -385,21 +390,25 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
         const int i = q * 32 + lane;
         const int arow = mma_row_to_actual(i);
         const int grp = (warp - EPI_WARP0) >> 2;  // R = 2: the accumulator (row tile) this group drains; R = 1: the tiles ti with ti & 1 == grp
-        const uint32_t empty_leader = mapa_shared(smem_u32(&acc_empty_bar[grp]), 0);
         int ti = 0;
         for (int tile = pair; tile < total_tiles; tile += npairs, ++ti) {
-            if (R == 1 && (ti & 1) != grp) continue;
+            // R = 1: this group's tiles, its half of every tile (ONE), or its half of this CTA's last tile, with which the other has nothing
+            // left to do
+            const bool shared = ONE || (R == 1 && !MULTI && ti == my_tiles - 1);
+            if (R == 1 && !shared && (ti & 1) != grp) continue;
+            const int aset = R == 2 ? grp : ONE ? 0 : ti & 1;
             int mq, nt;
             tile_coords(tile, mquads, p.ntiles, p.group_m, &mq, &nt);
             const int n0 = nt * BN;
             // the four warps of a group leave the loop together (they meet at named barriers below)
-            const bool got = wait_warp(&acc_full_bar[grp], R == 1 ? (uint32_t)(ti >> 1) & 1u : (uint32_t)ti & 1u, abort_flag, p.status,
+            const bool got = wait_warp(&acc_full_bar[aset], R == 1 && !ONE ? (uint32_t)(ti >> 1) & 1u : (uint32_t)ti & 1u, abort_flag, p.status,
                                        DEV_TIMEOUT_EPILOGUE);
-            if (!named_barrier_and(1 + grp, 128, got)) break;
+            if (MULTI ? !named_barrier_and(1 + grp, 128, got) : !got) break;
             tc_fence_after();
             {
                 const int rt = R == 1 ? 0 : grp;  // row tile of this CTA
                 const int mt = row_tile(mq, rt);
+                const uint32_t empty_leader = mapa_shared(smem_u32(&acc_empty_bar[aset]), 0);
                 auto release = [&] {
                     tc_fence_before();
                     __syncwarp();
@@ -408,9 +417,23 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
                 if constexpr (!MULTI) {
                     // straight from tensor memory; with two row tiles per CTA the next tile's MMAs wait for both accumulators, so
                     // they are read into registers whole before the first store
-                    const uint32_t tacc = tmem_base + ((uint32_t)(q * 32) << 16) + acc_col(grp);
-                    if (p.layout == 0) store_tile<BN, R == 2>(TileStoreMN(tacc, q, (int64_t)mt * TILE_M, n0, p), release);
-                    else store_tile<BN, R == 2>(TileStoreNM(tacc, q, (int64_t)mt * TILE_M, n0, p), release);
+                    const uint32_t tacc = tmem_base + ((uint32_t)(q * 32) << 16) + acc_col(aset);
+                    auto store = [&](auto width, auto hold, int first) {
+                        constexpr int W = decltype(width)::value;
+                        constexpr bool HOLD = decltype(hold)::value;
+                        if (p.layout == 0) store_tile<W, HOLD>(TileStoreMN(tacc + (uint32_t)first, q, (int64_t)mt * TILE_M, n0 + first, p), release);
+                        else store_tile<W, HOLD>(TileStoreNM(tacc + (uint32_t)first, q, (int64_t)mt * TILE_M, n0 + first, p), release);
+                    };
+                    using std::integral_constant;
+                    if constexpr (ONE) {
+                        store(integral_constant<int, 128>(), integral_constant<bool, false>(), grp * 128);
+                    } else if (!shared) {
+                        store(integral_constant<int, BN>(), integral_constant<bool, R == 2>(), 0);
+                    } else if (grp == 0) {
+                        store(integral_constant<int, 128>(), integral_constant<bool, false>(), 0);
+                    } else {
+                        store(integral_constant<int, BN - 128>(), integral_constant<bool, false>(), 128);
+                    }
                 } else {
                 const int64_t row = (int64_t)mt * TILE_M + arow;
                 const bool row_ok = mt < p.mtiles && row < p.M;
@@ -507,7 +530,7 @@ int g_pair_clusters = 0;  // co-resident clusters of two CTAs on this device (0 
 
 }  // namespace
 
-#define VNM_PAIR_INSTANCES(X) X(1, 192, false) X(1, 224, false) X(1, 240, false) X(1, 240, true) X(2, 192, false) X(2, 224, false) X(2, 240, false) X(2, 240, true)
+#define VNM_PAIR_INSTANCES(X) X(1, 256, false) X(1, 192, false) X(1, 224, false) X(1, 240, false) X(1, 240, true) X(2, 192, false) X(2, 224, false) X(2, 240, false) X(2, 240, true)
 
 cudaError_t spmm_dense_b_pair_init()
 {
@@ -537,17 +560,17 @@ cudaError_t spmm_dense_b_pair_init()
     return cudaSuccess;
 }
 
-// Pair tiles have 512 rows (two row tiles per CTA) or 256 (one row tile per CTA, two alternating accumulators) and 240, 224 or
-// 192 columns.  The tall form reads every B stage once per 512 rows, but its accumulators are drained between tiles (3 to 4 us a
-// wave against 1.1 to 1.5) and it needs twice the rows for a full wave; row tiles that do not divide evenly are padded
-// (computed, never stored).  A [K,N] operand in tiles of 240 columns costs half as much again a k-tile: the peer's half, 240 bytes
-// further, starts inside a 32-byte sector.  The constants are us a k-tile and us a wave, fitted to 18 shapes from 512 to 49152 rows, 512 to
-// 12288 k and 512 to 16384 columns; the smallest estimate wins.  They are a ranking more than a time: calls at the full clock (1965
-// MHz) on inputs that change from call to call take 1.08 to 1.48 of them (seven shapes, both layouts, all six tiles: 0.94 to
-// 1.48), least with [K,N] and many waves, most with a single wave that reads everything from HBM.  Of those 14 problems the tile
-// chosen is the fastest or within 1 % of it for 11; it is 512 x 192 instead of 256 x 240 (20.0 us instead of 15.9) for [K,N] 2976 x
-// 2040, N = 1368, and 256 x 240 instead of 512 x 224 for [N,K] 4096 x 1024 (72.5, 68.0) and 1024 x 1024 (25.2, 22.8), N = 16384, where
-// the stores of a wave outweigh its few k-tiles.
+// Pair tiles have 512 rows (two row tiles per CTA) or 256 (one row tile per CTA) and 256, 240, 224 or 192 columns.  The tall form reads every
+// B stage once per 512 rows, but its accumulators are drained between tiles and it needs twice the rows for a full wave; row tiles that
+// do not divide evenly are padded (computed, never stored).  256 columns leave tensor memory for one accumulator only: the MMAs wait
+// while it is drained, by both epilogue groups.  A [K,N] operand never takes 240 columns: the peer's half, 240 bytes further, starts
+// inside a 32-byte sector (0.65 us a k-tile instead of 0.48); 256 are aligned, and one wave of such tiles is what it wants most often:
+// 1024 x 4096, N = 4096 26.1 us as 512 x 192 (44 tiles for 74 pairs), 19.8 as 256 x 256; 8192 x 2048, N = 1024 25.2, 18.7; 4096 x 4096, N =
+// 4096 70.9, 64.2.  [N,K]: 256 x 240 or 256 where tiles are few, else 512 x 240.
+// The cost of a call, us: a start, and per wave a k-tile's time and a drain, with waves between the whole number that the last tile makes
+// and the fraction that the SMs' power and memory see.  Fitted to steady calls on inputs that change, 22 shapes from 512 to 49152 rows, 512
+// to 12288 k and 512 to 16384 columns, both layouts, all seven tiles (ratio to the measured time 0.7 to 1.25); the tile chosen takes
+// 1.007 of the fastest one's time on average, 1.16 at most (2048 x 8192, N = 1000, whose rows of 2000 bytes are not aligned to sectors).
 float spmm_dense_b_pair_config(int M, int N, int K, int b_nk, int max_ctas, int force_rows, bool multi, SpmmConfig *cfg)
 {
     if (g_pair_clusters <= 0) return -1.0f;
@@ -555,17 +578,22 @@ float spmm_dense_b_pair_config(int M, int N, int K, int b_nk, int max_ctas, int 
     int clusters = g_pair_clusters;
     if (max_ctas > 0 && max_ctas / 2 < clusters) clusters = max_ctas / 2;
     if (clusters < 1) return -1.0f;
-    static const int widths[3] = {240, 224, 192};
-    static const float kt_us[2][2][3] = {{{0.635f, 0.365f, 0.376f}, {0.31f, 0.30f, 0.295f}}, {{0.72f, 0.505f, 0.48f}, {0.54f, 0.50f, 0.465f}}};   // [row tiles - 1][b_nk][width]
-    static const float wave_us[2][3] = {{1.2f, 1.45f, 1.1f}, {3.4f, 3.9f, 2.9f}}, start_us[2] = {5.2f, 4.7f};
+    static const int widths[4] = {256, 240, 224, 192};
+    struct Cost { float start, kt, wave; };
+    static const Cost cost[2][2][4] = {   // [row tiles - 1][b_nk][width], us
+        {{{4.2f, 0.533f, 1.3f}, {6.0f, 0.692f, 0.95f}, {5.2f, 0.519f, 1.1f}, {5.45f, 0.506f, 0.85f}}, {{4.4f, 0.507f, 1.5f}, {4.5f, 0.474f, 1.25f}, {4.7f, 0.462f, 1.05f}, {4.95f, 0.429f, 0.9f}}},
+        {{{0.0f, 0.0f, 0.0f}, {4.85f, 1.006f, 2.75f}, {4.65f, 0.847f, 3.0f}, {4.1f, 0.792f, 2.45f}}, {{0.0f, 0.0f, 0.0f}, {4.2f, 0.853f, 2.75f}, {4.9f, 0.808f, 2.95f}, {4.4f, 0.729f, 2.25f}}}};
     float best = 1e30f;
-    for (int w = 0; w < (multi ? 1 : 3); w++) {
+    for (int w = 0; w < 4; w++) {
+        if (multi ? widths[w] != 6 * PART : !b_nk && widths[w] == 240) continue;
         const long long ntiles = (N + widths[w] - 1) / widths[w];
         for (int rt = 1; rt <= RT; rt++) {
+            if (rt == RT && widths[w] == 256) continue;   // its accumulators would fill tensor memory
             if ((force_rows == 1 && rt == RT) || (force_rows == 2 && mtiles > 2 && rt == 1)) continue;
             const long long tiles = (long long)((mtiles + 2 * rt - 1) / (2 * rt)) * ntiles;
-            const float waves = (float)((tiles + clusters - 1) / clusters);
-            const float us = start_us[rt - 1] + waves * (ktiles * kt_us[rt - 1][b_nk != 0][w] + wave_us[rt - 1][w]);
+            const float waves = 0.6f * (float)((tiles + clusters - 1) / clusters) + 0.4f * (float)tiles / clusters;
+            const Cost &c = cost[rt - 1][b_nk != 0][w];
+            const float us = c.start + waves * (ktiles * c.kt + c.wave);
             if (us < best) {
                 best = us;
                 cfg->bn = widths[w];
