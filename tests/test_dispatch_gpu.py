@@ -44,6 +44,29 @@ def test_few_columns(N, cfg, form):
     assert prep.device_status() == 0
 
 
+# Few tiles: one CTA an SM with the deep ring (eight k-tiles a CTA and more), two, and several waves of them; rings that do and do not go round.
+@pytest.mark.parametrize("V", [128, 64, 32])
+@pytest.mark.parametrize("ktiles", [7, 8, 9, 21])
+@pytest.mark.parametrize("N", [72, 104, 200, 264])
+@pytest.mark.parametrize("form", ["gather", "dense_b"])
+def test_few_tiles_with_the_deep_ring(form, N, ktiles, V):
+    import torch
+    from venom_b200 import capi
+    M, m = 160 if V == 32 else 192 if V == 64 else 256, 8
+    K = 128 * ktiles - 56 if form == "dense_b" else 256 * ktiles - 40       # the last k-tile is ragged
+    d, _, _, _, prep = _operand(M, K, V, m, capi.STRATEGY_GATHER if form == "gather" else capi.STRATEGY_DENSE_B, seed=M + K)
+    prep.set_pair_mode(0)
+    cfg = prep.config(N)
+    assert cfg["tile_m"] == 128 and (cfg["smem_bytes"] > 110 * 1024) == (ktiles >= 8 or cfg["tile_n"] * (128 // V if form == "gather" else 1) > 128)
+    B, bias = _ints((K, N), N), _ints((M,), 3)
+    want = (d @ B.float()).half()
+    assert torch.equal(prep.spmm(B), want)
+    assert torch.equal(prep.spmm(B, bias=bias, layout=capi.VNM_LAYOUT_NM), (want + bias[:, None]).T)
+    if form == "dense_b":
+        assert torch.equal(prep.spmm_nk(B.T.contiguous()), want.T)
+    assert prep.device_status() == 0
+
+
 # SM pairs, 256 rows a tile: every width, columns that end inside a tile; one tile a cluster, whose columns both epilogue groups share,
 # and two or three, the last of which they share; ragged rows.
 @pytest.mark.parametrize("tiles", [1, 2, 3])

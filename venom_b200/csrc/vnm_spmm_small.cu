@@ -1,4 +1,4 @@
-// SpMM kernel for few columns: C[M,N] = A * B for decoding steps and other products with too few 128 x 240 tiles to occupy the
+// SpMM kernel for few columns: C[M,N] = A * B for decoding steps and other products with too few large tiles to occupy the
 // GPU.  Both operand forms: the V:N:M form (rows of B gathered, NB = 128/V blocks) and the dense-B form (B as [K,N] or [N,K]
 // tiles shared by all blocks, NB = 1).
 //
@@ -9,17 +9,21 @@
 // results are the same on every call.
 //
 // One ring stage is a whole k-tile: the 18 KiB block of A (values and metadata, one bulk copy) and its rows of B.
-// Warps: 0..7 B producers (gather4 loads dealt to all of them; a warp needs about 65 clocks for each it issues), 8 A
-// producer, 9 tensor-memory owner and MMA issuer, 12..15 epilogue.  Every wait is bounded.
+// Warps: 0..7 B producers (gather4 loads dealt to all of them; plain tiles: warps 0 and 1 in turn), 8 A producer (with warp 10 in turn in the
+// deep instances), 9 tensor-memory owner and MMA issuer, 12..15 epilogue.  Every wait is bounded.  One thread needs up to 420 clocks to issue
+// a stage: 15.9 us a layer at 2048 x 8192, 128:2:8, 96 tokens with one issuing warp for B and A each, 13.8 with two.  Deep instances issue gathers
+// from one elected lane (see vnm_spmm.cu): 18.8 -> 15.8 us at 2048 x 8192, 128:2:8, N = 96 in tiles of 128 columns, 10.7 -> 9.5 at 1024 x 4096, 64:2:8,
+// N = 64; with two CTAs an SM it is bound by A and a gather4 a lane is as fast or faster (36864 x 12288, 128:2:16, 16 tokens 27.5, 27.8).
 #include "vnm_internal.h"
 
+#include <cmath>
 #include <cstring>
 
 namespace vnm {
 
 namespace {
 
-template <int BN, int NB>
+template <int BN, int NB, bool DEEP>
 struct Small {
     static_assert(NB == 1 || NB == 2 || NB == 4, "128 rows hold 1, 2 or 4 vector blocks");
     static constexpr int RB = BN >= 64 ? 128 : 2 * BN;        // bytes of a row of B in one slice (its swizzle span)
@@ -32,13 +36,18 @@ struct Small {
     static constexpr int PW = 8;
     static constexpr int GATHERS = NB * KT_GROUPS * CH;       // per k-tile
     static constexpr int PER_WARP = GATHERS / PW;
-    static_assert(PER_WARP <= 32 && GATHERS % PW == 0, "gathers are dealt to the lanes of the producer warps");
-    static constexpr int STAGES = 104 * 1024 / STAGE_BYTES < 2 ? 2 : 104 * 1024 / STAGE_BYTES > 5 ? 5 : 104 * 1024 / STAGE_BYTES;
+    static_assert(PER_WARP <= 32 && GATHERS % PW == 0 && KT_GROUPS % (NB * KT_GROUPS / PW) == 0, "gathers are dealt to the producer warps, groups of one block");
+    // Gathers: a lane issues one each, or (where one CTA has the SM, and the eight groups of a warp fit every lane's registers) one lane all of a warp's
+    static constexpr bool BY_LANE = !DEEP || NB == 4;
+    // Two CTAs share an SM and each has half of its shared memory for the ring; one that has its SM to itself (DEEP) has all of it.
+    static constexpr int RING_BYTES = (DEEP ? 210 : 104) * 1024, MOST = DEEP ? 8 : 5;
+    static constexpr int STAGES = RING_BYTES / STAGE_BYTES < 2 ? 2 : RING_BYTES / STAGE_BYTES > MOST ? MOST : RING_BYTES / STAGE_BYTES;
     static constexpr int RED_BYTES = (BN + 8) * TILE_M * 4;   // split over K: this CTA's columns from every rank (8: its share is rounded up); in the idle rings
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 256 + 1024;
     static_assert(SMEM_BYTES <= 227 * 1024 && (BN > 64 || RED_BYTES <= STAGES * STAGE_BYTES), "shared memory per CTA");
-    static constexpr int CTAS = 2 * (SMEM_BYTES + 1024) <= 227 * 1024 ? 2 : 1;   // resident per SM
-    static constexpr int A_WARP = PW, MMA_WARP = PW + 1, EPI_WARP0 = 12;
+    static constexpr int CTAS = !DEEP && 2 * (SMEM_BYTES + 1024) <= 227 * 1024 ? 2 : 1;   // resident per SM
+    static constexpr int A_WARP = PW, MMA_WARP = PW + 1, A_WARP2 = PW + 2, EPI_WARP0 = 12;
+    static constexpr int A_WARPS = DEEP ? 2 : 1;              // warps that load A
     static constexpr int NUM_THREADS = 16 * 32;
     static constexpr int META_COL = BN < 64 ? 64 : BN;        // the epilogue reads 64 columns at a time
     static constexpr int META_SETS = 4;
@@ -61,11 +70,11 @@ __device__ __forceinline__ uint32_t mapa_shared(uint32_t saddr, uint32_t rank)
 }
 __device__ __forceinline__ void st_cluster(uint32_t addr, uint32_t v) { asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
 
-template <int BN, int NB>
-__global__ void __launch_bounds__(Small<BN, NB>::NUM_THREADS, 2)
+template <int BN, int NB, bool DEEP>
+__global__ void __launch_bounds__(Small<BN, NB, DEEP>::NUM_THREADS, 2)
     spmm_small_kernel(const __grid_constant__ CUtensorMap tmap_b, const SpmmParams p)
 {
-    using T = Small<BN, NB>;
+    using T = Small<BN, NB, DEEP>;
     constexpr int S = T::STAGES;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -114,33 +123,61 @@ __global__ void __launch_bounds__(Small<BN, NB>::NUM_THREADS, 2)
         // ---------------- B producers ----------------
         if (p.early) grid_dependency_wait();   // B is still being written; A, barriers and tensor memory do not depend on it
         if (mode == GATHER_TMA4) {
-            const int q = warp * T::PER_WARP + lane;
-            const bool on = lane < T::PER_WARP;
-            const int gc = q % T::CH, gg = (q / T::CH) % KT_GROUPS, gb = on ? q / (T::CH * KT_GROUPS) : 0;
-            const int4 *rows = p.rows + ((size_t)(mt * NB + gb) * p.ktiles) * KT_GROUPS + gg;
-            if (lane == 0) tma_prefetch_desc(&tmap_b);
-            int4 r = make_int4(0, 0, 0, 0);
-            if (on && k0 < k1) r = __ldg(rows + (size_t)k0 * KT_GROUPS);
-            int s = 0;
-            uint32_t ph = 1;
             int kt = k0;
-            for (; kt < k1; ++kt) {
-                const int4 cur = r;
-                if (on && kt + 1 < k1) r = __ldg(rows + (size_t)(kt + 1) * KT_GROUPS);
-                if (!__all_sync(0xffffffffu, wait_quiet(&freed[s], ph, abort_flag, p.status, DEV_TIMEOUT_PRODUCER))) break;
-                if (lane == 0) mbar_arrive_expect_tx(&full[s], T::PER_WARP * 4 * T::RB);
-                __syncwarp();
-                if (on) tma_gather4(b_ring + s * T::B_BYTES + gb * T::B_BLOCK_BYTES + gc * T::B_CHUNK_BYTES + gg * 4 * T::RB, &tmap_b, n0 + gc * 64, cur, &full[s]);
-                if (++s == S) { s = 0; ph ^= 1; }
+            if constexpr (T::BY_LANE) {
+                const int q = warp * T::PER_WARP + lane;
+                const bool on = lane < T::PER_WARP;
+                const int gc = q % T::CH, gg = (q / T::CH) % KT_GROUPS, gb = on ? q / (T::CH * KT_GROUPS) : 0;
+                const int4 *rows = p.rows + ((size_t)(mt * NB + gb) * p.ktiles) * KT_GROUPS + gg;
+                if (lane == 0) tma_prefetch_desc(&tmap_b);
+                int4 r = make_int4(0, 0, 0, 0);
+                if (on && k0 < k1) r = __ldg(rows + (size_t)k0 * KT_GROUPS);
+                int s = 0;
+                uint32_t ph = 1;
+                for (; kt < k1; ++kt) {
+                    const int4 cur = r;
+                    if (on && kt + 1 < k1) r = __ldg(rows + (size_t)(kt + 1) * KT_GROUPS);
+                    if (!__all_sync(0xffffffffu, wait_quiet(&freed[s], ph, abort_flag, p.status, DEV_TIMEOUT_PRODUCER))) break;
+                    if (lane == 0) mbar_arrive_expect_tx(&full[s], T::PER_WARP * 4 * T::RB);
+                    __syncwarp();
+                    if (on) tma_gather4(b_ring + s * T::B_BYTES + gb * T::B_BLOCK_BYTES + gc * T::B_CHUNK_BYTES + gg * 4 * T::RB, &tmap_b, n0 + gc * 64, cur, &full[s]);
+                    if (++s == S) { s = 0; ph ^= 1; }
+                }
+            } else {
+                // this warp's groups of a k-tile are warp * G ..; group q is group q % KT_GROUPS of vector block q / KT_GROUPS
+                constexpr int G = NB * KT_GROUPS / T::PW;
+                const int mine = warp * G;
+                const int4 *entry = p.rows + ((size_t)(mt * NB + mine / KT_GROUPS) * p.ktiles + k0) * KT_GROUPS + mine % KT_GROUPS;
+                uint8_t *const first = b_ring + mine / KT_GROUPS * T::B_BLOCK_BYTES + mine % KT_GROUPS * 4 * T::RB;
+                if (lane == 0) tma_prefetch_desc(&tmap_b);
+                int s = 0;
+                uint32_t ph = 1;
+                for (; kt < k1; ++kt) {
+                    int4 rows[G];                    // on their way while the warp waits for the slot
+#pragma unroll
+                    for (int g = 0; g < G; g++) rows[g] = __ldg(entry + g);
+                    entry += KT_GROUPS;
+                    if (!__all_sync(0xffffffffu, wait_quiet(&freed[s], ph, abort_flag, p.status, DEV_TIMEOUT_PRODUCER))) break;
+                    uint8_t *dst = first + s * T::B_BYTES;
+                    if (elect_one()) {
+                        mbar_arrive_expect_tx(&full[s], T::PER_WARP * 4 * T::RB);
+#pragma unroll
+                        for (int g = 0; g < G; g++) {
+#pragma unroll
+                            for (int c = 0; c < T::CH; c++) tma_gather4(dst + c * T::B_CHUNK_BYTES + g * 4 * T::RB, &tmap_b, n0 + c * 64, rows[g], &full[s]);
+                        }
+                    }
+                    if (++s == S) { s = 0; ph ^= 1; }
+                }
             }
             if (*abort_flag && lane == 0)
                 for (int k = kt - k0 > S ? kt - k0 - S : 0; k < kt - k0; ++k) drain_slot(&full[k % S], (uint32_t)(k / S) & 1u, p.status);
-        } else if (warp == 0 && elect_one()) {
+        } else if (warp < 2 && elect_one()) {
             tma_prefetch_desc(&tmap_b);
-            int s = 0;
+            int s = warp;
             uint32_t ph = 1;
-            int kt = k0;
-            for (; kt < k1; ++kt) {
+            int kt = k0 + warp;
+            for (; kt < k1; kt += 2) {
                 if (!wait_quiet(&freed[s], ph, abort_flag, p.status, DEV_TIMEOUT_PRODUCER)) break;
                 uint8_t *st = b_ring + s * T::B_BYTES;
                 if (mode == GATHER_NONE) {
@@ -153,27 +190,29 @@ __global__ void __launch_bounds__(Small<BN, NB>::NUM_THREADS, 2)
                     for (int b = 0; b < NB; b++)
                         for (int c = 0; c < T::CH; c++) tma_load_2d(st + b * T::B_BLOCK_BYTES + c * T::B_CHUNK_BYTES, &tmap_b, n0 + c * 64, kt * KT_ROWS, &full[s]);
                 }
-                if (++s == S) { s = 0; ph ^= 1; }
+                if ((s += 2) >= S) { s -= S; ph ^= 1; }
             }
             if (*abort_flag && mode != GATHER_NONE)
-                for (int k = kt - k0 > S ? kt - k0 - S : 0; k < kt - k0; ++k) drain_slot(&full[k % S], (uint32_t)(k / S) & 1u, p.status);
+                for (int k = kt - k0 > S + 1 ? kt - k0 - (S + 1) / 2 * 2 : warp; k < kt - k0; k += 2) drain_slot(&full[k % S], (uint32_t)(k / S) & 1u, p.status);
         }
         __syncwarp();
-    } else if (warp == T::A_WARP) {
-        // ---------------- A producer ----------------
+    } else if (warp == T::A_WARP || (T::A_WARPS == 2 && warp == T::A_WARP2)) {
+        // ---------------- A producers, alternate k-tiles ----------------
         if (elect_one()) {
             const uint8_t *src = p.am + (size_t)mt * p.ktiles * AM_BLOCK_BYTES;
-            int s = 0;
+            constexpr int step = T::A_WARPS;
+            const int half = warp == T::A_WARP ? 0 : 1;
+            int s = half;
             uint32_t ph = 1;
-            int kt = k0;
-            for (; kt < k1; ++kt) {
+            int kt = k0 + half;
+            for (; kt < k1; kt += step) {
                 if (!wait_quiet(&freed[s], ph, abort_flag, p.status, DEV_TIMEOUT_PRODUCER)) break;
                 mbar_arrive_expect_tx(&full[s], AM_BLOCK_BYTES);
                 bulk_g2s(a_ring + s * AM_BLOCK_BYTES, src + (size_t)kt * AM_BLOCK_BYTES, AM_BLOCK_BYTES, &full[s]);
-                if (++s == S) { s = 0; ph ^= 1; }
+                if ((s += step) >= S) { s -= S; ph ^= 1; }
             }
             if (*abort_flag)
-                for (int k = kt - k0 > S ? kt - k0 - S : 0; k < kt - k0; ++k) drain_slot(&full[k % S], (uint32_t)(k / S) & 1u, p.status);
+                for (int k = kt - k0 > S + 1 ? kt - k0 - (S + 1) / step * step : half; k < kt - k0; k += step) drain_slot(&full[k % S], (uint32_t)(k / S) & 1u, p.status);
         }
         __syncwarp();
     } else if (warp == T::MMA_WARP) {
@@ -315,16 +354,16 @@ __global__ void wait_expiry_selftest_kernel(int *status)
 template <int BN, int NB>
 cudaError_t init_one()
 {
-    return cudaFuncSetAttribute(spmm_small_kernel<BN, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, Small<BN, NB>::SMEM_BYTES);
+    const cudaError_t e = cudaFuncSetAttribute(spmm_small_kernel<BN, NB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Small<BN, NB, false>::SMEM_BYTES);
+    return e == cudaSuccess ? cudaFuncSetAttribute(spmm_small_kernel<BN, NB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Small<BN, NB, true>::SMEM_BYTES) : e;
 }
 
 template <int BN, int NB>
 cudaError_t launch_one(const SpmmConfig &cfg, const CUtensorMap &tmap_b, const SpmmParams &p, cudaStream_t stream)
 {
-    using T = Small<BN, NB>;
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3((unsigned)cfg.grid, 1, 1);
-    lc.blockDim = dim3(T::NUM_THREADS, 1, 1);
+    lc.blockDim = dim3(Small<BN, NB, false>::NUM_THREADS, 1, 1);
     lc.dynamicSmemBytes = (size_t)cfg.smem_bytes;
     lc.stream = stream;
     cudaLaunchAttribute attr[2];
@@ -337,15 +376,16 @@ cudaError_t launch_one(const SpmmConfig &cfg, const CUtensorMap &tmap_b, const S
         attr[lc.numAttrs++].val.clusterDim.z = 1;
     }
     attr[lc.numAttrs++] = early_launch();
-    return cudaLaunchKernelEx(&lc, spmm_small_kernel<BN, NB>, tmap_b, p);
+    return cfg.resident == 1 ? cudaLaunchKernelEx(&lc, spmm_small_kernel<BN, NB, true>, tmap_b, p) : cudaLaunchKernelEx(&lc, spmm_small_kernel<BN, NB, false>, tmap_b, p);
 }
 
+// The instance for a grid: the deep ring where every CTA has an SM to itself.
 template <int BN, int NB>
-void fill(SpmmConfig *cfg)
+void fill(SpmmConfig *cfg, bool deep)
 {
-    cfg->smem_bytes = Small<BN, NB>::SMEM_BYTES;
-    cfg->threads = Small<BN, NB>::NUM_THREADS;
-    cfg->resident = Small<BN, NB>::CTAS;
+    cfg->smem_bytes = deep ? Small<BN, NB, true>::SMEM_BYTES : Small<BN, NB, false>::SMEM_BYTES;
+    cfg->threads = Small<BN, NB, false>::NUM_THREADS;
+    cfg->resident = deep ? Small<BN, NB, true>::CTAS : Small<BN, NB, false>::CTAS;
 }
 
 #define VNM_SMALL_DISPATCH(bn, nb, CALL)                                                                                  \
@@ -374,45 +414,49 @@ cudaError_t spmm_small_init()
     return cudaDeviceGetAttribute(&g_num_sms_small, cudaDevAttrMultiProcessorCount, dev);
 }
 
-// Tile width and split with the smallest estimated time (microseconds, returned).  The estimate is a fit to a sweep over
-// 1024 x 1024 .. 12288 x 12288, N = 8 .. 512, all widths and splits: a fixed part for launch, set-up, first loads and
-// epilogue; a k-tile's time in a CTA that has its SM to itself (latency of the ring for narrow tiles, the shared-memory port
-// for wide ones); a second CTA on an SM costs its set-up and shares the port; and A cannot be read faster than HBM delivers
-// it.  Widths of 16 and more CTAs than SMs lose more often than they win, which is what the fit expresses.  Only up to
-// SMALL_SPLIT_N columns are k-tiles split: beyond, the order of summation stays that of the other kernels, so that results do
-// not depend on how a caller cuts its columns.
+// Tile width and split with the smallest estimated time (microseconds, returned).  A fit to calls replayed from a graph, 512 x 4096 .. 36864 x
+// 12288, N = 8 .. 1024, all widths, splits 1, 2, 3, 4, 6 and 8: a fixed part for launch, set-up, first loads and epilogue; a k-tile's time, with the
+// deep ring where each CTA has an SM to itself and eight k-tiles or more to fill it with (4096 x 4096, N = 256, 64-column tiles 12.3 us a layer with two
+// CTAs' rings, 10.9 with the deep one; fewer k-tiles, or a cluster of such CTAs, gain nothing or lose: 8.2 -> 10.8 at 1024 x 4096, N = 64, split by 8);
+// the exchange of a split; a second CTA on an SM costs its set-up and shares the port; clusters of more than four do not
+// fill the last SMs of a GPC; and A cannot be read faster than HBM delivers it.  The choice takes 1.006 of the fastest one's time on average, 1.06 at most,
+// over 42 shapes (the fit to older kernels took 1.06 and 1.34: 14.2 us split by 3 instead of 10.6 by 2 at 12288 x 12288, 128:2:16, N = 16, 7.1 split by 8
+// instead of 5.5 by 4 at 1024 x 4096, 64:2:8, N = 64).  Only up to SMALL_SPLIT_N columns are k-tiles split: beyond, the
+// order of summation stays that of the other kernels, so that results do not depend on how a caller cuts its columns.
 float spmm_small_config(int mtiles, int ktiles, int N, int nb, bool gather, SpmmConfig *cfg)
 {
     const int sms = g_num_sms_small > 0 ? g_num_sms_small : 148;
     static const int widths[4] = {16, 32, 64, 128};
-    static const float fixed[4] = {3.9f, 4.1f, 4.6f, 5.3f};
-    static const float dense_kt[4] = {0.185f, 0.19f, 0.25f, 0.43f}, gather_kt[4] = {0.32f, 0.33f, 0.36f, 0.53f};
-    const float hbm = 3.5f + (float)mtiles * ktiles * AM_BLOCK_BYTES / 5.6e6f;
+    static const float fixed[4] = {3.15f, 3.3f, 4.0f, 4.65f};
+    static const float kt_time[2][2][4] = {{{0.165f, 0.17f, 0.25f, 0.43f}, {0.165f, 0.17f, 0.172f, 0.24f}},      // [gather][deep][width]
+                                           {{0.285f, 0.29f, 0.34f, 0.5f}, {0.285f, 0.29f, 0.27f, 0.35f}}};
+    const float a_bytes = (float)mtiles * ktiles * AM_BLOCK_BYTES;
     float best = 1e30f;
     for (int w = 0; w < 4; w++) {
         const int bn = widths[w];
         if ((bn == 128 && nb > 1) || (bn > 16 && bn >= 2 * N)) continue;
-        SpmmConfig c;
-        memset(&c, 0, sizeof(c));
-#define VNM_FILL(BN, NB) fill<BN, NB>(&c)
+        SpmmConfig shared, alone;
+        memset(&shared, 0, sizeof(shared));
+        memset(&alone, 0, sizeof(alone));
+#define VNM_FILL(BN, NB) (fill<BN, NB>(&shared, false), fill<BN, NB>(&alone, true))
         VNM_SMALL_DISPATCH(bn, nb, VNM_FILL);
 #undef VNM_FILL
-        const float kt_us = (gather ? gather_kt[w] : dense_kt[w]) * (nb == 4 ? 1.4f : nb == 2 ? 1.15f : 1.0f);
         const int tiles = mtiles * ((N + bn - 1) / bn);
         for (int split = 1; split <= 8 && split <= ktiles; split++) {
-            const int ctas = tiles * split, per = (ctas + sms - 1) / sms;
-            const int kts = (ktiles + split - 1) / split;
-            const int both = per < c.resident ? per : c.resident;      // CTAs that share an SM
-            float t = fixed[w] + (gather && nb > 1 ? 1.4f : 0.0f) + (split > 1 ? 0.3f + 0.006f * bn : 0.0f);
-            if (per <= c.resident) {
-                t += 2.2f * (both - 1) + kts * kt_us * (1.0f + 0.45f * (both - 1));
-            } else {   // several waves: the port is busy all the time and nothing is gained from the second CTA
-                t += (float)ctas / (float)(sms * c.resident) * (kts * kt_us * both * 1.25f + 3.0f);
-            }
-            t = t > hbm ? t : hbm + 0.01f * t;
+            const int ctas = tiles * split, kts = (ktiles + split - 1) / split;
+            const bool deep = split == 1 && kts >= 8 && ctas <= sms;
+            const bool one_each = (float)ctas <= (split <= 4 ? 1.0f : 0.72f) * sms;
+            const float fit = (split <= 2 ? 1.0f : 0.89f) * (float)(sms * shared.resident);       // CTAs at a time
+            const float kt_us = kt_time[gather][deep][w] * (nb == 4 ? 2.1f : nb == 2 ? 1.38f : 1.0f);
+            float t = fixed[w] + (nb == 4 ? 1.0f : nb == 2 ? 0.2f : 0.0f);
+            if (split > 1) t += 0.25f + 0.016f * bn + 0.004f * (float)(ctas < sms ? ctas : sms);
+            if (one_each) t += kts * kt_us * (1.0f + (gather ? 0.1f * ctas / sms : 0.0f));
+            else t += ceilf((float)ctas / fit) * (kts * kt_us * 1.45f + 2.0f);
+            const float hbm = 3.5f + a_bytes / (gather && one_each ? 4.2e6f : 5.6e6f);
+            t = (t > hbm ? t : hbm) + 0.05f * t;
             if (t < best) {
                 best = t;
-                *cfg = c;
+                *cfg = deep ? alone : shared;
                 cfg->bn = bn;
                 cfg->nb = nb;
                 cfg->part = bn;
