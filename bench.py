@@ -49,7 +49,7 @@ CONFIG = {"workload": "cfg4", "M": CFG4["M"], "K": CFG4["K"], "N": CFG4["N"], "V
 # dram__bytes_read.sum + dram__bytes_write.sum of one launch of the headline kernel at full size on one GPU, from the
 # one-pass ncu capture summarised under profiles/ (re-capture whenever the kernel or its tile order changes; reported for the
 # form that was captured only).
-NCU_TRAFFIC = {"bytes_per_launch": 15800000000 + 3270000000, "form": "gather",
+NCU_TRAFFIC = {"bytes_per_launch": 14760000000 + 3250000000, "form": "gather",
                "source": "profiles/spmm_kernel_cfg4_launch.md: one-pass ncu capture of a full-size launch (1 GPU, N = 32768)"}
 CPU_SAMPLE_ROWS = 256
 CPU_SAMPLE_DESC = ("first %d of the %d rows of the cfg4 sparse operand (2 vector blocks), full K and N: reference to_dense + restated "

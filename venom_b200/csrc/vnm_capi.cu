@@ -155,16 +155,14 @@ int ensure_kernels_ready(int *device_out)
 // m/4 times the MMA work and shares B between all blocks.  Measured on B200, [K,N] to [M,N], new inputs from call to call, each form
 // by itself until the clock is steady (both run into the power limit: the dense-B form at 1040 to 1500 MHz, the gather form at 1500
 // to 1700), us gather / dense-B:
-//   V = 128, m = 8, 1024 rows and more: 100 / 110 at 12288 x 4096, N = 2048;  250 / 258 at 4096 x 4096 and 76.5 / 75.3 at 1024 x 4096, N =
-//     16384;  1057 / 1125 at 12288 x 12288, N = 8192;  16.2 / 18.2 ms at 49152 x 12288, N = 32768; from 0.64 of the dense-B time (512 columns) to
-//     1.05 (1024 x 1024, N = 8192) over 54 sizes.  Calls of the two forms in turn show the opposite (1128 / 949 and 4554 / 3890 at 12288 and
-//     49152 x 12288, N = 8192), because each then runs at the clock that the other one left behind; after a pause, at the full clock,
-//     913 / 971 and 3580 / 3926, but 69 / 62 at 1024 x 4096, N = 16384.
-//   V = 128, m = 8, fewer rows: the line at 1024 is older than these figures, which have the gather form at 0.55 to 1.19 there (11.7 / 18.5
-//     at 128 x 4096, 24.6 / 26.2 at 512 x 4096, 11.6 / 9.8 at 768 x 512, N = 8192).
-//   4096 x 4096, N = 16384 (at N = 2048 and at 12288 x 12288 the ratios are the same or smaller):  m = 4 420 / 266;  V = 128: m = 16 147 / 248;
-//     V = 64: m = 8 388 / 252, m = 16 215 / 246, m = 32 127 / 243;  V = 32: m = 16 397 / 246, m = 32 220 / 243, m = 64 131 / 240.  The
-//     lines that leave V = 64, m = 16 and V = 32, m = 32 to the dense-B form are older than these figures, too.
+//   V = 128, m = 8, 1024 rows and more: 78 / 102 at 12288 x 4096, N = 2048;  198 / 248 at 4096 x 4096 and 62 / 71 at 1024 x 4096, N = 16384;
+//     806 / 1069 at 12288 x 12288, N = 8192;  13.3 / 17.8 ms at 49152 x 12288, N = 32768.  (After a pause, at the full clock: 72 / 90, 176 / 217, 55 / 62,
+//     718 / 926, 11.8 / 15.2 ms.)  Calls of two forms in turn each run at the clock that the other one left behind, so forms are compared by themselves.
+//   V = 128, m = 8, fewer rows: the line at 1024 is older than these figures (9.9 / 13.8 at 128 x 4096, 22.3 / 22.4 at 512 x 4096, 9.6 / 9.9 at 768 x
+//     512, N = 8192).
+//   4096 x 4096, N = 16384:  m = 4 520 / 259;  V = 128: m = 16 121 / 238;  V = 64: m = 8 349 / 246, m = 16 193 / 238, m = 32 116 / 234;  V = 32:
+//     m = 16 376 / 239, m = 32 208 / 235, m = 64 121 / 232.  The lines that leave V = 64, m = 16 and V = 32, m = 32 to the dense-B form are older than
+//     these figures, too; they stay, because an operand's form decides which calls it takes ([N,K] activations without a workspace).
 bool choose_dense_b(int M, int K, int V, int m, int strategy)
 {
     const bool possible = (m % 4 == 0) && (K % m == 0);
