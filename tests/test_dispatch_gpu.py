@@ -95,6 +95,37 @@ def test_pair_tiles_shared_by_both_epilogue_groups(N, tiles):
     assert prep.device_status() == 0
 
 
+# SM pairs: fewer k-tiles than the rings hold (three with 512 rows a tile, four with 256), as many, and more; one tile a cluster and several. The
+# slots of the last round of the rings are not reported free, all others are.
+@pytest.mark.parametrize("ktiles", [1, 2, 3, 4, 5, 8])
+@pytest.mark.parametrize("tiles", [1, 2])
+@pytest.mark.parametrize("rows", [3, 4])
+def test_pair_kernel_ends_in_any_round_of_its_rings(rows, tiles, ktiles):
+    import torch
+    from venom_b200 import capi
+    from venom_b200.synth import random_vnm_dense_cuda
+    pairs = torch.cuda.get_device_properties(0).multi_processor_count // 2
+    tile_m = 256 if rows == 3 else 512
+    M, K, V, m, N = tile_m * (3 if tiles == 1 else pairs + 2), 128 * ktiles - 64, 32, 8, 216
+    dense, cols = random_vnm_dense_cuda(M, K, V, m, seed=M + K)
+    dense = torch.sign(dense) * torch.ceil(dense.abs() * 3)
+    values, meta, bad = capi.compress(dense, cols, V, m)
+    assert bad == 0
+    prep = capi.Prepared(values, meta, cols, M, K, V, m, strategy=capi.STRATEGY_DENSE_B)
+    prep.set_pair_mode(rows)
+    assert prep.config(N)["tile_m"] == tile_m
+    B = _ints((K, N), N)
+    want = (dense.float() @ B.float()).half()
+    for _ in range(20):      # launches of one shape behind one another, each beside the end of the one ahead
+        out = prep.spmm(B)
+        out_nk = prep.spmm_nk(B.T.contiguous())
+    assert torch.equal(out, want) and torch.equal(out_nk, want.T)
+    outs = [torch.empty((M, N), dtype=torch.float16, device="cuda") for _ in range(2)]
+    prep.spmm_multi(B, outs)
+    assert torch.equal(outs[0], want) and torch.equal(outs[1], want)
+    assert prep.device_status() == 0
+
+
 # Gather kernel: a last wave of at most half of the SMs has its tiles cut in two, a fuller one has not.  Column tiles that end inside
 # the first and the second half; more tiles than one a SM, so that whole and half tiles follow one another on it.
 @pytest.mark.parametrize("N", [96, 200, 256 + 72])

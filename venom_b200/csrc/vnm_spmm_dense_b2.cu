@@ -336,6 +336,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
             const uint32_t kb_step = b_nk ? 64u : 32u * 128u;  // bytes between the K=32 blocks of a stage
             int sa = 0;            // A slot and metadata set; the k-tile's B stages are slots STAGES_PER_KT * sa ...
             uint32_t ph = 0;       // phase of all of them
+            int left = total_it;   // k-tiles, this one included
             bool alive = true;
             for (int ti = 0; alive && ti < my_tiles; ++ti) {
                 // accumulator set: R = 2 both (phase ti), R = 1 set ti & 1 (phase ti / 2)
@@ -345,6 +346,9 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
                     if (kt == 0 && !wait_one(&acc_empty_bar[aset], aphase ^ 1u, abort_flag, p.status, DEV_TIMEOUT_MMA)) { alive = false; break; }
                     if (!wait_one(&a_full[sa], ph, abort_flag, p.status, DEV_TIMEOUT_MMA)) { alive = false; break; }  // both CTAs' blocks
                     tc_fence_after();
+                    // A slot is reported free only where a later k-tile will fill it: the peer leaves once the last accumulator is full and
+                    // stored, and an arrival that none of its threads waits for could come after that.
+                    const bool refilled = left > SA;
                     const uint32_t mcol = tmem_base + meta_col<R, BN>(sa);
                     const uint32_t aoff = (uint32_t)(sa * A_STAGE_BYTES) >> 4;
 #pragma unroll
@@ -372,13 +376,14 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
                                 tc_mma2_sp_f16(tmem_base + acc_col(R == 1 ? aset : rt), adesc0 + aoff + (uint32_t)((rt * AM_BLOCK_BYTES + kb * 32) >> 4), bdesc0 + boff,
                                                mcol + rt * 4 + (uint32_t)(kb & ~1), idesc0 | (uint32_t)(kb & 1), (kt | kb) != 0 ? 1u : 0u);
                             }
-                            if (rt == R - 1) tc_commit2(&b_free[sb]);
+                            if (rt == R - 1 && refilled) tc_commit2(&b_free[sb]);
                         }
                         if (!alive) break;
                         if (kt == p.ktiles - 1) tc_commit2(&acc_full_bar[R == 1 ? aset : rt]);
                     }
                     if (!alive) break;
-                    tc_commit2(&a_free[sa]);
+                    if (refilled) tc_commit2(&a_free[sa]);
+                    --left;
                     if (++sa == SA) { sa = 0; ph ^= 1; }
                 }
             }
@@ -519,7 +524,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
     if (MULTI && warp >= EPI_WARP0 && ((warp - EPI_WARP0) & 3) == 0 && lane == 0) bulk_wait_group_read0();  // this thread's TMA stores have read shared memory (their global writes complete with the grid)
     tc_fence_before();
     __syncthreads();
-    cluster_sync_all();  // the peer's shared and tensor memory stay alive until the leader's last MMA and commit are done
+    cluster_sync_all();  // the peer's shared and tensor memory stay alive until the leader's last MMA and commit are done: the epilogues have seen the last commit arrive
     if (warp == 3) {
         tc_fence_after();
         tmem_dealloc2(tmem_base, TMEM_COLS);
