@@ -120,9 +120,29 @@ def test_pair_kernel_ends_in_any_round_of_its_rings(rows, tiles, ktiles):
         out = prep.spmm(B)
         out_nk = prep.spmm_nk(B.T.contiguous())
     assert torch.equal(out, want) and torch.equal(out_nk, want.T)
-    outs = [torch.empty((M, N), dtype=torch.float16, device="cuda") for _ in range(2)]
-    prep.spmm_multi(B, outs)
-    assert torch.equal(outs[0], want) and torch.equal(outs[1], want)
+    assert prep.device_status() == 0
+
+
+# Several destinations: the last tile is staged in the operand rings, in slots that its last k-tile (any of them) was read from.
+@pytest.mark.parametrize("ktiles", [1, 2, 3, 4])
+@pytest.mark.parametrize("tiles", [1, 2])
+@pytest.mark.parametrize("rows", [3, 4])
+def test_last_tile_staged_in_the_rings(rows, tiles, ktiles):
+    import torch
+    from venom_b200 import capi
+    pairs = torch.cuda.get_device_properties(0).multi_processor_count // 2
+    M, K, V, m = 1024, 128 * ktiles, 64, 8
+    N = 240 * 2 if tiles == 1 else 240 * pairs
+    d, _, _, _, prep = _operand(M, K, V, m, capi.STRATEGY_DENSE_B, seed=K)
+    prep.set_pair_mode(rows)
+    B, bias = _ints((K, N), N), _ints((M,), 3)
+    want = (d @ B.float()).half()
+    for _ in range(10):
+        outs = [torch.zeros((M, N), dtype=torch.float16, device="cuda") for _ in range(2)]
+        outs_nm = [torch.zeros((N, M), dtype=torch.float16, device="cuda") for _ in range(2)]
+        prep.spmm_multi(B, outs)
+        prep.spmm_multi(B, outs_nm, bias=bias, layout=capi.VNM_LAYOUT_NM)
+        assert all(torch.equal(o, want) for o in outs) and all(torch.equal(o, (want + bias[:, None]).T) for o in outs_nm)
     assert prep.device_status() == 0
 
 

@@ -409,6 +409,11 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
             const bool got = wait_warp(&acc_full_bar[aset], R == 1 && !ONE ? (uint32_t)(ti >> 1) & 1u : (uint32_t)ti & 1u, abort_flag, p.status,
                                        DEV_TIMEOUT_EPILOGUE);
             if (MULTI ? !named_barrier_and(1 + grp, 128, got) : !got) break;
+            if constexpr (MULTI && R == 2) {
+                // the last tile is staged in the rings, which the MMAs of the other row tile read half a k-tile longer than those of the first
+                if (ti == my_tiles - 1 && grp == 0 &&
+                    !named_barrier_and(1 + grp, 128, wait_warp(&acc_full_bar[1], (uint32_t)ti & 1u, abort_flag, p.status, DEV_TIMEOUT_EPILOGUE))) break;
+            }
             tc_fence_after();
             {
                 const int rt = R == 1 ? 0 : grp;  // row tile of this CTA
@@ -465,7 +470,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
                 };
                 // Several destinations: one part -> staging buffer -> one TMA store for each (which clips at M and N).  In the CTA's last tile nothing hides the
                 // stores behind later MMAs any more, and the operand rings are idle (every load has landed and every MMA that
-                // read them has completed, or this tile's accumulator would not be full): each part then gets a buffer of its
+                // read them has completed, or this CTA's accumulators would not be full): each part then gets a buffer of its
                 // own inside the rings, so no part waits for the previous store to release the staging buffer (final epilogue 9.6k ->
                 // 6.5k clocks; laying the six parts side by side and storing the 128 x 240 image at once measured slower, 8.1k).
                 const bool last_tile = ti == my_tiles - 1;
