@@ -318,7 +318,9 @@ __global__ void __launch_bounds__(THREADS, 768 / THREADS) prune_candidates_kerne
     }
     if (m > 4 && m <= 4 * TASK_MAX_BLOCKS) {
         // ---- sums of the columns
-        __shared__ uint32_t s_sum[PRUNE_MAX_COLUMNS];
+        __shared__ uint4 s_sum4[PRUNE_MAX_COLUMNS / 4];      // read four at a time: the type aligns them
+        uint32_t *const s_sum = reinterpret_cast<uint32_t *>(s_sum4);
+        static_assert(PRUNE_MAX_COLUMNS % 4 == 0 && alignof(decltype(s_sum4)) == sizeof(uint4), "whole vectors, aligned whatever else is in shared memory");
         const Divisor by_mp(mp);
         for (int e = tid; e < ng * mp; e += THREADS) {
             const int g = by_mp.div(e);
@@ -355,7 +357,7 @@ __global__ void __launch_bounds__(THREADS, 768 / THREADS) prune_candidates_kerne
                     for (int j = 0; j < 4; j++) s2[i][j] = max2(t2, ds[j]) * p.one + s2[i][j];
                 }
             }
-            const uint4 sa = *reinterpret_cast<const uint4 *>(s_sum + g * mp + A);
+            const uint4 sa = s_sum4[(g * mp + A) / 4];
             const uint32_t sas[4] = {sa.x, sa.y, sa.z, sa.w};
             uint32_t mine = 0, valid = idx < ng * tasks && quantised(g) ? task >> 16 : 0u;
             if (m % 4 != 0) {                                // the last block's columns are not all there
