@@ -274,6 +274,22 @@ def _two_forms(M, K, V, m):
     return first[capi.STRATEGY_GATHER], first[capi.STRATEGY_DENSE_B]
 
 
+# Token counts that are no multiple of 16: the form that was measured to be the faster one by more than a tenth, where a product is mostly its start
+# (few tokens, gather form) and where the gathers of unaligned rows count (dense-B form); and a multiple of 16 beside each.
+@pytest.mark.parametrize("cfg", [(8192, 2048, 128, 16, 8, "gather"), (8192, 2048, 128, 16, 24, "gather"), (8192, 2048, 128, 16, 56, "gather"), (1024, 4096, 128, 16, 72, "gather"),
+                                 (1024, 4096, 128, 16, 136, "gather"), (36864, 12288, 128, 16, 8, "gather"), (36864, 12288, 128, 16, 40, "gather"), (12288, 4096, 128, 32, 104, "gather"),
+                                 (4096, 4096, 64, 32, 1368, "gather"), (12288, 12288, 128, 16, 1000, "gather"), (12288, 4096, 128, 8, 8, "dense_b"), (12288, 4096, 128, 8, 56, "dense_b"),
+                                 (8192, 12288, 32, 8, 8, "dense_b"), (8192, 12288, 32, 8, 24, "dense_b"), (12288, 12288, 64, 16, 520, "dense_b"), (6912, 3784, 128, 8, 8152, "dense_b"),
+                                 (8192, 2048, 128, 16, 32, "gather"), (36864, 12288, 128, 16, 48, "gather"), (8192, 12288, 32, 8, 64, "dense_b")])
+def test_form_of_a_layer_at_odd_token_counts(cfg):
+    import ctypes as C
+    from venom_b200 import capi
+    M, K, V, m, N, want = cfg
+    form = C.c_int()
+    assert capi.lib().vnm_choose_form(M, K, V, 2, m, N, 1, C.byref(form)) == 0
+    assert form.value == (capi.STRATEGY_GATHER if want == "gather" else capi.STRATEGY_DENSE_B)
+
+
 def _layer_of(values, meta, c, M, K, V, m):
     import torch
     from venom_b200.nmv import SrnmSpmm

@@ -807,16 +807,21 @@ int vnm_choose_form(int M, int K, int V, int n, int m, int N, int b_nk, int *str
     // at about 4.5 TB/s, and a launch)
     vnm_prepared_s h;
     float us[2] = {-1.0f, -1.0f};
+    Kernel kernel[2] = {KERNEL_GATHER, KERNEL_GATHER};
     for (int form = 0; form < 2; form++) {
         memset(&h, 0, sizeof(h));
         shape_handle(&h, M, K, V, n, m, form == 1);
-        Kernel kernel;
         SpmmConfig cfg;
-        if (!choose_kernel(&h, N, b_nk && form == 1, 0, &kernel, &cfg, &us[form])) us[form] = -1.0f;
+        if (!choose_kernel(&h, N, b_nk && form == 1, 0, &kernel[form], &cfg, &us[form])) us[form] = -1.0f;
     }
-    // rows of the transpose that do not start at a 32-byte sector: 128 gathered bytes are five sectors instead of four (6912 x 3784, 128:2:8, N = 8152,
-    // whose estimates are 194 and 196 us without this: 249 in gather form, 217 in dense-B form)
-    if (us[0] >= 0.0f && N % 16 != 0) us[0] *= 1.2f;
+    // Rows of the transpose that do not start at a 32-byte sector: a gathered piece reads a sector more (128 bytes five instead of four, the 32 of a
+    // 16-column tile two instead of one).  That slows the gathers, not the launch, first loads and epilogue, which are about the first 5 us of a product:
+    // beyond them N tokens against N + 8, 107 pairs of layers from 1024 x 1024 to 36864 x 12288, 8 to 8152 tokens: gather kernel 1.27 (0.9 to
+    // 1.6), kernel for few tiles 1.12 at V = 128, 1.27 at V = 64, 1.7 at V = 32 (0.84 to 2.3).  With 1.2 and 1.4 the form taken costs 1.012 of the
+    // faster one's time on average over 185 such layers, 1.20 at most; without them 1.029 and 2.1, with 1.2 on the whole product 1.019 and 1.22.  Gather / dense-B,
+    // us:  8192 x 2048, 128:2:16, 8 tokens 5.7 / 7.0;  12288 x 4096, 128:2:8, 8 tokens 14.4 / 11.7;  8192 x 12288, 32:2:8, 24 tokens 33.9 / 21.8;
+    // 6912 x 3784, 128:2:8, 8152 tokens 244 / 210;  4096 x 4096, 64:2:32, 1000 tokens 17.6 / 19.3.
+    if (us[0] > 5.0f && N % 16 != 0) us[0] += (us[0] - 5.0f) * (kernel[0] == KERNEL_SMALL ? 0.4f : 0.2f);
     if (us[0] >= 0.0f) us[0] += m == 4 ? 1e6f : 2.0f + 4.0f * (float)N * (float)K / 4.5e6f;
     *strategy = us[0] >= 0.0f && (us[1] < 0.0f || us[0] < us[1]) ? VNM_STRATEGY_GATHER : VNM_STRATEGY_DENSE_B;
     return VNM_OK;
