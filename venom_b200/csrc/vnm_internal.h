@@ -206,6 +206,31 @@ __device__ __forceinline__ void drain_slot(uint64_t *bar, uint32_t parity, int *
     atomicOr(status, DEV_TIMEOUT_DRAIN);
 }
 
+// Fill j of a ring goes to slot j % slots in phase j / slots.  The last of `fills` fills that slot `slot` got, or -1.
+__host__ __device__ constexpr int last_fill(int slot, int slots, int fills) { return fills > slot ? fills - 1 - (fills - 1 - slot) % slots : -1; }
+// Whatever the number of slots and fills: a fill of this slot, none of a later round beside it (whose phase has the parity that the wait for an
+// older one waits for, so that it never ends), and no slot forgotten.
+constexpr bool last_fill_holds()
+{
+    for (int slots = 2; slots <= 9; slots++)
+        for (int fills = 0; fills <= 3 * slots; fills++)
+            for (int slot = 0; slot < slots; slot++) {
+                const int j = last_fill(slot, slots, fills);
+                if (j < 0 ? fills > slot : j % slots != slot || j >= fills || j + slots < fills) return false;
+            }
+    return true;
+}
+static_assert(last_fill_holds(), "the fills that a drain waits for");
+
+// After an abort, one warp, when no other issues loads any more: waits until the last fill of every slot has landed.  Older ones have: their slot was free
+// again before it was refilled, whichever warp did that.
+__device__ __forceinline__ void drain_ring(uint64_t *full, int slots, int fills, int *status)
+{
+    const int lane = threadIdx.x & 31, j = lane < slots ? last_fill(lane, slots, fills) : -1;
+    if (j >= 0) drain_slot(&full[lane], (uint32_t)(j / slots) & 1u, status);
+    __syncwarp();
+}
+
 // ---- epilogue of one warp straight from tensor memory to global memory (32 accumulator lanes x BN columns) ----
 // Nothing of it passes through shared memory, whose port the mainloop needs: the operand reads of the MMAs and the TMA
 // writes of the rings together keep it busy all the time.  What the stores must not do is flood L2 with small pieces, behind

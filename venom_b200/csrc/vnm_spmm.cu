@@ -112,6 +112,7 @@ __global__ void __launch_bounds__(Traits<BN, NB>::NUM_THREADS, 1)
     uint64_t *acc_empty = acc_full + 2;    // [2]
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty + 2);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    int *b_fills = reinterpret_cast<int *>(tmem_slot + 2);   // B stages that a warp has issued loads of
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -125,6 +126,7 @@ __global__ void __launch_bounds__(Traits<BN, NB>::NUM_THREADS, 1)
         for (int s = 0; s < SB; s++) { mbar_init(&b_full[s], T::H * per_warp); mbar_init(&b_free[s], 1); }
         for (int a = 0; a < 2; a++) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], T::ACCS == 1 ? 8 : 4); }
         *abort_flag = 0;
+        *b_fills = 0;
         fence_barrier_init();
     }
     grid_dependency_wait();
@@ -253,12 +255,7 @@ __global__ void __launch_bounds__(Traits<BN, NB>::NUM_THREADS, 1)
             ++issued;
         }
         if (gmode == GATHER_CPASYNC) cp_async_wait_all();
-        if (*abort_flag && lane == 0 && gmode != GATHER_NONE) {   // this warp's copies still in flight: its stages of the last round of the ring
-            for (int back = 1; back <= (SB + ng - 1) / ng && back <= issued; back++) {
-                const int j = first + (issued - back) * ng;
-                drain_slot(&b_full[j % SB], (uint32_t)(j / SB) & 1u, p.status);
-            }
-        }
+        if (lane == 0 && issued > 0) atomicMax(b_fills, first + (issued - 1) * ng + 1);
         __syncwarp();
     } else if (warp == T::A_WARP) {
         // ---------------- A producer ----------------
@@ -419,6 +416,7 @@ __global__ void __launch_bounds__(Traits<BN, NB>::NUM_THREADS, 1)
 
     tc_fence_before();
     __syncthreads();
+    if (warp == 0 && *abort_flag) drain_ring(b_full, SB, *b_fills, p.status);
     if (warp == T::MMA_WARP) {
         tc_fence_after();
         tmem_dealloc(tmem_base, T::TMEM_COLS);

@@ -85,8 +85,9 @@ __global__ void __launch_bounds__(Small<BN, NB, DEEP>::NUM_THREADS, 2)
     uint64_t *acc_full = freed + S;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_full + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    int *fills = reinterpret_cast<int *>(tmem_slot + 2);      // k-tiles that a warp has issued loads of
     float *red = reinterpret_cast<float *>(smem);
-    static_assert(T::B_BYTES % 1024 == 0 && (2 * S + 1) * 8 + 8 <= 256, "shared-memory plan");
+    static_assert(T::B_BYTES % 1024 == 0 && (2 * S + 1) * 8 + 12 <= 256, "shared-memory plan");
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -106,6 +107,7 @@ __global__ void __launch_bounds__(Small<BN, NB, DEEP>::NUM_THREADS, 2)
         }
         mbar_init(acc_full, 1);
         *abort_flag = 0;
+        *fills = 0;
         fence_barrier_init();
     }
     if (!p.early) grid_dependency_wait();
@@ -170,8 +172,7 @@ __global__ void __launch_bounds__(Small<BN, NB, DEEP>::NUM_THREADS, 2)
                     if (++s == S) { s = 0; ph ^= 1; }
                 }
             }
-            if (*abort_flag && lane == 0)
-                for (int k = kt - k0 > S ? kt - k0 - S : 0; k < kt - k0; ++k) drain_slot(&full[k % S], (uint32_t)(k / S) & 1u, p.status);
+            if (lane == 0) atomicMax(fills, kt - k0);
         } else if (warp < 2 && elect_one()) {
             tma_prefetch_desc(&tmap_b);
             int s = warp;
@@ -192,8 +193,7 @@ __global__ void __launch_bounds__(Small<BN, NB, DEEP>::NUM_THREADS, 2)
                 }
                 if ((s += 2) >= S) { s -= S; ph ^= 1; }
             }
-            if (*abort_flag && mode != GATHER_NONE)
-                for (int k = kt - k0 > S + 1 ? kt - k0 - (S + 1) / 2 * 2 : warp; k < kt - k0; k += 2) drain_slot(&full[k % S], (uint32_t)(k / S) & 1u, p.status);
+            atomicMax(fills, kt - k0 - 1);
         }
         __syncwarp();
     } else if (warp == T::A_WARP || (T::A_WARPS == 2 && warp == T::A_WARP2)) {
@@ -211,8 +211,7 @@ __global__ void __launch_bounds__(Small<BN, NB, DEEP>::NUM_THREADS, 2)
                 bulk_g2s(a_ring + s * AM_BLOCK_BYTES, src + (size_t)kt * AM_BLOCK_BYTES, AM_BLOCK_BYTES, &full[s]);
                 if ((s += step) >= S) { s -= S; ph ^= 1; }
             }
-            if (*abort_flag)
-                for (int k = kt - k0 > S + 1 ? kt - k0 - (S + 1) / step * step : half; k < kt - k0; k += step) drain_slot(&full[k % S], (uint32_t)(k / S) & 1u, p.status);
+            atomicMax(fills, kt - k0 - step + 1);
         }
         __syncwarp();
     } else if (warp == T::MMA_WARP) {
@@ -326,6 +325,7 @@ __global__ void __launch_bounds__(Small<BN, NB, DEEP>::NUM_THREADS, 2)
     }
     tc_fence_before();
     __syncthreads();
+    if (warp == 0 && *abort_flag) drain_ring(full, S, *fills, p.status);
     if (warp == T::MMA_WARP) {
         tc_fence_after();
         tmem_dealloc(tmem_base, T::TMEM_COLS);
