@@ -72,6 +72,7 @@ struct SpmmConfig {
     int grid;    // CTAs (persistent ones, except in the small kernel)
     int split;   // small kernel: CTAs that share a tile's k-tiles
     int resident;  // small kernel: CTAs per SM
+    int deep;      // small kernel: the instance whose ring takes an SM's whole shared memory
     int tiles;     // gather kernel: tiles of the launch, halves counted
     int cut_from;  // gather kernel: first of the tiles that are cut in two (`tiles`: none)
 };

@@ -45,7 +45,8 @@ struct Small {
     static constexpr int RED_BYTES = (BN + 8) * TILE_M * 4;   // split over K: this CTA's columns from every rank (8: its share is rounded up); in the idle rings
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 256 + 1024;
     static_assert(SMEM_BYTES <= 227 * 1024 && (BN > 64 || RED_BYTES <= STAGES * STAGE_BYTES), "shared memory per CTA");
-    static constexpr int CTAS = !DEEP && 2 * (SMEM_BYTES + 1024) <= 227 * 1024 ? 2 : 1;   // resident per SM
+    static constexpr bool TWO_FIT = 2 * (SMEM_BYTES + 1024) <= 227 * 1024;
+    static constexpr int CTAS = !DEEP && TWO_FIT ? 2 : 1;     // resident per SM
     static constexpr int A_WARP = PW, MMA_WARP = PW + 1, A_WARP2 = PW + 2, EPI_WARP0 = 12;
     static constexpr int A_WARPS = DEEP ? 2 : 1;              // warps that load A
     static constexpr int NUM_THREADS = 16 * 32;
@@ -75,6 +76,7 @@ __global__ void __launch_bounds__(Small<BN, NB, DEEP>::NUM_THREADS, 2)
     spmm_small_kernel(const __grid_constant__ CUtensorMap tmap_b, const SpmmParams p)
 {
     using T = Small<BN, NB, DEEP>;
+    static_assert(DEEP || T::TWO_FIT, "a CTA that has its SM to itself runs the deep instance");
     constexpr int S = T::STAGES;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -351,20 +353,33 @@ __global__ void wait_expiry_selftest_kernel(int *status)
     __syncthreads();
 }
 
+// The deep instance is the only one of a tile whose ring never lets a second CTA on the SM (64 columns of four blocks).
+template <int BN, int NB>
+constexpr bool only_deep = !Small<BN, NB, false>::TWO_FIT;
+
+template <int BN, int NB, bool DEEP>
+cudaError_t init_instance()
+{
+    return cudaFuncSetAttribute(spmm_small_kernel<BN, NB, DEEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, Small<BN, NB, DEEP>::SMEM_BYTES);
+}
 template <int BN, int NB>
 cudaError_t init_one()
 {
-    const cudaError_t e = cudaFuncSetAttribute(spmm_small_kernel<BN, NB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Small<BN, NB, false>::SMEM_BYTES);
-    return e == cudaSuccess ? cudaFuncSetAttribute(spmm_small_kernel<BN, NB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Small<BN, NB, true>::SMEM_BYTES) : e;
+    if constexpr (!only_deep<BN, NB>) {
+        const cudaError_t e = init_instance<BN, NB, false>();
+        if (e != cudaSuccess) return e;
+    }
+    return init_instance<BN, NB, true>();
 }
 
-template <int BN, int NB>
-cudaError_t launch_one(const SpmmConfig &cfg, const CUtensorMap &tmap_b, const SpmmParams &p, cudaStream_t stream)
+template <int BN, int NB, bool DEEP>
+cudaError_t launch_instance(const SpmmConfig &cfg, const CUtensorMap &tmap_b, const SpmmParams &p, cudaStream_t stream)
 {
+    using T = Small<BN, NB, DEEP>;
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3((unsigned)cfg.grid, 1, 1);
-    lc.blockDim = dim3(Small<BN, NB, false>::NUM_THREADS, 1, 1);
-    lc.dynamicSmemBytes = (size_t)cfg.smem_bytes;
+    lc.blockDim = dim3(T::NUM_THREADS, 1, 1);
+    lc.dynamicSmemBytes = T::SMEM_BYTES;
     lc.stream = stream;
     cudaLaunchAttribute attr[2];
     lc.attrs = attr;
@@ -376,16 +391,27 @@ cudaError_t launch_one(const SpmmConfig &cfg, const CUtensorMap &tmap_b, const S
         attr[lc.numAttrs++].val.clusterDim.z = 1;
     }
     attr[lc.numAttrs++] = early_launch();
-    return cfg.resident == 1 ? cudaLaunchKernelEx(&lc, spmm_small_kernel<BN, NB, true>, tmap_b, p) : cudaLaunchKernelEx(&lc, spmm_small_kernel<BN, NB, false>, tmap_b, p);
+    return cudaLaunchKernelEx(&lc, spmm_small_kernel<BN, NB, DEEP>, tmap_b, p);
+}
+template <int BN, int NB>
+cudaError_t launch_one(const SpmmConfig &cfg, const CUtensorMap &tmap_b, const SpmmParams &p, cudaStream_t stream)
+{
+    if constexpr (!only_deep<BN, NB>) {
+        if (!cfg.deep) return launch_instance<BN, NB, false>(cfg, tmap_b, p, stream);
+    }
+    return launch_instance<BN, NB, true>(cfg, tmap_b, p, stream);
 }
 
-// The instance for a grid: the deep ring where every CTA has an SM to itself.
+// What a grid of the deep instance, or of the one that shares an SM, takes.
 template <int BN, int NB>
 void fill(SpmmConfig *cfg, bool deep)
 {
-    cfg->smem_bytes = deep ? Small<BN, NB, true>::SMEM_BYTES : Small<BN, NB, false>::SMEM_BYTES;
-    cfg->threads = Small<BN, NB, false>::NUM_THREADS;
-    cfg->resident = deep ? Small<BN, NB, true>::CTAS : Small<BN, NB, false>::CTAS;
+    using Deep = Small<BN, NB, true>;
+    using Shared = Small<BN, NB, false>;
+    cfg->deep = deep || only_deep<BN, NB>;
+    cfg->smem_bytes = cfg->deep ? Deep::SMEM_BYTES : Shared::SMEM_BYTES;
+    cfg->threads = Deep::NUM_THREADS;
+    cfg->resident = cfg->deep ? Deep::CTAS : Shared::CTAS;
 }
 
 #define VNM_SMALL_DISPATCH(bn, nb, CALL)                                                                                  \
