@@ -405,22 +405,12 @@ __device__ __forceinline__ void store_tile(const Store &st, Release release)
         uint32_t pk[CHUNKS][32];
 #pragma unroll
         for (int k = 0; k < CHUNKS; k++) {
-            if (BN > 128 || k == 0) {
-                uint32_t v0[32], v1[32];   // both groups in flight before the wait: the next tile's MMAs wait for this
-                tc_ld_16x256b(st.taddr + (uint32_t)(64 * k), v0);
-                tc_ld_16x256b(st.taddr + (16u << 16) + (uint32_t)(64 * k), v1);
-                tc_wait_ld();
-                Store::pack(v0, pk[k]);
-                Store::pack(v1, pk[k] + 16);
-            } else {                       // kernels of fewer registers: one after the other
-#pragma unroll
-                for (int g = 0; g < 2; g++) {
-                    uint32_t v[32];
-                    tc_ld_16x256b(st.taddr + ((uint32_t)(16 * g) << 16) + (uint32_t)(64 * k), v);
-                    tc_wait_ld();
-                    Store::pack(v, pk[k] + 16 * g);
-                }
-            }
+            uint32_t v0[32], v1[32];   // both groups in flight before the wait: the next tile's MMAs wait for this
+            tc_ld_16x256b(st.taddr + (uint32_t)(64 * k), v0);
+            tc_ld_16x256b(st.taddr + (16u << 16) + (uint32_t)(64 * k), v1);
+            tc_wait_ld();
+            Store::pack(v0, pk[k]);
+            Store::pack(v1, pk[k] + 16);
         }
         release();
 #pragma unroll
