@@ -647,7 +647,8 @@ cudaError_t launch_candidates(PruneParams p, cudaStream_t stream)
     const size_t smem = prune_smem_bytes(p.V, p.m, p.G, elem);
     const unsigned blocks = (unsigned)((p.M / p.V) * ((p.Ksp / 2 + p.G - 1) / p.G));
     // 128 threads: five or six CTAs of an SM are in different phases and their tasks fill the warps better (12288 x 12288, m = 16, V = 32: 2044 us, with
-    // 256 threads 2411, before the last change of the loop).  With few CTAs 256 (1024 x 1024, m = 32, V = 128: 235, with 128 threads 296).
+    // 256 threads 2411, before the last change of the loop).  With fewer than four CTAs for each of a B200's 148 SMs 256 (1024 x 1024, m = 32, V = 128: 235, with
+    // 128 threads 296); where exactly the line lies was not measured.
     const bool few = blocks < 4 * 148;
     auto launch = [&](auto kernel, int threads) -> cudaError_t {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);

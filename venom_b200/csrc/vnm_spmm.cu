@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(Traits<BN, NB>::NUM_THREADS, 1)
     } else if (warp >= T::EPI_WARP0) {
         // ---------------- epilogue ----------------
         constexpr int PART = T::PART;
-        const int grp = (warp - T::EPI_WARP0) >> 2;     // drains the tiles ti with ti & 1 == grp
+        const int grp = (warp - T::EPI_WARP0) >> 2;     // one accumulator: drains its half of every tile's columns; two: the tiles ti with ti & 1 == grp
         const int q = warp & 3;                         // tensor-memory lane quadrant this warp may read
         const int arow = mma_row_to_actual(q * 32 + lane);
         const bool leader = ((warp - T::EPI_WARP0) & 3) == 0 && lane == 0;
@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(Traits<BN, NB>::NUM_THREADS, 1)
             int mt, n0, slices;
             locate_tile(tile, &mt, &n0, &slices);
             const int aset = T::ACCS == 1 ? 0 : grp;
-            // the four warps of a group leave the loop together (they meet at named barriers below)
+            // with stores through shared memory the four warps of a group leave the loop together (they meet at named barriers below)
             const bool got = wait_warp(&acc_full[aset], (uint32_t)(T::ACCS == 1 ? ti : ti >> 1) & 1u, abort_flag, p.status, DEV_TIMEOUT_EPILOGUE);
             if (p.tma_out ? !named_barrier_and(1 + grp, 128, got) : !got) break;
             tc_fence_after();

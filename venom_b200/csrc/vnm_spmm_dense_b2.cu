@@ -405,7 +405,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) spmm_dense_b_pair_kernel(const
             int mq, nt;
             tile_coords(tile, mquads, p.ntiles, p.group_m, &mq, &nt);
             const int n0 = nt * BN;
-            // the four warps of a group leave the loop together (they meet at named barriers below)
+            // with several destinations the four warps of a group leave the loop together (they meet at named barriers below)
             const bool got = wait_warp(&acc_full_bar[aset], R == 1 && !ONE ? (uint32_t)(ti >> 1) & 1u : (uint32_t)ti & 1u, abort_flag, p.status,
                                        DEV_TIMEOUT_EPILOGUE);
             if (MULTI ? !named_barrier_and(1 + grp, 128, got) : !got) break;
