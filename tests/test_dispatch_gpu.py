@@ -147,7 +147,8 @@ def test_last_tile_staged_in_the_rings(rows, tiles, ktiles):
 
 
 # Gather kernel: a last wave of at most half of the SMs has its tiles cut in two, a fuller one has not.  Column tiles that end inside
-# the first and the second half; more tiles than one a SM, so that whole and half tiles follow one another on it.
+# the first and the second half; more tiles than one a SM, so that whole and half tiles follow one another on it; five k-tiles a tile or more, the
+# last one ragged, so that the rings go round and half-filled stages take the slots of whole ones.
 @pytest.mark.parametrize("N", [96, 200, 256 + 72])
 @pytest.mark.parametrize("rest", ["few", "one", "half", "more"])
 @pytest.mark.parametrize("cfg", [(128, 16), (64, 16), (32, 8)])
@@ -160,15 +161,22 @@ def test_last_tiles_cut_in_two(cfg, rest, N):
     bn = {128: 256, 64: 128, 32: 64}[V]
     ntiles = -(-N // bn)
     want_tiles = {"few": 5, "one": sms + 1, "half": sms + sms // 2, "more": sms + sms // 2 + 3}[rest]
-    M, K = 128 * -(-want_tiles // ntiles), 320
+    M, K = 128 * -(-want_tiles // ntiles), 32 * m * 4 + 320
     dense, cols = random_vnm_dense_cuda(M, K, V, m, seed=M + N)
     dense = torch.sign(dense) * torch.ceil(dense.abs() * 3)
     values, meta, bad = capi.compress(dense, cols, V, m)
     assert bad == 0
     prep = capi.Prepared(values, meta, cols, M, K, V, m, strategy=capi.STRATEGY_GATHER)
     prep.set_pair_mode(3)   # not the kernel for few tiles
+    tiles = M // 128 * ntiles
+    cut = V != 32 and 0 < tiles % sms <= sms // 2
+    assert cut == (V != 32 and rest != "more")
+    assert prep.config(N)["grid"] == min(sms, tiles + (tiles % sms if cut else 0))
     B, bias = _ints((K, N), N), _ints((M,), 3)
     want = (dense.float() @ B.float()).half()
+    outs = [torch.zeros((N, M), dtype=torch.float16, device="cuda") for _ in range(2)]
+    prep.spmm_multi(B, outs, bias=bias, layout=capi.VNM_LAYOUT_NM)
+    assert all(torch.equal(o, (want + bias[:, None]).T) for o in outs)
     for mode in (0, 2):     # stores from tensor memory, through shared memory
         prep.set_epilogue(mode)
         assert torch.equal(prep.spmm(B), want)
