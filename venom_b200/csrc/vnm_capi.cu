@@ -160,7 +160,7 @@ int ensure_kernels_ready(int *device_out)
 //     718 / 926, 11.8 / 15.2 ms.)  Calls of two forms in turn each run at the clock that the other one left behind, so forms are compared by themselves.
 //   V = 128, m = 8, fewer rows: the line at 1024 is older than these figures (9.9 / 13.8 at 128 x 4096, 22.3 / 22.4 at 512 x 4096, 9.6 / 9.9 at 768 x
 //     512, N = 8192).
-//   4096 x 4096, N = 16384:  m = 4 520 / 259;  V = 128: m = 16 121 / 238;  V = 64: m = 8 349 / 246, m = 16 193 / 238, m = 32 116 / 234;  V = 32:
+//   4096 x 4096, N = 16384:  m = 4, V = 128 333 / 259 (V = 64 630, V = 32 1373);  V = 128: m = 16 121 / 238;  V = 64: m = 8 349 / 246, m = 16 193 / 238, m = 32 116 / 234;  V = 32:
 //     m = 16 376 / 239, m = 32 208 / 235, m = 64 121 / 232.  The lines that leave V = 64, m = 16 and V = 32, m = 32 to the dense-B form are older than
 //     these figures, too; they stay, because an operand's form decides which calls it takes ([N,K] activations without a workspace).
 bool choose_dense_b(int M, int K, int V, int m, int strategy)
@@ -522,7 +522,7 @@ bool choose_kernel(vnm_handle_t h, int N, int b_nk, int n_more, Kernel *kernel, 
     memset(cfg, 0, sizeof(*cfg));
     float big = -1.0f;
     if (!h->dense_b) {
-        big = spmm_select_config(h->V, N, h->M, h->ktiles, h->max_ctas, h->gather_mode == GATHER_TMA4, cfg);
+        big = spmm_select_config(h->V, N, h->M, h->ktiles, h->max_ctas, h->gather_mode, cfg);
         cfg->stages = h->producer_warps;
         *kernel = KERNEL_GATHER;
     } else {
@@ -533,7 +533,7 @@ bool choose_kernel(vnm_handle_t h, int N, int b_nk, int n_more, Kernel *kernel, 
     // The small kernel has one destination, no cap on its CTAs (it is not persistent) and none of the other kernels' ablations.
     if (n_more == 0 && h->max_ctas == 0 && !h->nm_tma_always && !h->out32 && h->producer_warps == GATHER_PRODUCER_WARPS && h->pair_rows == 0 && h->gather_mode != GATHER_CPASYNC) {
         SpmmConfig small_cfg;
-        const float small = spmm_small_config(h->mtiles, h->ktiles, N, h->nb, h->gather_mode == GATHER_TMA4, &small_cfg);
+        const float small = spmm_small_config(h->mtiles, h->ktiles, N, h->nb, h->gather_mode == GATHER_TMA4, !h->dense_b && h->gather_mode == GATHER_CONTIG, &small_cfg);
         // up to SMALL_SPLIT_N columns it alone is used: its split makes the order of summation its own
         if (N <= SMALL_SPLIT_N || big < 0.0f || small < big) {
             *cfg = small_cfg;

@@ -108,7 +108,7 @@ cudaError_t launch_sparsify(const void *w, bool half, int64_t ldw, int M, int K,
 
 // Tile configuration of the gather kernel.
 constexpr int GATHER_PRODUCER_WARPS = 16;   // all of them, in the units of vnm_set_producer_warps
-float spmm_select_config(int V, int N, int M, int ktiles, int max_ctas, bool may_cut, SpmmConfig *cfg);  // max_ctas: 0 = one per SM; may_cut: the last tiles, in two; returns an estimate in microseconds, < 0 for an unsupported V
+float spmm_select_config(int V, int N, int M, int ktiles, int max_ctas, int gather_mode, SpmmConfig *cfg);  // max_ctas: 0 = one per SM; returns an estimate in microseconds, < 0 for an unsupported V
 // Opt-in to large dynamic shared memory for every kernel instance on the CURRENT device (call once per device).
 cudaError_t spmm_init_kernels();
 cudaError_t launch_spmm(const SpmmConfig &cfg, const CUtensorMap &tmap_rows, const CUtensorMap &tmap_tile, const CUtensorMap &tmap_out,
@@ -120,7 +120,7 @@ cudaError_t launch_spmm(const SpmmConfig &cfg, const CUtensorMap &tmap_rows, con
 constexpr int SMALL_SPLIT_N = 64;
 cudaError_t spmm_small_init();
 cudaError_t launch_wait_expiry_selftest(int *status, cudaStream_t stream);
-float spmm_small_config(int mtiles, int ktiles, int N, int nb, bool gather, SpmmConfig *cfg);   // returns its estimate in microseconds
+float spmm_small_config(int mtiles, int ktiles, int N, int nb, bool gather, bool every_row, SpmmConfig *cfg);   // returns its estimate in microseconds
 CUresult spmm_small_encode(EncodeTiledFn enc, CUtensorMap *map, const void *B, int64_t ldb, int K, int N, int b_nk, int gather_mode, int bn);
 cudaError_t launch_spmm_small(const SpmmConfig &cfg, const CUtensorMap &tmap_b, const SpmmParams &p, cudaStream_t stream);
 

@@ -115,7 +115,7 @@ extern "C" int vnm_spmm_f16_noalloc(const void *values, const uint32_t *meta, co
     if (e != cudaSuccess) return nfail(VNM_ERR_CUDA, "re-pack launch: %s", cudaGetErrorString(e));
 
     SpmmConfig cfg;
-    if (spmm_select_config(V, N, M, ktiles, 0, m != 4, &cfg) < 0.0f) return nfail(VNM_ERR_UNSUPPORTED, "unsupported V");
+    if (spmm_select_config(V, N, M, ktiles, 0, m == 4 ? GATHER_CONTIG : GATHER_TMA4, &cfg) < 0.0f) return nfail(VNM_ERR_UNSUPPORTED, "unsupported V");
     EncodeTiledFn enc = get_encode_fn();
     if (!enc) return nfail(VNM_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
     CUtensorMap tmap_rows, tmap_tile;

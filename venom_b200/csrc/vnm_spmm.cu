@@ -455,12 +455,15 @@ int g_num_sms = 0;
 // 4096 x 12288, m = 8, N = 4096 (68 beyond three) 165.9 (152.8), 160.5 (144.1);  12288 x 12288, V = 64, m = 32, N = 2048 (56 beyond ten) 114.6
 // (110.9), 113.0 (108.7).  More than half (124 beyond 13 waves, 4096 x 4096, m = 8, N = 16384), which makes two waves of halves: 217.0, 221.2.
 //
-// The estimate, in us: start-up and last epilogue, then per wave a k-tile's 1330 clocks and what a tile change costs.  It is 0.97 to 1.03 of a call
-// after a pause from 8 k-tiles a tile and 3 waves on.
+// The estimate, in us: start-up and last epilogue, then per wave a k-tile's time (0.76 us: 1340 clocks at the 1760 MHz of a call among many) and what a tile
+// change costs.  Calls among many take 0.93 to 1.16 of it (ten sizes from 62 us to 14 ms, V = 128, 64 and 32; after a pause less, at the full clock).  With
+// boxes of rows instead of gathers (m = 4) a line of its own for each V, fitted to 168 sizes of 512 to 12288 rows and k and 256 to 16384 columns: between this
+// kernel and the one for few tiles the faster one is taken but for 1.08 of its time at most beyond 12 us.  (With the cost of gathers up to 1.72: 4096 x 4096,
+// 128:2:4, N = 16384 took 565 us in the other kernel and takes 333 in this one.)
 //
 // Tile configurations: V=128 -> one block per tile, BN 256; V=64 -> two blocks, BN 128; V=32 -> four blocks, BN 64 (NB * BN = 256:
 // every B stage is 16 KiB).
-float spmm_select_config(int V, int N, int M, int ktiles, int max_ctas, bool may_cut, SpmmConfig *cfg)
+float spmm_select_config(int V, int N, int M, int ktiles, int max_ctas, int gather_mode, SpmmConfig *cfg)
 {
     const int mtiles = (M + TILE_M - 1) / TILE_M;
     cfg->stages = GATHER_PRODUCER_WARPS;
@@ -480,10 +483,15 @@ float spmm_select_config(int V, int N, int M, int ktiles, int max_ctas, bool may
     if (max_ctas > 0 && max_ctas < sms) sms = max_ctas;  // the caller keeps some SMs free (e.g. for a collective that runs beside the product)
     const long long waves = tiles / sms;
     const int rest = (int)(tiles - waves * sms);
-    const bool cut = may_cut && cfg->bn > 64 && rest > 0 && 2 * rest <= sms;
+    const bool cut = gather_mode == GATHER_TMA4 && cfg->bn > 64 && rest > 0 && 2 * rest <= sms;
     cfg->tiles = (int)tiles + (cut ? rest : 0);
     cfg->cut_from = cut ? (int)(waves * sms) : cfg->tiles;
     cfg->grid = cfg->tiles < sms ? cfg->tiles : sms;
+    if (gather_mode == GATHER_CONTIG) {
+        static const float kt_us[3] = {0.58f, 0.645f, 0.76f}, tile_us[3] = {1.9f, 0.8f, 0.3f};   // 1, 2 and 4 vector blocks
+        const int i = V == 128 ? 0 : V == 64 ? 1 : 2;
+        return 4.6f + (float)(waves + (rest != 0)) * (ktiles * kt_us[i] + tile_us[i]);
+    }
     return 5.5f + ((float)waves + (rest == 0 ? 0.0f : cut ? 0.65f : 1.0f)) * (V == 128 ? ktiles * 0.76f + 1.7f : ktiles * 0.68f + 1.35f);
 }
 

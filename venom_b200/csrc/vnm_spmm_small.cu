@@ -447,9 +447,10 @@ cudaError_t spmm_small_init()
 // the exchange of a split; a second CTA on an SM costs its set-up and shares the port; clusters of more than four do not
 // fill the last SMs of a GPC; and A cannot be read faster than HBM delivers it.  The choice takes 1.006 of the fastest one's time on average, 1.06 at most,
 // over 42 shapes (the fit to older kernels took 1.06 and 1.34: 14.2 us split by 3 instead of 10.6 by 2 at 12288 x 12288, 128:2:16, N = 16, 7.1 split by 8
-// instead of 5.5 by 4 at 1024 x 4096, 64:2:8, N = 64).  Only up to SMALL_SPLIT_N columns are k-tiles split: beyond, the
+// instead of 5.5 by 4 at 1024 x 4096, 64:2:8, N = 64).  Operands of every row (m = 4 in gather form) in several waves, where each vector block of a tile reads the
+// same rows of B again, take 1.23, 1.40 and 1.66 of that fit on average and up to 2.4 (1, 2 and 4 blocks, 113 sizes), which is added beyond SMALL_SPLIT_N columns.  Only up to SMALL_SPLIT_N columns are k-tiles split: beyond, the
 // order of summation stays that of the other kernels, so that results do not depend on how a caller cuts its columns.
-float spmm_small_config(int mtiles, int ktiles, int N, int nb, bool gather, SpmmConfig *cfg)
+float spmm_small_config(int mtiles, int ktiles, int N, int nb, bool gather, bool every_row, SpmmConfig *cfg)
 {
     const int sms = g_num_sms_small > 0 ? g_num_sms_small : 148;
     static const int widths[4] = {16, 32, 64, 128};
@@ -477,7 +478,7 @@ float spmm_small_config(int mtiles, int ktiles, int N, int nb, bool gather, Spmm
             float t = fixed[w] + (nb == 4 ? 1.0f : nb == 2 ? 0.2f : 0.0f);
             if (split > 1) t += 0.25f + 0.016f * bn + 0.004f * (float)(ctas < sms ? ctas : sms);
             if (one_each) t += kts * kt_us * (1.0f + (gather ? 0.1f * ctas / sms : 0.0f));
-            else t += ceilf((float)ctas / fit) * (kts * kt_us * 1.45f + 2.0f);
+            else t += ceilf((float)ctas / fit) * (kts * kt_us * (every_row && N > SMALL_SPLIT_N ? 1.45f + 0.36f * nb : 1.45f) + 2.0f);
             const float hbm = 3.5f + a_bytes / (gather && one_each ? 4.2e6f : 5.6e6f);
             t = (t > hbm ? t : hbm) + 0.05f * t;
             if (t < best) {
