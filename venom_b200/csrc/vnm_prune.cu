@@ -209,13 +209,14 @@ struct Divisor {
 };
 __device__ __forceinline__ uint32_t halves_sum(uint32_t x) { return (x & 0xFFFFu) + (x >> 16); }
 
-// M_: m where it is known at compile time (8, 16, 32), else 0
+// M_: m where it is known at compile time (8, 16, 32), 0 for any m up to 32, LARGER_M beyond, whose loop needs fewer registers
+constexpr int LARGER_M = -1;
 template <int WT, bool FUSED, int M_, int THREADS>
-__global__ void __launch_bounds__(THREADS, 768 / THREADS) prune_candidates_kernel(const PruneParams p)
+__global__ void __launch_bounds__(THREADS, M_ == LARGER_M ? 1 : 768 / THREADS) prune_candidates_kernel(const PruneParams p)
 {
     using W = typename WeightOf<WT>::T;
     extern __shared__ __align__(16) uint8_t psm[];
-    const int V = p.V, m = M_ ? M_ : p.m, mp = M_ ? M_ : p.mp, G = p.G;
+    const int V = p.V, m = M_ > 0 ? M_ : p.m, mp = M_ > 0 ? M_ : p.mp, G = p.G;
     uint32_t *q = reinterpret_cast<uint32_t *>(psm);                        // [G][V / 2][mp] pairs of rows
     W *tile = reinterpret_cast<W *>(q + (size_t)G * (V / 2) * mp);          // [V][pitch] weights
     PruneGroup *grp = reinterpret_cast<PruneGroup *>(tile + (size_t)V * p.pitch);
@@ -316,7 +317,7 @@ __global__ void __launch_bounds__(THREADS, 768 / THREADS) prune_candidates_kerne
         }
         __syncthreads();
     }
-    if (m > 4 && m <= 4 * TASK_MAX_BLOCKS) {
+    if (M_ != LARGER_M && m > 4) {
         // ---- sums of the columns
         __shared__ uint4 s_sum4[PRUNE_MAX_COLUMNS / 4];      // read four at a time: the type aligns them
         uint32_t *const s_sum = reinterpret_cast<uint32_t *>(s_sum4);
@@ -395,7 +396,7 @@ __global__ void __launch_bounds__(THREADS, 768 / THREADS) prune_candidates_kerne
     }
     // ---- larger m: a warp takes 32 tasks of one group at a time
     int tasks = 0;                 // (c, b, pair of a, four of d): floor(c^2 / 4) pairs (b, a pair) for every c
-    if (M_ == 0 && m > 4 * TASK_MAX_BLOCKS)
+    if (M_ == LARGER_M)
         for (int c = 2; c <= m - 2; c++) tasks += (mp / 4 - (c + 1) / 4) * (c * c / 4);
     const int wtasks = (tasks + 31) / 32;
     for (int wt = warp; wt < ng * wtasks; wt += THREADS / 32) {
@@ -664,7 +665,11 @@ cudaError_t launch_candidates(PruneParams p, cudaStream_t stream)
     case 8: return either(std::integral_constant<int, 8>());
     case 16: return either(std::integral_constant<int, 16>());
     case 32: return either(std::integral_constant<int, 32>());
-    default: return either(std::integral_constant<int, 0>());
+    default:
+        // larger m: an instance with the registers that its loop needs, and 256 threads: 4096 x 4096, fp32, V = 64, m = 64 22.2 ms (29.2 with 128 threads and
+        // the registers of the other loop), fp16, V = 64, m = 40 4.91 (5.52), V = 32, m = 64 29.2 (31.1)
+        if (p.m > 4 * TASK_MAX_BLOCKS) return launch(prune_candidates_kernel<WT, FUSED, LARGER_M, 256>, 256);
+        return either(std::integral_constant<int, 0>());
     }
 }
 
