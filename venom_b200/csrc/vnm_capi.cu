@@ -533,7 +533,7 @@ bool choose_kernel(vnm_handle_t h, int N, int b_nk, int n_more, Kernel *kernel, 
     // The small kernel has one destination, no cap on its CTAs (it is not persistent) and none of the other kernels' ablations.
     if (n_more == 0 && h->max_ctas == 0 && !h->nm_tma_always && !h->out32 && h->producer_warps == GATHER_PRODUCER_WARPS && h->pair_rows == 0 && h->gather_mode != GATHER_CPASYNC) {
         SpmmConfig small_cfg;
-        const float small = spmm_small_config(h->mtiles, h->ktiles, N, h->nb, h->gather_mode == GATHER_TMA4, !h->dense_b && h->gather_mode == GATHER_CONTIG, &small_cfg);
+        const float small = spmm_small_config(h->mtiles, h->ktiles, N, h->nb, h->gather_mode == GATHER_TMA4, !h->dense_b && h->gather_mode == GATHER_CONTIG, b_nk != 0, &small_cfg);
         // up to SMALL_SPLIT_N columns it alone is used: its split makes the order of summation its own
         if (N <= SMALL_SPLIT_N || big < 0.0f || small < big) {
             *cfg = small_cfg;

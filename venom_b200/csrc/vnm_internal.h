@@ -120,7 +120,7 @@ cudaError_t launch_spmm(const SpmmConfig &cfg, const CUtensorMap &tmap_rows, con
 constexpr int SMALL_SPLIT_N = 64;
 cudaError_t spmm_small_init();
 cudaError_t launch_wait_expiry_selftest(int *status, cudaStream_t stream);
-float spmm_small_config(int mtiles, int ktiles, int N, int nb, bool gather, bool every_row, SpmmConfig *cfg);   // returns its estimate in microseconds
+float spmm_small_config(int mtiles, int ktiles, int N, int nb, bool gather, bool every_row, bool b_nk, SpmmConfig *cfg);   // returns its estimate in microseconds
 CUresult spmm_small_encode(EncodeTiledFn enc, CUtensorMap *map, const void *B, int64_t ldb, int K, int N, int b_nk, int gather_mode, int bn);
 cudaError_t launch_spmm_small(const SpmmConfig &cfg, const CUtensorMap &tmap_b, const SpmmParams &p, cudaStream_t stream);
 

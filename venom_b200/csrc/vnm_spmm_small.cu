@@ -448,9 +448,13 @@ cudaError_t spmm_small_init()
 // fill the last SMs of a GPC; and A cannot be read faster than HBM delivers it.  The choice takes 1.006 of the fastest one's time on average, 1.06 at most,
 // over 42 shapes (the fit to older kernels took 1.06 and 1.34: 14.2 us split by 3 instead of 10.6 by 2 at 12288 x 12288, 128:2:16, N = 16, 7.1 split by 8
 // instead of 5.5 by 4 at 1024 x 4096, 64:2:8, N = 64).  Operands of every row (m = 4 in gather form) in several waves, where each vector block of a tile reads the
-// same rows of B again, take 1.23, 1.40 and 1.66 of that fit on average and up to 2.4 (1, 2 and 4 blocks, 113 sizes), which is added beyond SMALL_SPLIT_N columns.  Only up to SMALL_SPLIT_N columns are k-tiles split: beyond, the
-// order of summation stays that of the other kernels, so that results do not depend on how a caller cuts its columns.
-float spmm_small_config(int mtiles, int ktiles, int N, int nb, bool gather, bool every_row, SpmmConfig *cfg)
+// same rows of B again, take 1.23, 1.40 and 1.66 of that fit on average and up to 2.4 (1, 2 and 4 blocks, 113 sizes), which is added beyond SMALL_SPLIT_N columns.
+// Up to SMALL_SPLIT_N columns that fit prices the kernel against others, but its choice among widths and splits took up to 1.75 of the fastest one's time (1.041
+// on average over 352 problems of 1024 x 1024 to 36864 x 12288, 8 to 64 columns, V = 128, 64 and 32, every width and split, weights in L2 where they fit): a cluster's exchange costs
+// more the wider the tile, clusters of three leave SMs idle, a row of 16 bytes is slow to load, and a ring that shares its SM takes in the weights of the call behind.  So
+// the choice has a cost of its own, with which it takes 1.016 and 1.31 (12288 x 4096, 128:2:8, N = 32, [K,N] 15.1 us as 32 columns split by 2, 8.5 unsplit; 2944 x 2048, N = 64
+// 9.9 as 32 columns split by 3, 5.7 unsplit).  Only up to SMALL_SPLIT_N columns are k-tiles split: beyond, the order of summation stays that of the other kernels, so that results do not depend on how a caller cuts its columns.
+float spmm_small_config(int mtiles, int ktiles, int N, int nb, bool gather, bool every_row, bool b_nk, SpmmConfig *cfg)
 {
     const int sms = g_num_sms_small > 0 ? g_num_sms_small : 148;
     static const int widths[4] = {16, 32, 64, 128};
@@ -458,7 +462,8 @@ float spmm_small_config(int mtiles, int ktiles, int N, int nb, bool gather, bool
     static const float kt_time[2][2][4] = {{{0.165f, 0.17f, 0.25f, 0.43f}, {0.165f, 0.17f, 0.172f, 0.24f}},      // [gather][deep][width]
                                            {{0.285f, 0.29f, 0.34f, 0.5f}, {0.285f, 0.29f, 0.27f, 0.35f}}};
     const float a_bytes = (float)mtiles * ktiles * AM_BLOCK_BYTES;
-    float best = 1e30f;
+    const bool few = N <= SMALL_SPLIT_N;
+    float estimate = 1e30f, best = 1e30f;
     for (int w = 0; w < 4; w++) {
         const int bn = widths[w];
         if ((bn == 128 && nb > 1) || (bn > 16 && bn >= 2 * N)) continue;
@@ -478,23 +483,40 @@ float spmm_small_config(int mtiles, int ktiles, int N, int nb, bool gather, bool
             float t = fixed[w] + (nb == 4 ? 1.0f : nb == 2 ? 0.2f : 0.0f);
             if (split > 1) t += 0.25f + 0.016f * bn + 0.004f * (float)(ctas < sms ? ctas : sms);
             if (one_each) t += kts * kt_us * (1.0f + (gather ? 0.1f * ctas / sms : 0.0f));
-            else t += ceilf((float)ctas / fit) * (kts * kt_us * (every_row && N > SMALL_SPLIT_N ? 1.45f + 0.36f * nb : 1.45f) + 2.0f);
+            else t += ceilf((float)ctas / fit) * (kts * kt_us * (every_row && !few ? 1.45f + 0.36f * nb : 1.45f) + 2.0f);
             const float hbm = 3.5f + a_bytes / (gather && one_each ? 4.2e6f : 5.6e6f);
             t = (t > hbm ? t : hbm) + 0.05f * t;
-            if (t < best) {
-                best = t;
-                *cfg = deep ? alone : shared;
+            estimate = t < estimate ? t : estimate;
+            auto take = [&](float cost, bool deep_ring) {
+                if (cost >= best) return;
+                best = cost;
+                *cfg = deep_ring ? alone : shared;
                 cfg->bn = bn;
                 cfg->nb = nb;
                 cfg->part = bn;
                 cfg->stages = 1;
                 cfg->split = split;
                 cfg->grid = ctas;
+            };
+            if (!few) {
+                take(t, deep);
+                break;
             }
-            if (N > SMALL_SPLIT_N) break;
+            const bool at_once = (float)ctas <= (split > 4 ? 0.72f : split == 3 ? 0.81f : 1.0f) * sms;
+            for (int ring = deep ? 1 : 0; ring >= 0; ring--) {
+                float kt = kt_time[gather][ring][w] * (nb == 4 ? 2.1f : nb == 2 ? 1.38f : 1.0f);
+                if (nb == 4) kt *= (bn == 64 ? 0.77f : 1.0f) * (every_row ? 1.54f : 1.0f);
+                if (N < 16 && !b_nk) kt *= 1.0f + (gather ? 0.55f : 0.5f * nb);      // rows of 16 bytes
+                float cost = fixed[w] + (nb == 4 ? 1.0f : nb == 2 ? 0.2f : 0.0f);
+                if (split > 1) cost += (0.038f + 0.15f / split) * bn - 0.4f;
+                if (at_once) cost += kts * kt * (1.0f + (gather ? 0.1f * ctas / sms : 0.0f));
+                else cost += ceilf((float)ctas / fit) * (split > 1 ? kts * kt * 1.32f + 3.1f : kts * kt * 1.45f + 2.0f);
+                const float a_time = 3.5f + a_bytes / (gather && at_once && (ring || split > 1) ? 4.7e6f : 5.6e6f);
+                take((cost > a_time ? cost : a_time) + 0.05f * cost, ring != 0);
+            }
         }
     }
-    return best;
+    return estimate;
 }
 
 // Tensor map of the dense operand for this kernel: rows of at most 64 columns, gathered four at a time or as boxes of 128
