@@ -25,7 +25,7 @@ def _ints(shape, seed):
     return torch.randint(-4, 5, shape, generator=g, device="cuda").half()
 
 
-# Few columns: tile widths 16 .. 128 and their edges; k-tiles that split evenly, raggedly and not at all; ragged rows.
+# Few columns: every N up to 64 and beyond at the edges of tiles; k-tiles that split evenly, raggedly and not at all; ragged rows.
 @pytest.mark.parametrize("N", [8, 16, 24, 32, 40, 64, 72, 136])
 @pytest.mark.parametrize("cfg", [(128, 1024, 128, 16), (96, 520, 32, 8), (192, 2048, 64, 8), (704, 4480, 64, 32), (128, 512, 128, 4)])
 @pytest.mark.parametrize("form", ["gather", "dense_b"])
@@ -41,6 +41,38 @@ def test_few_columns(N, cfg, form):
     assert torch.equal(prep.spmm(B, bias=bias, layout=capi.VNM_LAYOUT_NM), (want.half() + bias[:, None]).T)
     if form == "dense_b":
         assert torch.equal(prep.spmm_nk(B.T.contiguous()), want.half().T)
+    assert prep.device_status() == 0
+
+
+# Few columns: widths of 32 and 64 as well as 16, unsplit and split by 2 to 8, of 1, 2 and 4 vector blocks a tile: (form, V, row tiles, k-tiles, N, width, split).  The
+# last k-tile is ragged.  Among them the sizes at which a split was taken that is slower than none (V = 128, 96 row tiles and 16 k-tiles; 23 and 8).
+@pytest.mark.parametrize("cfg", [("dense_b", 64, 12, 20, 64, 32, 4), ("dense_b", 64, 23, 20, 40, 16, 2), ("dense_b", 64, 8, 7, 40, 16, 4), ("dense_b", 64, 1, 6, 8, 16, 6),
+                                 ("dense_b", 64, 1, 7, 8, 16, 7), ("dense_b", 64, 75, 8, 40, 64, 1), ("dense_b", 64, 48, 8, 64, 32, 1), ("gather", 128, 32, 24, 40, 32, 2),
+                                 ("gather", 128, 75, 32, 24, 32, 3), ("gather", 128, 23, 24, 64, 32, 5), ("gather", 128, 5, 32, 64, 32, 8), ("gather", 128, 32, 32, 40, 64, 4),
+                                 ("gather", 128, 75, 8, 40, 64, 1), ("gather", 128, 96, 16, 32, 32, 1), ("gather", 128, 96, 16, 16, 16, 1), ("gather", 128, 23, 8, 64, 16, 1),
+                                 ("gather", 64, 48, 32, 40, 64, 5), ("gather", 64, 12, 13, 24, 32, 8), ("gather", 64, 12, 8, 64, 32, 4), ("gather", 32, 8, 24, 40, 32, 6),
+                                 ("gather", 32, 12, 24, 64, 64, 8), ("gather", 32, 23, 16, 64, 64, 4), ("gather", 32, 23, 8, 64, 64, 1), ("gather", 32, 74, 8, 24, 32, 1),
+                                 ("gather", 32, 48, 13, 24, 32, 5), ("gather", 32, 75, 20, 24, 32, 3), ("gather", 32, 48, 12, 24, 32, 2), ("gather", 32, 288, 4, 64, 64, 1)])
+def test_widths_and_splits_of_few_columns(cfg):
+    import torch
+    from venom_b200 import capi
+    from venom_b200.synth import random_vnm_dense_cuda
+    form, V, mtiles, ktiles, N, width, split = cfg
+    M, K, m = 128 * mtiles, (128 * ktiles - 56 if form == "dense_b" else 256 * ktiles - 40), 8
+    dense, cols = random_vnm_dense_cuda(M, K, V, m, seed=M + K)
+    dense = torch.sign(dense) * torch.ceil(dense.abs() * 3)
+    values, meta, bad = capi.compress(dense, cols, V, m)
+    assert bad == 0
+    prep = capi.Prepared(values, meta, cols, M, K, V, m, strategy=capi.STRATEGY_GATHER if form == "gather" else capi.STRATEGY_DENSE_B)
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        got = prep.config(N)
+        assert got["tile_n"] == width and got["grid"] == mtiles * -(-N // width) * split
+    B, bias = _ints((K, N), N), _ints((M,), 3)
+    want = (dense.float() @ B.float()).half()
+    assert torch.equal(prep.spmm(B), want)
+    assert torch.equal(prep.spmm(B, bias=bias, layout=capi.VNM_LAYOUT_NM), (want + bias[:, None]).T)
+    if form == "dense_b":
+        assert torch.equal(prep.spmm_nk(B.T.contiguous()), want.T)
     assert prep.device_status() == 0
 
 

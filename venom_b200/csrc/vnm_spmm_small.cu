@@ -450,9 +450,9 @@ cudaError_t spmm_small_init()
 // instead of 5.5 by 4 at 1024 x 4096, 64:2:8, N = 64).  Operands of every row (m = 4 in gather form) in several waves, where each vector block of a tile reads the
 // same rows of B again, take 1.23, 1.40 and 1.66 of that fit on average and up to 2.4 (1, 2 and 4 blocks, 113 sizes), which is added beyond SMALL_SPLIT_N columns.
 // Up to SMALL_SPLIT_N columns that fit prices the kernel against others, but its choice among widths and splits took up to 1.75 of the fastest one's time (1.041
-// on average over 352 problems of 1024 x 1024 to 36864 x 12288, 8 to 64 columns, V = 128, 64 and 32, every width and split, weights in L2 where they fit): a cluster's exchange costs
+// on average over 352 problems of 1024 x 1024 to 36864 x 12288, 8 to 64 columns, V = 128, 64 and 32, every width and split, weights in L2 where they fit; 1.76 and 1.038 from HBM): a cluster's exchange costs
 // more the wider the tile, clusters of three leave SMs idle, a row of 16 bytes is slow to load, and a ring that shares its SM takes in the weights of the call behind.  So
-// the choice has a cost of its own, with which it takes 1.016 and 1.31 (12288 x 4096, 128:2:8, N = 32, [K,N] 15.1 us as 32 columns split by 2, 8.5 unsplit; 2944 x 2048, N = 64
+// the choice has a cost of its own, with which it takes 1.31 and 1.015 (1.32 and 1.022;  12288 x 4096, 128:2:8, N = 32, [K,N] 15.1 us as 32 columns split by 2, 8.5 unsplit; 2944 x 2048, N = 64
 // 9.9 as 32 columns split by 3, 5.7 unsplit).  Only up to SMALL_SPLIT_N columns are k-tiles split: beyond, the order of summation stays that of the other kernels, so that results do not depend on how a caller cuts its columns.
 float spmm_small_config(int mtiles, int ktiles, int N, int nb, bool gather, bool every_row, bool b_nk, SpmmConfig *cfg)
 {
@@ -505,13 +505,14 @@ float spmm_small_config(int mtiles, int ktiles, int N, int nb, bool gather, bool
             const bool at_once = (float)ctas <= (split > 4 ? 0.72f : split == 3 ? 0.81f : 1.0f) * sms;
             for (int ring = deep ? 1 : 0; ring >= 0; ring--) {
                 float kt = kt_time[gather][ring][w] * (nb == 4 ? 2.1f : nb == 2 ? 1.38f : 1.0f);
-                if (nb == 4) kt *= (bn == 64 ? 0.77f : 1.0f) * (every_row ? 1.54f : 1.0f);
+                if (nb == 4) kt *= (bn == 64 ? 0.7f : 1.0f) * (every_row ? 1.54f : 1.0f);
+                if (gather && ring) kt *= 1.15f;
                 if (N < 16 && !b_nk) kt *= 1.0f + (gather ? 0.55f : 0.5f * nb);      // rows of 16 bytes
                 float cost = fixed[w] + (nb == 4 ? 1.0f : nb == 2 ? 0.2f : 0.0f);
                 if (split > 1) cost += (0.038f + 0.15f / split) * bn - 0.4f;
                 if (at_once) cost += kts * kt * (1.0f + (gather ? 0.1f * ctas / sms : 0.0f));
                 else cost += ceilf((float)ctas / fit) * (split > 1 ? kts * kt * 1.32f + 3.1f : kts * kt * 1.45f + 2.0f);
-                const float a_time = 3.5f + a_bytes / (gather && at_once && (ring || split > 1) ? 4.7e6f : 5.6e6f);
+                const float a_time = 3.5f + a_bytes / (!gather || !at_once ? 5.6e6f : ring ? 4.0e6f : split > 1 ? 4.7e6f : 5.6e6f);
                 take((cost > a_time ? cost : a_time) + 0.05f * cost, ring != 0);
             }
         }
