@@ -453,7 +453,8 @@ cudaError_t spmm_small_init()
 // on average over 352 problems of 1024 x 1024 to 36864 x 12288, 8 to 64 columns, V = 128, 64 and 32, every width and split, weights in L2 where they fit; 1.76 and 1.038 from HBM): a cluster's exchange costs
 // more the wider the tile, clusters of three leave SMs idle, a row of 16 bytes is slow to load, and a ring that shares its SM takes in the weights of the call behind.  So
 // the choice has a cost of its own, with which it takes 1.31 and 1.015 (1.32 and 1.022;  12288 x 4096, 128:2:8, N = 32, [K,N] 15.1 us as 32 columns split by 2, 8.5 unsplit; 2944 x 2048, N = 64
-// 9.9 as 32 columns split by 3, 5.7 unsplit).  Only up to SMALL_SPLIT_N columns are k-tiles split: beyond, the order of summation stays that of the other kernels, so that results do not depend on how a caller cuts its columns.
+// 9.9 as 32 columns split by 3, 5.8 unsplit).  Only up to SMALL_SPLIT_N columns are k-tiles split: beyond, the order of summation stays that of the other kernels,
+// so that results do not depend on how a caller cuts its columns.
 float spmm_small_config(int mtiles, int ktiles, int N, int nb, bool gather, bool every_row, bool b_nk, SpmmConfig *cfg)
 {
     const int sms = g_num_sms_small > 0 ? g_num_sms_small : 148;
