@@ -507,7 +507,7 @@ float spmm_small_config(int mtiles, int ktiles, int N, int nb, bool gather, bool
             for (int ring = deep ? 1 : 0; ring >= 0; ring--) {
                 float kt = kt_time[gather][ring][w] * (nb == 4 ? 2.1f : nb == 2 ? 1.38f : 1.0f);
                 if (nb == 4) kt *= (bn == 64 ? 0.7f : 1.0f) * (every_row ? 1.54f : 1.0f);
-                if (gather && ring) kt *= 1.15f;
+                if (ring && (gather || (N < 16 && !b_nk))) kt *= 1.15f;
                 if (N < 16 && !b_nk) kt *= 1.0f + (gather ? 0.55f : 0.5f * nb);      // rows of 16 bytes
                 float cost = fixed[w] + (nb == 4 ? 1.0f : nb == 2 ? 0.2f : 0.0f);
                 if (split > 1) cost += (0.038f + 0.15f / split) * bn - 0.4f;
